@@ -452,7 +452,7 @@ sunny_geneig_status_t sunny_geneig_launch_sigma_intensity(sunny_geneig_solver_t 
     try {
         const sgeig::PlainPlan& p = solver->plan;
         cudaError_t e = with_device(solver->device, [&]() {
-            return sgeig::cta_launch_intensity(p.n, p.nmax, p.smem, reinterpret_cast<const void*>(d_S),
+            return sgeig::cta_launch_intensity(p.n, p.nmax, reinterpret_cast<const void*>(d_S),
                                                reinterpret_cast<const void*>(d_O),
                                                reinterpret_cast<const double*>(d_qhat),
                                                reinterpret_cast<const double*>(d_energies), n_energies, fwhm,

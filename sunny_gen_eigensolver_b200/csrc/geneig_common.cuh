@@ -49,19 +49,24 @@ __device__ __forceinline__ double2 cfms_bc(double2 acc, double2 a, double2 b) {
 }
 
 // ---------------------------------------------------------------- reductions
+// One FP64 tensor-core step D += A B on an 8x8x4 tile (mma.m8n8k4.f64).
+// Fragments: lane l holds A(l/4, l%4), B(l%4, l/4) and D(l/4, 2(l%4)+{0,1}).
+__device__ __forceinline__ void mma884(double (&d)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+        : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
+}
+// Sum over the warp's lanes, the same value in every lane, as two tensor-core
+// steps with A = 1: the first sums each B column (four lanes), leaving columns
+// 2q and 2q + 1 in the lanes l%4 == q; their sum as the second step's B adds
+// the four pairs. Two dependent steps and an add (60 cycles, 3 instructions)
+// where five shuffle-and-add rounds take 175 cycles and 15 instructions.
 __device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+    double c[2] = {0.0, 0.0}, t[2] = {0.0, 0.0};
+    mma884(c, 1.0, v);
+    mma884(t, 1.0, c[0] + c[1]);
+    return t[0];
 }
-__device__ __forceinline__ double2 warp_sum2(double2 v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-        v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-    }
-    return v;
-}
+__device__ __forceinline__ double2 warp_sum2(double2 v) { return c2(warp_sum(v.x), warp_sum(v.y)); }
 // Sum over the G consecutive lanes of one column group (G a power of two).
 template <int G>
 __device__ __forceinline__ double2 group_sum2(unsigned mask, double2 v) {
@@ -117,8 +122,8 @@ __host__ __device__ __forceinline__ double fast_rcp(double x) {
 // The NT threads that solve one pencil in a CTA of BLOCK threads: the whole
 // CTA when BLOCK == NT, else one of its BLOCK / NT teams of consecutive whole
 // warps (several pencils per CTA). team_sync is the team's barrier:
-// __syncthreads for a whole-CTA team, named barrier 1 + team otherwise
-// (barrier 0 stays the CTA's own).
+// __syncwarp for a team of one warp, __syncthreads for a whole-CTA team,
+// named barrier 1 + team otherwise (barrier 0 stays the CTA's own).
 template <int NT, int BLOCK>
 __device__ __forceinline__ unsigned team_tid() {
     if constexpr (BLOCK == NT) return threadIdx.x;
@@ -127,9 +132,15 @@ __device__ __forceinline__ unsigned team_tid() {
 template <int NT, int BLOCK>
 __device__ __forceinline__ void team_sync() {
     static_assert(NT % 32 == 0 && BLOCK % NT == 0 && BLOCK / NT <= 15, "team shape");
-    if constexpr (BLOCK == NT) __syncthreads();
+    if constexpr (NT == 32) __syncwarp();
+    else if constexpr (BLOCK == NT) __syncthreads();
     else asm volatile("bar.sync %0, %1;" :: "r"(1 + (int)(threadIdx.x / NT)), "n"(NT) : "memory");
 }
+
+// Makes the compiler forget what it knows of x, so that address arithmetic
+// derived from x is redone where it is used instead of being kept (or
+// spilled) across the phases of a long kernel.
+__device__ __forceinline__ void forget(int& x) { asm volatile("" : "+r"(x)); }
 
 // ---------------------------------------------------------------- constants
 // LAPACK dlamch convention: eps = 2^-53 (relative machine precision).

@@ -1,35 +1,29 @@
 // Batched generalized Hermitian-definite eigensolver, shared-memory regime
-// (N <= 64): a team of NT threads (64 to 256 by N) holds one matrix pair in
-// shared memory and solves it end to end; a CTA is one team or, with
-// several pencils per CTA, up to four, each with its own named barrier and
-// shared-memory slice; CTAs loop over the batch. A second kernel form
-// assembles S(q) from Fourier terms in the load stage (the metric solve of
-// a spin-wave dynamical matrix that never exists in memory).
+// (N <= 64): a team of NT threads (32 to 128 by N) holds one matrix per pencil
+// in shared memory and solves it end to end; a CTA is one team or, with
+// several pencils per CTA, up to four, each with its own barrier and
+// shared-memory slice; CTAs loop over the batch. Further kernel forms
+// assemble S(q) from Fourier terms in the load stage (the metric solve of a
+// spin-wave dynamical matrix that never exists in memory) and reduce the
+// metric solve to intensities.
 //
 // Stage chain (reference: src/unified/kernel_source.hpp:233-276):
-//   a1  load S -> A, H -> B                                   (:233-242)
-//   a2  Cholesky S = L L^H fused with X = L^-1: each row lives in the
-//       registers of a four-lane group, one barrier per column   (:244)
-//   a3+a4  C = L^-1 H L^-H as two complex GEMMs on the FP64 tensor cores
-//       (mma.m8n8k4.f64): T = H X^H, then C = X T (lower tiles, mirrored);
-//       H is read in full, as the reference's two triangular solves do (:246-248)
-//   a5  Householder tridiagonalisation (lower, look-ahead reflector, two
-//       barriers per step), divide and conquer on the tridiagonal,
-//       back-transform V = Q Z in compact-WY blocks of 16 reflectors on the
-//       FP64 tensor cores, one 8-column panel of V per warp          (:250)
-//   a6  U = L^-H V = X^H V on the FP64 tensor cores            (:252)
+//   a1  load the lower triangle of S                          (:233-242)
+//   a2  Cholesky S = L L^H fused with X = L^-1, in place, 8-column panels on
+//       the FP64 tensor cores (mma.m8n8k4.f64), two barriers per panel (:244)
+//   a3+a4  C = L^-1 H L^-H, 8 columns at a time: T = H X^H (H from global
+//       memory, in full, as the reference's two triangular solves read it),
+//       then C = X T; C fills the upper triangle beside X       (:246-248)
+//   a5  Householder tridiagonalisation (lower; the rank-2 update and the next
+//       matrix-vector product share one pass, one barrier per step), divide
+//       and conquer on the tridiagonal, back-transform V = Q Z in compact-WY
+//       blocks of 8 reflectors on the FP64 tensor cores, 8-column panels of
+//       V per warp                                                  (:250)
+//   a6  U = L^-H V = X^H V, on the same panels                     (:252)
 //   a7  W (ascending) and U, columns permuted by eigenvalue rank (:268-276)
-//
-// Thread layouts (NT threads): groups of four lanes (g = tid / 4, q = tid % 4)
-// owning one row or one column for the Cholesky/inverse and the Householder
-// updates; warps owning 8x8 output tiles or 8-column panels for the
-// tensor-core GEMMs; an NT/16 x 16 grid (tr, tc) for the copies.
-//
-// A variant that kept C in registers for the Householder steps (16 x 16
-// thread grid, rank-2 updates in registers) was measured slower on B200 at
-// N = 24 and 54 (80 K vs 75 K and 365 K vs 229 K cycles per solve): the
-// per-warp redundant reflector arithmetic and whole-block predicated
-// updates cost more issue slots than the shared-memory traffic they saved.
+// X and the reflectors wait for a5/a6 in the pencil's own block of the output
+// U, so that one n x n matrix and ~10 KB of vectors per pencil are all the
+// shared memory it takes.
 
 #include "geneig_cta_body.cuh"
 
@@ -37,59 +31,31 @@ namespace sgeig {
 using namespace cta;
 namespace {
 
-// Threads per pencil (one pencil per CTA) and CTAs per SM that the register
-// allocation is sized for, by row bound (at least 4 NMAX threads: the
-// Cholesky gives each row a four-lane group). Small pencils run on narrow
-// CTAs, several resident per SM: their steps are latency chains (a barrier
-// per Cholesky column, two per Householder step), so more pencils in flight
-// raise throughput more than more threads per pencil. Measured on B200
-// (solves/s at batch 65,536, against 256 threads and 2-3 CTAs/SM):
-//   NMAX 16: 64 x 8   N=16 9.09 M (3.80 M); 64 x 16 (spills) 7.36 M
-//   NMAX 24: 128 x 4  N=24 4.45 M (2.42 M); 96 x 4 4.39 M, 128 x 6 2.85 M
-//   NMAX 32: 128 x 4  N=32 2.26 M (1.96 M); 128 x 5 2.09 M
-//   NMAX 40: 256 x 3  N=40 1.36 M; 160 x 3 1.31 M, 192 x 3 1.34 M
-//   NMAX 48: 192 x 2  N=44 1.16 M (1.08 M); N=48 0.97 M either way
-//   NMAX 56: 256 x 2  N=54 832 K; 224 x 2 748 K
-template <int NMAX> struct CtaShape { static constexpr int nt = kNT, minb = 2; };
-template <> struct CtaShape<16> { static constexpr int nt = 64, minb = 8; };
-template <> struct CtaShape<24> { static constexpr int nt = 128, minb = 4; };
-template <> struct CtaShape<32> { static constexpr int nt = 128, minb = 4; };
-template <> struct CtaShape<40> { static constexpr int nt = kNT, minb = 3; };
-template <> struct CtaShape<48> { static constexpr int nt = 192, minb = 2; };
+// Pencils per SM that the register allocation is sized for, by row bound.
+template <int NMAX> struct CtaShape {
+    static constexpr int nt = cta_team_threads(NMAX);
+    static constexpr int per_sm = NMAX <= 16 ? 16 : NMAX <= 32 ? 8 : NMAX <= 56 ? 4 : 3;
+};
 
 // TEAMS pencils per CTA at a time (the reference's batches per block): the
 // CTA has TEAMS teams of CtaShape<NMAX>::nt threads, each with its own
 // barrier and shared-memory slice, team t taking pencils TEAMS * cta + t,
-// then a grid's stride on. TEAMS = 1 is the default launch.
-template <int NMAX, int TEAMS>
-__global__ void __launch_bounds__(CtaShape<NMAX>::nt * TEAMS, (CtaShape<NMAX>::minb + TEAMS - 1) / TEAMS)
-geneig_cta_kernel(CtaArgs a) {
+// then a grid's stride on. FS: S from Fourier terms. SPEC: intensities.
+template <int NMAX, int TEAMS, bool FS, bool SPEC>
+__global__ void __launch_bounds__(CtaShape<NMAX>::nt * TEAMS, (CtaShape<NMAX>::per_sm + TEAMS - 1) / TEAMS)
+geneig_cta_kernel(CtaArgs a, CtaFourier f) {
     constexpr int NT = CtaShape<NMAX>::nt;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     phase_start();
-    if constexpr (TEAMS == 1) {
-        for (long long b = blockIdx.x; b < a.batch; b += gridDim.x) cta_solve<NMAX, NT, NT>(a, b, smem_raw);
-    } else {
-        const int t = (int)(threadIdx.x / NT);
-        unsigned char* sm = smem_raw + (size_t)t * cta_team_bytes(a.n);
-        for (long long b = (long long)blockIdx.x * TEAMS + t; b < a.batch; b += (long long)gridDim.x * TEAMS)
-            cta_solve<NMAX, NT, NT * TEAMS>(a, b, sm);
-    }
-}
-
-// S assembled on the device from Fourier terms (one pencil per CTA).
-template <int NMAX>
-__global__ void __launch_bounds__(CtaShape<NMAX>::nt, CtaShape<NMAX>::minb)
-geneig_cta_fourier_kernel(CtaArgs a, CtaFourier f) {
-    constexpr int NT = CtaShape<NMAX>::nt;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    phase_start();
-    for (long long b = blockIdx.x; b < a.batch; b += gridDim.x) cta_solve<NMAX, NT, NT, true>(a, b, smem_raw, &f);
+    const int t = TEAMS == 1 ? 0 : (int)(threadIdx.x / NT);
+    unsigned char* sm = smem_raw + (TEAMS == 1 ? 0 : (size_t)t * cta_bytes(a.n, NT / 32, SPEC));
+    for (long long b = (long long)blockIdx.x * TEAMS + t; b < a.batch; b += (long long)gridDim.x * TEAMS)
+        cta_solve<NMAX, NT, NT * TEAMS, FS, SPEC>(a, b, sm, &f);
 }
 
 }  // namespace
 
-size_t cta_smem_bytes(int n) { return (size_t)2 * n * (n | 1) * 16 + cta_vec_bytes(n); }
+size_t cta_smem_bytes(int n, bool spec) { return cta_bytes(n, cta_team_threads(cta_nmax_for(n)) / 32, spec); }
 
 // Compile-time row bounds: the register arrays and unrolled loops are sized by
 // NMAX, so a bound close above n wastes less (56 covers the N=54 workload).
@@ -97,32 +63,32 @@ int cta_nmax_for(int n) {
     return n <= 16 ? 16 : n <= 24 ? 24 : n <= 32 ? 32 : n <= 40 ? 40 : n <= 48 ? 48 : n <= 56 ? 56 : 64;
 }
 
-using CtaKernelFn = void (*)(CtaArgs);
+using CtaKernelFn = void (*)(CtaArgs, CtaFourier);
+template <int NMAX, bool FS, bool SPEC>
+static CtaKernelFn cta_kernel_teams(int teams) {
+    if constexpr (!FS && NMAX <= 16) {
+        if (teams == 4) return geneig_cta_kernel<NMAX, 4, FS, SPEC>;
+    }
+    if constexpr (!FS && NMAX <= 32) {
+        if (teams == 2) return geneig_cta_kernel<NMAX, 2, FS, SPEC>;
+    }
+    return geneig_cta_kernel<NMAX, 1, FS, SPEC>;
+}
+template <bool FS, bool SPEC>
 static CtaKernelFn cta_kernel_for(int nmax, int teams) {
     switch (nmax) {
-        case 16: return teams == 4 ? geneig_cta_kernel<16, 4> : teams == 2 ? geneig_cta_kernel<16, 2>
-                                                                          : geneig_cta_kernel<16, 1>;
-        case 24: return teams == 2 ? geneig_cta_kernel<24, 2> : geneig_cta_kernel<24, 1>;
-        case 32: return teams == 2 ? geneig_cta_kernel<32, 2> : geneig_cta_kernel<32, 1>;
-        case 40: return geneig_cta_kernel<40, 1>;
-        case 48: return geneig_cta_kernel<48, 1>;
-        case 56: return geneig_cta_kernel<56, 1>;
-        default: return geneig_cta_kernel<64, 1>;
+        case 16: return cta_kernel_teams<16, FS, SPEC>(teams);
+        case 24: return cta_kernel_teams<24, FS, SPEC>(teams);
+        case 32: return cta_kernel_teams<32, FS, SPEC>(teams);
+        case 40: return cta_kernel_teams<40, FS, SPEC>(teams);
+        case 48: return cta_kernel_teams<48, FS, SPEC>(teams);
+        case 56: return cta_kernel_teams<56, FS, SPEC>(teams);
+        default: return cta_kernel_teams<64, FS, SPEC>(teams);
     }
 }
-
-// The assembled-S (Fourier) form, one pencil per CTA.
-using CtaFourierKernelFn = void (*)(CtaArgs, CtaFourier);
-static CtaFourierKernelFn cta_fourier_kernel_for(int nmax) {
-    switch (nmax) {
-        case 16: return geneig_cta_fourier_kernel<16>;
-        case 24: return geneig_cta_fourier_kernel<24>;
-        case 32: return geneig_cta_fourier_kernel<32>;
-        case 40: return geneig_cta_fourier_kernel<40>;
-        case 48: return geneig_cta_fourier_kernel<48>;
-        case 56: return geneig_cta_fourier_kernel<56>;
-        default: return geneig_cta_fourier_kernel<64>;
-    }
+static CtaKernelFn cta_kernel(int nmax, int teams, bool fs, bool spec) {
+    return fs ? (spec ? cta_kernel_for<true, true>(nmax, 1) : cta_kernel_for<true, false>(nmax, 1))
+              : (spec ? cta_kernel_for<false, true>(nmax, teams) : cta_kernel_for<false, false>(nmax, teams));
 }
 
 int cta_max_teams(int nmax) { return nmax <= 16 ? 4 : nmax <= 32 ? 2 : 1; }
@@ -135,43 +101,36 @@ int cta_max_teams(int nmax) { return nmax <= 16 ? 4 : nmax <= 32 ? 2 : 1; }
 // 1.16 M, N=48 1.05 M vs 0.98 M, N=54 810 K vs 836 K.
 int cta_default_teams(int nmax) { return nmax <= 16 ? 4 : nmax == 32 ? 2 : 1; }
 
-size_t cta_teams_smem_bytes(int n, int teams) { return teams <= 1 ? cta_smem_bytes(n) : teams * cta_team_bytes(n); }
+size_t cta_teams_smem_bytes(int n, int teams, bool spec) { return teams * cta_smem_bytes(n, spec); }
 
-int cta_threads_for(int nmax) {
-    switch (nmax) {
-        case 16: return CtaShape<16>::nt;
-        case 24: return CtaShape<24>::nt;
-        case 32: return CtaShape<32>::nt;
-        case 40: return CtaShape<40>::nt;
-        case 48: return CtaShape<48>::nt;
-        case 56: return CtaShape<56>::nt;
-        default: return CtaShape<64>::nt;
-    }
-}
+int cta_threads_for(int nmax) { return cta_team_threads(nmax); }
 
 // `smem` is the per-CTA shared-memory limit; the kernel's own static shared
 // memory (profiling builds have some) comes off the dynamic allowance.
 cudaError_t cta_set_attributes(int nmax, size_t smem) {
-    {
-        cudaFuncAttributes fa{};
-        cudaError_t e = cudaFuncGetAttributes(&fa, cta_fourier_kernel_for(nmax));
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(cta_fourier_kernel_for(nmax), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(smem - fa.sharedSizeBytes));
-        if (e != cudaSuccess) return e;
-    }
-    for (int teams = 1; teams <= cta_max_teams(nmax); teams *= 2) {
-        cudaFuncAttributes fa{};
-        cudaError_t e = cudaFuncGetAttributes(&fa, cta_kernel_for(nmax, teams));
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(cta_kernel_for(nmax, teams), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(smem - fa.sharedSizeBytes));
-        if (e != cudaSuccess) return e;
-    }
+    for (int form = 0; form < 4; ++form)
+        for (int teams = 1; teams <= cta_max_teams(nmax); teams *= 2) {
+            const CtaKernelFn k = cta_kernel(nmax, teams, (form & 1) != 0, (form & 2) != 0);
+            cudaFuncAttributes fa{};
+            cudaError_t e = cudaFuncGetAttributes(&fa, k);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(smem - fa.sharedSizeBytes));
+            if (e != cudaSuccess) return e;
+        }
     return cudaSuccess;
 }
 
-cudaError_t cta_launch(int n, int nmax, size_t smem, int stage, const void* H, const void* S, double* W, void* U,
+static cudaError_t cta_start(const CtaArgs& a, const CtaFourier& f, int nmax, int teams, bool fs, bool spec,
+                             cudaStream_t stream) {
+    const long long ctas = (a.batch + teams - 1) / teams;
+    const long long grid = ctas < 0x7fffffffLL ? ctas : 0x7fffffffLL;
+    cta_kernel(nmax, teams, fs, spec)<<<(unsigned)grid, teams * cta_threads_for(nmax),
+                                        cta_teams_smem_bytes(a.n, teams, spec), stream>>>(a, f);
+    return cudaGetLastError();
+}
+
+cudaError_t cta_launch(int n, int nmax, int stage, const void* H, const void* S, double* W, void* U,
                        int* info, long long batch, cudaStream_t stream, bool sigma, int teams) {
     CtaArgs a{};
     a.H = static_cast<const double2*>(H);
@@ -181,34 +140,16 @@ cudaError_t cta_launch(int n, int nmax, size_t smem, int stage, const void* H, c
     a.info = info;
     a.batch = batch;
     a.n = n;
-    a.ld = n | 1;
+    a.ld = cta_ld(n, false);
     a.stage = stage;
     a.sigma = sigma ? 1 : 0;
-    a.O = nullptr;
-    a.qhat = a.energies = nullptr;
-    a.spec = nullptr;
-    a.ne = 0;
-    a.gnorm = a.ginv2 = 0.0;
-    const long long ctas = (batch + teams - 1) / teams;
-    const long long grid = ctas < 0x7fffffffLL ? ctas : 0x7fffffffLL;
-    cta_kernel_for(nmax, teams)<<<(unsigned)grid, teams * cta_threads_for(nmax), smem, stream>>>(a);
-    return cudaGetLastError();
+    return cta_start(a, CtaFourier{}, nmax, teams, false, false, stream);
 }
 
-cudaError_t cta_launch_intensity(int n, int nmax, size_t smem, const void* S, const void* O, const double* qhat,
-                                 const double* energies, int ne, double fwhm, double* W, double* spec, int* info,
-                                 long long batch, cudaStream_t stream, int teams) {
-    CtaArgs a{};
-    a.H = nullptr;
-    a.S = static_cast<const double2*>(S);
-    a.W = W;
-    a.U = nullptr;
-    a.info = info;
-    a.batch = batch;
-    a.n = n;
-    a.ld = n | 1;
-    a.stage = kStageIntensity;
-    a.sigma = 1;
+// Arguments of the intensity form (no U).
+static void spec_args(CtaArgs& a, int n, const void* O, const double* qhat, const double* energies, int ne,
+                      double fwhm, double* spec) {
+    a.ld = cta_ld(n, true);
     a.O = static_cast<const double2*>(O);
     a.qhat = qhat;
     a.energies = energies;
@@ -217,12 +158,22 @@ cudaError_t cta_launch_intensity(int n, int nmax, size_t smem, const void* S, co
     const double sigma_e = fwhm / (2.0 * std::sqrt(2.0 * std::log(2.0)));
     a.gnorm = 1.0 / (sigma_e * std::sqrt(2.0 * M_PI));
     a.ginv2 = 1.0 / (2.0 * sigma_e * sigma_e);
-    const long long ctas = (batch + teams - 1) / teams;
-    const long long grid = ctas < 0x7fffffffLL ? ctas : 0x7fffffffLL;
-    cta_kernel_for(nmax, teams)<<<(unsigned)grid, teams * cta_threads_for(nmax), smem, stream>>>(a);
-    return cudaGetLastError();
 }
 
+cudaError_t cta_launch_intensity(int n, int nmax, const void* S, const void* O, const double* qhat,
+                                 const double* energies, int ne, double fwhm, double* W, double* spec, int* info,
+                                 long long batch, cudaStream_t stream, int teams) {
+    CtaArgs a{};
+    a.S = static_cast<const double2*>(S);
+    a.W = W;
+    a.info = info;
+    a.batch = batch;
+    a.n = n;
+    a.stage = 4;
+    a.sigma = 1;
+    spec_args(a, n, O, qhat, energies, ne, fwhm, spec);
+    return cta_start(a, CtaFourier{}, nmax, teams, false, true, stream);
+}
 
 cudaError_t cta_launch_fourier(int n, int nmax, const FourierTerms& ft, const double* q,
                                const void* O, const double* qhat, const double* energies, int ne, double fwhm,
@@ -233,7 +184,8 @@ cudaError_t cta_launch_fourier(int n, int nmax, const FourierTerms& ft, const do
     a.info = info;
     a.batch = batch;
     a.n = n;
-    a.ld = n | 1;
+    a.ld = cta_ld(n, false);
+    a.stage = 4;
     a.sigma = 1;
     CtaFourier f{};
     f.start = ft.start;
@@ -241,22 +193,8 @@ cudaError_t cta_launch_fourier(int n, int nmax, const FourierTerms& ft, const do
     f.disp = ft.disp;
     f.q = q;
     f.nterms = ft.nterms;
-    if (O) {
-        a.stage = kStageIntensity;
-        a.O = static_cast<const double2*>(O);
-        a.qhat = qhat;
-        a.energies = energies;
-        a.spec = spec;
-        a.ne = ne;
-        const double sigma_e = fwhm / (2.0 * std::sqrt(2.0 * std::log(2.0)));
-        a.gnorm = 1.0 / (sigma_e * std::sqrt(2.0 * M_PI));
-        a.ginv2 = 1.0 / (2.0 * sigma_e * sigma_e);
-    } else {
-        a.stage = 4;
-    }
-    const long long grid = batch < 0x7fffffffLL ? batch : 0x7fffffffLL;
-    cta_fourier_kernel_for(nmax)<<<(unsigned)grid, cta_threads_for(nmax), cta_smem_bytes(n), stream>>>(a, f);
-    return cudaGetLastError();
+    if (O) spec_args(a, n, O, qhat, energies, ne, fwhm, spec);
+    return cta_start(a, f, nmax, 1, true, O != nullptr, stream);
 }
 
 }  // namespace sgeig

@@ -19,12 +19,6 @@
 namespace sgeig {
 namespace cta {
 
-constexpr int kNT = 256;
-constexpr int kG = 4;
-// stage number of the intensity form (the spin-wave metric solve that
-// reduces U to S(q, E) on the device instead of storing it)
-constexpr int kStageIntensity = 5;
-
 struct CtaArgs {
     const double2* __restrict__ H;
     const double2* __restrict__ S;
@@ -34,7 +28,7 @@ struct CtaArgs {
     long long batch;
     int n, ld, stage;
     int sigma;      // H = diag(I_{n/2}, -I_{n/2}), not read from memory
-    // stage kStageIntensity (spin-wave intensities in place of U):
+    // intensity form (SPEC): spin-wave intensities in place of U
     const double2* O;        // 3 x n observable matrix per problem (column-major)
     const double*  qhat;     // 3 per problem
     const double*  energies; // ne
@@ -55,726 +49,829 @@ struct CtaFourier {
     int            nterms;  // terms are read only from [0, nterms)
 };
 
-struct CtaVec {
-    double2* tau;   // n   Householder scalars
-    double2* vb;    // n   Householder vector of even steps
-    double2* vb2;   // n   Householder vector of odd steps (written one step ahead)
-    double2* pb;    // n   tau * A22 * v
-    double2* wred;  // 8   per-warp partial dots
-    double2* colv;  // 2n  column k of the Cholesky working matrix (double-buffered)
-    double2* rowv;  // 2n  row k of the inverse accumulator (double-buffered)
-    double*  d;     // n
-    double*  e;     // n
-    double*  rdg;   // n   1 / L_kk
-    double*  dcd;   // D&C doubles
-    int*     dci;   // D&C ints
-    int*     rank;  // n
-    int*     ctl;   // 8
-};
+// Threads that solve one pencil, by row bound. One matrix per pencil is kept
+// in shared memory, so the pencils per SM are bounded by registers for small
+// n and by shared memory above; narrow teams keep many pencils, whose steps
+// are chains of dependent operations, in flight.
+constexpr int cta_team_threads(int nmax) { return nmax <= 16 ? 32 : nmax <= 32 ? 64 : 128; }
 
-__host__ __device__ inline size_t cta_vec_bytes(int n) {
-    return (size_t)n * 16 * 8 + 8 * 16 + (size_t)n * 8 * 3 + (size_t)dc_vec_doubles(n) * 8 +
-           (size_t)dc_vec_ints(n) * 4 + (size_t)n * 4 + 8 * 4;
+// Rows of a pencil's matrix in shared memory: the intensity form appends the
+// three rows of P = O X^H, which the Householder updates turn into P Q.
+constexpr int kSpecRows = 3;
+__host__ __device__ inline int cta_rows(int n, bool spec) { return spec ? n + kSpecRows : n; }
+// Leading dimension: odd, so that walks along a row and the fragment accesses
+// below (rows lane/4, columns 2 (lane%4) + s) are free of bank conflicts.
+__host__ __device__ inline int cta_ld(int n, bool spec) { return cta_rows(n, spec) | 1; }
+
+// Shared memory of one pencil's team after its n x ld matrix:
+//   work   phase by phase: the 8-column panel of the Cholesky and reduction,
+//          the Householder partial products and vectors, the divide and
+//          conquer scratch with the WY factors after it
+//   de     (d_k, e_k) of the tridiagonal, when the matrix has no padding row
+//          to hold them
+//   rank   ascending position of each eigenvalue
+__host__ __device__ inline size_t cta_dc_bytes(int n, bool spec) {   // (d, e) first, then the scratch
+    const size_t b = (size_t)n * 16 + (size_t)dc_vec_doubles(n) * 8 + (size_t)(spec ? kRowsTracked * n : 0) * 8 +
+                     (size_t)dc_vec_ints(n) * 4;
+    return (b + 15) & ~(size_t)15;
+}
+constexpr int kDElems = 72;       // an 8 x 8 tile with leading dimension 9
+__host__ __device__ inline size_t cta_work_bytes(int n, int nw, bool spec) {
+    const size_t panel = ((size_t)8 * (n | 1) + 2 * kDElems) * 16;
+    const size_t hh = (size_t)(nw + 3) * cta_rows(n, spec) * 16;
+    const size_t dc = cta_dc_bytes(n, spec) + (spec ? 0 : (size_t)((n + 7) / 8) * 36 * 16);
+    const size_t m = panel > hh ? panel : hh;
+    return m > dc ? m : dc;
+}
+// Complex entries of the matrix area (the leaves of the divide and conquer
+// keep their rows there too, which for tiny n take more than n x ld).
+__host__ __device__ inline size_t cta_mat_elems(int n, bool spec) {
+    const size_t mat = (size_t)n * cta_ld(n, spec), leaf = ((size_t)dc_leaf_doubles(n) + 1) / 2;
+    return mat > leaf ? mat : leaf;
+}
+__host__ __device__ inline bool cta_pad_row(int n, bool spec) { return cta_ld(n, spec) > cta_rows(n, spec); }
+__host__ __device__ inline size_t cta_bytes(int n, int nw, bool spec) {
+    const size_t b = cta_mat_elems(n, spec) * 16 + cta_work_bytes(n, nw, spec) +
+                     (cta_pad_row(n, spec) ? 0 : (size_t)n * 16) + (size_t)n * 4;
+    return (b + 15) & ~(size_t)15;
 }
 
-// Shared-memory bytes of one pencil's team (both matrices and the vector
-// area), rounded up to 16 so that consecutive teams stay aligned.
-__host__ __device__ inline size_t cta_team_bytes(int n) {
-    return ((size_t)2 * n * (n | 1) * 16 + cta_vec_bytes(n) + 15) & ~(size_t)15;
+// Complex step: D += A B with four real ones.
+__device__ __forceinline__ void zmma(double (&re)[2], double (&im)[2], double2 a, double2 b) {
+    mma884(re, a.x, b.x);
+    mma884(re, -a.y, b.y);
+    mma884(im, a.x, b.y);
+    mma884(im, a.y, b.x);
 }
 
-__device__ inline CtaVec cta_carve(unsigned char* p, int n) {
-    CtaVec v;
-    v.tau  = reinterpret_cast<double2*>(p);
-    v.vb   = v.tau + n;
-    v.vb2  = v.vb + n;
-    v.pb   = v.vb2 + n;
-    v.wred = v.pb + n;
-    v.colv = v.wred + 8;
-    v.rowv = v.colv + 2 * n;
-    v.d    = reinterpret_cast<double*>(v.rowv + 2 * n);
-    v.e    = v.d + n;
-    v.rdg  = v.e + n;
-    v.dcd  = v.rdg + n;
-    v.dci  = reinterpret_cast<int*>(v.dcd + dc_vec_doubles(n));
-    v.rank = v.dci + dc_vec_ints(n);
-    v.ctl  = v.rank + n;
-    return v;
-}
+template <int V> struct IntC { static constexpr int value = V; };
 
-// One FP64 tensor-core step D += A B on an 8x8x4 tile (mma.m8n8k4.f64).
-// Fragments: lane l holds A(l/4, l%4), B(l%4, l/4) and D(l/4, 2(l%4)+{0,1}).
-__device__ __forceinline__ void mma884(double& d0, double& d1, double a, double b) {
-    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-        : "+d"(d0), "+d"(d1) : "d"(a), "d"(b));
-}
-
-// Complex product on 8x8 output tiles, one warp per tile (round robin over
-// the CTA's warps), four real MMAs per 8x8x4 step:
-//   Dr += Ar Br - Ai Bi,  Di += Ar Bi + Ai Br.
-// fa(i, k) / fb(k, j) return the operands (zero outside their nonzero
-// pattern and outside the matrix); kr(ti, tj, k0, k1) bounds the k loop of
-// tile (ti, tj); keep(ti, tj) selects the tiles to compute. The results stay
-// in registers (acc) so that the caller can barrier before overwriting an
-// operand, then call `put` for every computed element.
-template <int MAXT>
-struct ZTiles {
-    double re[MAXT][2], im[MAXT][2];
-};
-
-template <int MAXT, int NT, int BLOCK, class FA, class FB, class FK, class FKeep>
-__device__ __forceinline__ void ztiles_compute(ZTiles<MAXT>& acc, int tm, int tn, FA fa, FB fb, FK kr, FKeep keep) {
-    const int lane = team_tid<NT, BLOCK>() & 31, warp = team_tid<NT, BLOCK>() >> 5;
-    constexpr int NW = NT / 32;
-#pragma unroll
-    for (int u = 0; u < MAXT; ++u) {
-        acc.re[u][0] = acc.re[u][1] = acc.im[u][0] = acc.im[u][1] = 0.0;
-        const int t = warp + NW * u;
-        if (t >= tm * tn) continue;
-        const int ti = t / tn, tj = t - ti * tn;
-        if (!keep(ti, tj)) continue;
-        int k0, k1;
-        kr(ti, tj, k0, k1);
-        const int ia = 8 * ti + (lane >> 2), ka = lane & 3;   // A fragment element
-        const int kb = lane & 3, jb = 8 * tj + (lane >> 2);   // B fragment element
-        for (int k = k0; k < k1; k += 4) {
-            const double2 av = fa(ia, k + ka);
-            const double2 bv = fb(k + kb, jb);
-            mma884(acc.re[u][0], acc.re[u][1], av.x, bv.x);
-            mma884(acc.re[u][0], acc.re[u][1], -av.y, bv.y);
-            mma884(acc.im[u][0], acc.im[u][1], av.x, bv.y);
-            mma884(acc.im[u][0], acc.im[u][1], av.y, bv.x);
-        }
-    }
-}
-
-template <int MAXT, int NT, int BLOCK, class FKeep, class FPut>
-__device__ __forceinline__ void ztiles_store(const ZTiles<MAXT>& acc, int tm, int tn, FKeep keep, FPut put) {
-    const int lane = team_tid<NT, BLOCK>() & 31, warp = team_tid<NT, BLOCK>() >> 5;
-    constexpr int NW = NT / 32;
-#pragma unroll
-    for (int u = 0; u < MAXT; ++u) {
-        const int t = warp + NW * u;
-        if (t >= tm * tn) continue;
-        const int ti = t / tn, tj = t - ti * tn;
-        if (!keep(ti, tj)) continue;
-        const int i = 8 * ti + (lane >> 2), j = 8 * tj + 2 * (lane & 3);
-        put(i, j, c2(acc.re[u][0], acc.im[u][0]));
-        put(i, j + 1, c2(acc.re[u][1], acc.im[u][1]));
-    }
+__device__ __forceinline__ double2 shfl2(double2 v, int src) {
+    return c2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
 
 // One pencil b, solved end to end by a team of NT threads (every thread of
 // the team calls this with the same b and the team's shared memory): the
 // whole CTA when BLOCK == NT, else one of the BLOCK / NT teams of a CTA of
-// BLOCK threads. NT >= 4 NMAX: the Cholesky gives each row a column group
-// of four lanes. FS: S is assembled from the Fourier terms `fs` instead of
-// loaded (a separate instantiation, so that the plain solve's register
-// allocation is untouched).
-template <int NMAX, int NT = kNT, int BLOCK = NT, bool FS = false>
+// BLOCK threads. FS: S is assembled from the Fourier terms `fs` instead of
+// loaded. SPEC: the metric solve reduced to intensities (no U).
+//
+// Products run on the FP64 tensor cores in 8 x 8 tiles. In every k block of 8
+// the MMA's k slot q of step s is column 2 q + s (any assignment that A and B
+// share is valid), which makes the fragment accesses conflict-free for odd ld
+// and an accumulator's layout (row l/4, columns 2 (l%4) + e) that of an A
+// fragment.
+//
+// Global memory: the pencil's own output block U serves as scratch between
+// the reduction and the back-transforms: X^H above and on its diagonal, the
+// Householder vectors and their tau below. All of H and S is read before.
+template <int NMAX, int NT, int BLOCK = NT, bool FS = false, bool SPEC = false>
 __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, unsigned char* smem_raw,
                                                 const CtaFourier* fs = nullptr) {
-    constexpr int R = NMAX / kG;    // rows per lane in a column group
     constexpr int NW = NT / 32;     // warps
-    constexpr int NG = NT / kG;     // column groups
-    constexpr int TR = NT / 16;     // thread rows of the 16-wide copy loops
-    static_assert(NG >= NMAX && NW >= 2 && NW <= 8 && NT % 32 == 0, "CTA shape");
+    constexpr int NB = NMAX / 8;    // 8-row tiles
+    constexpr int R = (NMAX + (SPEC ? kSpecRows : 0) + 31) / 32;   // Householder rows per lane
+    constexpr int PP = (NB + NW - 1) / NW;                         // 8-column panels per warp
+    static_assert(NT % 32 == 0 && NW >= 1 && NW <= 8 && NMAX % 8 == 0, "team shape");
     const int n = a.n, ld = a.ld;
-    const size_t mat = (size_t)n * ld;
-    double2* A = reinterpret_cast<double2*>(smem_raw);
-    double2* B = A + mat;
-    CtaVec v = cta_carve(reinterpret_cast<unsigned char*>(B + mat), n);
+    const int rows = cta_rows(n, SPEC);
+    double2* M = reinterpret_cast<double2*>(smem_raw);
+    double2* work = M + cta_mat_elems(n, SPEC);
+    unsigned char* after = reinterpret_cast<unsigned char*>(work) + cta_work_bytes(n, NW, SPEC);
+    const bool pad = cta_pad_row(n, SPEC);
+    double2* de = pad ? M + rows : reinterpret_cast<double2*>(after);   // (d_k, e_k) at de[k * des]
+    const int des = pad ? ld : 1;
+    int* rank = reinterpret_cast<int*>(after + (pad ? 0 : (size_t)n * 16));
 
-    // (threadIdx.x read here directly: through team_tid the register
-    // allocation of the 56- and 64-row kernels spilled 300+ bytes)
-    const int tid = BLOCK == NT ? (int)threadIdx.x : (int)(threadIdx.x % NT), lane = tid & 31, warp = tid >> 5;
-    const int tr = tid >> 4, tc = tid & 15;
-    const int g = tid >> 2, q = tid & 3;
-    const unsigned gmask = 0xFu << (lane & ~3);
+    int tid = BLOCK == NT ? (int)threadIdx.x : (int)(threadIdx.x % NT), lane = tid & 31, warp = tid >> 5;
+    int fr = lane >> 2, fq = lane & 3;           // fragment row / column index, k slots 2 fq + s
+    auto phase = [&]() { forget(tid); forget(lane); forget(warp); forget(fr); forget(fq); };
+    const int nb = (n + 7) >> 3;
     const size_t nn = (size_t)n * n;
+    const double2 zero = c2(0.0, 0.0);
 
     const double2* Hb = a.H + (size_t)b * nn;
     const double2* Sb = a.S + (size_t)b * nn;
     double*  Wb = a.W + (size_t)b * n;
     double2* Ub = a.U + (size_t)b * nn;
 
-    team_sync<NT, BLOCK>();
+    team_sync<NT, BLOCK>();   // the previous pencil's shared memory is free
     phase_mark(8);
-    // ---- a1: load (rows by tc so that global reads are contiguous)
+    // ---- a1: lower triangle of S -> M
     if constexpr (FS) {
-        // S(q) from its Fourier terms, lower triangle (the only part the
-        // Cholesky reads); the terms are shared by all pencils (L1/L2-resident).
-        // Term values first, one term per thread (coalesced, independent
-        // loads), into B, which the metric solve leaves free until a3; then
-        // each lower entry sums its terms in table order.
+        // S(q) from its Fourier terms; they are shared by all pencils
+        // (L1/L2-resident). Term values first, one term per thread (coalesced,
+        // independent loads), into M's strict upper triangle, which is free
+        // until a4, as many at a time as it holds; then each lower entry adds
+        // its terms in table order. The triangle is folded into n/2 lines of
+        // n1 = n - 1 slots (n even): line c holds column c (c entries), then
+        // column n1 - c (n1 - c entries).
         const double q0 = __ldg(fs->q + 3 * b), q1 = __ldg(fs->q + 3 * b + 1), q2 = __ldg(fs->q + 3 * b + 2);
         const int nt = fs->nterms;
-        auto term = [&](int t) {
-            const double x = fma(q0, __ldg(fs->disp + 3 * t),
-                             fma(q1, __ldg(fs->disp + 3 * t + 1), q2 * __ldg(fs->disp + 3 * t + 2)));
-            double sn, cs;
-            sincospi(2.0 * x, &sn, &cs);
-            return cmul(__ldg(fs->coef + t), c2(cs, sn));
+        const int n1 = n - 1, cap = (n >> 1) * n1;
+        auto upper = [&](int s) -> double2* {
+            const int c = s / n1, r = s - c * n1;
+            return r < c ? M + r + (size_t)c * ld : M + (r - c) + (size_t)(n1 - c) * ld;
         };
-        const bool staged = nt <= n * ld;
-        if (staged) {
-            for (int t = tid; t < nt; t += NT) B[t] = term(t);
-            team_sync<NT, BLOCK>();
-        }
+#pragma unroll 1
         for (int idx = tid; idx < n * n; idx += NT) {
             const int j = idx / n, i = idx - j * n;
-            if (i < j) continue;
-            double2 acc = c2(0.0, 0.0);
-            const int t1 = min(__ldg(fs->start + idx + 1), nt);
-            for (int t = max(__ldg(fs->start + idx), 0); t < t1; ++t) acc = cadd(acc, staged ? B[t] : term(t));
-            A[i + (size_t)j * ld] = acc;
+            if (i >= j) M[i + (size_t)j * ld] = zero;
         }
-    } else {
-        for (int j = tr; j < n; j += TR)
-            for (int i = tc; i < n; i += 16) {
-                A[i + (size_t)j * ld] = __ldg(Sb + i + (size_t)j * n);
-                if (!a.sigma) B[i + (size_t)j * ld] = __ldg(Hb + i + (size_t)j * n);
+#pragma unroll 1
+        for (int t0 = 0; t0 < nt; t0 += cap) {
+            const int t1 = min(nt, t0 + cap);
+#pragma unroll 1
+            for (int t = t0 + tid; t < t1; t += NT) {
+                const double x = fma(q0, __ldg(fs->disp + 3 * t),
+                                 fma(q1, __ldg(fs->disp + 3 * t + 1), q2 * __ldg(fs->disp + 3 * t + 2)));
+                double sn, cs;
+                sincospi(2.0 * x, &sn, &cs);
+                *upper(t - t0) = cmul(__ldg(fs->coef + t), c2(cs, sn));
             }
-    }
-    if (tid < 8) v.ctl[tid] = 0;
-
-    // ---- a2: Cholesky S = L L^H fused with X = L^-1, in registers.
-    // Group g owns row i = g; lane q holds slots j = q + 4t (t < R). Slot j
-    // holds the Cholesky working value a_ij while j > k and, from step j
-    // on, the inverse accumulator acc(i, j), so that at the end
-    // X(i, j) = acc(i, j) r_i with r_k = 1/sqrt(a_kk). Step k reads, from
-    // shared memory, column k (colv: a_jk, final after step k-1) and row k
-    // of acc (rowv: acc(k, j), j < k), and for i > k applies
-    //   a_ij -= a_ik conj(a_jk) r_k^2           k < j <= i
-    //   acc(i, j) -= a_ik r_k^2 acc(k, j)       j < k
-    //   acc(i, k) = -a_ik r_k^2
-    // then publishes column k+1 and row k+1 into the other buffers; one
-    // barrier per step. The step loop is unrolled so that slot k is a
-    // register known at compile time.
-    int fail = 0;
-    team_sync<NT, BLOCK>();   // the loads above are complete
-    phase_mark(0);
-    {
-        const int i = g;
-        double2 x[R];
-#pragma unroll
-        for (int t = 0; t < R; ++t) {
-            const int j = q + kG * t;
-            x[t] = (i < n && j <= i) ? A[i + (size_t)j * ld] : c2(0.0, 0.0);
-        }
-        if (i < n && q == 0) v.colv[i] = x[0];   // column 0, buffer 0
-        double ri = 0.0;
-#pragma unroll
-        for (int k = 0; k < NMAX; ++k) {
-            if (k >= n) break;
             team_sync<NT, BLOCK>();
-            const double2* colk = v.colv + (k & 1) * n;
-            const double2* rowk = v.rowv + (k & 1) * n;
-            double2* coln = v.colv + ((k + 1) & 1) * n;
-            double2* rown = v.rowv + ((k + 1) & 1) * n;
-            const double akk = colk[k].x;
-            if (!(akk > 0.0)) { fail = k + 1; break; }   // uniform: every thread reads akk
-            const double r = rsqrt(akk);
-            const double r2 = r * r;
-            if (i == k) ri = r;
-            if (tid == 0) v.rdg[k] = r;
-            if (a.stage == 1) {   // stage-wise output: column k of L
-                for (int jj = k + tid; jj < n; jj += NT)
-                    A[jj + (size_t)k * ld] = (jj == k) ? c2(1.0 / r, 0.0) : cscale(colk[jj], r);
+#pragma unroll 1
+            for (int idx = tid; idx < n * n; idx += NT) {
+                const int j = idx / n, i = idx - j * n;
+                if (i < j) continue;
+                const int lo = max(__ldg(fs->start + idx), t0), hi = min(__ldg(fs->start + idx + 1), t1);
+                if (lo >= hi) continue;
+                double2 acc = M[i + (size_t)j * ld];
+#pragma unroll 1
+                for (int t = lo; t < hi; ++t) acc = cadd(acc, *upper(t - t0));
+                M[i + (size_t)j * ld] = acc;
             }
-            if (i > k && i < n) {
-                const double2 aik = cscale(colk[i], r2);
+            team_sync<NT, BLOCK>();
+        }
+        if (nt == 0) team_sync<NT, BLOCK>();
+    } else {
+        // one warp per column, copied asynchronously (every load in flight
+        // at once, no registers)
+#pragma unroll 1
+        for (int j = warp; j < n; j += NW)
+#pragma unroll 1
+            for (int i = j + lane; i < n; i += 32) {
+                const unsigned dst = (unsigned)__cvta_generic_to_shared(M + i + (size_t)j * ld);
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(Sb + i + (size_t)j * n)
+                             : "memory");
+            }
+        if (!a.sigma && a.stage >= 2) {   // H follows in a3: start it towards L2
+            const char* hp = reinterpret_cast<const char*>(Hb);
+#pragma unroll 1
+            for (size_t o = (size_t)tid * 128; o < nn * 16; o += (size_t)NT * 128)
+                asm volatile("prefetch.global.L2 [%0];" :: "l"(hp + o));
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        team_sync<NT, BLOCK>();
+    }
+    phase_mark(0);
+    phase();
+
+    // ---- a2: Cholesky S = L L^H together with X = L^-1, 8-column panels,
+    // right-looking. In M's lower triangle, columns right of the current
+    // panel p hold the Cholesky working matrix, columns up to p the inverse
+    // accumulators Acc. With D = L_pp^-1 (from warp 0, in shared memory):
+    //   L(i, p) = A(i, p) D^H  (i > p, into `work`),   X(p, c) = D Acc(p, c)  (c < p, in place)
+    // barrier
+    //   Acc(i, c) -= L(i, p) X(p, c)  (c < p),  Acc(i, p) = -L(i, p) D,  A(i, j) -= L(i, p) L(j, p)^H
+    // barrier; warp 0 updates the next diagonal tile first and factors it
+    // while the other warps do the rest. Two barriers per 8 columns and all
+    // products on the tensor cores; one barrier per column with a row in each
+    // four-lane group's registers took 90 K CTA cycles at n = 54 and needed
+    // 256 threads. Fragment rows past n read whatever lies there: they reach
+    // discarded rows or columns of the result only.
+    double2* Pn = work;                // n x 8 panel of L
+    const int ldp = n | 1;
+    double2* Ds = work + 8 * ldp;      // D of even and odd panels: element (i, j) at i + 9 j
+    auto factor = [&](int p) {         // warp 0; lane: row fr, columns 2 fq + s of the tile
+        const int o = 8 * p;
+        double2* Dp = Ds + (p & 1) * kDElems;
+        double2 x[2];
 #pragma unroll
-                for (int t = 0; t < R; ++t) {
-                    const int j = q + kG * t;
-                    if (j > k && j <= i) x[t] = cfms_bc(x[t], aik, colk[j]);
-                    else if (j < k) x[t] = cfms(x[t], aik, rowk[j]);
+        for (int s = 0; s < 2; ++s) {
+            const int j = 2 * fq + s;
+            x[s] = (o + fr < n && j <= fr) ? M[o + fr + (o + j) * ld] : c2(fr == j ? 1.0 : 0.0, 0.0);
+        }
+        int bad = 0;
+        double rr = 0.0;               // 1 / L of this lane's row
+#pragma unroll 1
+        for (int h = 0; h < 4; ++h) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int c = 2 * h + u;
+                const double akk = __shfl_sync(0xffffffffu, x[u].x, 4 * c + h);
+                if (!bad && o + c < n && !(akk > 0.0)) bad = o + c + 1;
+                const double r = rsqrt(akk), r2 = r * r;
+                if (fr == c) rr = r;
+                const double2 aic = shfl2(x[u], (lane & 28) + h);
+                double2 ajc[2], rc[2];
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    ajc[s] = shfl2(x[u], 4 * (2 * fq + s) + h);      // column c, row j
+                    rc[s] = shfl2(x[s], 4 * c + fq);                 // row c, column j
                 }
-                if (q == (k & 3)) x[k >> 2] = cscale(aik, -1.0);
-            }
-            // publish column k+1 (rows >= k+1) and row k+1 of acc (j <= k)
-            if (k + 1 < n) {
-                if (i >= k + 1 && i < n && q == ((k + 1) & 3)) coln[i] = x[(k + 1) >> 2];
-                if (i == k + 1) {
+                if (a.stage == 1 && fq == h && o + fr < n && fr >= c && !bad)
+                    Ub[o + fr + (size_t)(o + c) * n] = fr == c ? c2(1.0 / r, 0.0) : cscale(aic, r);
+                if (fr > c) {
+                    const double2 aik = cscale(aic, r2);
 #pragma unroll
-                    for (int t = 0; t < R; ++t) {
-                        const int j = q + kG * t;
-                        if (j <= k) rown[j] = x[t];
+                    for (int s = 0; s < 2; ++s) {
+                        const int j = 2 * fq + s;
+                        if (j > c) { if (j <= fr) x[s] = cfms_bc(x[s], aik, ajc[s]); }
+                        else if (j < c) x[s] = cfms(x[s], aik, rc[s]);
+                        else x[s] = cscale(aik, -1.0);
                     }
                 }
             }
         }
-        team_sync<NT, BLOCK>();
-        if (!fail && a.stage >= 2 && i < n) {
-            // X(i, j) = acc(i, j) r_i, X(i, i) = r_i, into A's lower triangle
+        if (lane == 0) rank[0] = bad;
 #pragma unroll
-            for (int t = 0; t < R; ++t) {
-                const int j = q + kG * t;
-                if (j < i) A[i + (size_t)j * ld] = cscale(x[t], ri);
-                else if (j == i) A[i + (size_t)i * ld] = c2(ri, 0.0);
-            }
+        for (int s = 0; s < 2; ++s) {
+            const int j = 2 * fq + s;
+            Dp[fr + 9 * j] = j < fr ? cscale(x[s], rr) : c2(j == fr ? rr : 0.0, 0.0);
         }
+    };
+    int fail = 0;
+#pragma unroll 1
+    for (int p = -1; p < nb; ++p) {    // p = -1: the first diagonal tile only
+        const int o = 8 * p;
+        const double2* Dp = Ds + (p & 1) * kDElems;
+        if (p >= 0) {
+            fail = rank[0];
+            if (fail) break;
+#pragma unroll 1
+            for (int t = warp; t < nb - 1; t += NW) {
+                double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
+                const bool xt = t < p;     // X(p, t) = D Acc(p, t), else L(t + 1, p) = A(t + 1, p) D^H
+                const int i = 8 * (t + 1) + fr;
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    const int k = 2 * fq + s;
+                    const double2 dd = Dp[fr + 9 * k];
+                    const double2 m = xt ? M[min(o + k, n - 1) + (8 * t + fr) * ld] : M[i + (o + k) * ld];
+                    zmma(re, im, xt ? dd : m, xt ? m : cconj(dd));
+                }
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int j = 2 * fq + e;
+                    if (xt) {
+                        if (o + fr < n) M[o + fr + (8 * t + j) * ld] = c2(re[e], im[e]);
+                    } else if (i < n) {
+                        Pn[i + j * ldp] = c2(re[e], im[e]);
+                        if (a.stage == 1) Ub[i + (size_t)(o + j) * n] = c2(re[e], im[e]);
+                    }
+                }
+            }
+            team_sync<NT, BLOCK>();
+        }
+        auto update = [&](int i8, int j8) {
+            const int i = 8 * i8 + fr;
+            double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
+            if (j8 != p) {
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const double2 c = M[i + (8 * j8 + 2 * fq + e) * ld];
+                    re[e] = c.x; im[e] = c.y;
+                }
+            }
+            // B(k, j) = conj(L(j, p)), X(p, j) or D, by the tile's column
+            const double2* bp = j8 > p ? Pn + 8 * j8 + fr + 2 * fq * ldp
+                              : j8 < p ? M + o + 2 * fq + (8 * j8 + fr) * ld : Dp + 2 * fq + 9 * fr;
+            const int bs = j8 > p ? ldp : 1;
+            const double sg = j8 > p ? 1.0 : -1.0;      // conj(B) for j8 > p, -A in place of A
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                const double2 l = Pn[i + (2 * fq + s) * ldp], bv = bp[s * bs];
+                mma884(re, -l.x, bv.x);
+                mma884(re, -sg * l.y, bv.y);
+                mma884(im, sg * l.x, bv.y);
+                mma884(im, -l.y, bv.x);
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int j = 8 * j8 + 2 * fq + e;
+                if (i < n && j < n) M[i + j * ld] = c2(re[e], im[e]);
+            }
+        };
+        // warp 0: the next diagonal tile, then its factor; the others (a lone
+        // warp: the same one) the remaining tiles (i8, j8 <= i8), row by row
+        if (p >= 0) {
+            if (warp == 0 && o + fr < n) {
+#pragma unroll
+                for (int s = 0; s < 2; ++s)
+                    if (2 * fq + s <= fr) M[o + fr + (o + 2 * fq + s) * ld] = Dp[fr + 9 * (2 * fq + s)];
+            }
+            int i8 = p + 1, j8 = NW == 1 ? 0 : warp == 0 ? p + 1 : warp - 1;
+#pragma unroll 1
+            for (;;) {
+                while (i8 < nb && j8 > i8) { j8 -= i8 + 1; ++i8; }
+                if (i8 >= nb) break;
+                if (NW == 1 || warp == 0 || i8 != p + 1 || j8 != p + 1) update(i8, j8);
+                j8 += NW == 1 ? 1 : warp == 0 ? nb * nb : NW - 1;
+            }
+            __syncwarp();
+        }
+        if (warp == 0 && p + 1 < nb) factor(p + 1);
+        team_sync<NT, BLOCK>();
     }
-    team_sync<NT, BLOCK>();
     phase_mark(1);
+    phase();
     int code = fail ? n + fail : 0;   // zhegv: info = n + order of the failing minor
 
     if (!code && a.stage == 1) {
-        for (int j = tr; j < n; j += TR)
-            for (int i = tc; i < n; i += 16)
-                Ub[i + (size_t)j * n] = (i >= j) ? A[i + (size_t)j * ld] : c2(0.0, 0.0);
+#pragma unroll 1
+        for (int j = warp; j < n; j += NW)
+#pragma unroll 1
+            for (int i = lane; i < j; i += 32) Ub[i + (size_t)j * n] = zero;
         if (tid == 0) a.info[b] = 0;
         return;
     }
 
     if (!code) {
-        // A now holds X = L^-1 in its lower triangle (diagonal real).
-        // ---- a3: T = H X^H, T(i, j) = sum_{k <= j} H(i, k) conj(X(j, k)),
-        // FP64 tensor-core tiles; T overwrites H after the barrier.
-        constexpr int MAXT = ((NMAX / 8) * (NMAX / 8) + NW - 1) / NW;
-        const int tn8 = (n + 7) >> 3;
-        if (a.sigma) {
-            // H = diag(I, -I): T(i, j) = sigma_i conj(X(j, i)), no product needed
+        // M holds X = L^-1 in its lower triangle (diagonal real); the upper
+        // triangle receives C below, so the tiles on the diagonal are masked.
+        // C(i, j) of tile (ti, tj) (ti >= tj): conj into M(j, i), the diagonal's
+        // real part into de[.].x
+        auto put_c = [&](int ti, int tj, const double (&re)[2], const double (&im)[2]) {
+            const int i = 8 * ti + fr;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int j = 8 * tj + 2 * fq + e;
+                if (i < n && j < i) M[j + i * ld] = c2(re[e], -im[e]);
+                else if (i < n && j == i) de[i * des] = c2(re[e], 0.0);
+            }
+        };
+        if (SPEC || a.sigma) {
+            // ---- a3 + a4, H = diag(I, -I): C = X diag(I, -I) X^H directly
             const int m = n >> 1;
-            for (int j = tr; j < n; j += TR)
-                for (int i = tc; i < n; i += 16) {
-                    const double2 x = (i <= j) ? cconj(A[j + (size_t)i * ld]) : c2(0.0, 0.0);
-                    B[i + (size_t)j * ld] = (i < m) ? x : c2(-x.x, -x.y);
-                }
-            team_sync<NT, BLOCK>();
-        } else {
-            ZTiles<MAXT> acc;
-            ztiles_compute<MAXT, NT, BLOCK>(acc, tn8, tn8,
-                [&](int i, int k) { return (i < n && k < n) ? B[i + (size_t)k * ld] : c2(0.0, 0.0); },
-                [&](int k, int j) { return (j < n && k <= j) ? cconj(A[j + (size_t)k * ld]) : c2(0.0, 0.0); },
-                [&](int, int tj, int& k0, int& k1) { k0 = 0; k1 = min(n, 8 * tj + 8); },
-                [](int, int) { return true; });
-            team_sync<NT, BLOCK>();
-            ztiles_store<MAXT, NT, BLOCK>(acc, tn8, tn8, [](int, int) { return true; },
-                [&](int i, int j, double2 c) { if (i < n && j < n) B[i + (size_t)j * ld] = c; });
-            team_sync<NT, BLOCK>();
-        }
-        phase_mark(2);
-        // ---- a4: C = X T, C(i, j) = sum_{k <= i} X(i, k) T(k, j); lower
-        // tiles only, each lower element written with its mirror, so that
-        // C is exactly Hermitian.
-        {
-            ZTiles<MAXT> acc;
-            ztiles_compute<MAXT, NT, BLOCK>(acc, tn8, tn8,
-                [&](int i, int k) { return (i < n && k <= i) ? A[i + (size_t)k * ld] : c2(0.0, 0.0); },
-                [&](int k, int j) { return (k < n && j < n) ? B[k + (size_t)j * ld] : c2(0.0, 0.0); },
-                [&](int ti, int, int& k0, int& k1) { k0 = 0; k1 = min(n, 8 * ti + 8); },
-                [](int ti, int tj) { return ti >= tj; });
-            team_sync<NT, BLOCK>();
-            ztiles_store<MAXT, NT, BLOCK>(acc, tn8, tn8, [](int ti, int tj) { return ti >= tj; },
-                [&](int i, int j, double2 c) {
-                    if (i < n && j < n && i >= j) {
-                        if (i == j) c.y = 0.0;
-                        B[i + (size_t)j * ld] = c;
-                        B[j + (size_t)i * ld] = cconj(c);
+            int i8 = 0, j8 = warp;
+#pragma unroll 1
+            for (;;) {
+                while (i8 < nb && j8 > i8) { j8 -= i8 + 1; ++i8; }
+                if (i8 >= nb) break;
+                double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
+                const double2* xi = M + 8 * i8 + fr;
+                const double2* xj = M + 8 * j8 + fr;
+#pragma unroll 1
+                for (int kb = 0; kb <= j8; ++kb) {
+#pragma unroll
+                    for (int s = 0; s < 2; ++s) {
+                        const int kr = 2 * fq + s, k = 8 * kb + kr;
+                        double2 av = xi[k * ld], y = xj[k * ld];
+                        if (kb == j8 && kr > fr) {       // above X's diagonal
+                            y = zero;
+                            if (i8 == j8) av = zero;
+                        }
+                        const double sg = k < m ? 1.0 : -1.0;
+                        zmma(re, im, av, c2(sg * y.x, -sg * y.y));
                     }
-                });
-            team_sync<NT, BLOCK>();
-            phase_mark(3);
+                }
+                put_c(i8, j8, re, im);
+                j8 += NW;
+            }
+            phase_mark(2);
+        } else {
+            // ---- a3 + a4, one 8-column block of C at a time:
+            // T(:, tj) = H X(tj, :)^H into `work` (H read in full, from global
+            // memory, L2 after the first blocks), then C(ti, tj) = X(ti, :) T,
+            // ti >= tj. Two row tiles per warp share each fragment of X.
+            double2* Tp = work;
+#pragma unroll 1
+            for (int tj = 0; tj < nb; ++tj) {
+#pragma unroll 1
+                for (int t0 = warp; t0 < nb; t0 += 2 * NW) {
+                    const int i0 = 8 * t0 + fr, i1 = i0 + 8 * NW;
+                    double re0[2] = {0.0, 0.0}, im0[2] = {0.0, 0.0}, re1[2] = {0.0, 0.0}, im1[2] = {0.0, 0.0};
+                    const double2* xj = M + 8 * tj + fr;
+                    const double2* h0 = Hb + min(i0, n - 1);
+                    const double2* h1 = Hb + min(i1, n - 1);
+                    const bool two = t0 + NW < nb;
+                    double2 y0[2], y1[2];        // the next k block's H, loaded ahead
+#pragma unroll
+                    for (int s = 0; s < 2; ++s) {
+                        const int k = min(2 * fq + s, n - 1);
+                        y0[s] = __ldg(h0 + k * n);
+                        y1[s] = __ldg(h1 + k * n);
+                    }
+#pragma unroll 1
+                    for (int kb = 0; kb <= tj; ++kb) {
+                        const double2 a0[2] = {y0[0], y0[1]}, a1[2] = {y1[0], y1[1]};
+                        if (kb < tj) {
+#pragma unroll
+                            for (int s = 0; s < 2; ++s) {
+                                const int k = min(8 * kb + 8 + 2 * fq + s, n - 1);
+                                y0[s] = __ldg(h0 + k * n);
+                                y1[s] = __ldg(h1 + k * n);
+                            }
+                        }
+#pragma unroll
+                        for (int s = 0; s < 2; ++s) {
+                            const int kr = 2 * fq + s;
+                            double2 bv = cconj(xj[(8 * kb + kr) * ld]);
+                            if (kb == tj && kr > fr) bv = zero;
+                            zmma(re0, im0, a0[s], bv);
+                            if (two) zmma(re1, im1, a1[s], bv);
+                        }
+                    }
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        double2* tc = Tp + (2 * fq + e) * ldp;
+                        if (i0 < n) tc[i0] = c2(re0[e], im0[e]);
+                        if (i1 < n) tc[i1] = c2(re1[e], im1[e]);
+                    }
+                }
+                team_sync<NT, BLOCK>();
+#pragma unroll 1
+                for (int ti = tj + warp; ti < nb; ti += NW) {
+                    double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
+                    const double2* xi = M + 8 * ti + fr;
+                    const double2* tc = Tp + fr * ldp;
+#pragma unroll 1
+                    for (int kb = 0; kb <= ti; ++kb) {
+#pragma unroll
+                        for (int s = 0; s < 2; ++s) {
+                            const int kr = 2 * fq + s, k = 8 * kb + kr;
+                            double2 av = xi[k * ld];
+                            if (kb == ti && kr > fr) av = zero;
+                            zmma(re, im, av, tc[min(k, n - 1)]);
+                        }
+                    }
+                    put_c(ti, tj, re, im);
+                }
+                team_sync<NT, BLOCK>();
+            }
+            phase_mark(2);
         }
+        if constexpr (SPEC) {
+            // P = O X^H (3 x n) into rows n .. n+2
+            const double2* Ob = a.O + (size_t)b * 3 * n;
+#pragma unroll 1
+            for (int idx = tid; idx < 3 * n; idx += NT) {
+                const int c = idx / n, k = idx - c * n;
+                double2 acc = zero;
+#pragma unroll 1
+                for (int i = 0; i <= k; ++i) acc = cfma(acc, __ldg(Ob + c + 3 * i), cconj(M[k + (size_t)i * ld]));
+                M[n + c + (size_t)k * ld] = acc;
+            }
+        } else if (a.stage == 4) {
+            // X^H into the upper triangle and the diagonal of U's block
+#pragma unroll 1
+            for (int k = warp; k < n; k += NW)
+#pragma unroll 1
+                for (int i = lane; i <= k; i += 32) Ub[i + (size_t)k * n] = cconj(M[k + (size_t)i * ld]);
+        }
+        team_sync<NT, BLOCK>();
+        // C to the lower triangle and the diagonal: M is exactly Hermitian
+#pragma unroll 1
+        for (int j = warp; j < n; j += NW)
+#pragma unroll 1
+            for (int i = j + lane; i < n; i += 32)
+                M[i + (size_t)j * ld] = i == j ? c2(de[j * des].x, 0.0) : cconj(M[j + (size_t)i * ld]);
+        team_sync<NT, BLOCK>();
+        phase_mark(3);
+    phase();
     }
 
     if (!code && a.stage == 2) {
-        for (int j = tr; j < n; j += TR)
-            for (int i = tc; i < n; i += 16) Ub[i + (size_t)j * n] = B[i + (size_t)j * ld];
+#pragma unroll 1
+        for (int j = warp; j < n; j += NW)
+#pragma unroll 1
+            for (int i = lane; i < n; i += 32) Ub[i + (size_t)j * n] = M[i + (size_t)j * ld];
         if (tid == 0) a.info[b] = 0;
         return;
     }
 
+    double2* tpk = reinterpret_cast<double2*>(reinterpret_cast<unsigned char*>(work) + cta_dc_bytes(n, SPEC));
+    auto tidx = [](int c, int l, int i) { return 36 * c + ((i * (i + 1)) >> 1) + l; };   // T_c(l, i), l <= i
+    const int nref = n - 1;                      // reflectors 0 .. n-2
+    const int nblk = (nref + 7) >> 3;            // WY blocks of 8
+    DCShared dc;
+    dc.Z = reinterpret_cast<double*>(M); dc.ldz = ld;
+    dc.U = dc.Z + (size_t)n * ld;        dc.ldu = ld;
+    dc.Zo = nullptr;
+    dc.leaf = dc.Z; dc.leaf_lanes = kLeaf * nb;
+    {
+        double* dv = reinterpret_cast<double*>(work + n);
+        dc.rows = SPEC ? dv + dc_vec_doubles(n) : nullptr;
+        int* iv = reinterpret_cast<int*>(dv + dc_vec_doubles(n) + (SPEC ? kRowsTracked * n : 0));
+        dc_carve(dc, dv, iv, n);
+    }
+    dc.d = reinterpret_cast<const double*>(work); dc.ds = 2;
+    dc.e = dc.d + 1;                              dc.es = 2;
+
     if (!code) {
-        // ---- a5a: Householder tridiagonalisation of C (lower). Reflector k:
-        // I - tau_k v v^H on rows k+1.., v[k+1] = 1, v[k+2..] kept in A's
-        // strict upper triangle (row k), tau_k in v.tau. Look-ahead: during
-        // the rank-2 update of step k, warp 0 updates column k+1 first and
-        // computes reflector k+1 (into the other vector buffer) while the
-        // other warps update the rest, so each step needs two barriers.
-        auto reflect = [&](int k, double2* vbuf) {   // warp 0
-            const double2* bk = B + (size_t)k * ld;
-            double ss = 0.0;
-            for (int i = k + 2 + lane; i < n; i += 32) { const double2 x = bk[i]; ss = fma(x.x, x.x, fma(x.y, x.y, ss)); }
-            ss = warp_sum(ss);
-            const double2 alpha = bk[k + 1];
-            double2 taui, scal = c2(0.0, 0.0);
-            double beta;
-            if (ss == 0.0 && alpha.y == 0.0) {
-                taui = c2(0.0, 0.0);
-                beta = alpha.x;
-            } else {
-                beta = -copysign(sqrt(fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, ss))), alpha.x);
-                const double rb = fast_rcp(beta);
-                taui = c2((beta - alpha.x) * rb, -alpha.y * rb);
-                const double2 z = c2(alpha.x - beta, alpha.y);
-                const double inv = fast_rcp(fma(z.x, z.x, z.y * z.y));
-                scal = c2(z.x * inv, -z.y * inv);
-            }
-            for (int i = k + 2 + lane; i < n; i += 32) {
-                const double2 vi = cmul(bk[i], scal);
-                vbuf[i] = vi;
-                A[k + (size_t)i * ld] = vi;
-            }
-            if (lane == 0) {
-                vbuf[k + 1] = c2(1.0, 0.0);
-                v.tau[k] = taui;
-                v.d[k] = bk[k].x;
-                v.e[k] = beta;
-            }
-        };
-        if (n >= 2 && warp == 0) reflect(0, v.vb);
-        team_sync<NT, BLOCK>();
-        for (int k = 0; k < n - 1; ++k) {
-            double2* vk = (k & 1) ? v.vb2 : v.vb;
-            double2* vn = (k & 1) ? v.vb : v.vb2;
-            const double2 taui = v.tau[k];
-            const bool has = !(taui.x == 0.0 && taui.y == 0.0);
-            if (has) {
-                // p = tau A22 v: four lanes per row; per-warp partial of p^H v
-                double2 dotp = c2(0.0, 0.0);
-                for (int i = k + 1 + g; i < n; i += NG) {
-                    double2 acc = c2(0.0, 0.0);
-                    for (int j = k + 1 + q; j < n; j += kG) acc = cfma(acc, B[i + (size_t)j * ld], vk[j]);
-                    acc = group_sum2<kG>(gmask, acc);
-                    const double2 pi = cmul(taui, acc);
-                    if (q == 0) { v.pb[i] = pi; dotp = cfmac(dotp, pi, vk[i]); }
-                }
-                dotp = warp_sum2(dotp);
-                if (lane == 0) v.wred[warp] = dotp;
-                team_sync<NT, BLOCK>();
-            }
-            // A22 -= v w^H + w v^H, w = p + alpha2 v, alpha2 = -tau/2 (p^H v)
-            double2 alpha2 = c2(0.0, 0.0);
-            if (has) {
-                double2 dot = c2(0.0, 0.0);
+        // ---- a5a: Householder tridiagonalisation of C (lower), one pass over
+        // the trailing matrix per step. Lane l of a warp holds the rows counted
+        // l, l + 32, ... from the last one up (so that the row blocks in use
+        // follow the trailing matrix); warp w owns the columns j = w mod NW.
+        // Step c (column c):
+        //   one warp (a different one each step, so that the pencils of an SM
+        //   spread over its schedulers): y = A v from the warps' partial
+        //     products (v: reflector c - 1), p = tau y, w = p + alpha2 v
+        //     (alpha2 = -|tau|^2/2 v^H A v, real), column c of the updated
+        //     matrix and from it reflector c, v_c; w, v_c to shared memory
+        //   barrier; every warp over its own columns j > c, one load and one
+        //   store of each element:
+        //     A(:, j) -= v conj(w_j) + w conj(v_j),   y_next += A(:, j) v_c(j)
+        //   barrier
+        // The update and the next product share one pass, where separate
+        // ones took 232 K CTA cycles at n = 54. With every warp doing the
+        // first part for itself (one barrier) a step took twice the
+        // instructions.
+        // Reflector k: I - tau_k v v^H on rows k+1.., v[k+1] = 1; column k of M
+        // keeps v[k+2..] and tau_k at row k + 1. SPEC: rows n .. n+2 see the
+        // same update with v = 0 there, which is P <- P (I - tau v v^H), so
+        // that P Q is in their place at the end.
+        double2* part = work;                    // NW x rows partial products
+        double2* vb = part + NW * rows;          // 2 x rows reflectors (this one, the next)
+        double2* wb = vb + 2 * rows;             // rows
+        const int last = rows - 1 - lane;        // row of slot t: last - 32 t
+#pragma unroll 1
+        for (int i = tid; i < rows; i += NT) vb[rows + i] = wb[i] = zero;   // "reflector -1"
+#pragma unroll 1
+        for (int c = 0; c < n; ++c) {
+            if (warp == (unsigned)(c + (int)b) % NW) {
+                const double2* vk = vb + ((c + 1) & 1) * rows;
+                double2* vc = vb + (c & 1) * rows;
+                double2 x[R], w[R], v[R];
+                const int ic = rows - 1 - c;     // slot of row c
 #pragma unroll
-                for (int w = 0; w < NW; ++w) dot = cadd(dot, v.wred[w]);
-                alpha2 = cscale(cmul(taui, dot), -0.5);
-            }
-            if (warp == 0) {
-                if (has) {
-                    const int j = k + 1;
-                    const double2 vj = vk[j];
-                    const double2 wj = cfma(v.pb[j], alpha2, vj);
-                    for (int i = j + lane; i < n; i += 32) {
-                        const double2 vi = vk[i];
-                        const double2 wi = cfma(v.pb[i], alpha2, vi);
-                        double2* p = B + i + (size_t)j * ld;
-                        *p = cfms_bc(cfms_bc(*p, vi, wj), wi, vj);
-                    }
-                    __syncwarp();
+                for (int t = 0; t < R; ++t) {
+                    const int i = last - 32 * t;
+                    x[t] = M[max(i, 0) + c * ld];
+                    w[t] = zero;
                 }
-                if (k + 1 < n - 1) reflect(k + 1, vn);
-            } else if (has) {
-                // group g - 8 of warps 1.. takes rows k+1+(g-8), + NG-8, ...;
-                // its lanes take columns j = k+2+q step 4 (column k+1 is warp 0's)
-                for (int i = k + 1 + (g - 8); i < n; i += NG - 8) {
-                    const double2 vi = vk[i];
-                    const double2 wi = cfma(v.pb[i], alpha2, vi);
-                    double2* bi = B + i;
-                    int j = k + 2 + q;
-                    for (; j + 4 < n; j += 8) {
-                        const double2 x0 = bi[(size_t)j * ld], x1 = bi[(size_t)(j + 4) * ld];
-                        const double2 v0 = vk[j], v1 = vk[j + 4];
-                        const double2 w0 = cfma(v.pb[j], alpha2, v0), w1 = cfma(v.pb[j + 4], alpha2, v1);
-                        bi[(size_t)j * ld] = cfms_bc(cfms_bc(x0, vi, w0), wi, v0);
-                        bi[(size_t)(j + 4) * ld] = cfms_bc(cfms_bc(x1, vi, w1), wi, v1);
+                if (c > 0) {
+                    const double2 tau = M[c + (c - 1) * ld];
+                    double s = 0.0;
+#pragma unroll
+                    for (int t = 0; t < R; ++t) {
+                        const int i = last - 32 * t, im = max(i, 0);
+                        double2 acc = part[im];
+                        v[t] = vk[im];
+#pragma unroll
+                        for (int u = 1; u < NW; ++u) acc = cadd(acc, part[u * rows + im]);
+                        const bool in = i >= c;
+                        w[t] = c2(in ? acc.x : 0.0, in ? acc.y : 0.0);
+                        v[t] = c2(in ? v[t].x : 0.0, in ? v[t].y : 0.0);
+                        s = fma(w[t].x, v[t].x, fma(w[t].y, v[t].y, s));
                     }
-                    if (j < n) {
-                        const double2 v0 = vk[j];
-                        const double2 w0 = cfma(v.pb[j], alpha2, v0);
-                        bi[(size_t)j * ld] = cfms_bc(cfms_bc(bi[(size_t)j * ld], vi, w0), wi, v0);
+                    const double h = -0.5 * fma(tau.x, tau.x, tau.y * tau.y) * warp_sum(s);
+#pragma unroll
+                    for (int t = 0; t < R; ++t) {
+                        w[t] = cmul(tau, w[t]);
+                        w[t] = c2(fma(h, v[t].x, w[t].x), fma(h, v[t].y, w[t].y));
+                    }
+                    double2 wc = w[0];
+#pragma unroll
+                    for (int t = 1; t < R; ++t) if ((ic >> 5) == t) wc = w[t];
+                    wc = shfl2(wc, ic & 31);
+#pragma unroll
+                    for (int t = 0; t < R; ++t) {
+                        const int i = last - 32 * t;
+                        x[t] = csub(cfms_bc(x[t], v[t], wc), w[t]);      // v(c) = 1
+                        if (i >= c) wb[i] = w[t];
+                        if (SPEC && i >= n) M[i + c * ld] = x[t];        // the final P of column c
                     }
                 }
+                // reflector c from column c (1 / beta comes with the root)
+                double ss = 0.0, dk = x[0].x;
+#pragma unroll
+                for (int t = 0; t < R; ++t) {
+                    const int i = last - 32 * t;
+                    const bool in = i > c + 1 && i < n;
+                    const double xr = in ? x[t].x : 0.0, xi = in ? x[t].y : 0.0;
+                    ss = fma(xr, xr, fma(xi, xi, ss));
+                    if (t > 0 && (ic >> 5) == t) dk = x[t].x;
+                }
+                double2 tau = zero;
+                double beta = 0.0;
+                if (c < n - 1) {
+                    double2 alpha = x[0];
+#pragma unroll
+                    for (int t = 1; t < R; ++t) if (((ic - 1) >> 5) == t) alpha = x[t];
+                    alpha = shfl2(alpha, (ic - 1) & 31);
+                    ss = warp_sum(ss);
+                    double2 scal = zero;
+                    beta = alpha.x;
+                    if (!(ss == 0.0 && alpha.y == 0.0)) {
+                        const double nn = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, ss));
+                        const double rn = rsqrt(nn);
+                        beta = -copysign(nn * rn, alpha.x);
+                        const double rb = -copysign(rn, alpha.x);
+                        tau = c2((beta - alpha.x) * rb, -alpha.y * rb);
+                        const double2 z = c2(alpha.x - beta, alpha.y);
+                        const double inv = fast_rcp(fma(z.x, z.x, z.y * z.y));
+                        scal = c2(z.x * inv, -z.y * inv);
+                    }
+#pragma unroll
+                    for (int t = 0; t < R; ++t) {
+                        const int i = last - 32 * t;
+                        if (i > c) {
+                            const double2 vi = i >= n ? zero : i == c + 1 ? c2(1.0, 0.0) : cmul(x[t], scal);
+                            vc[i] = vi;
+                            if (i < n) M[i + c * ld] = i == c + 1 ? tau : vi;
+                        }
+                    }
+                }
+                if (lane == (ic & 31)) de[c * des] = c2(dk, beta);
             }
+            if (c >= n - 1) break;
+            team_sync<NT, BLOCK>();
+            const double2* vk = vb + ((c + 1) & 1) * rows;
+            const double2* vc = vb + (c & 1) * rows;
+            double2 v[R], w[R], y[R];
+            int off[R];                          // this lane's rows (none: any row, not stored)
+#pragma unroll
+            for (int t = 0; t < R; ++t) {
+                const int i = last - 32 * t;
+                off[t] = max(i, 0);
+                const bool in = i > c;           // rows up to c get no update
+                v[t] = vk[off[t]];
+                w[t] = wb[off[t]];
+                v[t] = c2(in ? v[t].x : 0.0, in ? v[t].y : 0.0);
+                w[t] = c2(in ? w[t].x : 0.0, in ? w[t].y : 0.0);
+                y[t] = zero;
+            }
+            const int j0 = c + 1 + (warp - (c + 1) % NW + NW) % NW;
+            // the own columns, U of them at a time so that their loads and
+            // chains overlap, on the first RT row blocks
+            auto pass = [&](auto rt) {
+                constexpr int RT = decltype(rt)::value, U = RT == 1 ? 4 : 2;
+                double2* q = M + j0 * ld;
+                const double2 *pv = vk + j0, *pw = wb + j0, *pn = vc + j0;
+#pragma unroll 1
+                for (int j = j0; j < n; j += U * NW, q += U * NW * ld, pv += U * NW, pw += U * NW, pn += U * NW) {
+                    double2 z[U][RT];
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+#pragma unroll
+                        for (int t = 0; t < RT; ++t)
+                            if (u == 0 || j + u * NW < n) z[u][t] = q[off[t] + u * NW * ld];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        if (u > 0 && j + u * NW >= n) break;
+                        const double2 vj = pv[u * NW], wj = pw[u * NW], nj = pn[u * NW];
+#pragma unroll
+                        for (int t = 0; t < RT; ++t) {
+                            z[u][t] = cfms_bc(cfms_bc(z[u][t], v[t], wj), w[t], vj);
+                            y[t] = cfma(y[t], z[u][t], nj);
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+#pragma unroll
+                        for (int t = 0; t < RT; ++t)
+                            if ((u == 0 || j + u * NW < n) && last - 32 * t >= 0) q[off[t] + u * NW * ld] = z[u][t];
+                }
+            };
+            const int blocks = (rows - 1 - c + 31) >> 5;         // row blocks that hold rows c + 1 ..
+            if (R == 1 || blocks == 1) pass(IntC<1>{});
+            else if (R == 2 || blocks == 2) pass(IntC<R < 2 ? R : 2>{});
+            else pass(IntC<R>{});
+#pragma unroll
+            for (int t = 0; t < R; ++t)
+                if (last - 32 * t > c) part[warp * rows + last - 32 * t] = y[t];
             team_sync<NT, BLOCK>();
         }
-        if (tid == 0) v.d[n - 1] = B[(n - 1) + (size_t)(n - 1) * ld].x;
         team_sync<NT, BLOCK>();
+#pragma unroll 1
+        for (int k = tid; k < n; k += NT) work[k] = de[k * des];
         phase_mark(4);
-        // ---- a5b: divide and conquer; Z (real) and its workspace in B
-        DCShared dc;
-        dc.Z = reinterpret_cast<double*>(B); dc.ldz = ld;
-        dc.U = dc.Z + (size_t)n * ld;        dc.ldu = ld;
-        dc.d = v.d; dc.e = v.e;
-        dc.w = v.dcd; dc.z = dc.w + n; dc.dl = dc.z + n; dc.zz = dc.dl + n; dc.zh = dc.zz + n;
-        dc.rt = dc.zh + n; dc.rho = dc.rt + n; dc.scal = dc.rho + n;
-        dc.org = v.dci; dc.nd = dc.org + n; dc.perm = dc.nd + n; dc.kcnt = dc.perm + n;
-        tridiag_dc<NT, NMAX, BLOCK>(n, dc);
-        if (tid == 0) {
-            bool bad = false;
-            for (int i = 0; i < n; ++i) bad |= !isfinite(dc.w[i]);
-            v.ctl[4] = bad ? kEigFailCode : 0;
+    phase();
+        if constexpr (SPEC) {
+            // rows of P Q (re, im of each of the three) for the divide and conquer
+#pragma unroll 1
+            for (int idx = tid; idx < 3 * n; idx += NT) {
+                const int c = idx / n, j = idx - c * n;
+                const double2 p = M[n + c + (size_t)j * ld];
+                double* rj = dc.rows + kRowsTracked * j;
+                rj[2 + 2 * c] = p.x;
+                rj[3 + 2 * c] = p.y;
+                if (c == 0) rj[0] = rj[1] = 0.0;
+            }
+        } else {
+            // WY factors: block c (reflectors 8c .. 8c+7) is I - Y_c T_c Y_c^H
+            // (zlarft, forward columnwise: T(l, l) = tau_l, T(0:l, l) =
+            // -tau_l T(0:l, 0:l) Y^H y_l), G = Y^H Y first, one warp per block,
+            // while Y is still in M.
+#pragma unroll 1
+            for (int c = warp; c < nblk; c += NW) {
+                double gr[2] = {0.0, 0.0}, gi[2] = {0.0, 0.0};
+                const int ky = 8 * c + fr;       // reflector of both fragments
+#pragma unroll 1
+                for (int kb = c; kb < nb; ++kb) {
+#pragma unroll
+                    for (int s = 0; s < 2; ++s) {
+                        const int r = 8 * kb + 2 * fq + s;
+                        const double2 yr = (ky >= nref || r <= ky || r >= n) ? zero
+                                         : r == ky + 1 ? c2(1.0, 0.0) : M[r + (size_t)ky * ld];
+                        zmma(gr, gi, cconj(yr), yr);
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int i = 2 * fq + e;
+                    if (fr < i && 8 * c + i < nref) tpk[tidx(c, fr, i)] = c2(gr[e], gi[e]);
+                }
+                __syncwarp();
+                const int mc = min(8, nref - 8 * c), l = lane;
+                double2 trow[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    trow[i] = zero;
+                    if (i < mc && l <= i) {
+                        const int k = 8 * c + i;
+                        const double2 ti = M[k + 1 + (size_t)k * ld];
+                        if (l == i) {
+                            trow[i] = ti;
+                        } else {
+                            double2 s0 = zero, s1 = zero;
+#pragma unroll
+                            for (int m = 0; m < i; ++m) {
+                                if (m < l) continue;
+                                const double2 gm = tpk[tidx(c, m, i)];
+                                if (m & 1) s1 = cfma(s1, trow[m], gm); else s0 = cfma(s0, trow[m], gm);
+                            }
+                            trow[i] = cscale(cmul(ti, cadd(s0, s1)), -1.0);
+                        }
+                    }
+                    __syncwarp();                 // column i of G read before T overwrites it
+                    if (i < mc && l <= i) tpk[tidx(c, l, i)] = trow[i];
+                }
+                __syncwarp();
+            }
+            // reflectors into the lower triangle of U's block
+#pragma unroll 1
+            for (int k = warp; k < nref; k += NW)
+#pragma unroll 1
+                for (int i = k + 1 + lane; i < n; i += 32)
+                    Ub[i + (size_t)k * n] = i == k + 1 ? c2(1.0, 0.0) : M[i + k * ld];
         }
         team_sync<NT, BLOCK>();
+        // ---- a5b: divide and conquer; Z (real) and its workspace in M
+        tridiag_dc<NT, NMAX, BLOCK, SPEC>(n, dc);
+        // a failed eigensolve shows as a non-finite value (every warp looks at
+        // all of them: the verdict is uniform without a barrier)
+        bool bad = false;
+#pragma unroll 1
+        for (int i = lane; i < n; i += 32) bad |= !isfinite(dc.w[i]);
+        if (__any_sync(0xffffffffu, bad)) code = kEigFailCode;
         phase_mark(5);
-        if (v.ctl[4]) code = v.ctl[4];
+    phase();
     }
 
     if (code) {
         const double qnan = __longlong_as_double(0x7ff8000000000000LL);
-        if (a.stage == kStageIntensity) {
+        if constexpr (SPEC) {
+#pragma unroll 1
             for (int e = tid; e < a.ne; e += NT) a.spec[(size_t)b * a.ne + e] = qnan;
         } else {
+            team_sync<NT, BLOCK>();   // earlier writes to U's block come first
+#pragma unroll 1
             for (size_t idx = tid; idx < nn; idx += NT) Ub[idx] = c2(qnan, qnan);
         }
-        if (a.stage >= 3) for (int i = tid; i < n; i += NT) Wb[i] = qnan;
+        if (SPEC || a.stage >= 3) for (int i = tid; i < n; i += NT) Wb[i] = qnan;
         if (tid == 0) a.info[b] = code == kEigFailCode ? eig_fail_info(n) : code;
         return;
     }
 
-    // ---- ascending rank of each eigenvalue
-    for (int j = tid; j < n; j += NT) {
-        const double dj = order_key(v.dcd[j]);
-        int r = 0;
-        for (int k2 = 0; k2 < n; ++k2) {
-            const double dk = order_key(v.dcd[k2]);
-            r += (dk < dj) || (dk == dj && k2 < j);
-        }
-        v.rank[j] = r;
-        Wb[r] = v.dcd[j];
+    // ---- ascending eigenvalues
+#pragma unroll 1
+    for (int t = tid; t < n; t += NT) {
+        const int slot = dc.ord[t];
+        rank[slot] = t;
+        Wb[t] = dc.w[slot];
     }
-    // ---- a5c: V = Q Z with Q = H_0 H_1 ... H_{n-2} in compact-WY blocks of
-    // 16 reflectors on the FP64 tensor cores. Block c (reflectors 16c ..,
-    // m_c of them) is Q_c = I - Y_c T_c Y_c^H (the zlarft forward,
-    // columnwise T: T(l, l) = tau_l, T(0:l, l) = -tau_l T(0:l, 0:l) Y^H y_l),
-    // and V = Q_0 (Q_1 (... Q_last Z)). Steps:
-    //   1. G_c = Y_c^H Y_c (MMA tiles, upper 8x8 tiles), packed into the
-    //      vector area (free from here on); Z (real) into registers.
-    //   2. V = Z as complex in B; T_c by its column recurrence, one warp per
-    //      block, written over G_c column by column.
-    //   3. warp p owns columns [8p, 8p+8) of V and applies the blocks, last
-    //      first, with no CTA barrier: W1 = Y_c^H V_p, W2 = T_c W1,
-    //      V_p -= Y_c W2, the 8-column intermediates passed between MMA
-    //      fragment layouts by shuffles.
-    {
-        const int nref = n - 1;                      // reflectors 0 .. n-2
-        const int nblk = (nref + 15) >> 4;
-        double2* tpk = v.vb;                         // packed upper T_c (G_c before)
-        auto tidx = [](int c, int l, int i) { return 136 * c + ((i * (i + 1)) >> 1) + l; };
-        // Y_c(r, l): reflector k = 16c + l, v_k[k+1] = 1, v_k[r] in A's row k
-        auto yv = [&](int c, int r, int l) -> double2 {
-            const int k = 16 * c + l;
-            if (k >= nref || r <= k || r >= n) return c2(0.0, 0.0);
-            return (r == k + 1) ? c2(1.0, 0.0) : A[k + (size_t)r * ld];
-        };
-        // 1. Gram blocks: tiles (c, hr, hc) with hr <= hc, dealt to the warps
-        for (int t = warp; t < 3 * nblk; t += NW) {
-            const int c = t / 3, hh = t - 3 * c;
-            const int hr = hh == 2 ? 1 : 0, hc = hh == 0 ? 0 : 1;
-            double gr[2] = {0.0, 0.0}, gi[2] = {0.0, 0.0};
-            const int la = 8 * hr + (lane >> 2), lb = 8 * hc + (lane >> 2);
-            for (int k0 = 16 * c; k0 < n; k0 += 4) {
-                const int r = k0 + (lane & 3);
-                const double2 ya = yv(c, r, la);   // A(l, r) = conj(Y(r, l))
-                const double2 yb = yv(c, r, lb);   // B(r, l') = Y(r, l')
-                mma884(gr[0], gr[1], ya.x, yb.x);
-                mma884(gr[0], gr[1], ya.y, yb.y);
-                mma884(gi[0], gi[1], ya.x, yb.y);
-                mma884(gi[0], gi[1], -ya.y, yb.x);
-            }
-            const int l = 8 * hr + (lane >> 2);
-#pragma unroll
-            for (int e2 = 0; e2 < 2; ++e2) {
-                const int i = 8 * hc + 2 * (lane & 3) + e2;
-                if (l < i && 16 * c + i < nref) tpk[tidx(c, l, i)] = c2(gr[e2], gi[e2]);
-            }
-        }
-        // Z (real) into registers, then V = Z as complex in place
-        constexpr int ZR = (NMAX * NMAX + NT - 1) / NT;
-        double zr[ZR];
-        const double* Z = reinterpret_cast<const double*>(B);
-#pragma unroll
-        for (int u = 0; u < ZR; ++u) {
-            const int idx = tid + NT * u, j = idx / n, i = idx - j * n;
-            zr[u] = (idx < n * n) ? Z[i + (size_t)j * ld] : 0.0;
-        }
-        team_sync<NT, BLOCK>();
-#pragma unroll
-        for (int u = 0; u < ZR; ++u) {
-            const int idx = tid + NT * u, j = idx / n, i = idx - j * n;
-            if (idx < n * n) B[i + (size_t)j * ld] = c2(zr[u], 0.0);
-        }
-        // 2. T_c: lane l of warp c holds row l of T_c; column i needs
-        // T(l, m < i) and G(m, i) (l <= m < i); every lane reads column i of
-        // G before any lane overwrites it with column i of T.
-        for (int c = warp; c < nblk; c += NW) {
-            const int l = lane;
-            const int mc = min(16, nref - 16 * c);
-            double2 trow[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                trow[i] = c2(0.0, 0.0);
-                if (i < mc && l < 16 && l <= i) {
-                    const double2 ti = v.tau[16 * c + i];
-                    if (l == i) {
-                        trow[i] = ti;
-                    } else {
-                        double2 s0 = c2(0.0, 0.0), s1 = c2(0.0, 0.0);
-#pragma unroll
-                        for (int m = 0; m < i; ++m) {
-                            if (m < l) continue;
-                            const double2 gm = tpk[tidx(c, m, i)];
-                            if (m & 1) s1 = cfma(s1, trow[m], gm); else s0 = cfma(s0, trow[m], gm);
-                        }
-                        trow[i] = cscale(cmul(ti, cadd(s0, s1)), -1.0);
-                    }
-                }
-                __syncwarp();
-                if (i < mc && l < 16 && l <= i) tpk[tidx(c, l, i)] = trow[i];
-                __syncwarp();
-            }
-        }
-        team_sync<NT, BLOCK>();
-        // 3. per-warp panels: columns [8p, 8p+8), p = warp, warp + NW, ...
-        for (int p = warp; 8 * p < n; p += NW) {
-            const int jb = 8 * p + (lane >> 2);   // B-fragment column of this lane
-            // W (16 x 8, accumulator layout: rows 8h + lane/4, columns
-            // 2(lane%4) + e) -> B-fragment layout for k-step s: element
-            // (4s + lane%4, lane/4), returned as (re, im) scaled by `sgn`
-            auto to_bfrag = [&](const double (&wr)[2][2], const double (&wi)[2][2], int s, double sgn,
-                                double& br, double& bi) {
-                const int src = 16 * (s & 1) + 4 * (lane & 3) + (lane >> 3);
-                const int h = s >> 1, e2 = (lane >> 2) & 1;
-                const double r0 = __shfl_sync(0xffffffffu, wr[h][0], src);
-                const double r1 = __shfl_sync(0xffffffffu, wr[h][1], src);
-                const double i0 = __shfl_sync(0xffffffffu, wi[h][0], src);
-                const double i1 = __shfl_sync(0xffffffffu, wi[h][1], src);
-                br = sgn * (e2 ? r1 : r0);
-                bi = sgn * (e2 ? i1 : i0);
-            };
-            for (int c = nblk - 1; c >= 0; --c) {
-                // W1 = Y_c^H V_p  (16 x 8, K = rows 16c .. n-1)
-                double w1r[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, w1i[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-                for (int k0 = 16 * c; k0 < n; k0 += 4) {
-                    const int r = k0 + (lane & 3);
-                    const double2 vb_ = (r < n && jb < n) ? B[r + (size_t)jb * ld] : c2(0.0, 0.0);
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const double2 ya = yv(c, r, 8 * h + (lane >> 2));
-                        mma884(w1r[h][0], w1r[h][1], ya.x, vb_.x);
-                        mma884(w1r[h][0], w1r[h][1], ya.y, vb_.y);
-                        mma884(w1i[h][0], w1i[h][1], ya.x, vb_.y);
-                        mma884(w1i[h][0], w1i[h][1], -ya.y, vb_.x);
-                    }
-                }
-                // W2 = T_c W1 (T upper, K = 16), negated for the update
-                double w2r[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, w2i[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-#pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    double br, bi;
-                    to_bfrag(w1r, w1i, s, -1.0, br, bi);
-                    const int kk = 4 * s + (lane & 3);
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int l = 8 * h + (lane >> 2);
-                        const double2 ta = (l <= kk && 16 * c + kk < nref) ? tpk[tidx(c, l, kk)] : c2(0.0, 0.0);
-                        mma884(w2r[h][0], w2r[h][1], ta.x, br);
-                        mma884(w2r[h][0], w2r[h][1], -ta.y, bi);
-                        mma884(w2i[h][0], w2i[h][1], ta.x, bi);
-                        mma884(w2i[h][0], w2i[h][1], ta.y, br);
-                    }
-                }
-                // V_p += Y_c (-W2) on row tiles from 2c (rows < 16c + 1 get 0)
-                double bfr[4], bfi[4];
-#pragma unroll
-                for (int s = 0; s < 4; ++s) to_bfrag(w2r, w2i, s, 1.0, bfr[s], bfi[s]);
-                const int j0 = 8 * p + 2 * (lane & 3);
-                for (int t = 2 * c; 8 * t < n; ++t) {
-                    const int r = 8 * t + (lane >> 2);
-                    double ar[2], ai[2];
-#pragma unroll
-                    for (int e2 = 0; e2 < 2; ++e2) {
-                        const double2 x = (r < n && j0 + e2 < n) ? B[r + (size_t)(j0 + e2) * ld] : c2(0.0, 0.0);
-                        ar[e2] = x.x; ai[e2] = x.y;
-                    }
-#pragma unroll
-                    for (int s = 0; s < 4; ++s) {
-                        const double2 ya = yv(c, r, 4 * s + (lane & 3));   // A(r, l) = Y(r, l)
-                        mma884(ar[0], ar[1], ya.x, bfr[s]);
-                        mma884(ar[0], ar[1], -ya.y, bfi[s]);
-                        mma884(ai[0], ai[1], ya.x, bfi[s]);
-                        mma884(ai[0], ai[1], ya.y, bfr[s]);
-                    }
-#pragma unroll
-                    for (int e2 = 0; e2 < 2; ++e2)
-                        if (r < n && j0 + e2 < n) B[r + (size_t)(j0 + e2) * ld] = c2(ar[e2], ai[e2]);
-                }
-                __syncwarp();
-            }
-        }
-    }
-    team_sync<NT, BLOCK>();
-    phase_mark(6);
-    if (a.stage == 3) {
-        for (int jj = tr; jj < n; jj += TR) {
-            double2* uo = Ub + (size_t)v.rank[jj] * n;
-            for (int i = tc; i < n; i += 16) uo[i] = B[i + (size_t)jj * ld];
-        }
-        if (tid == 0) a.info[b] = 0;
-        return;
-    }
-    // ---- a6: U = X^H V, U(i, j) = sum_{k >= i} conj(X(k, i)) V(k, j), FP64
-    // tensor-core tiles; U overwrites V after the barrier.
-    {
-        constexpr int MAXT = ((NMAX / 8) * (NMAX / 8) + NW - 1) / NW;
-        const int tn8 = (n + 7) >> 3;
-        ZTiles<MAXT> acc;
-        ztiles_compute<MAXT, NT, BLOCK>(acc, tn8, tn8,
-            [&](int i, int k) { return (i < n && k >= i && k < n) ? cconj(A[k + (size_t)i * ld]) : c2(0.0, 0.0); },
-            [&](int k, int j) { return (k < n && j < n) ? B[k + (size_t)j * ld] : c2(0.0, 0.0); },
-            [&](int ti, int, int& k0, int& k1) { k0 = 8 * ti; k1 = n; },
-            [](int, int) { return true; });
-        team_sync<NT, BLOCK>();
-        ztiles_store<MAXT, NT, BLOCK>(acc, tn8, tn8, [](int, int) { return true; },
-            [&](int i, int j, double2 c) { if (i < n && j < n) B[i + (size_t)j * ld] = c; });
-        team_sync<NT, BLOCK>();
-        phase_mark(7);
-    }
-    if (a.stage == kStageIntensity) {
-        // ---- spin-wave intensities from U (in B, column jj = eigenvalue
-        // dcd[jj]) without storing U: for each positive eigenvalue lambda,
-        // t = u / sqrt(lambda) is the Bogoliubov vector of the mode of
-        // energy omega = 1 / lambda; Y = O t (3 components) and
+
+    if constexpr (SPEC) {
+        // ---- spin-wave intensities: column jj of P Q Z = O U is Y = O u of
+        // eigenvalue w[jj]. For each positive eigenvalue lambda, t = u /
+        // sqrt(lambda) is the Bogoliubov vector of the mode of energy omega =
+        // 1 / lambda; Y = O t (3 components) and
         // I = sum_ab (delta_ab - q_a q_b) conj(Y_a) Y_b = |Y|^2 - |q . Y|^2;
         // then S(E_e) = sum_modes I g(E_e - omega) with the Gaussian g.
-        // A (X) is free after a6 and takes O (3 n <= n ld for even n);
-        // the modes go to the dead Householder vector pb.
-        const double2* Ob = a.O + (size_t)b * 3 * n;
-        double2* Os = A;
-        double* om = reinterpret_cast<double*>(v.pb);
+        double* om = reinterpret_cast<double*>(M);
         double* it = om + n;
-        for (int idx = tid; idx < 3 * n; idx += NT) Os[idx] = __ldg(Ob + idx);
         const double q0 = __ldg(a.qhat + 3 * b), q1 = __ldg(a.qhat + 3 * b + 1), q2 = __ldg(a.qhat + 3 * b + 2);
-        team_sync<NT, BLOCK>();
-        for (int jj = g; jj < n; jj += NG) {
-            const double lam = v.dcd[jj];
-            double2 y0 = c2(0.0, 0.0), y1 = c2(0.0, 0.0), y2 = c2(0.0, 0.0);
-            for (int i = q; i < n; i += kG) {
-                const double2 u = B[i + (size_t)jj * ld];
-                y0 = cfma(y0, Os[3 * i], u);
-                y1 = cfma(y1, Os[3 * i + 1], u);
-                y2 = cfma(y2, Os[3 * i + 2], u);
-            }
-            const unsigned gm = 0xFu << (lane & ~3);
-            y0 = group_sum2<kG>(gm, y0);
-            y1 = group_sum2<kG>(gm, y1);
-            y2 = group_sum2<kG>(gm, y2);
-            if (q == 0) {
-                const double yy = fma(y0.x, y0.x, fma(y0.y, y0.y, fma(y1.x, y1.x, fma(y1.y, y1.y,
-                                  fma(y2.x, y2.x, y2.y * y2.y)))));
-                const double2 qy = c2(fma(q0, y0.x, fma(q1, y1.x, q2 * y2.x)), fma(q0, y0.y, fma(q1, y1.y, q2 * y2.y)));
-                const bool pos = lam > 0.0;
-                om[jj] = pos ? 1.0 / lam : -1.0;
-                it[jj] = pos ? (yy - fma(qy.x, qy.x, qy.y * qy.y)) / lam : 0.0;
-            }
+#pragma unroll 1
+        for (int jj = tid; jj < n; jj += NT) {
+            const double lam = dc.w[jj];
+            const double* yj = dc.rows + kRowsTracked * jj + 2;
+            const double yy = fma(yj[0], yj[0], fma(yj[1], yj[1], fma(yj[2], yj[2], fma(yj[3], yj[3],
+                              fma(yj[4], yj[4], yj[5] * yj[5])))));
+            const double2 qy = c2(fma(q0, yj[0], fma(q1, yj[2], q2 * yj[4])),
+                                  fma(q0, yj[1], fma(q1, yj[3], q2 * yj[5])));
+            const bool pos = lam > 0.0;
+            om[jj] = pos ? 1.0 / lam : -1.0;
+            it[jj] = pos ? (yy - fma(qy.x, qy.x, qy.y * qy.y)) / lam : 0.0;
         }
         team_sync<NT, BLOCK>();
+#pragma unroll 1
         for (int e = tid; e < a.ne; e += NT) {
             const double E = __ldg(a.energies + e);
             double acc = 0.0;
+#pragma unroll 1
             for (int jj = 0; jj < n; ++jj) {
                 if (!(om[jj] > 0.0)) continue;
                 const double x = E - om[jj];
@@ -784,13 +881,179 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
         }
         if (tid == 0) a.info[b] = 0;
         return;
+    } else {
+        // ---- a5c: V = Q Z in compact-WY blocks of 8 reflectors, last block
+        // first, V = Q_0 (Q_1 (... Q_last Z)), and a6: U = X^H V. Warp p owns
+        // the 8-column panels p, p + NW of V and takes them through both
+        // without a CTA barrier; they share every fragment of Y and X, which
+        // are read from U's block (L2). Per block: W1 = Y_c^H V_p, W2 = T_c W1,
+        // V_p -= Y_c W2, the 8 x 8 intermediates turned from accumulator into
+        // B-fragment layout by shuffles.
+        {   // Z (real) -> V (complex) in place, through registers, the last
+            // columns first (column j of V lies at or above Z's columns 2j, 2j + 1)
+            constexpr int CU = 8, RB = (NMAX + 31) / 32;
+#pragma unroll 1
+            for (int j0 = (n - 1) / (CU * NW) * (CU * NW); j0 >= 0; j0 -= CU * NW) {
+                double zr[CU][RB];
+#pragma unroll
+                for (int u = 0; u < CU; ++u)
+#pragma unroll
+                    for (int t = 0; t < RB; ++t) {
+                        const int j = j0 + warp + NW * u, i = lane + 32 * t;
+                        zr[u][t] = (j < n && i < n) ? dc.Z[i + j * ld] : 0.0;
+                    }
+                team_sync<NT, BLOCK>();
+#pragma unroll
+                for (int u = 0; u < CU; ++u)
+#pragma unroll
+                    for (int t = 0; t < RB; ++t) {
+                        const int j = j0 + warp + NW * u, i = lane + 32 * t;
+                        if (j < n && i < n) M[i + j * ld] = c2(zr[u][t], 0.0);
+                    }
+                team_sync<NT, BLOCK>();
+            }
+        }
+        // accumulator (row fr, columns 2 fq + e) -> B fragment (row 2 fq + s, column fr)
+        auto to_b = [&](const double (&re)[2], const double (&im)[2], int s) -> double2 {
+            const int src = 4 * (2 * fq + s) + (fr >> 1);
+            const double2 y0 = shfl2(c2(re[0], im[0]), src), y1 = shfl2(c2(re[1], im[1]), src);
+            return (fr & 1) ? y1 : y0;
+        };
+        // Y_c(r, l) is at Ub[r + k n], k = 8c + l, for r > k; the tile row c is
+        // masked and rows past n are zero (clamped reads)
+        const int np = (nb - warp + NW - 1) / NW;   // panels of this warp
+        double2* vp[PP];                            // panel columns: B fragment column fr
+#pragma unroll
+        for (int u = 0; u < PP; ++u) vp[u] = M + min(8 * (warp + NW * u) + fr, n - 1) * ld;
+#pragma unroll 1
+        for (int c = nblk - 1; c >= 0; --c) {
+            double wr[PP][2], wi[PP][2];
+#pragma unroll
+            for (int u = 0; u < PP; ++u) wr[u][0] = wr[u][1] = wi[u][0] = wi[u][1] = 0.0;
+            const int ky = 8 * c + fr;
+            const double2* yc = Ub + min(ky, n - 1) * n;
+            double2 yn[2];                       // the next tile's Y, loaded ahead
+#pragma unroll
+            for (int s = 0; s < 2; ++s) yn[s] = yc[min(8 * c + 2 * fq + s, n - 1)];
+#pragma unroll 1
+            for (int kb = c; kb < nb; ++kb) {    // W1 = Y_c^H V
+                const double2 yl[2] = {yn[0], yn[1]};
+                if (kb + 1 < nb) {
+#pragma unroll
+                    for (int s = 0; s < 2; ++s) yn[s] = yc[min(8 * kb + 8 + 2 * fq + s, n - 1)];
+                }
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    const int r = 8 * kb + 2 * fq + s, rc = min(r, n - 1);
+                    const bool in = r > ky && r < n;
+                    const double2 ya = c2(in ? yl[s].x : 0.0, in ? -yl[s].y : 0.0);
+#pragma unroll
+                    for (int u = 0; u < PP; ++u)
+                        if (u < np) zmma(wr[u], wi[u], ya, vp[u][rc]);
+                }
+            }
+            const double2* yr[2];                // A fragments of Y: column 8 c + 2 fq + s
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                yr[s] = Ub + min(8 * c + 2 * fq + s, n - 1) * n;
+                yn[s] = yr[s][min(8 * c + fr, n - 1)];
+            }
+            double2 bw[PP][2];
+#pragma unroll
+            for (int u = 0; u < PP; ++u) {       // W2 = T_c W1, negated
+                if (u >= np) continue;
+                double tr[2] = {0.0, 0.0}, ti[2] = {0.0, 0.0};
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    const int k = 2 * fq + s;
+                    const double2 ta = (fr <= k && 8 * c + k < nref) ? tpk[tidx(c, fr, k)] : zero;
+                    zmma(tr, ti, c2(-ta.x, -ta.y), to_b(wr[u], wi[u], s));
+                }
+#pragma unroll
+                for (int s = 0; s < 2; ++s) bw[u][s] = to_b(tr, ti, s);
+            }
+#pragma unroll 1
+            for (int t = c; t < nb; ++t) {       // V -= Y_c W2 (rows up to 8c get 0)
+                const int r = 8 * t + fr;
+                double2 ya[2];
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    const bool in = t > c || r > 8 * c + 2 * fq + s;
+                    ya[s] = c2(in ? yn[s].x : 0.0, in ? yn[s].y : 0.0);
+                    if (t + 1 < nb) yn[s] = yr[s][min(r + 8, n - 1)];
+                }
+#pragma unroll
+                for (int u = 0; u < PP; ++u) {
+                    if (u >= np) continue;
+                    const int j = 8 * (warp + NW * u) + 2 * fq;
+                    double2* q = M + r + j * ld;
+                    double vr[2], vi[2];
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) { const double2 x = q[e * ld]; vr[e] = x.x; vi[e] = x.y; }
+#pragma unroll
+                    for (int s = 0; s < 2; ++s) zmma(vr, vi, ya[s], bw[u][s]);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        if (r < n && j + e < n) q[e * ld] = c2(vr[e], vi[e]);
+                }
+            }
+            __syncwarp();
+        }
+        phase_mark(6);
+    phase();
+        if (a.stage == 4) {
+            // U(i, j) = sum_{k >= i} conj(X(k, i)) V(k, j), in place from the top:
+            // row tile ti needs the rows of V from 8 ti on only
+#pragma unroll 1
+            for (int ti = 0; ti < nb; ++ti) {
+                double ur[PP][2], ui[PP][2];
+#pragma unroll
+                for (int u = 0; u < PP; ++u) ur[u][0] = ur[u][1] = ui[u][0] = ui[u][1] = 0.0;
+                const int i = 8 * ti + fr;
+                const double2* xi = Ub + min(i, n - 1);
+                double2 xn[2];                   // the next tile's X^H, loaded ahead
+#pragma unroll
+                for (int s = 0; s < 2; ++s) xn[s] = xi[min(8 * ti + 2 * fq + s, n - 1) * n];
+#pragma unroll 1
+                for (int kb = ti; kb < nb; ++kb) {
+                    const double2 xl[2] = {xn[0], xn[1]};
+                    if (kb + 1 < nb) {
+#pragma unroll
+                        for (int s = 0; s < 2; ++s) xn[s] = xi[min(8 * kb + 8 + 2 * fq + s, n - 1) * n];
+                    }
+#pragma unroll
+                    for (int s = 0; s < 2; ++s) {
+                        const int k = 8 * kb + 2 * fq + s, kc = min(k, n - 1);
+                        const bool in = k >= i && k < n;
+                        const double2 xa = c2(in ? xl[s].x : 0.0, in ? xl[s].y : 0.0);
+#pragma unroll
+                        for (int u = 0; u < PP; ++u)
+                            if (u < np) zmma(ur[u], ui[u], xa, vp[u][kc]);
+                    }
+                }
+                __syncwarp();
+#pragma unroll
+                for (int u = 0; u < PP; ++u) {
+                    if (u >= np) continue;
+                    const int j = 8 * (warp + NW * u) + 2 * fq;
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        if (i < n && j + e < n) M[i + (j + e) * ld] = c2(ur[u][e], ui[u][e]);
+                }
+                __syncwarp();
+            }
+        }
+        team_sync<NT, BLOCK>();   // the last reads of X and Y from U's block come before its results
+        phase_mark(7);
+        // ---- a7: store V or U, column j to position rank[j]
+#pragma unroll 1
+        for (int jj = warp; jj < n; jj += NW) {
+            double2* uo = Ub + (size_t)rank[jj] * n;
+#pragma unroll 1
+            for (int i = lane; i < n; i += 32) uo[i] = M[i + (size_t)jj * ld];
+        }
+        if (tid == 0) a.info[b] = 0;
     }
-    // ---- a7: store U, column j to position rank[j]
-    for (int jj = tr; jj < n; jj += TR) {
-        double2* uo = Ub + (size_t)v.rank[jj] * n;
-        for (int i = tc; i < n; i += 16) uo[i] = B[i + (size_t)jj * ld];
-    }
-    if (tid == 0) a.info[b] = 0;
 }
 
 }  // namespace cta

@@ -1,20 +1,26 @@
 // Divide-and-conquer eigensolver for the real symmetric tridiagonal matrix
-// T = tridiag(e, d, e), one CTA, everything in shared memory.
+// T = tridiag(e, d, e), one team of threads.
 //
 // Method (Cuppen's divide and conquer with the Gu-Eisenstat correction, the
 // algorithm of LAPACK dstedc / dlaed0-dlaed4):
-//   * T is torn at every index k in [1, n): d[k-1] and d[k] each lose |e[k-1]|,
-//     so that T = blockdiag(T1', T2') + |e| v v^T with v = e_{k-1} + sign(e) e_k.
-//   * Leaves are 1x1 (Z = I). Blocks are merged bottom-up along a power-of-two
-//     tree: level `half` merges [a, a+half) with [a+half, a+2*half).
+//   * T is torn at every multiple k of kLeaf in [1, n): d[k-1] and d[k] each
+//     lose |e[k-1]|, so that T = blockdiag(T1', T2') + |e| v v^T with
+//     v = e_{k-1} + sign(e) e_k.
+//   * Leaves (kLeaf rows) are solved by the implicit QL iteration (Wilkinson
+//     shift, as EISPACK imtql2), eight lanes per leaf: every lane runs the
+//     same scalar recurrence on its own copy of d and e and keeps one row of
+//     the leaf's eigenvectors, so a leaf needs no communication. Blocks are then merged
+//     bottom-up: level `half` merges [a, a+half) with [a+half, a+2*half).
 //   * A merge forms z = (last row of Q1, sign(e) * first row of Q2)/sqrt(2),
 //     rho = 2|e|, deflates entries with rho|z_j| <= tol and pairs of nearly
 //     equal poles (Givens rotation of the two eigenvector columns), solves the
 //     secular equation 1 + rho sum_j z_j^2/(d_j - lambda) = 0 for the K
-//     remaining roots (one thread per root), recomputes z from the computed
+//     remaining roots (P lanes per root), recomputes z from the computed
 //     roots with Loewner's formula so that the new eigenvectors are orthogonal
 //     to working precision, and multiplies the old eigenvector columns by the
-//     K x K eigenvector matrix of the rank-one problem.
+//     K x K eigenvector matrix of the rank-one problem. Rows of the first half
+//     only meet columns of the first half (the others are zero there) unless
+//     a rotation has mixed the halves, so the product runs over half of K.
 // The secular solver is this file's own: each root is bracketed between its
 // two poles, measured from the nearer pole (so that every d_j - lambda is
 // formed without cancellation), and iterated with a two-pole rational model
@@ -22,45 +28,64 @@
 // point, solve the resulting quadratic), safeguarded by bisection.
 //
 // Output: Z (n x n, column slot j holds the eigenvector of w[j]); w[] in the
-// caller's units. Eigenvalues are not sorted here.
+// caller's units; ord[t] the slot of the t-th smallest eigenvalue.
 //
 // NMAX > 0 bounds n at compile time (Z, U in shared memory; merge products
 // accumulate in registers). NMAX == 0 is the any-n form for matrices kept in
 // global memory: merges wider than 32 columns are 16 x 16 FP64 tensor-core
 // tiles written to the separate buffer Zo and copied back.
+//
+// ROWS: instead of Z, the caller wants only a few combinations of Z's rows
+// (R Z for 6 real rows R). Then only those rows and the first and last row of
+// every block are carried through the merges (kRowsTracked doubles per column
+// slot), which needs neither Z nor U and replaces the O(n^3) merge products by
+// O(n^2) ones.
 #pragma once
 
 #include "geneig_common.cuh"
 
 namespace sgeig {
 
+constexpr int kLeaf = 8;          // rows of a leaf
+constexpr int kLeafStride = 25;   // d, e and a row of z of a lane's leaf (odd: no bank conflicts)
+constexpr int kRowsTracked = 8;   // ROWS: first row, last row, 6 caller rows per column slot
+
 struct DCShared {
     double* Z;  int ldz;    // eigenvectors
     double* U;  int ldu;    // K x K blocks of each merge at [a, a+K)^2
     double* Zo;             // NMAX == 0 only: n x ldz product buffer of the merge GEMMs
-    double* d;  double* e;  // tridiagonal (modified)
+    const double* d; int ds;  // diagonal, element i at d[i * ds]
+    const double* e; int es;  // off-diagonal, element i at e[i * es]
     double* w;              // eigenvalue of column slot j
     double* z;              // merge z-vector by column slot
-    double* dl;             // non-deflated poles [a, a+K)
+    double* dl;             // non-deflated poles [a, a+K), ascending
     double* zz;             // their z
     double* zh;             // Loewner z-hat
     double* rt;             // root offsets from their origin pole
-    int* org;               // origin pole (merge-local index) of each root
-    int* nd;                // non-deflated column slots [a, a+K)
-    int* perm;              // ascending order of the merge's eigenvalues
-    int* kcnt;              // K per merge, indexed by a
     double* rho;            // rho per merge, indexed by a
-    double* scal;           // [0] = scale applied to T
+    double* leaf;           // kLeafStride doubles for each of leaf_lanes lanes (may overlap Z)
+    int leaf_lanes;         // multiple of kLeaf; fewer than n: several passes, which must not overlap Z
+    double* rows;           // ROWS only: rows[kRowsTracked * slot + r]
+    int* org;               // origin pole (merge-local index) of each root
+    int* nd;                // column slots of a merge: the K non-deflated ones ascending, then the deflated ones
+    int* perm;              // ascending order of the merge's poles before deflation
+    int* ord;               // ascending order of each block's eigenvalues
+    int* kl;                // non-deflated (position | slot << 16): first-half slots, then second-half slots
+    int* kcnt;              // per merge at a: K (-1: ord is current), K of the first half, rotated flag
 };
 
-// Largest power of two strictly below x (x >= 2).
-__host__ __device__ constexpr int top_bit(int x) { return (x & (x - 1)) ? top_bit(x & (x - 1)) : x; }
-__host__ __device__ constexpr int pow2_below(int x) { return (x & (x - 1)) ? top_bit(x) : x / 2; }
-static_assert(pow2_below(48) == 32 && pow2_below(64) == 32 && pow2_below(32) == 16 && pow2_below(16) == 8, "pow2_below");
+// Number of doubles / ints of scratch DCShared needs for size n (excluding Z, U, rows).
+__host__ __device__ inline int dc_vec_doubles(int n) { return 7 * n + 1; }
+__host__ __device__ inline int dc_vec_ints(int n) { return 6 * n; }
 
-// Number of doubles / ints of scratch DCShared needs for size n (excluding Z, U).
-__host__ __device__ inline int dc_vec_doubles(int n) { return 8 * n + 2; }
-__host__ __device__ inline int dc_vec_ints(int n) { return 4 * n; }
+__host__ __device__ inline int dc_leaf_doubles(int n) { return kLeafStride * kLeaf * ((n + kLeaf - 1) / kLeaf); }
+
+// Points the scratch members at `dbl` (dc_vec_doubles(n), eigenvalues first)
+// and `ints` (dc_vec_ints(n)).
+__host__ __device__ inline void dc_carve(DCShared& s, double* dbl, int* ints, int n) {
+    s.w = dbl; s.z = s.w + n; s.dl = s.z + n; s.zz = s.dl + n; s.zh = s.zz + n; s.rt = s.zh + n; s.rho = s.rt + n;
+    s.org = ints; s.nd = s.org + n; s.perm = s.nd + n; s.ord = s.perm + n; s.kl = s.ord + n; s.kcnt = s.kl + n;
+}
 
 // Sum over the P consecutive lanes that share one root (P = 1, 2 or 4); on
 // the host (P = 1) it is the identity. Every lane ends with the same value
@@ -100,7 +125,7 @@ __host__ __device__ inline int secular_root_p(int i, int K, const double* dl, co
         const double gap = dl[i + 1] - dl[i];
         const double mid = 0.5 * gap;
         double gs = 0.0;
-#pragma unroll 4
+#pragma unroll 2
         for (int j = qq; j < K; j += P) {
             const double del = (dl[j] - dl[i]) - mid;
             gs = fma(rho * zz[j], zz[j] * fast_rcp(del), gs);
@@ -135,7 +160,7 @@ __host__ __device__ inline int secular_root_p(int i, int K, const double* dl, co
         const double m = 0.5 * hi;
         if (m > 0.0) {
             double gs = 0.0;
-#pragma unroll 4
+#pragma unroll 2
             for (int j = qq; j < K; j += P) {
                 const double del = (dl[j] - dl[K - 1]) - m;
                 gs = fma(rho * zz[j], zz[j] * fast_rcp(del), gs);
@@ -153,25 +178,28 @@ __host__ __device__ inline int secular_root_p(int i, int K, const double* dl, co
     const double q = (i < K - 1) ? dl[i + 1] - dlo : 0.0;
     int it = 0;
     for (; it < 80; ++it) {
-        double psi = 0.0, dpsi = 0.0, phi = 0.0, dphi = 0.0, erra = 0.0;
-#pragma unroll 4
-        for (int j = qq; j < K; j += P) {
-            const double del = (dl[j] - dlo) - tau;
-            const double t = zz[j] * fast_rcp(del);
-            const double term = rho * zz[j] * t;
-            const double dterm = rho * t * t;
-            const bool left = j <= i;       // poles left of the root go to psi
-            psi += left ? term : 0.0;
-            dpsi += left ? dterm : 0.0;
-            phi += left ? 0.0 : term;
-            dphi += left ? 0.0 : dterm;
-            erra += fabs(term);
+        // poles up to i (left of the root) give psi <= 0, the others phi >= 0
+        double psi = 0.0, dpsi = 0.0, phi = 0.0, dphi = 0.0;
+        int j = qq;
+#pragma unroll 2
+        for (; j <= i; j += P) {
+            const double zj = zz[j];
+            const double t = zj * fast_rcp((dl[j] - dlo) - tau);
+            psi = fma(zj, t, psi);
+            dpsi = fma(t, t, dpsi);
         }
-        psi = lanes_sum<P>(psi, mask);
-        dpsi = lanes_sum<P>(dpsi, mask);
-        phi = lanes_sum<P>(phi, mask);
-        dphi = lanes_sum<P>(dphi, mask);
-        erra = lanes_sum<P>(erra, mask);
+#pragma unroll 2
+        for (; j < K; j += P) {
+            const double zj = zz[j];
+            const double t = zj * fast_rcp((dl[j] - dlo) - tau);
+            phi = fma(zj, t, phi);
+            dphi = fma(t, t, dphi);
+        }
+        psi = rho * lanes_sum<P>(psi, mask);
+        dpsi = rho * lanes_sum<P>(dpsi, mask);
+        phi = rho * lanes_sum<P>(phi, mask);
+        dphi = rho * lanes_sum<P>(dphi, mask);
+        const double erra = fabs(psi) + fabs(phi);
         const double g = 1.0 + psi + phi;
         const double err = kEps * (2.0 + 8.0 * erra + 3.0 * fabs(tau) * (dpsi + dphi));
         if (fabs(g) <= err) break;
@@ -226,42 +254,54 @@ __host__ __device__ inline int secular_root(int i, int K, const double* dl, cons
     return secular_root_p<1>(i, K, dl, zz, rho, 0, 0u, tau_out, org_out);
 }
 
-// Phase E of a level whose single merge covers [0, n): 8x8 output tiles on
-// the FP64 tensor cores (mma.m8n8k4.f64), one warp per tile, accumulators in
-// registers (n <= NMAX); all reads finish before the barrier, then the tiles
-// are written back to the gathered columns.
+// Phase E of a level for NMAX > 0: the merges' products on the FP64 tensor
+// cores (mma.m8n8k4.f64), a warp per 8-row tile with all K columns of the
+// result in registers, so that the tile is read (and its old columns used up)
+// before the same warp overwrites it, without a barrier. A row tile lies in
+// one half of its merge (half is a multiple of 8), so its k loop runs over the
+// columns of that half only, unless a rotation mixed them. Columns past K are
+// computed from whatever lies there and not stored.
 template <int NT, int NMAX, int BLOCK = NT>
-__device__ __forceinline__ void dc_merge_top_regs(int n, const DCShared& s) {
+__device__ __forceinline__ void dc_merge_panels(int n, int half, int span, const DCShared& s) {
     const int lane = team_tid<NT, BLOCK>() & 31, warp = team_tid<NT, BLOCK>() >> 5;
-    constexpr int NW = NT / 32;
-    const int K = s.kcnt[0];
-    const int tm = (n + 7) >> 3, tn = (K + 7) >> 3;
-    constexpr int MAXT = ((NMAX / 8) * (NMAX / 8) + NW - 1) / NW;
-    double acc[MAXT][2];
+    constexpr int NW = NT / 32, NB = NMAX / 8;
+    const int fr = lane >> 2, fq = lane & 3;
+#pragma unroll 1
+    for (int r0 = 8 * warp; r0 < n; r0 += 8 * NW) {
+        const int a = r0 - r0 % span;
+        const int K = a + half < n ? s.kcnt[a] : 0;
+        if (K == 0) continue;
+        const int K1 = s.kcnt[a + 1], r = r0 + fr;
+        const bool dense = s.kcnt[a + 2] != 0, upper = r0 - a < half;
+        const int k0 = (dense || upper) ? 0 : K1, k1 = (dense || !upper) ? K : K1;
+        const int* kl = s.kl + a;
+        const double* zr = s.Z + min(r, n - 1);
+        const double* uc = s.U + a + (size_t)(a + fr) * s.ldu;
+        double acc[NB][2];
 #pragma unroll
-    for (int u = 0; u < MAXT; ++u) {
-        acc[u][0] = acc[u][1] = 0.0;
-        const int t = warp + NW * u;
-        if (K == 0 || t >= tm * tn) continue;
-        const int ti = t / tn, tj = t - ti * tn;
-        const int ia = 8 * ti + (lane >> 2), jb = 8 * tj + (lane >> 2);
-        for (int k = 0; k < K; k += 4) {
-            const int ka = k + (lane & 3);
-            const double av = (ia < n && ka < K) ? s.Z[ia + (size_t)s.nd[ka] * s.ldz] : 0.0;
-            const double bv = (ka < K && jb < K) ? s.U[ka + (size_t)jb * s.ldu] : 0.0;
-            asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                : "+d"(acc[u][0]), "+d"(acc[u][1]) : "d"(av), "d"(bv));
+        for (int t = 0; t < NB; ++t) acc[t][0] = acc[t][1] = 0.0;
+#pragma unroll 1
+        for (int k = k0; k < k1; k += 4) {
+            const int ka = k + fq;
+            const int ps = kl[min(ka, k1 - 1)];
+            double av = zr[(size_t)(ps >> 16) * s.ldz];
+            if (ka >= k1) av = 0.0;
+            const double* ur = uc + (ps & 0xffff);
+#pragma unroll
+            for (int t = 0; t < NB; ++t) {
+                if (8 * t >= K) continue;
+                const double bv = ur[(size_t)(8 * t) * s.ldu];
+                asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                    : "+d"(acc[t][0]), "+d"(acc[t][1]) : "d"(av), "d"(bv));
+            }
         }
-    }
-    team_sync<NT, BLOCK>();
+        __syncwarp();
 #pragma unroll
-    for (int u = 0; u < MAXT; ++u) {
-        const int t = warp + NW * u;
-        if (K == 0 || t >= tm * tn) continue;
-        const int ti = t / tn, tj = t - ti * tn;
-        const int r = 8 * ti + (lane >> 2), j = 8 * tj + 2 * (lane & 3);
-        if (r < n && j < K) s.Z[r + (size_t)s.nd[j] * s.ldz] = acc[u][0];
-        if (r < n && j + 1 < K) s.Z[r + (size_t)s.nd[j + 1] * s.ldz] = acc[u][1];
+        for (int t = 0; t < NB; ++t) {
+            const int j = 8 * t + 2 * fq;
+            if (r < n && j < K) s.Z[r + (size_t)s.nd[a + j] * s.ldz] = acc[t][0];
+            if (r < n && j + 1 < K) s.Z[r + (size_t)s.nd[a + j + 1] * s.ldz] = acc[t][1];
+        }
     }
 }
 
@@ -364,150 +404,388 @@ __device__ __forceinline__ void dc_merge_tiled(int n, int half, int span, const 
     }
 }
 
-// All NT threads of the CTA call this. n >= 1. On return Z, w hold the
-// eigen-decomposition of the tridiagonal (d, e) given on entry.
-template <int NT, int NMAX, int BLOCK = NT>
+// Implicit QL with Wilkinson shift on a leaf of m <= kLeaf rows: d, e (e[i]
+// couples i and i+1) and one row z of the eigenvector matrix, all private to
+// the calling lane (shared memory: the indices are data-dependent); every
+// lane of the leaf's group runs the same recurrence on the same data. Returns
+// false when it did not converge (non-finite input).
+__device__ __forceinline__ bool leaf_ql(int m, double* d, double* e, double* z) {
+#pragma unroll 1
+    for (int it = 0; it < 30 * kLeaf; ++it) {
+        unsigned small = ~0u << (m - 1);
+#pragma unroll 1
+        for (int i = 0; i < m - 1; ++i)
+            if (fabs(e[i]) <= kEps * (fabs(d[i]) + fabs(d[i + 1]))) small |= 1u << i;
+        if (small == ~0u) return true;
+        const int l = __ffs(~small) - 1;                       // first off-diagonal left
+        const int top = l + __ffs(small >> l) - 1;             // its block is [l, top]
+        const double dl = d[l], el = e[l];
+        const double hd = 0.5 * (d[l + 1] - dl);
+        const double qs = hd + copysign(sqrt(fma(hd, hd, el * el)), hd);
+        double dnext = d[top];
+        double g = dnext - dl + (qs != 0.0 ? el * el * fast_rcp(qs) : 0.0);
+        double s = 1.0, c = 1.0, p = 0.0;
+        int i = top - 1;
+        double znext = z[top];
+#pragma unroll 1
+        for (; i >= l; --i) {
+            const double ei = e[i], di = d[i], zi = z[i];
+            const double f = s * ei, b = c * ei;
+            const double q = fma(f, f, g * g);
+            if (q == 0.0) break;                               // the chase ended early: the block splits here
+            const double inv = rsqrt(q);
+            e[i + 1] = q * inv;
+            s = f * inv;
+            c = g * inv;
+            g = dnext - p;
+            const double r = fma(di - g, s, 2.0 * c * b);
+            p = s * r;
+            d[i + 1] = g + p;
+            g = fma(c, r, -b);
+            z[i + 1] = fma(s, zi, c * znext);
+            znext = fma(c, zi, -s * znext);
+            dnext = di;
+        }
+        z[i + 1] = znext;
+        d[i + 1] = dnext - p;
+        if (i < l) e[l] = g; else e[i + 1] = 0.0;
+        e[top] = 0.0;
+    }
+    return false;
+}
+
+// One warp: ord[a, b), the ascending order of a block, from its last merge
+// (nothing to do when it has had none since ord was written). Roots and
+// deflated values are two ascending lists, merged by binary search, unless a
+// rotation changed deflated values (then by counting). The counts form a
+// permutation for finite values; with NaN they may collide, which leaves
+// stale but valid slots of the block in ord.
+__device__ __forceinline__ void dc_order(int a, int b, const DCShared& s, int lane) {
+    const int K = s.kcnt[a];
+    if (K < 0) return;
+    const int m = b - a;
+    const int* nd = s.nd + a;
+    const bool rotated = s.kcnt[a + 2] != 0;
+    for (int t = lane; t < m; t += 32) {
+        const int slot = nd[t];
+        const double key = order_key(s.w[slot]);
+        int pos;
+        if (rotated) {
+            pos = 0;
+            for (int q = 0; q < m; ++q) {
+                const double kq = order_key(s.w[nd[q]]);
+                pos += (kq < key) || (kq == key && q < t);
+            }
+        } else {
+            // first element of the other list that goes after this one
+            int lo = t < K ? K : 0, hi = t < K ? m : K;
+            const int lo0 = lo;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                const double km = order_key(s.w[nd[mid]]);
+                if (t < K ? km < key : km <= key) lo = mid + 1; else hi = mid;
+            }
+            pos = (lo - lo0) + (t < K ? t : t - K);
+        }
+        s.ord[a + pos] = slot;
+    }
+}
+
+// All NT threads of the team call this. n >= 1. On return Z (or rows), w and
+// ord hold the eigen-decomposition of the tridiagonal (d, e), which is only
+// read. ROWS: on entry rows[kRowsTracked * j + 2 ..] hold the six caller rows
+// R (R[.][j]) and Z is scratch for the leaves (at least n x kLeaf, ldz >= n).
+template <int NT, int NMAX, int BLOCK = NT, bool ROWS = false>
 __device__ void tridiag_dc(int n, DCShared s) {
     const int tid = team_tid<NT, BLOCK>(), lane = tid & 31, warp = tid >> 5;
     constexpr int NW = NT / 32;
+    // lanes per secular root and rank-one column: as many as let one pass of
+    // the team cover every root (more lanes shorten each root's term loop)
+    constexpr int P = NMAX == 0 || NT >= 4 * NMAX ? 4 : NT >= 2 * NMAX ? 2 : 1;
 
-    // ---- scale T by a power of two so that max |T_ij| is in [0.5, 1)
-    if (tid < 32) {
+    // ---- scale T by a power of two so that max |T_ij| is in [0.5, 1); every
+    // warp finds the scale by itself (no barrier)
+    double sc = 1.0;
+    {
         double mx = 0.0;
-        for (int i = lane; i < n; i += 32) mx = fmax(mx, fabs(s.d[i]));
-        for (int i = lane; i < n - 1; i += 32) mx = fmax(mx, fabs(s.e[i]));
+#pragma unroll 1
+        for (int i = lane; i < n; i += 32) mx = fmax(mx, fabs(s.d[(size_t)i * s.ds]));
+#pragma unroll 1
+        for (int i = lane; i < n - 1; i += 32) mx = fmax(mx, fabs(s.e[(size_t)i * s.es]));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (lane == 0) {
+        if (mx > 0.0 && isfinite(mx)) {
             int ex = 0;
-            double sc = 1.0;
-            if (mx > 0.0 && isfinite(mx)) { frexp(mx, &ex); sc = ldexp(1.0, -ex); }
-            s.scal[0] = sc;
+            frexp(mx, &ex);
+            sc = ldexp(1.0, -ex);
+        }
+    }
+    // ---- leaves: torn at multiples of kLeaf, solved by eight lanes each, as
+    // many at a time as the leaf buffer holds
+    const int lanes = min(s.leaf_lanes, NT) & ~(kLeaf - 1);
+#pragma unroll 1
+    for (int f0 = 0; f0 * kLeaf < n; f0 += lanes / kLeaf) {
+        const int f = f0 + tid / kLeaf, o = f * kLeaf, m = min(kLeaf, n - o), r = tid % kLeaf;
+        const bool mine = tid < lanes && o < n;
+        double zr[kLeaf], dr = 0.0;
+        int pos = 0;
+        if (mine) {
+            double* d = s.leaf + tid * kLeafStride;
+            double* e = d + kLeaf;
+            double* z = e + kLeaf;
+            bool ok = true;
+#pragma unroll 1
+            for (int i = 0; i < m; ++i) {
+                double di = s.d[(o + i) * s.ds] * sc, ei = i < m - 1 ? s.e[(o + i) * s.es] * sc : 0.0;
+                if (i == 0 && o > 0) di -= fabs(s.e[(o - 1) * s.es] * sc);
+                if (i == kLeaf - 1 && o + kLeaf < n) di -= fabs(s.e[(o + i) * s.es] * sc);
+                ok = ok && isfinite(di) && isfinite(ei);
+                d[i] = di;
+                e[i] = ei;
+                z[i] = i == r ? 1.0 : 0.0;
+            }
+            if (ok) ok = leaf_ql(m, d, e, z);
+            if (!ok) for (int i = 0; i < m; ++i) d[i] = __longlong_as_double(0x7ff8000000000000LL);
+            if (r < m) {
+                dr = d[r];
+                const double key = order_key(dr);
+#pragma unroll 1
+                for (int i = 0; i < m; ++i) {
+                    const double ki = order_key(d[i]);
+                    pos += (ki < key) || (ki == key && i < r);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < kLeaf; ++i) zr[i] = i < m ? z[i] : 0.0;
+        }
+        if (lanes >= n) team_sync<NT, BLOCK>();               // every leaf is done before Z overwrites the buffer
+        if (!ROWS && f0 == 0) {
+#pragma unroll 1
+            for (int j = warp; j < n; j += NW)
+#pragma unroll 1
+                for (int i = lane; i < n; i += 32)
+                    if ((i ^ j) >= kLeaf) s.Z[i + (size_t)j * s.ldz] = 0.0;   // outside the leaves' blocks
+        }
+        if (mine && r < m) {
+            s.ord[o + pos] = o + r;
+            s.w[o + r] = dr;
+            if (r == 0) s.kcnt[o] = -1;
+#pragma unroll
+            for (int i = 0; i < kLeaf; ++i) {
+                if (i >= m) continue;
+                s.Z[o + r + (size_t)(ROWS ? i : o + i) * s.ldz] = zr[i];
+                if (ROWS) {
+                    if (r == 0) s.rows[kRowsTracked * (o + i)] = zr[i];
+                    if (r == m - 1) s.rows[kRowsTracked * (o + i) + 1] = zr[i];
+                }
+            }
         }
     }
     team_sync<NT, BLOCK>();
-    const double sc = s.scal[0];
-    // ---- scale, tear at every split, leaves: Z = I, w = d
-    for (int i = tid; i < n; i += NT) {
-        double di = s.d[i] * sc;
-        if (i > 0) di -= fabs(s.e[i - 1] * sc);
-        if (i < n - 1) di -= fabs(s.e[i] * sc);
-        s.w[i] = di;
+    if constexpr (ROWS) {
+        // the caller's rows times the leaves' eigenvectors
+        constexpr int RQ = (6 * NMAX + NT - 1) / NT;
+        double v[RQ];
+#pragma unroll
+        for (int u = 0; u < RQ; ++u) {
+            const int idx = tid + NT * u, j = idx / 6, q = idx - 6 * j;
+            v[u] = 0.0;
+            if (j < n) {
+                const int o = j & ~(kLeaf - 1), m = min(kLeaf, n - o);
+#pragma unroll 1
+                for (int r = 0; r < m; ++r)
+                    v[u] = fma(s.rows[kRowsTracked * (o + r) + 2 + q], s.Z[o + r + (size_t)(j - o) * s.ldz], v[u]);
+            }
+        }
+        team_sync<NT, BLOCK>();
+#pragma unroll
+        for (int u = 0; u < RQ; ++u) {
+            const int idx = tid + NT * u, j = idx / 6, q = idx - 6 * j;
+            if (j < n) s.rows[kRowsTracked * j + 2 + q] = v[u];
+        }
+        team_sync<NT, BLOCK>();
     }
-    team_sync<NT, BLOCK>();   // every unscaled e[] read above before it is scaled in place
-    for (int i = tid; i < n - 1; i += NT) s.e[i] *= sc;
-    for (int idx = tid; idx < n * n; idx += NT) {
-        const int j = idx / n, i = idx - j * n;
-        s.Z[i + j * s.ldz] = (i == j) ? 1.0 : 0.0;
-    }
-    team_sync<NT, BLOCK>();
     phase_mark(10);
 
-    for (int half = 1; half < n; half <<= 1) {
+#pragma unroll 1
+    for (int half = kLeaf;; half <<= 1) {
         const int span = half << 1;
-        // ---- phase A: one warp per merge: z, order, deflation
+        // ---- phase A: one warp per merge: order, z, deflation (after the
+        // last merge only the order of the whole)
+#pragma unroll 1
         for (int a = warp * span; a < n; a += NW * span) {
             const int k = a + half;
-            if (k >= n) { if (lane == 0) s.kcnt[a] = 0; continue; }
             const int b = min(a + span, n);
             const int m = b - a;
-            const double er = s.e[k - 1];
-            if (er == 0.0) { if (lane == 0) s.kcnt[a] = 0; continue; }
+#pragma unroll 1
+            for (int h0 = a; h0 < b; h0 += half) dc_order(h0, min(h0 + half, b), s, lane);
+            if (k >= n) {
+                __syncwarp();
+                if (lane == 0) s.kcnt[a] = -1;
+                continue;
+            }
+#pragma unroll 1
+            for (int t = lane; t < m; t += 32) s.perm[a + t] = a + t;
+            __syncwarp();
+            // ascending order of the merged poles: two ascending lists
+#pragma unroll 1
+            for (int t = lane; t < m; t += 32) {
+                const bool first = t < half;
+                const int slot = s.ord[a + t];
+                const double key = order_key(s.w[slot]);
+                int lo = first ? half : 0, hi = first ? m : half;
+                const int lo0 = lo;
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    const double km = order_key(s.w[s.ord[a + mid]]);
+                    if (first ? km < key : km <= key) lo = mid + 1; else hi = mid;
+                }
+                s.perm[a + (lo - lo0) + (first ? t : t - half)] = slot;
+            }
+            const double er = s.e[(size_t)(k - 1) * s.es] * sc;
             const double sgn = er < 0.0 ? -1.0 : 1.0;
             const double rho = 2.0 * fabs(er);
-            double zmax = 0.0, dmax = 0.0;
+            double mx = 0.0;
+#pragma unroll 1
             for (int j = a + lane; j < b; j += 32) {
-                const double zj = (j < k ? s.Z[(k - 1) + j * s.ldz] : sgn * s.Z[k + j * s.ldz]) * 0.70710678118654752440;
+                double zj;
+                if constexpr (ROWS) {
+                    // last row of the first half, first row of the second; the
+                    // merged block's first (last) row is zero in the second
+                    // (first) half's columns
+                    double* rj = s.rows + kRowsTracked * j;
+                    zj = (j < k ? rj[1] : sgn * rj[0]) * 0.70710678118654752440;
+                    rj[j < k ? 1 : 0] = 0.0;
+                } else {
+                    zj = (j < k ? s.Z[(k - 1) + (size_t)j * s.ldz] : sgn * s.Z[k + (size_t)j * s.ldz]) *
+                         0.70710678118654752440;
+                }
                 s.z[j] = zj;
-                zmax = fmax(zmax, fabs(zj));
-                dmax = fmax(dmax, fabs(s.w[j]));
+                mx = fmax(mx, fmax(fabs(zj), fabs(s.w[j])));
             }
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                zmax = fmax(zmax, __shfl_xor_sync(0xffffffffu, zmax, o));
-                dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
-            }
-            const double tol = 8.0 * kEps * fmax(dmax, zmax);
-            for (int j = a + lane; j < b; j += 32) {
-                const double wj = order_key(s.w[j]);
-                int r = 0;
-                for (int t = a; t < b; ++t) {
-                    const double wt = order_key(s.w[t]);
-                    r += (wt < wj) || (wt == wj && t < j);
-                }
-                s.perm[a + r] = j;   // r in [0, m): the keys are totally ordered
-            }
+            for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            const double tol = 8.0 * kEps * mx;
             __syncwarp();
-            // fast path: keep entries with rho|z| > tol, in ascending order
-            int base = 0;
+            // keep entries with rho|z| > tol, in ascending order (none when
+            // the tear is zero): counts first, then the lists
+            int K0 = 0, K1 = 0;
+#pragma unroll 1
             for (int t0 = 0; t0 < m; t0 += 32) {
                 const int t = t0 + lane;
-                int j = -1;
-                bool keep = false;
-                if (t < m) { j = s.perm[a + t]; keep = rho * fabs(s.z[j]) > tol; }
+                const int j = t < m ? s.perm[a + t] : a;
+                const bool keep = t < m && rho * fabs(s.z[j]) > tol;
                 const unsigned mask = __ballot_sync(0xffffffffu, keep);
-                const int pos = base + __popc(mask & ((1u << lane) - 1u));
-                if (keep) { s.nd[a + pos] = j; s.dl[a + pos] = s.w[j]; s.zz[a + pos] = s.z[j]; }
+                const unsigned mask1 = __ballot_sync(0xffffffffu, keep && j < k);
+                K0 += __popc(mask);
+                K1 += __popc(mask1);
+            }
+            int base = 0, base1 = 0;
+#pragma unroll 1
+            for (int t0 = 0; t0 < m; t0 += 32) {
+                const int t = t0 + lane;
+                const int j = t < m ? s.perm[a + t] : a;
+                const bool keep = t < m && rho * fabs(s.z[j]) > tol;
+                const unsigned mask = __ballot_sync(0xffffffffu, keep);
+                const unsigned mask1 = __ballot_sync(0xffffffffu, keep && j < k);
+                const unsigned below = (1u << lane) - 1u;
+                const int pos = base + __popc(mask & below);
+                const int pos1 = base1 + __popc(mask1 & below);
+                if (keep) {
+                    s.nd[a + pos] = j; s.dl[a + pos] = s.w[j]; s.zz[a + pos] = s.z[j];
+                    s.kl[a + (j < k ? pos1 : K1 + pos - pos1)] = pos | (j << 16);
+                } else if (t < m) {
+                    s.nd[a + K0 + t - pos] = j;
+                }
                 base += __popc(mask);
+                base1 += __popc(mask1);
             }
             __syncwarp();
-            const int K0 = base;
             bool close = false;
+#pragma unroll 1
             for (int p = 1 + lane; p < K0; p += 32) {
                 const double T = s.dl[a + p] - s.dl[a + p - 1];
                 const double zn = s.zz[a + p], zp = s.zz[a + p - 1];
                 close |= fabs(T) * fabs(zn * zp) <= tol * (zn * zn + zp * zp);
             }
             close = __any_sync(0xffffffffu, close);
-            if (close && lane == 0) {
-                // sequential deflation with rotations of nearly equal poles
-                int K = 0, pj = -1;
-                for (int t = 0; t < m; ++t) {
-                    const int nj = s.perm[a + t];
-                    if (!(rho * fabs(s.z[nj]) > tol)) continue;
-                    if (pj < 0) { pj = nj; continue; }
-                    const double T = s.w[nj] - s.w[pj];
-                    const double zn = s.z[nj], zp = s.z[pj];
-                    const double t2 = zn * zn + zp * zp;
-                    if (fabs(T) * fabs(zn * zp) <= tol * t2) {
-                        const double ta = sqrt(t2);
-                        const double c = zn / ta, sn = -zp / ta;
-                        s.z[nj] = ta; s.z[pj] = 0.0;
-                        for (int r = a; r < b; ++r) {
-                            const double x = s.Z[r + pj * s.ldz], y = s.Z[r + nj * s.ldz];
-                            s.Z[r + pj * s.ldz] = c * x + sn * y;
-                            s.Z[r + nj * s.ldz] = c * y - sn * x;
+            if (lane == 0) {
+                int K = K0;
+                if (close) {
+                    // sequential deflation with rotations of nearly equal
+                    // poles; deflated slots fill nd from the back
+                    K = 0;
+                    int pj = -1, back = m;
+#pragma unroll 1
+                    for (int t = 0; t < m; ++t) {
+                        const int nj = s.perm[a + t];
+                        if (!(rho * fabs(s.z[nj]) > tol)) { s.org[a + --back] = nj; continue; }
+                        if (pj < 0) { pj = nj; continue; }
+                        const double T = s.w[nj] - s.w[pj];
+                        const double zn = s.z[nj], zp = s.z[pj];
+                        const double t2 = zn * zn + zp * zp;
+                        if (fabs(T) * fabs(zn * zp) <= tol * t2) {
+                            const double ta = sqrt(t2);
+                            const double c = zn / ta, sn = -zp / ta;
+                            s.z[nj] = ta; s.z[pj] = 0.0;
+                            if constexpr (ROWS) {
+                                double* x = s.rows + kRowsTracked * pj;
+                                double* y = s.rows + kRowsTracked * nj;
+#pragma unroll 1
+                                for (int r = 0; r < kRowsTracked; ++r) {
+                                    const double xr = x[r], yr = y[r];
+                                    x[r] = c * xr + sn * yr;
+                                    y[r] = c * yr - sn * xr;
+                                }
+                            } else {
+#pragma unroll 1
+                                for (int r = a; r < b; ++r) {
+                                    const double x = s.Z[r + (size_t)pj * s.ldz], y = s.Z[r + (size_t)nj * s.ldz];
+                                    s.Z[r + (size_t)pj * s.ldz] = c * x + sn * y;
+                                    s.Z[r + (size_t)nj * s.ldz] = c * y - sn * x;
+                                }
+                            }
+                            const double wp = s.w[pj], wn = s.w[nj];
+                            s.w[pj] = wp * c * c + wn * sn * sn;
+                            s.w[nj] = wp * sn * sn + wn * c * c;
+                            s.org[a + --back] = pj;
+                        } else {
+                            s.nd[a + K] = pj; s.dl[a + K] = s.w[pj]; s.zz[a + K] = s.z[pj];
+                            s.kl[a + K] = K | (pj << 16);
+                            ++K;
                         }
-                        const double wp = s.w[pj], wn = s.w[nj];
-                        s.w[pj] = wp * c * c + wn * sn * sn;
-                        s.w[nj] = wp * sn * sn + wn * c * c;
-                        pj = nj;
-                    } else {
-                        s.nd[a + K] = pj; s.dl[a + K] = s.w[pj]; s.zz[a + K] = s.z[pj]; ++K;
                         pj = nj;
                     }
+                    if (pj >= 0) {
+                        s.nd[a + K] = pj; s.dl[a + K] = s.w[pj]; s.zz[a + K] = s.z[pj];
+                        s.kl[a + K] = K | (pj << 16);
+                        ++K;
+                    }
+#pragma unroll 1
+                    for (int t = K; t < m; ++t) s.nd[a + t] = s.org[a + t];   // back == K here
                 }
-                if (pj >= 0) { s.nd[a + K] = pj; s.dl[a + K] = s.w[pj]; s.zz[a + K] = s.z[pj]; ++K; }
                 s.kcnt[a] = K;
-                s.rho[a] = rho;
-            } else if (lane == 0) {
-                s.kcnt[a] = K0;
+                s.kcnt[a + 1] = K1;
+                s.kcnt[a + 2] = close ? 1 : 0;
                 s.rho[a] = rho;
             }
         }
         team_sync<NT, BLOCK>();
         phase_mark(11);
-        // ---- phase B: secular roots, four lanes per root (root slot = tid / 4)
-        for (int p0 = 0; p0 < 4 * n; p0 += NT) {
-            const int pidx = (p0 + tid) >> 2, qq = tid & 3;
-            const unsigned qmask = 0xFu << (lane & ~3);
+        if (half >= n) break;
+        // ---- phase B: secular roots, P lanes per root
+        const int qq = tid & (P - 1);
+        const unsigned qmask = (P == 4 ? 0xFu : P == 2 ? 0x3u : 0x1u) << (lane & ~(P - 1));
+#pragma unroll 1
+        for (int p0 = 0; p0 < P * n; p0 += NT) {
+            const int pidx = (p0 + tid) / P;
             if (pidx >= n) continue;
             const int a = pidx - pidx % span;
             if (a + half >= n) continue;
             const int i = pidx - a, K = s.kcnt[a];
             if (i >= K) continue;
             double t; int o;
-            const int its = secular_root_p<4>(i, K, s.dl + a, s.zz + a, s.rho[a], qq, qmask, t, o);
+            const int its = secular_root_p<P>(i, K, s.dl + a, s.zz + a, s.rho[a], qq, qmask, t, o);
             if (qq == 0) {
                 s.rt[pidx] = t; s.org[pidx] = o;
                 phase_count(27, (unsigned long long)its);
@@ -518,10 +796,10 @@ __device__ void tridiag_dc(int n, DCShared s) {
         team_sync<NT, BLOCK>();
         phase_mark(12);
         phase_level_flush(28);
-        // ---- phase C: Loewner z-hat, four lanes per root
-        for (int p0 = 0; p0 < 4 * n; p0 += NT) {
-            const int pidx = (p0 + tid) >> 2, qq = tid & 3;
-            const unsigned qmask = 0xFu << (lane & ~3);
+        // ---- phase C: Loewner z-hat, P lanes per root
+#pragma unroll 1
+        for (int p0 = 0; p0 < P * n; p0 += NT) {
+            const int pidx = (p0 + tid) / P;
             if (pidx >= n) continue;
             const int a = pidx - pidx % span;
             if (a + half >= n) continue;
@@ -530,54 +808,93 @@ __device__ void tridiag_dc(int n, DCShared s) {
             const double* dl = s.dl + a;
             const double dli = dl[i];
             double W = (qq == 0) ? (dli - dl[s.org[a + i]]) - s.rt[a + i] : 1.0;
-            for (int j = qq; j < K; j += 4) {
+#pragma unroll 2
+            for (int j = qq; j < K; j += P) {
                 if (j == i) continue;
                 const double del = (dli - dl[s.org[a + j]]) - s.rt[a + j];
                 W *= del * fast_rcp(dli - dl[j]);
             }
-            W = lanes_prod<4>(W, qmask);
+            W = lanes_prod<P>(W, qmask);
             if (qq == 0) s.zh[pidx] = copysign(sqrt(fmax(-W, 0.0)), s.zz[pidx]);
         }
         team_sync<NT, BLOCK>();
         phase_mark(13);
-        // ---- phase D: eigenvector columns of the rank-one problem (four lanes
-        // per column), new eigenvalues
-        for (int p0 = 0; p0 < 4 * n; p0 += NT) {
-            const int pidx = (p0 + tid) >> 2, qq = tid & 3;
-            const unsigned qmask = 0xFu << (lane & ~3);
-            if (pidx >= n) continue;
+        // ---- phase D: eigenvector columns of the rank-one problem (P lanes
+        // per column), new eigenvalues; ROWS: the tracked rows times them
+        if constexpr (ROWS) {
+            constexpr int RP = (P * NMAX + NT - 1) / NT;
+            static_assert(RP == 1, "one pass over the columns");
+            const int pidx = tid / P;
             const int a = pidx - pidx % span;
-            if (a + half >= n) continue;
-            const int j = pidx - a, K = s.kcnt[a];
-            if (j >= K) continue;
-            const double* dl = s.dl + a;
-            const double base = dl[s.org[a + j]], tj = s.rt[a + j];
-            double* ucol = s.U + a + (size_t)(a + j) * s.ldu;
-            double nrm = 0.0;
-            for (int l = qq; l < K; l += 4) {
-                const double v = s.zh[a + l] * fast_rcp((dl[l] - base) - tj);
-                ucol[l] = v;
-                nrm = fma(v, v, nrm);
+            double nr[kRowsTracked];
+#pragma unroll
+            for (int r = 0; r < kRowsTracked; ++r) nr[r] = 0.0;
+            const bool on = pidx < n && a + half < n && pidx - a < s.kcnt[a < n ? a : 0];
+            if (on) {
+                const int j = pidx - a, K = s.kcnt[a];
+                const double* dl = s.dl + a;
+                const double base = dl[s.org[a + j]], tj = s.rt[a + j];
+                double nrm = 0.0;
+#pragma unroll 1
+                for (int l = qq; l < K; l += P) {
+                    const double v = s.zh[a + l] * fast_rcp((dl[l] - base) - tj);
+                    nrm = fma(v, v, nrm);
+                    const double* rl = s.rows + kRowsTracked * s.nd[a + l];
+#pragma unroll
+                    for (int r = 0; r < kRowsTracked; ++r) nr[r] = fma(v, rl[r], nr[r]);
+                }
+                const double inv = rsqrt(lanes_sum<P>(nrm, qmask));
+#pragma unroll
+                for (int r = 0; r < kRowsTracked; ++r) nr[r] = lanes_sum<P>(nr[r], qmask) * inv;
+                if (qq == 0) s.w[s.nd[a + j]] = base + tj;
             }
-            const double inv = rsqrt(lanes_sum<4>(nrm, qmask));
-            for (int l = qq; l < K; l += 4) ucol[l] *= inv;
-            if (qq == 0) s.w[s.nd[a + j]] = base + tj;
-        }
-        team_sync<NT, BLOCK>();
-        phase_mark(14);
-        // ---- phase E: Z(:, nd) <- Z(:, nd) * U.
-        if constexpr (NMAX > 0) {
-            if (span >= n) dc_merge_top_regs<NT, NMAX, BLOCK>(n, s);
-            else dc_merge_rows_regs<NT, pow2_below(NMAX) / 4, BLOCK>(n, half, span, s);
+            team_sync<NT, BLOCK>();
+            phase_mark(14);
+            if (on && qq == 0) {
+                double* rj = s.rows + kRowsTracked * s.nd[pidx];
+#pragma unroll
+                for (int r = 0; r < kRowsTracked; ++r) rj[r] = nr[r];
+            }
         } else {
-            if (span <= 32) dc_merge_rows_regs<NT, 8, BLOCK>(n, half, span, s);
-            else dc_merge_tiled<NT, BLOCK>(n, half, span, s);
+#pragma unroll 1
+            for (int p0 = 0; p0 < P * n; p0 += NT) {
+                const int pidx = (p0 + tid) / P;
+                if (pidx >= n) continue;
+                const int a = pidx - pidx % span;
+                if (a + half >= n) continue;
+                const int j = pidx - a, K = s.kcnt[a];
+                if (j >= K) continue;
+                const double* dl = s.dl + a;
+                const double base = dl[s.org[a + j]], tj = s.rt[a + j];
+                double* ucol = s.U + a + (size_t)(a + j) * s.ldu;
+                double nrm = 0.0;
+#pragma unroll 2
+                for (int l = qq; l < K; l += P) {
+                    const double v = s.zh[a + l] * fast_rcp((dl[l] - base) - tj);
+                    ucol[l] = v;
+                    nrm = fma(v, v, nrm);
+                }
+                const double inv = rsqrt(lanes_sum<P>(nrm, qmask));
+#pragma unroll 1
+                for (int l = qq; l < K; l += P) ucol[l] *= inv;
+                if (qq == 0) s.w[s.nd[a + j]] = base + tj;
+            }
+            team_sync<NT, BLOCK>();
+            phase_mark(14);
+            // ---- phase E: Z(:, nd) <- Z(:, nd) * U.
+            if constexpr (NMAX > 0) {
+                dc_merge_panels<NT, NMAX, BLOCK>(n, half, span, s);
+            } else {
+                if (span <= 32) dc_merge_rows_regs<NT, 8, BLOCK>(n, half, span, s);
+                else dc_merge_tiled<NT, BLOCK>(n, half, span, s);
+            }
         }
         team_sync<NT, BLOCK>();
         phase_mark(15);
     }
     // ---- back to the caller's units
     const double inv = 1.0 / sc;
+#pragma unroll 1
     for (int i = tid; i < n; i += NT) s.w[i] *= inv;
     team_sync<NT, BLOCK>();
 }

@@ -28,7 +28,7 @@ enum class Regime : int {
 // kCtaPreferredMaxN (measured crossover with the l2-slot kernel on B200).
 constexpr int kCtaMaxN = 64;
 constexpr int kCtaPreferredMaxN = 60;
-size_t cta_smem_bytes(int n);
+size_t cta_smem_bytes(int n, bool spec = false);   // one pencil; `spec`: the intensity form
 int cta_nmax_for(int n);
 int cta_threads_for(int nmax);   // threads per pencil (per team) of that row bound's kernel
 // Pencils per CTA at a time (teams) that row bound's kernels exist for: 4 for
@@ -36,19 +36,18 @@ int cta_threads_for(int nmax);   // threads per pencil (per team) of that row bo
 // CTA of `teams` teams.
 int cta_max_teams(int nmax);
 int cta_default_teams(int nmax);   // pencils per CTA when none is requested
-size_t cta_teams_smem_bytes(int n, int teams);
+size_t cta_teams_smem_bytes(int n, int teams, bool spec = false);
 cudaError_t cta_set_attributes(int nmax, size_t smem);   // every teams form of the row bound
 // `sigma`: H is the metric diag(I_{n/2}, -I_{n/2}) and is not read (H may be NULL).
-// `teams`: pencils per CTA (1, or up to cta_max_teams(nmax)); smem from
-// cta_teams_smem_bytes.
-cudaError_t cta_launch(int n, int nmax, size_t smem, int stage, const void* H, const void* S, double* W, void* U,
+// `teams`: pencils per CTA (1, or up to cta_max_teams(nmax)).
+cudaError_t cta_launch(int n, int nmax, int stage, const void* H, const void* S, double* W, void* U,
                        int* info, long long batch, cudaStream_t stream, bool sigma = false, int teams = 1);
 
 // Spin-wave metric solve that reduces the eigenvectors to the spectrum
 // S(q, E) on the device (no U output): O is 3 x n complex per problem,
 // qhat 3 doubles per problem, energies ne doubles, spec ne doubles per
 // problem; Gaussian broadening of full width at half maximum fwhm.
-cudaError_t cta_launch_intensity(int n, int nmax, size_t smem, const void* S, const void* O, const double* qhat,
+cudaError_t cta_launch_intensity(int n, int nmax, const void* S, const void* O, const double* qhat,
                                  const double* energies, int ne, double fwhm, double* W, double* spec, int* info,
                                  long long batch, cudaStream_t stream, int teams = 1);
 
@@ -58,7 +57,7 @@ cudaError_t cta_launch_intensity(int n, int nmax, size_t smem, const void* S, co
 // start int32[n*n + 1], coef complex128, disp 3 doubles per term, q 3
 // doubles per problem. O == NULL: W and U as cta_launch (stage 4); else the
 // intensity form of cta_launch_intensity (W and spec, no U). One pencil per
-// CTA (its own kernel instantiation), dynamic smem cta_smem_bytes(n).
+// CTA (its own kernel instantiations).
 struct FourierTerms {
     const int*    start  = nullptr;
     const void*   coef   = nullptr;

@@ -278,30 +278,14 @@ __global__ void __launch_bounds__(kNT, 1) geneig_plain_kernel(PlainArgs a) {
                 dc.Z = reinterpret_cast<double*>(B); dc.ldz = ld;
                 dc.U = dc.Z + (size_t)n * ld;        dc.ldu = ld;
                 dc.Zo = nullptr;
-                dc.d = v.d; dc.e = v.e;
-                dc.w = v.dcd; dc.z = dc.w + n; dc.dl = dc.z + n; dc.zz = dc.dl + n; dc.zh = dc.zz + n;
-                dc.rt = dc.zh + n; dc.rho = dc.rt + n; dc.scal = dc.rho + n;
-                dc.org = v.dci; dc.nd = dc.org + n; dc.perm = dc.nd + n; dc.kcnt = dc.perm + n;
+                dc.leaf = dc.Z; dc.leaf_lanes = kLeaf * ((n + 7) / 8);
+                dc.d = v.d; dc.ds = 1; dc.e = v.e; dc.es = 1;
+                dc_carve(dc, v.dcd, v.dci, n);
                 tridiag_dc<kNT, NMAX>(n, dc);
-                if (tid == 0) {
-                    bool bad = false;
-                    for (int i = 0; i < n; ++i) bad |= !isfinite(dc.w[i]);
-                    v.ctl[4] = bad ? kEigFailCode : 0;
-                }
-                __syncthreads();
-                if (v.ctl[4]) code = v.ctl[4];
-            }
-            // ascending rank of each eigenvalue
-            if (!code) {
-                for (int j = tid; j < n; j += kNT) {
-                    const double dj = order_key(v.dcd[j]);
-                    int r = 0;
-                    for (int k2 = 0; k2 < n; ++k2) {
-                        const double dk = order_key(v.dcd[k2]);
-                        r += (dk < dj) || (dk == dj && k2 < j);
-                    }
-                    v.rank[j] = r;
-                }
+                bool bad = false;
+                for (int i = lane; i < n; i += 32) bad |= !isfinite(dc.w[i]);
+                if (__any_sync(0xffffffffu, bad)) code = kEigFailCode;
+                for (int t = tid; t < n; t += kNT) v.rank[dc.ord[t]] = t;
             }
             __syncthreads();
         }
@@ -515,7 +499,7 @@ cudaError_t plain_launch(const PlainPlan& plan, int stage, const void* H, const 
     a.stage = stage;
     a.sigma = sigma ? 1 : 0;
     if (plan.regime == Regime::SmemCta)
-        return cta_launch(plan.n, plan.nmax, plan.smem, stage, H, S, W, U, info, batch, stream, sigma, plan.teams);
+        return cta_launch(plan.n, plan.nmax, stage, H, S, W, U, info, batch, stream, sigma, plan.teams);
     if (plan.regime == Regime::L2Slot)
         return tiled_launch(plan.n, plan.slots, plan.smem, stage, H, S, W, U, info, batch, scratch, stream, sigma,
                             plan.mixed, plan.refine_max);
@@ -627,7 +611,7 @@ extern "C" sunny_geneig_status_t sunny_geneig_launch_noalloc(int n, uintptr_t d_
     if (n <= kCtaPreferredMaxN && cta_smem_bytes(n) <= (size_t)d->optin) {
         // the shared-memory kernel keeps everything on chip: no scratch at all
         const int nmax = cta_nmax_for(n), teams = cta_default_teams(nmax);
-        e = cta_launch(n, nmax, cta_teams_smem_bytes(n, teams), 4, reinterpret_cast<const void*>(d_H),
+        e = cta_launch(n, nmax, 4, reinterpret_cast<const void*>(d_H),
                        reinterpret_cast<const void*>(d_S), reinterpret_cast<double*>(d_W),
                        reinterpret_cast<void*>(d_U), reinterpret_cast<int*>(d_info), batch_size,
                        reinterpret_cast<cudaStream_t>(stream), false, teams);

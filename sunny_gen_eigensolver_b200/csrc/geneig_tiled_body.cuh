@@ -227,6 +227,10 @@ __device__ __forceinline__ void tri_tile(int t, int& ti, int& tj) {
     tj = t - r * (r + 1) / 2;
 }
 
+// The divide and conquer with a register allocation of its own: inlined, it
+// made the tile products around it spill (n = 216: 4 % slower).
+static __device__ __noinline__ void tiled_dc(int n, DCShared dc) { tridiag_dc<kNT, 0>(n, dc); }
+
 // One pencil b, solved end to end by the whole CTA in its global-memory
 // slot `slot` (tiled_slot_elems(n, mixed) complex entries) with the
 // launch's dynamic shared memory as the vector area.
@@ -798,29 +802,18 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
             dc.Z = reinterpret_cast<double*>(M2); dc.ldz = ld;
             dc.U = dc.Z + mat;                    dc.ldu = ld;
             dc.Zo = Zo;
-            dc.d = v.d; dc.e = v.e;
-            dc.w = v.dcd; dc.z = dc.w + n; dc.dl = dc.z + n; dc.zz = dc.dl + n; dc.zh = dc.zz + n;
-            dc.rt = dc.zh + n; dc.rho = dc.rt + n; dc.scal = dc.rho + n;
-            dc.org = v.dci; dc.nd = dc.org + n; dc.perm = dc.nd + n; dc.kcnt = dc.perm + n;
-            tridiag_dc<kNT, 0>(n, dc);
-            if (tid == 0) {
-                bool bad = false;
-                for (int i = 0; i < n; ++i) bad |= !isfinite(dc.w[i]);
-                v.ctl[4] = bad ? kEigFailCode : 0;
-            }
-            __syncthreads();
-            code = v.ctl[4];
-            if (!code) {
-                for (int j = tid; j < n; j += kNT) {
-                    const double dj = order_key(v.dcd[j]);
-                    int r = 0;
-                    for (int k2 = 0; k2 < n; ++k2) {
-                        const double dk = order_key(v.dcd[k2]);
-                        r += (dk < dj) || (dk == dj && k2 < j);
-                    }
-                    v.rank[j] = r;
-                }
-            }
+            // tb, gb and the partial vectors are free here
+            dc.leaf = reinterpret_cast<double*>(v.tb);
+            dc.leaf_lanes = (int)((768 + tiled_part_elems(n)) * 2 / (kLeafStride * kLeaf)) * kLeaf;
+            dc.d = v.d; dc.ds = 1; dc.e = v.e; dc.es = 1;
+            dc_carve(dc, v.dcd, v.dci, n);
+            tiled_dc(n, dc);
+            // a failed eigensolve shows as a non-finite value (every warp looks
+            // at all of them: the verdict is uniform without a barrier)
+            bool bad = false;
+            for (int i = lane; i < n; i += 32) bad |= !isfinite(dc.w[i]);
+            code = __any_sync(0xffffffffu, bad) ? kEigFailCode : 0;
+            for (int t = tid; t < n; t += kNT) v.rank[dc.ord[t]] = t;
             __syncthreads();
             phase_mark(21);
         }

@@ -10,10 +10,9 @@
 // per-pencil body as the size's own kernel (cta_solve / tiled_solve), so the
 // results are bitwise those of per-size launches. An l2-slot body uses the
 // CTA's own global-memory slot, sized for the largest l2-slot N of the mix.
-// Small pencils are solved several per CTA at a time: an item of N <= 16
-// goes to four 64-thread teams and one of N <= 32 to two 128-thread teams,
-// each team with its own barrier and shared-memory slice, taking the item's
-// pencils in turn (the thread counts of the sizes' own kernels).
+// The smem-cta sizes are solved several pencils per CTA at a time: 8, 4 or 2
+// teams of the sizes' own kernels (32, 64 or 128 threads), each with its own
+// barrier and shared-memory slice, taking the item's pencils in turn.
 
 // The smem-cta bodies are called, each with its own register allocation
 // (inlining all of them with the tiled body into one function made the
@@ -25,10 +24,11 @@
 namespace sgeig {
 namespace {
 
-constexpr int kTeams16 = 4;   // 64-thread teams per CTA for N <= 16
-constexpr int kTeams32 = 2;   // 128-thread teams per CTA for N <= 32
-
-size_t team_slice(int n) { return (cta_smem_bytes(n) + 15) & ~(size_t)15; }
+// Threads per CTA; a size's pencils are solved by its kernel's own team
+// shape, as many at a time as the CTA has teams.
+constexpr int kNT = 256;
+constexpr int kind_nmax(int kind) { return kind == 0 ? 16 : kind == 1 ? 32 : kind == 2 ? 48 : kind == 3 ? 56 : 64; }
+constexpr int kind_teams(int kind) { return kNT / cta::cta_team_threads(kind_nmax(kind)); }
 
 struct UnevenGroup {
     const double2* H;
@@ -41,7 +41,7 @@ struct UnevenGroup {
     int n;
     int kind;               // 0..4: smem-cta row bound 16/32/48/56/64; 5: l2-slot
     int per_item;           // pencils per work item
-    size_t slice;           // kinds 0, 1: shared-memory bytes of one team
+    size_t slice;           // kinds 0..4: shared-memory bytes of one team
 };
 
 struct UnevenArgs {
@@ -53,7 +53,17 @@ struct UnevenArgs {
     size_t slot_elems;
 };
 
-__global__ void __launch_bounds__(256, 2) geneig_uneven_kernel(UnevenArgs a) {
+// The pencils [b0, b1) of one smem-cta size, dealt to the CTA's teams.
+template <int KIND>
+__device__ __forceinline__ void team_items(const cta::CtaArgs& c, long long b0, long long b1, unsigned char* smem,
+                                           size_t slice) {
+    constexpr int NMAX = kind_nmax(KIND), NT = cta::cta_team_threads(NMAX);
+    const int t = threadIdx.x / NT;
+    for (long long b = b0 + t; b < b1; b += kind_teams(KIND))
+        cta::cta_solve<NMAX, NT, kNT>(c, b, smem + t * slice);
+}
+
+__global__ void __launch_bounds__(kNT, 2) geneig_uneven_kernel(UnevenArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned long long s_item;
     double2* slot = a.scratch ? a.scratch + (size_t)blockIdx.x * a.slot_elems : nullptr;
@@ -78,25 +88,15 @@ __global__ void __launch_bounds__(256, 2) geneig_uneven_kernel(UnevenArgs a) {
         } else {
             cta::CtaArgs c;
             c.H = G.H; c.S = G.S; c.W = G.W; c.U = G.U; c.info = G.info;
-            c.batch = G.count; c.n = G.n; c.ld = G.n | 1; c.stage = 4; c.sigma = 0;
+            c.batch = G.count; c.n = G.n; c.ld = cta::cta_ld(G.n, false); c.stage = 4; c.sigma = 0;
             c.O = nullptr; c.qhat = nullptr; c.energies = nullptr; c.spec = nullptr; c.ne = 0;
             c.gnorm = 0.0; c.ginv2 = 0.0;
             switch (G.kind) {
-                case 0: {
-                    const int t = threadIdx.x / 64;
-                    for (long long b = b0 + t; b < b1; b += kTeams16)
-                        cta::cta_solve<16, 64, 256>(c, b, smem_raw + t * G.slice);
-                    break;
-                }
-                case 1: {
-                    const int t = threadIdx.x / 128;
-                    for (long long b = b0 + t; b < b1; b += kTeams32)
-                        cta::cta_solve<32, 128, 256>(c, b, smem_raw + t * G.slice);
-                    break;
-                }
-                case 2: for (long long b = b0; b < b1; ++b) cta::cta_solve<48>(c, b, smem_raw); break;
-                case 3: for (long long b = b0; b < b1; ++b) cta::cta_solve<56>(c, b, smem_raw); break;
-                default: for (long long b = b0; b < b1; ++b) cta::cta_solve<64>(c, b, smem_raw); break;
+                case 0: team_items<0>(c, b0, b1, smem_raw, G.slice); break;
+                case 1: team_items<1>(c, b0, b1, smem_raw, G.slice); break;
+                case 2: team_items<2>(c, b0, b1, smem_raw, G.slice); break;
+                case 3: team_items<3>(c, b0, b1, smem_raw, G.slice); break;
+                default: team_items<4>(c, b0, b1, smem_raw, G.slice); break;
             }
         }
     }
@@ -119,9 +119,7 @@ int uneven_kind(int n, bool l2slot) {
 
 size_t uneven_smem_bytes(int n, int kind) {
     return kind == 5 ? tiled_vec_bytes(n)
-         : kind == 0 ? kTeams16 * team_slice(n)
-         : kind == 1 ? kTeams32 * team_slice(n)
-         : cta_smem_bytes(n);
+                     : kind_teams(kind) * cta_smem_bytes(n);
 }
 
 cudaError_t uneven_launch(const UnevenLaunch& L, unsigned long long* head, void* scratch, size_t slot_elems,
@@ -141,7 +139,7 @@ cudaError_t uneven_launch(const UnevenLaunch& L, unsigned long long* head, void*
         G.n = L.n[i];
         G.kind = L.kind[i];
         G.per_item = L.per_item[i] > 0 ? L.per_item[i] : 1;
-        G.slice = team_slice(G.n);
+        G.slice = G.kind == 5 ? 0 : cta_smem_bytes(G.n);
         G.first_item = first;
         first += (G.count + G.per_item - 1) / G.per_item;
     }
@@ -154,7 +152,7 @@ cudaError_t uneven_launch(const UnevenLaunch& L, unsigned long long* head, void*
     cudaError_t e = cudaMemsetAsync(head, 0, sizeof(unsigned long long), stream);
     if (e != cudaSuccess) return e;
     const long long g = first < grid ? first : grid;
-    geneig_uneven_kernel<<<(unsigned)g, 256, smem, stream>>>(a);
+    geneig_uneven_kernel<<<(unsigned)g, kNT, smem, stream>>>(a);
     return cudaGetLastError();
 }
 
