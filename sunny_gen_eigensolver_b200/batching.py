@@ -47,6 +47,8 @@ def size_configs(n: int) -> List[dict]:
         cands.insert(0, {"regime": "smem-cta", "slots_per_sm": 0})
     elif n <= 96:
         cands.append({"regime": "smem-wide", "slots_per_sm": 0})
+    if 60 < n <= 110:                          # the library's own choice for these sizes
+        cands.insert(0, {"regime": "l2-slot", "slots_per_sm": 0})
     return cands
 
 

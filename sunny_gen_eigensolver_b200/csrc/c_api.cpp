@@ -54,6 +54,7 @@ struct sunny_geneig_uneven {
     size_t slot_elems = 0;
     void* scratch = nullptr;
     unsigned long long* head = nullptr;
+    sgeig::UnevenSide side;      // for the sizes that run beside the persistent kernel
     cudaEvent_t done = nullptr;
     uintptr_t last_stream = 0;
     bool used = false;
@@ -84,6 +85,12 @@ cudaError_t with_device(int device, F&& fn) {
 }
 
 bool aligned(uintptr_t p, uintptr_t a) { return (p % a) == 0; }
+
+void release_side(sgeig::UnevenSide& s) {
+    if (s.stream) cudaStreamDestroy(s.stream);
+    if (s.fork) cudaEventDestroy(s.fork);
+    if (s.join) cudaEventDestroy(s.join);
+}
 
 // NVTX range around each entry point (header-only NVTX v3: a no-op unless a
 // profiler such as nsys or ncu --nvtx is attached), so that a timeline or an
@@ -146,8 +153,9 @@ sunny_geneig_solver_t create_impl(int n, int device_id, int bpb_request,
             const std::string key = sgeig::tune_key(n, (int)mode, device_id);
             std::string cfg;
             if (!sgeig::tune_lookup(key, (int)cache, &cfg)) {
-                const std::vector<std::pair<std::string, int>> cands = {
+                std::vector<std::pair<std::string, int>> cands = {
                     {"smem-cta", 0}, {"smem-wide", 0}, {"l2-slot", 1}, {"l2-slot", 2}};
+                if (n > sgeig::kCtaPreferredMaxN && n <= sgeig::kResidentMaxN) cands.push_back({"l2-slot", 0});
                 const int pick = sgeig::tune_pick(n, device_id, cands, &err);
                 if (pick < 0) return cudaErrorInvalidValue;
                 cfg = cands[pick].first + ":" + std::to_string(cands[pick].second);
@@ -526,7 +534,10 @@ sunny_geneig_uneven_t sunny_geneig_uneven_create(int num_sizes, const int* sizes
                 h->kind[g] = sgeig::uneven_kind(n, l2);
                 h->per_item[g] = (per_item && per_item[i] > 0) ? per_item[i] : (l2 ? 1 : 4);
                 h->smem = std::max(h->smem, sgeig::uneven_smem_bytes(n, h->kind[g]));
-                if (l2) slot = std::max(slot, sgeig::tiled_slot_elems(n));
+                if (h->kind[g] == sgeig::kUnevenResident) {
+                    ea = sgeig::cta_set_attributes(sgeig::cta_nmax_for(n), (size_t)optin);
+                    if (ea != cudaSuccess) { err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea); return ea; }
+                } else if (l2) slot = std::max(slot, sgeig::tiled_slot_elems(n));
             }
             if (h->smem > (size_t)optin) { err = "the mix needs more shared memory than a CTA has"; return cudaErrorInvalidValue; }
             ea = sgeig::uneven_set_attributes((size_t)optin);
@@ -539,13 +550,18 @@ sunny_geneig_uneven_t sunny_geneig_uneven_create(int num_sizes, const int* sizes
             }
             ea = cudaMalloc(reinterpret_cast<void**>(&h->head), sizeof(unsigned long long));
             if (ea != cudaSuccess) { err = std::string("cudaMalloc counter: ") + cudaGetErrorString(ea); return ea; }
-            return cudaEventCreateWithFlags(&h->done, cudaEventDisableTiming);
+            ea = cudaStreamCreateWithFlags(&h->side.stream, cudaStreamNonBlocking);
+            if (ea == cudaSuccess) ea = cudaEventCreateWithFlags(&h->side.fork, cudaEventDisableTiming);
+            if (ea == cudaSuccess) ea = cudaEventCreateWithFlags(&h->side.join, cudaEventDisableTiming);
+            if (ea == cudaSuccess) ea = cudaEventCreateWithFlags(&h->done, cudaEventDisableTiming);
+            return ea;
         });
         if (e != cudaSuccess) {
             set_error(std::string(fn) + ": " + (err.empty() ? cudaGetErrorString(e) : err));
             with_device(device_id, [&]() {
                 cudaFree(h->scratch);
                 cudaFree(h->head);
+                release_side(h->side);
                 if (h->done) cudaEventDestroy(h->done);
                 return cudaSuccess;
             });
@@ -608,7 +624,7 @@ sunny_geneig_status_t sunny_geneig_uneven_launch(sunny_geneig_uneven_t h, const 
                 cudaError_t w = cudaStreamWaitEvent(st, h->done, 0);
                 if (w != cudaSuccess) return w;
             }
-            cudaError_t l = sgeig::uneven_launch(L, h->head, h->scratch, h->slot_elems, h->grid, h->smem, st);
+            cudaError_t l = sgeig::uneven_launch(L, h->head, h->scratch, h->slot_elems, h->grid, h->smem, st, h->side);
             if (l != cudaSuccess || capturing) return l;
             l = cudaEventRecord(h->done, st);
             if (l == cudaSuccess) { h->used = true; h->last_stream = stream; }
@@ -630,6 +646,7 @@ void sunny_geneig_uneven_destroy(sunny_geneig_uneven_t h) {
     try {
         with_device(h->device, [&]() {
             if (h->done) { cudaEventSynchronize(h->done); cudaEventDestroy(h->done); }
+            release_side(h->side);
             cudaFree(h->scratch);
             cudaFree(h->head);
             return cudaSuccess;
@@ -643,7 +660,7 @@ int sunny_geneig_uneven_shape(sunny_geneig_uneven_t h, int* sizes, int* regimes,
     if (!h) return -1;
     for (int g = 0; g < h->ngroups; ++g) {
         if (sizes) sizes[g] = h->n[g];
-        if (regimes) regimes[g] = h->kind[g] == 5 ? 2 : 1;
+        if (regimes) regimes[g] = h->kind[g] >= 5 ? 2 : 1;
         if (per_item) per_item[g] = h->per_item[g];
     }
     return h->ngroups;

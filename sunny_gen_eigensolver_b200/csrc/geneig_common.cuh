@@ -197,6 +197,17 @@ __device__ __forceinline__ void phase_level_flush(int slot) {
         phase_level() = 0;
     }
 }
+// Adds this translation unit's counters to `out` (and clears them).
+static inline cudaError_t add_phase_cycles(unsigned long long* out, int count, bool reset) {
+    unsigned long long mine[kPhaseSlots] = {};
+    cudaError_t e = cudaMemcpyFromSymbol(mine, g_phase_cycles, sizeof(mine));
+    for (int i = 0; e == cudaSuccess && i < count && i < kPhaseSlots; ++i) out[i] += mine[i];
+    if (e == cudaSuccess && reset) {
+        static const unsigned long long zeros[kPhaseSlots] = {};
+        e = cudaMemcpyToSymbol(g_phase_cycles, zeros, sizeof(zeros));
+    }
+    return e;
+}
 #else
 __device__ __forceinline__ void phase_start() {}
 __device__ __forceinline__ void phase_mark(int) {}

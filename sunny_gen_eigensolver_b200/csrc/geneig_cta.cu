@@ -25,70 +25,22 @@
 // U, so that one n x n matrix and ~10 KB of vectors per pencil are all the
 // shared memory it takes.
 
-#include "geneig_cta_body.cuh"
+#include "geneig_cta_kernel.cuh"
 
 namespace sgeig {
-using namespace cta;
-namespace {
-
-// Pencils per SM that the register allocation is sized for, by row bound.
-template <int NMAX> struct CtaShape {
-    static constexpr int nt = cta_team_threads(NMAX);
-    static constexpr int per_sm = NMAX <= 16 ? 16 : NMAX <= 32 ? 8 : NMAX <= 56 ? 4 : 3;
-};
-
-// TEAMS pencils per CTA at a time (the reference's batches per block): the
-// CTA has TEAMS teams of CtaShape<NMAX>::nt threads, each with its own
-// barrier and shared-memory slice, team t taking pencils TEAMS * cta + t,
-// then a grid's stride on. FS: S from Fourier terms. SPEC: intensities.
-template <int NMAX, int TEAMS, bool FS, bool SPEC>
-__global__ void __launch_bounds__(CtaShape<NMAX>::nt * TEAMS, (CtaShape<NMAX>::per_sm + TEAMS - 1) / TEAMS)
-geneig_cta_kernel(CtaArgs a, CtaFourier f) {
-    constexpr int NT = CtaShape<NMAX>::nt;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    phase_start();
-    const int t = TEAMS == 1 ? 0 : (int)(threadIdx.x / NT);
-    unsigned char* sm = smem_raw + (TEAMS == 1 ? 0 : (size_t)t * cta_bytes(a.n, NT / 32, SPEC));
-    for (long long b = (long long)blockIdx.x * TEAMS + t; b < a.batch; b += (long long)gridDim.x * TEAMS)
-        cta_solve<NMAX, NT, NT * TEAMS, FS, SPEC>(a, b, sm, &f);
-}
-
-}  // namespace
 
 size_t cta_smem_bytes(int n, bool spec) { return cta_bytes(n, cta_team_threads(cta_nmax_for(n)) / 32, spec); }
 
 // Compile-time row bounds: the register arrays and unrolled loops are sized by
 // NMAX, so a bound close above n wastes less (56 covers the N=54 workload).
 int cta_nmax_for(int n) {
-    return n <= 16 ? 16 : n <= 24 ? 24 : n <= 32 ? 32 : n <= 40 ? 40 : n <= 48 ? 48 : n <= 56 ? 56 : 64;
+    return n <= 16 ? 16 : n <= 24 ? 24 : n <= 32 ? 32 : n <= 40 ? 40 : n <= 48 ? 48 : n <= 56 ? 56 : n <= 64 ? 64
+         : n <= 72 ? 72 : n <= 80 ? 80 : n <= 96 ? 96 : 112;
 }
 
-using CtaKernelFn = void (*)(CtaArgs, CtaFourier);
-template <int NMAX, bool FS, bool SPEC>
-static CtaKernelFn cta_kernel_teams(int teams) {
-    if constexpr (!FS && NMAX <= 16) {
-        if (teams == 4) return geneig_cta_kernel<NMAX, 4, FS, SPEC>;
-    }
-    if constexpr (!FS && NMAX <= 32) {
-        if (teams == 2) return geneig_cta_kernel<NMAX, 2, FS, SPEC>;
-    }
-    return geneig_cta_kernel<NMAX, 1, FS, SPEC>;
-}
-template <bool FS, bool SPEC>
-static CtaKernelFn cta_kernel_for(int nmax, int teams) {
-    switch (nmax) {
-        case 16: return cta_kernel_teams<16, FS, SPEC>(teams);
-        case 24: return cta_kernel_teams<24, FS, SPEC>(teams);
-        case 32: return cta_kernel_teams<32, FS, SPEC>(teams);
-        case 40: return cta_kernel_teams<40, FS, SPEC>(teams);
-        case 48: return cta_kernel_teams<48, FS, SPEC>(teams);
-        case 56: return cta_kernel_teams<56, FS, SPEC>(teams);
-        default: return cta_kernel_teams<64, FS, SPEC>(teams);
-    }
-}
 static CtaKernelFn cta_kernel(int nmax, int teams, bool fs, bool spec) {
-    return fs ? (spec ? cta_kernel_for<true, true>(nmax, 1) : cta_kernel_for<true, false>(nmax, 1))
-              : (spec ? cta_kernel_for<false, true>(nmax, teams) : cta_kernel_for<false, false>(nmax, teams));
+    if (fs || spec) return cta_kernel_spec(nmax, fs ? 1 : teams, fs, spec);
+    return nmax <= 32 ? cta_kernel_small(nmax, teams) : nmax <= kCtaMaxN ? cta_kernel_mid(nmax) : cta_kernel_wide(nmax);
 }
 
 int cta_max_teams(int nmax) { return nmax <= 16 ? 4 : nmax <= 32 ? 2 : 1; }
@@ -108,7 +60,7 @@ int cta_threads_for(int nmax) { return cta_team_threads(nmax); }
 // `smem` is the per-CTA shared-memory limit; the kernel's own static shared
 // memory (profiling builds have some) comes off the dynamic allowance.
 cudaError_t cta_set_attributes(int nmax, size_t smem) {
-    for (int form = 0; form < 4; ++form)
+    for (int form = 0; form < (nmax > kCtaMaxN ? 1 : 4); ++form)
         for (int teams = 1; teams <= cta_max_teams(nmax); teams *= 2) {
             const CtaKernelFn k = cta_kernel(nmax, teams, (form & 1) != 0, (form & 2) != 0);
             cudaFuncAttributes fa{};
@@ -131,7 +83,7 @@ static cudaError_t cta_start(const CtaArgs& a, const CtaFourier& f, int nmax, in
 }
 
 cudaError_t cta_launch(int n, int nmax, int stage, const void* H, const void* S, double* W, void* U,
-                       int* info, long long batch, cudaStream_t stream, bool sigma, int teams) {
+                       int* info, long long batch, cudaStream_t stream, bool sigma, int teams, bool retry) {
     CtaArgs a{};
     a.H = static_cast<const double2*>(H);
     a.S = static_cast<const double2*>(S);
@@ -143,6 +95,7 @@ cudaError_t cta_launch(int n, int nmax, int stage, const void* H, const void* S,
     a.ld = cta_ld(n, false);
     a.stage = stage;
     a.sigma = sigma ? 1 : 0;
+    a.retry = retry ? 1 : 0;
     return cta_start(a, CtaFourier{}, nmax, teams, false, false, stream);
 }
 
@@ -200,22 +153,19 @@ cudaError_t cta_launch_fourier(int n, int nmax, const FourierTerms& ft, const do
 }  // namespace sgeig
 
 #ifdef SGEIG_PHASE_TIMERS
-// Profiling builds only: copies the per-phase cycle counters of the
-// smem-cta kernel (see phase_mark in geneig_common.cuh) to `out` and, when
-// `reset` is nonzero, clears them. Not part of the product library's ABI.
+// Profiling builds only: the per-phase cycle counters of the kernels (see
+// phase_mark in geneig_common.cuh) into `out`; a nonzero `reset` clears them.
+// Not part of the product library's ABI.
 #pragma GCC visibility push(default)
 extern "C" int sunny_geneig_phase_cycles(unsigned long long* out, int count, int reset) {
-    if (count > sgeig::kPhaseSlots) count = sgeig::kPhaseSlots;
+    using namespace sgeig;
+    if (count > kPhaseSlots) count = kPhaseSlots;
     cudaError_t e = cudaDeviceSynchronize();
-    if (e == cudaSuccess && out && count > 0)
-        e = cudaMemcpyFromSymbol(out, sgeig::g_phase_cycles, sizeof(unsigned long long) * count);
-    if (e == cudaSuccess && reset) {
-        static const unsigned long long zeros[sgeig::kPhaseSlots] = {};
-        e = cudaMemcpyToSymbol(sgeig::g_phase_cycles, zeros, sizeof(zeros));
-    }
-    if (e == cudaSuccess && out && count > 0) e = sgeig::tiled_phase_cycles(out, count, reset != 0);
+    unsigned long long sum[kPhaseSlots] = {};
+    for (auto f : {cta_small_phase_cycles, cta_mid_phase_cycles, cta_wide_phase_cycles, tiled_phase_cycles})
+        if (e == cudaSuccess) e = f(sum, kPhaseSlots, reset != 0);
+    for (int i = 0; out && i < count; ++i) out[i] = sum[i];
     return e == cudaSuccess ? 0 : -1;
 }
 #pragma GCC visibility pop
 #endif
-

@@ -36,6 +36,7 @@ struct CtaArgs {
     int            ne;
     double         gnorm;    // Gaussian normalisation 1 / (sigma sqrt(2 pi))
     double         ginv2;    // 1 / (2 sigma^2)
+    int            retry;    // only the pencils whose info is kRetryInfo
 };
 
 // S assembled on the device instead of loaded (the FS form of cta_solve):
@@ -53,7 +54,9 @@ struct CtaFourier {
 // in shared memory, so the pencils per SM are bounded by registers for small
 // n and by shared memory above; narrow teams keep many pencils, whose steps
 // are chains of dependent operations, in flight.
-constexpr int cta_team_threads(int nmax) { return nmax <= 16 ? 32 : nmax <= 32 ? 64 : 128; }
+constexpr int cta_team_threads(int nmax) {
+    return nmax <= 16 ? 32 : nmax <= 32 ? 64 : nmax <= 64 ? 128 : nmax <= 80 ? 256 : 512;
+}
 
 // Rows of a pencil's matrix in shared memory: the intensity form appends the
 // three rows of P = O X^H, which the Householder updates turn into P Q.
@@ -78,7 +81,7 @@ __host__ __device__ inline size_t cta_dc_bytes(int n, bool spec) {   // (d, e) f
 constexpr int kDElems = 72;       // an 8 x 8 tile with leading dimension 9
 __host__ __device__ inline size_t cta_work_bytes(int n, int nw, bool spec) {
     const size_t panel = ((size_t)8 * (n | 1) + 2 * kDElems) * 16;
-    const size_t hh = (size_t)(nw + 3) * cta_rows(n, spec) * 16;
+    const size_t hh = ((size_t)32 * nw + 3 * cta_rows(n, spec)) * 16;
     const size_t dc = cta_dc_bytes(n, spec) + (spec ? 0 : (size_t)((n + 7) / 8) * 36 * 16);
     const size_t m = panel > hh ? panel : hh;
     return m > dc ? m : dc;
@@ -132,7 +135,7 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
     constexpr int NB = NMAX / 8;    // 8-row tiles
     constexpr int R = (NMAX + (SPEC ? kSpecRows : 0) + 31) / 32;   // Householder rows per lane
     constexpr int PP = (NB + NW - 1) / NW;                         // 8-column panels per warp
-    static_assert(NT % 32 == 0 && NW >= 1 && NW <= 8 && NMAX % 8 == 0, "team shape");
+    static_assert(NT % 32 == 0 && NW >= 1 && NW <= 16 && NMAX % 8 == 0, "team shape");
     const int n = a.n, ld = a.ld;
     const int rows = cta_rows(n, SPEC);
     double2* M = reinterpret_cast<double2*>(smem_raw);
@@ -446,22 +449,26 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
                     const double2* h0 = Hb + min(i0, n - 1);
                     const double2* h1 = Hb + min(i1, n - 1);
                     const bool two = t0 + NW < nb;
-                    double2 y0[2], y1[2];        // the next k block's H, loaded ahead
+                    double2 y0[2][2], y1[2][2];  // H of the next two k blocks, loaded ahead
 #pragma unroll
-                    for (int s = 0; s < 2; ++s) {
-                        const int k = min(2 * fq + s, n - 1);
-                        y0[s] = __ldg(h0 + k * n);
-                        y1[s] = __ldg(h1 + k * n);
-                    }
+                    for (int p = 0; p < 2; ++p)
+#pragma unroll
+                        for (int s = 0; s < 2; ++s) {
+                            const int k = min(8 * p + 2 * fq + s, n - 1);
+                            y0[p][s] = __ldg(h0 + k * n);
+                            y1[p][s] = __ldg(h1 + k * n);
+                        }
 #pragma unroll 1
                     for (int kb = 0; kb <= tj; ++kb) {
-                        const double2 a0[2] = {y0[0], y0[1]}, a1[2] = {y1[0], y1[1]};
-                        if (kb < tj) {
+                        const double2 a0[2] = {y0[0][0], y0[0][1]}, a1[2] = {y1[0][0], y1[0][1]};
 #pragma unroll
-                            for (int s = 0; s < 2; ++s) {
-                                const int k = min(8 * kb + 8 + 2 * fq + s, n - 1);
-                                y0[s] = __ldg(h0 + k * n);
-                                y1[s] = __ldg(h1 + k * n);
+                        for (int s = 0; s < 2; ++s) {
+                            const int k = min(8 * kb + 16 + 2 * fq + s, n - 1);
+                            y0[0][s] = y0[1][s];
+                            y1[0][s] = y1[1][s];
+                            if (kb + 2 <= tj) {
+                                y0[1][s] = __ldg(h0 + k * n);
+                                y1[1][s] = __ldg(h1 + k * n);
                             }
                         }
 #pragma unroll
@@ -561,9 +568,11 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
 
     if (!code) {
         // ---- a5a: Householder tridiagonalisation of C (lower), one pass over
-        // the trailing matrix per step. Lane l of a warp holds the rows counted
-        // l, l + 32, ... from the last one up (so that the row blocks in use
-        // follow the trailing matrix); warp w owns the columns j = w mod NW.
+        // the trailing matrix per step. Rows are counted from the last one up
+        // in blocks of 32 (so that the blocks in use follow the trailing
+        // matrix), a lane per row; with RB blocks in use, warp w takes block
+        // w % RB of the columns j = w / RB mod NW / RB, so that a row has only
+        // NW / RB partial products to add.
         // Step c (column c):
         //   one warp (a different one each step, so that the pencils of an SM
         //   spread over its schedulers): y = A v from the warps' partial
@@ -582,38 +591,43 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
         // keeps v[k+2..] and tau_k at row k + 1. SPEC: rows n .. n+2 see the
         // same update with v = 0 there, which is P <- P (I - tau v v^H), so
         // that P Q is in their place at the end.
-        double2* part = work;                    // NW x rows partial products
-        double2* vb = part + NW * rows;          // 2 x rows reflectors (this one, the next)
+        // Rows above the trailing matrix are carried along unmasked: v is zero
+        // there, so they only see A <- A (I - tau v v^H), which keeps them
+        // bounded, and nothing reads them.
+        double2* part = work;                    // 32 NW partial products
+        double2* vb = part + 32 * NW;            // 2 x rows reflectors (this one, the next)
         double2* wb = vb + 2 * rows;             // rows
-        const int last = rows - 1 - lane;        // row of slot t: last - 32 t
+        const int last = rows - 1 - lane;        // row of block t: last - 32 t
+        int off[R];                              // (no such row: row 0, not stored)
+#pragma unroll
+        for (int t = 0; t < R; ++t) off[t] = max(last - 32 * t, 0);
 #pragma unroll 1
         for (int i = tid; i < rows; i += NT) vb[rows + i] = wb[i] = zero;   // "reflector -1"
+        int rb = 0, G = 0, myt = 0, myg = 0;     // row blocks in use, column classes, this warp's block and class
 #pragma unroll 1
         for (int c = 0; c < n; ++c) {
+            const double2* vk = vb + ((c + 1) & 1) * rows;
+            double2* vc = vb + (c & 1) * rows;
             if (warp == (unsigned)(c + (int)b) % NW) {
-                const double2* vk = vb + ((c + 1) & 1) * rows;
-                double2* vc = vb + (c & 1) * rows;
-                double2 x[R], w[R], v[R];
+                double2 x[R], w[R];
+                double2* mc = M + c * ld;
                 const int ic = rows - 1 - c;     // slot of row c
 #pragma unroll
-                for (int t = 0; t < R; ++t) {
-                    const int i = last - 32 * t;
-                    x[t] = M[max(i, 0) + c * ld];
-                    w[t] = zero;
-                }
+                for (int t = 0; t < R; ++t) x[t] = mc[off[t]];
                 if (c > 0) {
-                    const double2 tau = M[c + (c - 1) * ld];
+                    const double2 tau = mc[c - ld];
+                    double2 v[R];
                     double s = 0.0;
+                    const double2* pt = part + lane;
 #pragma unroll
                     for (int t = 0; t < R; ++t) {
-                        const int i = last - 32 * t, im = max(i, 0);
-                        double2 acc = part[im];
-                        v[t] = vk[im];
-#pragma unroll
-                        for (int u = 1; u < NW; ++u) acc = cadd(acc, part[u * rows + im]);
-                        const bool in = i >= c;
-                        w[t] = c2(in ? acc.x : 0.0, in ? acc.y : 0.0);
-                        v[t] = c2(in ? v[t].x : 0.0, in ? v[t].y : 0.0);
+                        v[t] = vk[off[t]];
+                        w[t] = zero;
+                        if (t < rb) {
+                            w[t] = pt[32 * t];
+#pragma unroll 1
+                            for (int g = 1; g < G; ++g) w[t] = cadd(w[t], pt[32 * (t + g * rb)]);
+                        }
                         s = fma(w[t].x, v[t].x, fma(w[t].y, v[t].y, s));
                     }
                     const double h = -0.5 * fma(tau.x, tau.x, tau.y * tau.y) * warp_sum(s);
@@ -621,6 +635,7 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
                     for (int t = 0; t < R; ++t) {
                         w[t] = cmul(tau, w[t]);
                         w[t] = c2(fma(h, v[t].x, w[t].x), fma(h, v[t].y, w[t].y));
+                        wb[off[t]] = w[t];       // (lanes without a row repeat row 0, long dead or theirs alone)
                     }
                     double2 wc = w[0];
 #pragma unroll
@@ -628,38 +643,37 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
                     wc = shfl2(wc, ic & 31);
 #pragma unroll
                     for (int t = 0; t < R; ++t) {
-                        const int i = last - 32 * t;
-                        x[t] = csub(cfms_bc(x[t], v[t], wc), w[t]);      // v(c) = 1
-                        if (i >= c) wb[i] = w[t];
-                        if (SPEC && i >= n) M[i + c * ld] = x[t];        // the final P of column c
+                        x[t] = csub(cfms_bc(x[t], v[t], wc), w[t]);          // v(c) = 1
+                        if (SPEC && last - 32 * t >= n) mc[off[t]] = x[t];   // the final P of column c
                     }
                 }
                 // reflector c from column c (1 / beta comes with the root)
-                double ss = 0.0, dk = x[0].x;
+                double2 xc = x[0], alpha = x[0];
 #pragma unroll
-                for (int t = 0; t < R; ++t) {
-                    const int i = last - 32 * t;
-                    const bool in = i > c + 1 && i < n;
-                    const double xr = in ? x[t].x : 0.0, xi = in ? x[t].y : 0.0;
-                    ss = fma(xr, xr, fma(xi, xi, ss));
-                    if (t > 0 && (ic >> 5) == t) dk = x[t].x;
+                for (int t = 1; t < R; ++t) {
+                    if ((ic >> 5) == t) xc = x[t];
+                    if (((ic - 1) >> 5) == t) alpha = x[t];
                 }
-                double2 tau = zero;
                 double beta = 0.0;
                 if (c < n - 1) {
-                    double2 alpha = x[0];
-#pragma unroll
-                    for (int t = 1; t < R; ++t) if (((ic - 1) >> 5) == t) alpha = x[t];
                     alpha = shfl2(alpha, (ic - 1) & 31);
+                    double ss = 0.0;
+#pragma unroll
+                    for (int t = 0; t < R; ++t) {
+                        const int i = last - 32 * t;
+                        const bool in = i > c + 1 && (!SPEC || i < n);
+                        x[t] = c2(in ? x[t].x : 0.0, in ? x[t].y : 0.0);
+                        ss = fma(x[t].x, x[t].x, fma(x[t].y, x[t].y, ss));
+                    }
                     ss = warp_sum(ss);
-                    double2 scal = zero;
+                    double2 scal = zero, tau = zero;
                     beta = alpha.x;
                     if (!(ss == 0.0 && alpha.y == 0.0)) {
                         const double nn = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, ss));
                         const double rn = rsqrt(nn);
                         beta = -copysign(nn * rn, alpha.x);
-                        const double rb = -copysign(rn, alpha.x);
-                        tau = c2((beta - alpha.x) * rb, -alpha.y * rb);
+                        const double rbeta = -copysign(rn, alpha.x);
+                        tau = c2((beta - alpha.x) * rbeta, -alpha.y * rbeta);
                         const double2 z = c2(alpha.x - beta, alpha.y);
                         const double inv = fast_rcp(fma(z.x, z.x, z.y * z.y));
                         scal = c2(z.x * inv, -z.y * inv);
@@ -667,71 +681,52 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
 #pragma unroll
                     for (int t = 0; t < R; ++t) {
                         const int i = last - 32 * t;
-                        if (i > c) {
-                            const double2 vi = i >= n ? zero : i == c + 1 ? c2(1.0, 0.0) : cmul(x[t], scal);
-                            vc[i] = vi;
-                            if (i < n) M[i + c * ld] = i == c + 1 ? tau : vi;
-                        }
+                        x[t] = cmul(x[t], scal);
+                        if (i >= 0) vc[i] = i == c + 1 ? c2(1.0, 0.0) : x[t];
+                        if (i > c && (!SPEC || i < n)) mc[i] = i == c + 1 ? tau : x[t];
                     }
                 }
-                if (lane == (ic & 31)) de[c * des] = c2(dk, beta);
+                if (lane == (ic & 31)) de[c * des] = c2(xc.x, beta);
             }
             if (c >= n - 1) break;
             team_sync<NT, BLOCK>();
-            const double2* vk = vb + ((c + 1) & 1) * rows;
-            const double2* vc = vb + (c & 1) * rows;
-            double2 v[R], w[R], y[R];
-            int off[R];                          // this lane's rows (none: any row, not stored)
-#pragma unroll
-            for (int t = 0; t < R; ++t) {
-                const int i = last - 32 * t;
-                off[t] = max(i, 0);
-                const bool in = i > c;           // rows up to c get no update
-                v[t] = vk[off[t]];
-                w[t] = wb[off[t]];
-                v[t] = c2(in ? v[t].x : 0.0, in ? v[t].y : 0.0);
-                w[t] = c2(in ? w[t].x : 0.0, in ? w[t].y : 0.0);
-                y[t] = zero;
+            // this warp's row block and columns, four of them at a time so
+            // that their loads and chains overlap
+            if (const int r = (rows - 1 - c + 31) >> 5; r != rb) {
+                rb = r;
+                G = NW / rb;
+                myg = warp / rb;
+                myt = warp - myg * rb;
             }
-            const int j0 = c + 1 + (warp - (c + 1) % NW + NW) % NW;
-            // the own columns, U of them at a time so that their loads and
-            // chains overlap, on the first RT row blocks
-            auto pass = [&](auto rt) {
-                constexpr int RT = decltype(rt)::value, U = RT == 1 ? 4 : 2;
-                double2* q = M + j0 * ld;
-                const double2 *pv = vk + j0, *pw = wb + j0, *pn = vc + j0;
+            if (myg < G) {
+                const int i = last - 32 * myt, o = max(i, 0);
+                const double2 v = vk[o], w = wb[o];
+                double2 y = zero;
+                int j = c + 1 + myg;
+                const double2 *pv = vk + j, *pw = wb + j, *pn = vc + j;
+                double2* q = M + o + j * ld;
+                const int qs = G * ld;
 #pragma unroll 1
-                for (int j = j0; j < n; j += U * NW, q += U * NW * ld, pv += U * NW, pw += U * NW, pn += U * NW) {
-                    double2 z[U][RT];
+                for (; j + 3 * G < n; j += 4 * G, q += 4 * qs, pv += 4 * G, pw += 4 * G, pn += 4 * G) {
+                    double2 z[4];
 #pragma unroll
-                    for (int u = 0; u < U; ++u)
+                    for (int u = 0; u < 4; ++u) z[u] = q[u * qs];
 #pragma unroll
-                        for (int t = 0; t < RT; ++t)
-                            if (u == 0 || j + u * NW < n) z[u][t] = q[off[t] + u * NW * ld];
+                    for (int u = 0; u < 4; ++u) z[u] = cfms_bc(cfms_bc(z[u], v, pw[u * G]), w, pv[u * G]);
 #pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        if (u > 0 && j + u * NW >= n) break;
-                        const double2 vj = pv[u * NW], wj = pw[u * NW], nj = pn[u * NW];
-#pragma unroll
-                        for (int t = 0; t < RT; ++t) {
-                            z[u][t] = cfms_bc(cfms_bc(z[u][t], v[t], wj), w[t], vj);
-                            y[t] = cfma(y[t], z[u][t], nj);
-                        }
+                    for (int u = 0; u < 4; ++u) {
+                        if (i >= 0) q[u * qs] = z[u];
+                        y = cfma(y, z[u], pn[u * G]);
                     }
-#pragma unroll
-                    for (int u = 0; u < U; ++u)
-#pragma unroll
-                        for (int t = 0; t < RT; ++t)
-                            if ((u == 0 || j + u * NW < n) && last - 32 * t >= 0) q[off[t] + u * NW * ld] = z[u][t];
                 }
-            };
-            const int blocks = (rows - 1 - c + 31) >> 5;         // row blocks that hold rows c + 1 ..
-            if (R == 1 || blocks == 1) pass(IntC<1>{});
-            else if (R == 2 || blocks == 2) pass(IntC<R < 2 ? R : 2>{});
-            else pass(IntC<R>{});
-#pragma unroll
-            for (int t = 0; t < R; ++t)
-                if (last - 32 * t > c) part[warp * rows + last - 32 * t] = y[t];
+#pragma unroll 1
+                for (; j < n; j += G, q += qs, pv += G, pw += G, pn += G) {
+                    const double2 z = cfms_bc(cfms_bc(*q, v, *pw), w, *pv);
+                    if (i >= 0) *q = z;
+                    y = cfma(y, z, *pn);
+                }
+                part[32 * (myg * rb + myt) + lane] = y;
+            }
             team_sync<NT, BLOCK>();
         }
         team_sync<NT, BLOCK>();

@@ -28,6 +28,14 @@ enum class Regime : int {
 // kCtaPreferredMaxN (measured crossover with the l2-slot kernel on B200).
 constexpr int kCtaMaxN = 64;
 constexpr int kCtaPreferredMaxN = 60;
+// Above it, up to here, the l2-slot size class is also solved by that kernel
+// (one CTA of 256 or 512 threads per pencil, no slots) unless a number of
+// slots per SM is asked for: the largest N whose matrix and vectors fit one
+// CTA's shared memory.
+constexpr int kResidentMaxN = 110;
+// info of a pencil that the mixed form leaves to a following cta_launch with
+// `retry` (never seen by the caller).
+constexpr int kRetryInfo = -2147483647 - 1;
 size_t cta_smem_bytes(int n, bool spec = false);   // one pencil; `spec`: the intensity form
 int cta_nmax_for(int n);
 int cta_threads_for(int nmax);   // threads per pencil (per team) of that row bound's kernel
@@ -39,9 +47,11 @@ int cta_default_teams(int nmax);   // pencils per CTA when none is requested
 size_t cta_teams_smem_bytes(int n, int teams, bool spec = false);
 cudaError_t cta_set_attributes(int nmax, size_t smem);   // every teams form of the row bound
 // `sigma`: H is the metric diag(I_{n/2}, -I_{n/2}) and is not read (H may be NULL).
-// `teams`: pencils per CTA (1, or up to cta_max_teams(nmax)).
+// `teams`: pencils per CTA (1, or up to cta_max_teams(nmax)). `retry`: only
+// pencils whose info is kRetryInfo.
 cudaError_t cta_launch(int n, int nmax, int stage, const void* H, const void* S, double* W, void* U,
-                       int* info, long long batch, cudaStream_t stream, bool sigma = false, int teams = 1);
+                       int* info, long long batch, cudaStream_t stream, bool sigma = false, int teams = 1,
+                       bool retry = false);
 
 // Spin-wave metric solve that reduces the eigenvectors to the spectrum
 // S(q, E) on the device (no U output): O is 3 x n complex per problem,
@@ -86,11 +96,12 @@ __host__ __device__ inline size_t tiled_slot_bytes(int n, bool mixed = false) {
 size_t tiled_vec_bytes(int n);
 cudaError_t tiled_set_attributes(size_t smem);
 // `mixed`: FP32 Householder reduction, FP64 refinement (see geneig_tiled.cu).
-// `refine_max`: mixed form's refinement steps before it falls back to FP64.
+// `refine_max`: mixed form's refinement steps before it falls back to FP64;
+// `defer`: a pencil that needs it gets info = kRetryInfo instead.
 constexpr int kRefineMaxIters = 8;
 cudaError_t tiled_launch(int n, int slots, size_t smem, int stage, const void* H, const void* S, double* W, void* U,
                          int* info, long long batch, void* scratch, cudaStream_t stream, bool sigma,
-                         bool mixed = false, int refine_max = kRefineMaxIters);
+                         bool mixed = false, int refine_max = kRefineMaxIters, bool defer = false);
 
 struct PlainPlan {
     int    n        = 0;
@@ -100,10 +111,12 @@ struct PlainPlan {
     Regime regime   = Regime::SmemCta;
     int    nmax     = 0;      // SmemCta: compile-time row bound of the register arrays
     int    teams    = 1;      // SmemCta: pencils per CTA at a time (threads / teams each)
+    bool   resident = false;  // L2Slot solved by the shared-memory kernel (see kResidentMaxN)
     int    slots    = 0;      // L2Slot: number of resident CTAs (= scratch slots)
     size_t scratch_bytes = 0; // L2Slot: bytes of device scratch needed
     bool   mixed    = false;  // mixed-precision form (always the L2Slot regime)
-    int    refine_max = kRefineMaxIters;  // mixed: refinement steps before the FP64 fallback
+    int    refine_max = kRefineMaxIters;  // mixed: refinement steps before the FP64 fallback (by the
+                              // shared-memory kernel of row bound nmax when nmax > 0)
 };
 
 // Picks the regime and launch shape for size n on `device` and sets the
@@ -131,8 +144,11 @@ cudaError_t plain_launch(const PlainPlan& plan, int stage,
                          cudaStream_t stream, bool sigma = false);
 
 #ifdef SGEIG_PHASE_TIMERS
-// Profiling builds only: adds the tiled kernel's phase counters into out.
+// Profiling builds only: each kernel unit adds its phase counters to out.
 cudaError_t tiled_phase_cycles(unsigned long long* out, int count, bool reset);
+cudaError_t cta_small_phase_cycles(unsigned long long* out, int count, bool reset);
+cudaError_t cta_mid_phase_cycles(unsigned long long* out, int count, bool reset);
+cudaError_t cta_wide_phase_cycles(unsigned long long* out, int count, bool reset);
 #endif
 
 // Thread-local last-error text of the C ABI (defined in c_api.cpp), for
@@ -154,7 +170,7 @@ int tune_pick(int n, int device, const std::vector<std::pair<std::string, int>>&
 // Persistent uneven-size kernel (geneig_uneven.cu). One launch solves up to
 // kUnevenMaxGroups size groups, given in the order their work is handed out
 // (descending N); kind is uneven_kind(n, l2slot): 0..4 the smem-cta row
-// bound 16/32/48/56/64, 5 the l2-slot body; per_item pencils make one work
+// bound 16/32/48/56/64, 5 the l2-slot body, 6 below; per_item pencils make one work
 // item. `head` is a device counter (reset by the launch), `scratch` holds
 // `grid` slots of slot_elems complex entries when any group is l2-slot.
 constexpr int kUnevenMaxGroups = 8;
@@ -173,7 +189,15 @@ struct UnevenLaunch {
 int uneven_kind(int n, bool l2slot);
 size_t uneven_smem_bytes(int n, int kind);
 cudaError_t uneven_set_attributes(size_t smem);
+// Sizes of kind 6 (kResidentMaxN's class, whose pencils take a whole SM) run
+// as launches of the shared-memory kernel, on `side` beside the persistent
+// kernel when the mix has both.
+constexpr int kUnevenResident = 6;
+struct UnevenSide {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+};
 cudaError_t uneven_launch(const UnevenLaunch& L, unsigned long long* head, void* scratch, size_t slot_elems,
-                          int grid, size_t smem, cudaStream_t stream);
+                          int grid, size_t smem, cudaStream_t stream, const UnevenSide& side);
 
 }  // namespace sgeig

@@ -466,6 +466,14 @@ bool plain_plan(int n, int device, PlainPlan* plan, std::string* err, bool mixed
         p.smem = smem_wide;
         p.nmax = kWideNmax;
         e = cudaFuncSetAttribute(geneig_plain_kernel<kWideNmax>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    } else if (!mixed && slots_per_sm == 0 && std::getenv("SUNNY_GENEIG_SLOTS_PER_SM") == nullptr &&
+               n > kCtaPreferredMaxN && n <= kResidentMaxN && cta_smem_bytes(n) <= (size_t)optin) {
+        p.regime = Regime::L2Slot;
+        p.resident = true;
+        p.nmax = cta_nmax_for(n);
+        p.smem = cta_smem_bytes(n);
+        p.threads = cta_threads_for(p.nmax);
+        e = cta_set_attributes(p.nmax, (size_t)optin);
     } else {
         p.regime = Regime::L2Slot;
         p.smem = tiled_vec_bytes(n);
@@ -477,6 +485,10 @@ bool plain_plan(int n, int device, PlainPlan* plan, std::string* err, bool mixed
         p.slots = per_sm * sms;
         p.scratch_bytes = (size_t)p.slots * tiled_slot_bytes(n, mixed);
         e = tiled_set_attributes((size_t)optin);
+        if (mixed && n <= kResidentMaxN && cta_smem_bytes(n) <= (size_t)optin) {
+            p.nmax = cta_nmax_for(n);
+            if (e == cudaSuccess) e = cta_set_attributes(p.nmax, (size_t)optin);
+        }
     }
     if (e != cudaSuccess) { *err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e); return false; }
     *plan = p;
@@ -498,11 +510,23 @@ cudaError_t plain_launch(const PlainPlan& plan, int stage, const void* H, const 
     a.ld = plan.ld;
     a.stage = stage;
     a.sigma = sigma ? 1 : 0;
-    if (plan.regime == Regime::SmemCta)
+    if (plan.regime == Regime::SmemCta || plan.resident)
         return cta_launch(plan.n, plan.nmax, stage, H, S, W, U, info, batch, stream, sigma, plan.teams);
-    if (plan.regime == Regime::L2Slot)
-        return tiled_launch(plan.n, plan.slots, plan.smem, stage, H, S, W, U, info, batch, scratch, stream, sigma,
-                            plan.mixed, plan.refine_max);
+    if (plan.regime == Regime::L2Slot) {
+        // mixed: what does not converge is solved again from H and S by the
+        // plain kernel of that size, unless U lies over them
+        const size_t bytes = (size_t)plan.n * plan.n * 16 * (size_t)batch;
+        auto apart = [&](const void* p) {
+            const char *u = static_cast<const char*>(U), *q = static_cast<const char*>(p);
+            return u + bytes <= q || q + bytes <= u;
+        };
+        const bool defer = plan.mixed && plan.nmax > 0 && (sigma || apart(H)) && apart(S);
+        cudaError_t e = tiled_launch(plan.n, plan.slots, plan.smem, stage, H, S, W, U, info, batch, scratch, stream,
+                                     sigma, plan.mixed, plan.refine_max, defer);
+        if (e == cudaSuccess && defer)
+            e = cta_launch(plan.n, plan.nmax, stage, H, S, W, U, info, batch, stream, sigma, 1, true);
+        return e;
+    }
     const long long grid = batch < 0x7fffffffLL ? batch : 0x7fffffffLL;
     geneig_plain_kernel<kWideNmax><<<(unsigned)grid, kNT, plan.smem, stream>>>(a);
     return cudaGetLastError();
@@ -514,14 +538,14 @@ cudaError_t plain_launch(const PlainPlan& plan, int stage, const void* H, const 
 // Callers that cannot allocate device memory -- code running inside another
 // framework's memory pool or under a strict no-allocation policy, plugins
 // whose host forbids cudaMalloc on its streams, and graph-replay setups that
-// must not touch the allocator -- get, for n up to the smem-cta limit, the
+// must not touch the allocator -- get, for n up to kResidentMaxN, the
 // shared-memory kernel, which needs no scratch at all, and above it the
 // L2-slot kernel with its per-CTA scratch slots taken from the fixed array
 // below instead of a cudaMalloc'd buffer. The array is sized once
 // (kNoAllocScratchBytes) and every GPU that loads the library keeps it for
 // the life of the process. It holds floor(32 MiB / slot) slots, so the
-// number of resident CTAs, and with it the throughput, falls with n: 161
-// CTAs at n = 61, 12 at n = 216, 2 at n = 512 (the regular launch keeps
+// number of resident CTAs, and with it the throughput, falls with n: 48
+// CTAs at n = 111, 12 at n = 216, 2 at n = 512 (the regular launch keeps
 // 2 per SM, 296 on B200).
 namespace {
 
@@ -554,7 +578,7 @@ cudaError_t noalloc_setup(int dev, NoAllocDevice** out, std::string* err) {
         e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         if (e != cudaSuccess) { *err = std::string("cudaDeviceGetAttribute: ") + cudaGetErrorString(e); return e; }
         e = tiled_set_attributes((size_t)optin);
-        for (int nmax : {16, 24, 32, 40, 48, 56, 64})
+        for (int nmax : {16, 24, 32, 40, 48, 56, 64, 72, 80, 96, 112})
             if (e == cudaSuccess) e = cta_set_attributes(nmax, (size_t)optin);
         if (e != cudaSuccess) { *err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e); return e; }
         d.optin = optin;
@@ -608,7 +632,7 @@ extern "C" sunny_geneig_status_t sunny_geneig_launch_noalloc(int n, uintptr_t d_
         api_set_error("sunny_geneig_launch_noalloc: " + err);
         return SUNNY_GENEIG_DEVICE_ERROR;
     }
-    if (n <= kCtaPreferredMaxN && cta_smem_bytes(n) <= (size_t)d->optin) {
+    if (n <= kResidentMaxN && cta_smem_bytes(n) <= (size_t)d->optin) {
         // the shared-memory kernel keeps everything on chip: no scratch at all
         const int nmax = cta_nmax_for(n), teams = cta_default_teams(nmax);
         e = cta_launch(n, nmax, 4, reinterpret_cast<const void*>(d_H),

@@ -32,7 +32,9 @@
 // and conquer, the back-transform and everything else stay FP64; then
 // Ogita-Aishima refinement steps (FP64 tensor-core GEMMs against the FP64 C,
 // repeated until the correction is negligible) recover FP64 eigenpairs of C
-// before U = X^H V.
+// before U = X^H V. A pencil whose refinement does not converge is solved in
+// FP64: from C in this kernel, or (`defer`) by the shared-memory kernel, which
+// is the plain form of the sizes it holds.
 
 #include "geneig_tiled_body.cuh"
 #include "sunny_geneig.h"
@@ -67,7 +69,7 @@ cudaError_t tiled_set_attributes(size_t smem) {
 
 cudaError_t tiled_launch(int n, int slots, size_t smem, int stage, const void* H, const void* S, double* W, void* U,
                          int* info, long long batch, void* scratch, cudaStream_t stream, bool sigma, bool mixed,
-                         int refine_max) {
+                         int refine_max, bool defer) {
     if (batch <= 0) return cudaSuccess;
     TiledArgs a;
     a.H = static_cast<const double2*>(H);
@@ -83,6 +85,7 @@ cudaError_t tiled_launch(int n, int slots, size_t smem, int stage, const void* H
     a.sigma = sigma ? 1 : 0;
     a.mixed = mixed ? 1 : 0;
     a.refine_max = refine_max;
+    a.defer = defer ? 1 : 0;
     const long long grid = batch < slots ? batch : slots;
     geneig_tiled_kernel<<<(unsigned)grid, kNT, smem, stream>>>(a);
     return cudaGetLastError();
@@ -92,18 +95,6 @@ cudaError_t tiled_launch(int n, int slots, size_t smem, int stage, const void* H
 
 #ifdef SGEIG_PHASE_TIMERS
 namespace sgeig {
-// Profiling builds only: this translation unit's phase counters (the tiled
-// kernel's marks), added into `out` by sunny_geneig_phase_cycles.
-cudaError_t tiled_phase_cycles(unsigned long long* out, int count, bool reset) {
-    unsigned long long mine[kPhaseSlots] = {};
-    cudaError_t e = cudaMemcpyFromSymbol(mine, g_phase_cycles, sizeof(mine));
-    for (int i = 0; e == cudaSuccess && i < count && i < kPhaseSlots; ++i) out[i] += mine[i];
-    if (e == cudaSuccess && reset) {
-        static const unsigned long long zeros[kPhaseSlots] = {};
-        e = cudaMemcpyToSymbol(g_phase_cycles, zeros, sizeof(zeros));
-    }
-    return e;
-}
+cudaError_t tiled_phase_cycles(unsigned long long* out, int count, bool reset) { return add_phase_cycles(out, count, reset); }
 }  // namespace sgeig
 #endif
-

@@ -40,6 +40,7 @@ struct TiledArgs {
     int sigma;      // H = diag(I_{n/2}, -I_{n/2}), not read from memory
     int mixed;      // FP32 Householder reduction + FP64 refinement
     int refine_max; // mixed: refinement steps before the FP64 fallback
+    int defer;      // mixed: leave the fallback to the shared-memory kernel (info = kRetryInfo)
 };
 
 // Ogita-Aishima refinement of the mixed form: it stops as soon as the current
@@ -1022,6 +1023,10 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
                 // no convergence from the FP32 start (possible when C's
                 // spectrum is spread over many orders of magnitude): redo
                 // this pencil's eigensolve in FP64 from C, still intact in M0
+                if (a.defer) {
+                    if (tid == 0) a.info[b] = kRetryInfo;
+                    return;
+                }
                 use32 = false;
                 continue;
             }

@@ -1,5 +1,5 @@
 // Persistent kernel for batches of pencils of uneven sizes (one launch for
-// the whole mix). The host groups the problems by size N (up to kMaxGroups
+// the whole mix, but for the sizes whose pencils take a whole SM). The host groups the problems by size N (up to kMaxGroups
 // sizes, each group batch-contiguous in its own buffers, the layouts of
 // sunny_geneig_launch) and orders the groups by descending N. The groups are
 // cut into work items: one pencil for sizes in the l2-slot regime, `per_item`
@@ -113,22 +113,25 @@ cudaError_t uneven_set_attributes(size_t smem) {
 }
 
 int uneven_kind(int n, bool l2slot) {
-    if (l2slot) return 5;
+    if (l2slot) return n > kCtaPreferredMaxN && n <= kResidentMaxN ? kUnevenResident : 5;
     return n <= 16 ? 0 : n <= 32 ? 1 : n <= 48 ? 2 : n <= 56 ? 3 : 4;
 }
 
 size_t uneven_smem_bytes(int n, int kind) {
-    return kind == 5 ? tiled_vec_bytes(n)
+    return kind == kUnevenResident ? 0
+         : kind == 5 ? tiled_vec_bytes(n)
                      : kind_teams(kind) * cta_smem_bytes(n);
 }
 
 cudaError_t uneven_launch(const UnevenLaunch& L, unsigned long long* head, void* scratch, size_t slot_elems,
-                          int grid, size_t smem, cudaStream_t stream) {
+                          int grid, size_t smem, cudaStream_t stream, const UnevenSide& side) {
     UnevenArgs a{};
     long long first = 0;
     int ng = 0;
+    bool resident = false;
     for (int i = 0; i < L.ngroups; ++i) {
         if (L.count[i] <= 0) continue;
+        if (L.kind[i] == kUnevenResident) { resident = true; continue; }
         UnevenGroup& G = a.g[ng++];
         G.H = static_cast<const double2*>(L.H[i]);
         G.S = static_cast<const double2*>(L.S[i]);
@@ -143,17 +146,39 @@ cudaError_t uneven_launch(const UnevenLaunch& L, unsigned long long* head, void*
         G.first_item = first;
         first += (G.count + G.per_item - 1) / G.per_item;
     }
-    if (ng == 0) return cudaSuccess;
-    a.ngroups = ng;
-    a.nitems = first;
-    a.head = head;
-    a.scratch = static_cast<double2*>(scratch);
-    a.slot_elems = slot_elems;
-    cudaError_t e = cudaMemsetAsync(head, 0, sizeof(unsigned long long), stream);
-    if (e != cudaSuccess) return e;
-    const long long g = first < grid ? first : grid;
-    geneig_uneven_kernel<<<(unsigned)g, kNT, smem, stream>>>(a);
-    return cudaGetLastError();
+    // the persistent kernel first: its long items start at once, and the
+    // resident sizes fill the SMs that its CTAs leave
+    const bool both = resident && ng > 0;
+    cudaError_t e = cudaSuccess;
+    if (both) {
+        e = cudaEventRecord(side.fork, stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(side.stream, side.fork, 0);
+        if (e != cudaSuccess) return e;
+    }
+    if (ng > 0) {
+        a.ngroups = ng;
+        a.nitems = first;
+        a.head = head;
+        a.scratch = static_cast<double2*>(scratch);
+        a.slot_elems = slot_elems;
+        e = cudaMemsetAsync(head, 0, sizeof(unsigned long long), stream);
+        if (e != cudaSuccess) return e;
+        const long long g = first < grid ? first : grid;
+        geneig_uneven_kernel<<<(unsigned)g, kNT, smem, stream>>>(a);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    const cudaStream_t st = both ? side.stream : stream;
+    for (int i = 0; i < L.ngroups && resident; ++i) {
+        if (L.count[i] <= 0 || L.kind[i] != kUnevenResident) continue;
+        e = cta_launch(L.n[i], cta_nmax_for(L.n[i]), 4, L.H[i], L.S[i], L.W[i], L.U[i], L.info[i], L.count[i], st);
+        if (e != cudaSuccess) return e;
+    }
+    if (both) {
+        e = cudaEventRecord(side.join, side.stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, side.join, 0);
+    }
+    return e;
 }
 
 }  // namespace sgeig
