@@ -49,6 +49,8 @@ struct sunny_geneig_uneven {
     int n[sgeig::kUnevenMaxGroups] = {};
     int kind[sgeig::kUnevenMaxGroups] = {};
     int per_item[sgeig::kUnevenMaxGroups] = {};
+    void* big_scratch[sgeig::kUnevenMaxGroups] = {};   // kUnevenBig sizes: one slot per SM
+    int sms = 0;
     size_t smem = 0;
     int grid = 0;
     size_t slot_elems = 0;
@@ -87,9 +89,9 @@ cudaError_t with_device(int device, F&& fn) {
 bool aligned(uintptr_t p, uintptr_t a) { return (p % a) == 0; }
 
 void release_side(sgeig::UnevenSide& s) {
-    if (s.stream) cudaStreamDestroy(s.stream);
+    for (cudaStream_t st : s.stream) if (st) cudaStreamDestroy(st);
+    for (cudaEvent_t ev : s.join) if (ev) cudaEventDestroy(ev);
     if (s.fork) cudaEventDestroy(s.fork);
-    if (s.join) cudaEventDestroy(s.join);
 }
 
 // NVTX range around each entry point (header-only NVTX v3: a no-op unless a
@@ -537,12 +539,17 @@ sunny_geneig_uneven_t sunny_geneig_uneven_create(int num_sizes, const int* sizes
                 if (h->kind[g] == sgeig::kUnevenResident) {
                     ea = sgeig::cta_set_attributes(sgeig::cta_nmax_for(n), (size_t)optin);
                     if (ea != cudaSuccess) { err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea); return ea; }
+                } else if (h->kind[g] == sgeig::kUnevenBig) {
+                    ea = sgeig::tiled_set_attributes((size_t)optin);
+                    if (ea == cudaSuccess) ea = cudaMalloc(&h->big_scratch[g], (size_t)sms * sgeig::tiled_slot_bytes(n));
+                    if (ea != cudaSuccess) { err = std::string("cudaMalloc scratch: ") + cudaGetErrorString(ea); return ea; }
                 } else if (l2) slot = std::max(slot, sgeig::tiled_slot_elems(n));
             }
             if (h->smem > (size_t)optin) { err = "the mix needs more shared memory than a CTA has"; return cudaErrorInvalidValue; }
             ea = sgeig::uneven_set_attributes((size_t)optin);
             if (ea != cudaSuccess) { err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea); return ea; }
             h->grid = 2 * sms;
+            h->sms = sms;
             h->slot_elems = slot;
             if (slot) {
                 ea = cudaMalloc(&h->scratch, (size_t)h->grid * slot * 16);
@@ -550,9 +557,14 @@ sunny_geneig_uneven_t sunny_geneig_uneven_create(int num_sizes, const int* sizes
             }
             ea = cudaMalloc(reinterpret_cast<void**>(&h->head), sizeof(unsigned long long));
             if (ea != cudaSuccess) { err = std::string("cudaMalloc counter: ") + cudaGetErrorString(ea); return ea; }
-            ea = cudaStreamCreateWithFlags(&h->side.stream, cudaStreamNonBlocking);
-            if (ea == cudaSuccess) ea = cudaEventCreateWithFlags(&h->side.fork, cudaEventDisableTiming);
-            if (ea == cudaSuccess) ea = cudaEventCreateWithFlags(&h->side.join, cudaEventDisableTiming);
+            int nside = 0;
+            for (int g = 0; g < num_sizes; ++g) nside += h->kind[g] >= sgeig::kUnevenResident;
+            if (num_sizes < 2) nside = 0;      // a lone size runs on the caller's stream
+            for (int i = 0; i < nside && ea == cudaSuccess; ++i) {
+                ea = cudaStreamCreateWithFlags(&h->side.stream[i], cudaStreamNonBlocking);
+                if (ea == cudaSuccess) ea = cudaEventCreateWithFlags(&h->side.join[i], cudaEventDisableTiming);
+            }
+            if (ea == cudaSuccess && nside) ea = cudaEventCreateWithFlags(&h->side.fork, cudaEventDisableTiming);
             if (ea == cudaSuccess) ea = cudaEventCreateWithFlags(&h->done, cudaEventDisableTiming);
             return ea;
         });
@@ -561,6 +573,7 @@ sunny_geneig_uneven_t sunny_geneig_uneven_create(int num_sizes, const int* sizes
             with_device(device_id, [&]() {
                 cudaFree(h->scratch);
                 cudaFree(h->head);
+                for (void* p : h->big_scratch) cudaFree(p);
                 release_side(h->side);
                 if (h->done) cudaEventDestroy(h->done);
                 return cudaSuccess;
@@ -612,6 +625,8 @@ sunny_geneig_status_t sunny_geneig_uneven_launch(sunny_geneig_uneven_t h, const 
         L.W[g] = reinterpret_cast<double*>(d_W[i]);
         L.U[g] = reinterpret_cast<void*>(d_U[i]);
         L.info[g] = reinterpret_cast<int*>(d_info[i]);
+        L.scratch[g] = h->big_scratch[g];
+        L.slots[g] = h->sms;
     }
     try {
         std::lock_guard<std::mutex> lock(h->mu);
@@ -649,6 +664,7 @@ void sunny_geneig_uneven_destroy(sunny_geneig_uneven_t h) {
             release_side(h->side);
             cudaFree(h->scratch);
             cudaFree(h->head);
+            for (void* p : h->big_scratch) cudaFree(p);
             return cudaSuccess;
         });
         delete h;

@@ -93,13 +93,14 @@ __host__ __device__ inline size_t tiled_slot_elems(int n, bool mixed = false) {
 __host__ __device__ inline size_t tiled_slot_bytes(int n, bool mixed = false) {
     return tiled_slot_elems(n, mixed) * 16;
 }
-size_t tiled_vec_bytes(int n);
+size_t tiled_vec_bytes(int n, bool work = true);   // dynamic shared memory, with or without the work area
+int tiled_threads_for(int n);   // threads per CTA: 512 (one CTA per SM) above kResidentMaxN, else 256 (two)
 cudaError_t tiled_set_attributes(size_t smem);
 // `mixed`: FP32 Householder reduction, FP64 refinement (see geneig_tiled.cu).
 // `refine_max`: mixed form's refinement steps before it falls back to FP64;
 // `defer`: a pencil that needs it gets info = kRetryInfo instead.
 constexpr int kRefineMaxIters = 8;
-cudaError_t tiled_launch(int n, int slots, size_t smem, int stage, const void* H, const void* S, double* W, void* U,
+cudaError_t tiled_launch(int n, int slots, int stage, const void* H, const void* S, double* W, void* U,
                          int* info, long long batch, void* scratch, cudaStream_t stream, bool sigma,
                          bool mixed = false, int refine_max = kRefineMaxIters, bool defer = false);
 
@@ -170,7 +171,7 @@ int tune_pick(int n, int device, const std::vector<std::pair<std::string, int>>&
 // Persistent uneven-size kernel (geneig_uneven.cu). One launch solves up to
 // kUnevenMaxGroups size groups, given in the order their work is handed out
 // (descending N); kind is uneven_kind(n, l2slot): 0..4 the smem-cta row
-// bound 16/32/48/56/64, 5 the l2-slot body, 6 below; per_item pencils make one work
+// bound 16/32/48/56/64, 5 the l2-slot body (asked for, N <= 60), 6 and 7 below; per_item pencils make one work
 // item. `head` is a device counter (reset by the launch), `scratch` holds
 // `grid` slots of slot_elems complex entries when any group is l2-slot.
 constexpr int kUnevenMaxGroups = 8;
@@ -185,17 +186,21 @@ struct UnevenLaunch {
     double* W[kUnevenMaxGroups] = {};
     void* U[kUnevenMaxGroups] = {};
     int* info[kUnevenMaxGroups] = {};
+    void* scratch[kUnevenMaxGroups] = {};
+    int slots[kUnevenMaxGroups] = {};
 };
 int uneven_kind(int n, bool l2slot);
 size_t uneven_smem_bytes(int n, int kind);
 cudaError_t uneven_set_attributes(size_t smem);
-// Sizes of kind 6 (kResidentMaxN's class, whose pencils take a whole SM) run
-// as launches of the shared-memory kernel, on `side` beside the persistent
-// kernel when the mix has both.
-constexpr int kUnevenResident = 6;
+// Sizes whose pencils take a whole SM run as launches of their own kernels,
+// each on a stream of `side`, beside the persistent kernel: kind 6, up to
+// kResidentMaxN, the shared-memory kernel; kind 7, above, the tiled kernel with
+// L.slots[i] slots at L.scratch[i].
+constexpr int kUnevenResident = 6, kUnevenBig = 7;
 struct UnevenSide {
-    cudaStream_t stream = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
+    cudaStream_t stream[kUnevenMaxGroups] = {};
+    cudaEvent_t join[kUnevenMaxGroups] = {};
+    cudaEvent_t fork = nullptr;
 };
 cudaError_t uneven_launch(const UnevenLaunch& L, unsigned long long* head, void* scratch, size_t slot_elems,
                           int grid, size_t smem, cudaStream_t stream, const UnevenSide& side);

@@ -478,8 +478,9 @@ bool plain_plan(int n, int device, PlainPlan* plan, std::string* err, bool mixed
         p.regime = Regime::L2Slot;
         p.smem = tiled_vec_bytes(n);
         // resident CTAs (and scratch slots) per SM: SUNNY_GENEIG_SLOTS_PER_SM
-        // = 1 or 2 (default 2, the kernel's occupancy limit)
-        int per_sm = 2;
+        // = 1 or 2 (default: the kernel's occupancy limit, 1 above kResidentMaxN)
+        p.threads = tiled_threads_for(n);
+        int per_sm = n > kResidentMaxN ? 1 : 2;
         if (slots_per_sm != 0) per_sm = slots_per_sm;
         else if (const char* ps = std::getenv("SUNNY_GENEIG_SLOTS_PER_SM")) per_sm = std::atoi(ps) == 1 ? 1 : 2;
         p.slots = per_sm * sms;
@@ -521,7 +522,7 @@ cudaError_t plain_launch(const PlainPlan& plan, int stage, const void* H, const 
             return u + bytes <= q || q + bytes <= u;
         };
         const bool defer = plan.mixed && plan.nmax > 0 && (sigma || apart(H)) && apart(S);
-        cudaError_t e = tiled_launch(plan.n, plan.slots, plan.smem, stage, H, S, W, U, info, batch, scratch, stream,
+        cudaError_t e = tiled_launch(plan.n, plan.slots, stage, H, S, W, U, info, batch, scratch, stream,
                                      sigma, plan.mixed, plan.refine_max, defer);
         if (e == cudaSuccess && defer)
             e = cta_launch(plan.n, plan.nmax, stage, H, S, W, U, info, batch, stream, sigma, 1, true);
@@ -647,7 +648,7 @@ extern "C" sunny_geneig_status_t sunny_geneig_launch_noalloc(int n, uintptr_t d_
     }
     const long long fit = (long long)(kNoAllocScratchBytes / slot);
     const int slots = (int)(fit < 2LL * d->sms ? fit : 2LL * d->sms);
-    e = tiled_launch(n, slots, tiled_vec_bytes(n), 4, reinterpret_cast<const void*>(d_H),
+    e = tiled_launch(n, slots, 4, reinterpret_cast<const void*>(d_H),
                      reinterpret_cast<const void*>(d_S), reinterpret_cast<double*>(d_W), reinterpret_cast<void*>(d_U),
                      reinterpret_cast<int*>(d_info), batch_size, d->scratch, reinterpret_cast<cudaStream_t>(stream),
                      false);

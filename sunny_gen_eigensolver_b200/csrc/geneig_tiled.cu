@@ -43,31 +43,34 @@ namespace sgeig {
 using namespace tiled;
 namespace {
 
-__global__ void __launch_bounds__(kNT, 2) geneig_tiled_kernel(TiledArgs a) {
+template <int NT>
+__global__ void __launch_bounds__(NT, NT == kTiledWide ? 1 : 2) geneig_tiled_kernel(TiledArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* slot = a.scratch + (size_t)blockIdx.x * tiled_slot_elems(a.n, a.mixed != 0);
     phase_start();
-    for (long long b = blockIdx.x; b < a.batch; b += gridDim.x) tiled_solve(a, b, slot, smem_raw);
+    for (long long b = blockIdx.x; b < a.batch; b += gridDim.x) tiled_solve<NT>(a, b, slot, smem_raw);
 }
 
 }  // namespace
 
-size_t tiled_vec_bytes(int n) {
-    return (size_t)n * 16 * 3 + 32 * 16 + 3 * 256 * 16 + tiled_part_elems(n) * 16 + (size_t)n * 8 * 3 +
-           (size_t)dc_vec_doubles(n) * 8 + (size_t)n * 4 + 8 * 4 + (size_t)dc_vec_ints(n) * 4;
-}
+int tiled_threads_for(int n) { return tiled_threads(n); }
+
+size_t tiled_vec_bytes(int n, bool work) { return tiled_base_bytes(n) + (work ? tiled_work_elems(n) * 16 : 0); }
 
 // `smem` is the per-CTA shared-memory limit; the kernel's own static shared
 // memory (profiling builds have some) comes off the dynamic allowance.
 cudaError_t tiled_set_attributes(size_t smem) {
-    cudaFuncAttributes fa{};
-    cudaError_t e = cudaFuncGetAttributes(&fa, geneig_tiled_kernel);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(geneig_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(smem - fa.sharedSizeBytes));
+    for (auto k : {geneig_tiled_kernel<kTiledNarrow>, geneig_tiled_kernel<kTiledWide>}) {
+        cudaFuncAttributes fa{};
+        cudaError_t e = cudaFuncGetAttributes(&fa, k);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem - fa.sharedSizeBytes));
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
-cudaError_t tiled_launch(int n, int slots, size_t smem, int stage, const void* H, const void* S, double* W, void* U,
+cudaError_t tiled_launch(int n, int slots, int stage, const void* H, const void* S, double* W, void* U,
                          int* info, long long batch, void* scratch, cudaStream_t stream, bool sigma, bool mixed,
                          int refine_max, bool defer) {
     if (batch <= 0) return cudaSuccess;
@@ -86,8 +89,11 @@ cudaError_t tiled_launch(int n, int slots, size_t smem, int stage, const void* H
     a.mixed = mixed ? 1 : 0;
     a.refine_max = refine_max;
     a.defer = defer ? 1 : 0;
+    a.work = defer ? 0 : 1;
+    const size_t smem = tiled_vec_bytes(n, !defer);
     const long long grid = batch < slots ? batch : slots;
-    geneig_tiled_kernel<<<(unsigned)grid, kNT, smem, stream>>>(a);
+    if (tiled_threads(n) == kTiledWide) geneig_tiled_kernel<kTiledWide><<<(unsigned)grid, kTiledWide, smem, stream>>>(a);
+    else geneig_tiled_kernel<kTiledNarrow><<<(unsigned)grid, kTiledNarrow, smem, stream>>>(a);
     return cudaGetLastError();
 }
 

@@ -17,16 +17,12 @@
 namespace sgeig {
 namespace tiled {
 
-constexpr int kNT = 256;          // threads per CTA
-constexpr int kNW = kNT / 32;     // warps per CTA
-// Below this n the per-column (unblocked) Householder reduction is faster on
-// B200 than the 16-column panels (fewer barriers per column); above it the
-// panels' halved trailing-matrix traffic wins (measured crossover ~90).
-constexpr int kBlockedHetrdMinN = 96;
-// Up to this n the blocked reduction forms y = A v column by column with
-// per-warp partial vectors in shared memory (8 n complex entries, which keep
-// two CTAs per SM up to here); above it, a warp per row item.
-constexpr int kColMatvecMaxN = 352;
+// Threads per CTA: 512 (one CTA per SM) for the sizes this kernel solves by
+// default, whose steps want many loads in flight and whose slots then stay
+// closer to the L2's size; 256 (two per SM) up to kResidentMaxN, where only the
+// mixed form and explicit requests come here.
+constexpr int kTiledWide = 512, kTiledNarrow = 256;
+__host__ __device__ constexpr int tiled_threads(int n) { return n > kResidentMaxN ? kTiledWide : kTiledNarrow; }
 
 struct TiledArgs {
     const double2* __restrict__ H;
@@ -41,6 +37,7 @@ struct TiledArgs {
     int mixed;      // FP32 Householder reduction + FP64 refinement
     int refine_max; // mixed: refinement steps before the FP64 fallback
     int defer;      // mixed: leave the fallback to the shared-memory kernel (info = kRetryInfo)
+    int work;       // the launch's shared memory has the work area (tiled_work_elems)
 };
 
 // Ogita-Aishima refinement of the mixed form: it stops as soon as the current
@@ -98,7 +95,8 @@ struct TVec {
     double2* pb;    // n    tau * A22 * v
     double2* red;   // 32   reduction scratch
     double2* tb;    // 256  T factor of the current WY block (16 x 16, column-major)
-    double2* part;  // tiled_part_elems(n): per-warp partials of the blocked y = A v
+    double2* part;  // threads/32 x kMvRows: per-warp partials of y = A v
+    double2* ring;  // tiled_ring_elems(n): elements of A on their way
     double2* gb;    // 512  Y^H Y of the current WY block: two partial sums, then their sum
     double*  d;     // n    tridiagonal diagonal
     double*  e;     // n    tridiagonal off-diagonal
@@ -109,8 +107,20 @@ struct TVec {
     int*     dci;   // divide-and-conquer ints (dc_vec_ints(n))
 };
 
-__host__ __device__ inline size_t tiled_part_elems(int n) {
-    return (n >= kBlockedHetrdMinN && n <= kColMatvecMaxN) ? (size_t)8 * n : 0;
+// y = A v of the Householder steps: rows per warp, and the columns whose
+// elements a lane has on their way to shared memory.
+constexpr int kMvRows = 128, kMvDepth = 3;
+__host__ __device__ inline size_t tiled_part_elems(int n) { return (size_t)(tiled_threads(n) / 32) * kMvRows; }
+__host__ __device__ inline size_t tiled_ring_elems(int n) { return (size_t)kMvDepth * (kMvRows / 32) * tiled_threads(n); }
+// The work area of the FP64 reduction, last in shared memory: launches of the
+// mixed form that leave their fallback to the shared-memory kernel go without
+// it, which leaves the SM's L1 to the refinement's products (N=54: 7 %).
+__host__ __device__ inline size_t tiled_work_elems(int n) { return tiled_part_elems(n) + tiled_ring_elems(n); }
+
+__host__ __device__ inline size_t tiled_base_bytes(int n) {
+    const size_t b = (size_t)n * 16 * 3 + 32 * 16 + 3 * 256 * 16 + (size_t)n * 8 * 3 + (size_t)dc_vec_doubles(n) * 8 +
+                     (size_t)n * 4 + 8 * 4 + (size_t)dc_vec_ints(n) * 4;
+    return (b + 15) & ~(size_t)15;
 }
 
 __device__ inline TVec tcarve(unsigned char* p, int n) {
@@ -121,26 +131,22 @@ __device__ inline TVec tcarve(unsigned char* p, int n) {
     v.red = v.pb + n;
     v.tb  = v.red + 32;
     v.gb  = v.tb + 256;
-    v.part = v.gb + 512;
-    v.d   = reinterpret_cast<double*>(v.part + tiled_part_elems(n));
+    v.d   = reinterpret_cast<double*>(v.gb + 512);
     v.e   = v.d + n;
     v.rdg = v.e + n;
     v.dcd = v.rdg + n;
     v.rank = reinterpret_cast<int*>(v.dcd + dc_vec_doubles(n));
     v.ctl  = v.rank + n;
     v.dci  = v.ctl + 8;
+    v.part = reinterpret_cast<double2*>(p + tiled_base_bytes(n));
+    v.ring = v.part + tiled_part_elems(n);
     return v;
 }
 
 __device__ __forceinline__ double2 cneg(double2 a) { return c2(-a.x, -a.y); }
 
 // ---------------------------------------------------------------- 16x16 complex MMA tiles
-// D(8x8) += A(8x4) B(4x8) in FP64 on the tensor cores. Fragments: lane l
-// holds A(l/4, l%4), B(l%4, l/4) and D(l/4, 2(l%4) + {0, 1}).
-__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
-    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-        : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
-}
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) { mma884(d, a, b); }
 
 // A warp's 16 x 16 complex accumulator: 2 x 2 subtiles of 8 x 8, real and
 // imaginary parts apart. Element [h][g][e] is row i0 + 8h + lane/4, column
@@ -188,6 +194,19 @@ __device__ __forceinline__ void z16_store(const Z16& c, int i0, int j0, F f) {
                 f(i0 + 8 * h + (lane >> 2), j0 + 8 * g + 2 * (lane & 3) + e, c2(c.re[h][g][e], c.im[h][g][e]));
 }
 
+// One k step of 4: a = A fragments of rows r, r + 8, b = B fragments of columns r, r + 8.
+__device__ __forceinline__ void z16_step(Z16& c, const double2 (&a)[2], const double2 (&b)[2]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            dmma(c.re[h][g], a[h].x, b[g].x);
+            dmma(c.re[h][g], -a[h].y, b[g].y);
+            dmma(c.im[h][g], a[h].x, b[g].y);
+            dmma(c.im[h][g], a[h].y, b[g].x);
+        }
+}
+
 // c += A(i0:i0+16, k0:k1) B(k0:k1, j0:j0+16); a_at(i, k) and b_at(k, j)
 // return the operand elements (they must return 0 outside the operands;
 // k < k1 is checked here).
@@ -207,16 +226,51 @@ __device__ __forceinline__ void z16_mma(Z16& c, int i0, int j0, int k0, int k1, 
         } else {
             a[0] = a[1] = b[0] = b[1] = c2(0.0, 0.0);
         }
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int g = 0; g < 2; ++g) {
-                dmma(c.re[h][g], a[h].x, b[g].x);
-                dmma(c.re[h][g], -a[h].y, b[g].y);
-                dmma(c.im[h][g], a[h].x, b[g].y);
-                dmma(c.im[h][g], a[h].y, b[g].x);
-            }
+        z16_step(c, a, b);
     }
+}
+
+// The same for operands in memory, A(i, k) at pa[i si + k sk] and B(k, j) at
+// pb[k tk + j tj], conjugated where CA / CB say so, A negated for NA. Rows and
+// columns past ni, nj repeat the last one (they reach discarded results only);
+// k blocks are unmasked but for the last, whose A is zeroed past k1.
+template <bool CA, bool NA, bool CB>
+__device__ __forceinline__ void z16_gemm(Z16& c, int i0, int j0, int k0, int k1, const double2* pa, int si, int sk, int ni,
+                                         const double2* pb, int tk, int tj, int nj) {
+    const int lane = threadIdx.x & 31;
+    const int r = lane >> 2, kq = lane & 3;
+    const double2* a0 = pa + (size_t)min(i0 + r, ni - 1) * si;
+    const double2* a1 = pa + (size_t)min(i0 + r + 8, ni - 1) * si;
+    const double2* b0 = pb + (size_t)min(j0 + r, nj - 1) * tj;
+    const double2* b1 = pb + (size_t)min(j0 + r + 8, nj - 1) * tj;
+    auto fix_a = [](double2 x) { return c2(NA ? -x.x : x.x, NA != CA ? -x.y : x.y); };
+    auto fix_b = [](double2 x) { return c2(x.x, CB ? -x.y : x.y); };
+    int k = k0;
+#pragma unroll 4
+    for (; k + 4 <= k1; k += 4) {
+        const size_t ka = (size_t)(k + kq) * sk, kb = (size_t)(k + kq) * tk;
+        const double2 a[2] = {fix_a(a0[ka]), fix_a(a1[ka])}, b[2] = {fix_b(b0[kb]), fix_b(b1[kb])};
+        z16_step(c, a, b);
+    }
+    if (k < k1) {
+        const bool in = k + kq < k1;
+        const size_t ka = (size_t)min(k + kq, k1 - 1) * sk, kb = (size_t)min(k + kq, k1 - 1) * tk;
+        double2 a[2] = {fix_a(a0[ka]), fix_a(a1[ka])};
+        const double2 b[2] = {fix_b(b0[kb]), fix_b(b1[kb])};
+        if (!in) a[0] = a[1] = c2(0.0, 0.0);
+        z16_step(c, a, b);
+    }
+}
+
+// Work order of tm x tn tiles: 4 x 4 blocks of tiles after one another, so that
+// the warps of a CTA share 4 + 4 operand strips at a time. Returns false for a
+// number past the edge (numbers run to tile_blocks(tm, tn)).
+__device__ __forceinline__ int tile_blocks(int tm, int tn) { return ((tm + 3) >> 2) * ((tn + 3) >> 2) * 16; }
+__device__ __forceinline__ bool tile_at(int t, int tm, int tn, int& ti, int& tj) {
+    const int bn = (tn + 3) >> 2, blk = t >> 4, bi = blk / bn, bj = blk - bi * bn;
+    ti = 4 * bi + ((t >> 2) & 3);
+    tj = 4 * bj + (t & 3);
+    return ti < tm && tj < tn;
 }
 
 // t -> (ti, tj) with ti >= tj, enumerating the lower triangle row by row.
@@ -230,13 +284,142 @@ __device__ __forceinline__ void tri_tile(int t, int& ti, int& tj) {
 
 // The divide and conquer with a register allocation of its own: inlined, it
 // made the tile products around it spill (n = 216: 4 % slower).
+template <int kNT>
 static __device__ __noinline__ void tiled_dc(int n, DCShared dc) { tridiag_dc<kNT, 0>(n, dc); }
+
+// How y = A v over rows and columns lo .. n-1 is dealt to the warps: blocks of
+// kMvRows rows, counted from the last row up, each with a share of the warps
+// in proportion to its elements (first[q] .. first[q + 1] - 1 for block q).
+struct MatvecSplit {
+    int first[5];
+};
+template <int NW>
+__device__ __forceinline__ MatvecSplit matvec_split(int n, int lo) {
+    const int m = n - lo, nq = (m + kMvRows - 1) / kMvRows;
+    MatvecSplit s;
+    float total = 0.0f, sum = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) if (q < nq) total += (float)(m - kMvRows * q);
+    s.first[0] = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (q < nq) sum += (float)(m - kMvRows * q);
+        // at least one warp for each block
+        const int f = (int)(NW * sum / total + 0.5f);
+        s.first[q + 1] = q + 1 >= nq ? NW : min(max(f, s.first[q] + 1), NW - (nq - 1 - q));
+    }
+    return s;
+}
+
+// y = A v for the Hermitian trailing matrix A kept in its lower triangle, v zero
+// below lo. A warp has a block of rows, four per lane, and every G-th column j
+// of it, and gets from each element both halves of the product: y_i += A(i, j)
+// v_j for i > j (in registers, to part at the end) and y_j = sum_{i >= j}
+// conj(A(i, j)) v_i (each block's share to ydot[block]). The elements come
+// through shared memory by asynchronous copies, kMvDepth columns ahead; a lane
+// reads what it copied itself, so nothing but its own copies is waited for.
+// N=216, cycles per column: 18.4 K for the full matrix column by column with
+// two pencils per SM, 17.6 K with one column ahead in registers (one pencil of
+// 512 threads): the loads' latency, with some 30 KB in flight per SM.
+template <int kNT>
+__device__ __forceinline__ void sym_matvec(const double2* A, int ld, int n, int lo, const double2* vb, double2* part,
+                                           double2* const (&ydot)[4], double2* ring) {
+    constexpr int NW = kNT / 32, RB = kMvRows / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const MatvecSplit ms = matvec_split<NW>(n, lo);
+    int q = 0;
+#pragma unroll
+    for (int u = 1; u < 4; ++u) if (warp >= ms.first[u]) q = u;
+    int f = 0, G = 0;
+    double2* yd = nullptr;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) if (q == u) { f = ms.first[u]; G = ms.first[u + 1] - f; yd = ydot[u]; }
+    const int r1 = n - kMvRows * q, r0 = max(lo, r1 - kMvRows), g = warp - f;
+    double2 v[RB], y[RB];
+#pragma unroll
+    for (int t = 0; t < RB; ++t) {
+        const int i = r0 + lane + 32 * t;
+        v[t] = i < r1 ? vb[i] : c2(0.0, 0.0);
+        y[t] = c2(0.0, 0.0);
+    }
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(ring + threadIdx.x);
+    auto fetch = [&](int j, int stage) {
+        if (j < r1) {
+            const double2* cj = A + (size_t)j * ld + r0 + lane;
+#pragma unroll
+            for (int t = 0; t < RB; ++t) {
+                const int i = r0 + lane + 32 * t;
+                if (i >= j && i < r1)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                                 :: "r"(dst + (unsigned)((stage * RB + t) * kNT * 16)), "l"(cj + 32 * t) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int u = 0; u < kMvDepth - 1; ++u) fetch(lo + g + u * G, u);
+    int stage = 0;
+#pragma unroll 1
+    for (int j = lo + g; j < r1; j += G) {
+        fetch(j + (kMvDepth - 1) * G, stage == 0 ? kMvDepth - 1 : stage - 1);
+        asm volatile("cp.async.wait_group %0;" :: "n"(kMvDepth - 1) : "memory");
+        const double2* x = ring + stage * RB * kNT + threadIdx.x;
+        const double2 vj = vb[j];
+        double2 dot = c2(0.0, 0.0);
+#pragma unroll
+        for (int t = 0; t < RB; ++t) {
+            const int i = r0 + lane + 32 * t;
+            if (r0 + 32 * t + 31 < j || r0 + 32 * t >= r1) continue;
+            const double2 e = x[t * kNT];
+            const bool in = i >= j && i < r1;
+            const double2 z = c2(in ? e.x : 0.0, in ? e.y : 0.0);
+            dot = cfmac(dot, z, v[t]);
+            if (i != j) y[t] = cfma(y[t], z, vj);                    // the diagonal belongs to the dot
+        }
+        dot = warp_sum2(dot);
+        if (lane == 0) yd[j] = dot;
+        stage = stage == kMvDepth - 1 ? 0 : stage + 1;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+#pragma unroll
+    for (int t = 0; t < RB; ++t) part[warp * kMvRows + lane + 32 * t] = y[t];
+}
+
+// Element i of that product, after a barrier.
+template <int kNT>
+__device__ __forceinline__ double2 sym_matvec_row(int n, int lo, int i, const double2* part, double2* const (&ydot)[4]) {
+    const MatvecSplit ms = matvec_split<kNT / 32>(n, lo);
+    const int q = (n - 1 - i) / kMvRows, r0 = max(lo, n - kMvRows * (q + 1));
+    double2 y = c2(0.0, 0.0);
+    int f = 0, e = 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        if (u <= q) y = cadd(y, ydot[u][i]);     // this block and those below it
+        if (u == q) { f = ms.first[u]; e = ms.first[u + 1]; }
+    }
+#pragma unroll 4
+    for (int w = f; w < e; ++w) y = cadd(y, part[w * kMvRows + i - r0]);
+    return y;
+}
+
+// Sum over the CTA: every thread gets the value; red holds threads/32 entries
+// that no other sum since the last barrier has used.
+template <int kNT>
+__device__ __forceinline__ double cta_sum(double x, double* red) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    x = warp_sum(x);
+    if (lane == 0) red[warp] = x;
+    __syncthreads();
+    return warp_sum(lane < kNT / 32 ? red[lane] : 0.0);
+}
 
 // One pencil b, solved end to end by the whole CTA in its global-memory
 // slot `slot` (tiled_slot_elems(n, mixed) complex entries) with the
-// launch's dynamic shared memory as the vector area.
+// launch's dynamic shared memory as the vector area. kNT >= n.
+template <int kNT>
 __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long long b, double2* slot,
                                             unsigned char* smem_raw) {
+    constexpr int kNW = kNT / 32;
     const int n = a.n, ld = a.ld;
     const size_t mat = (size_t)n * ld;
     const bool mixed = a.mixed != 0;
@@ -308,9 +491,7 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
                 const int i0 = pe + 16 * ti, j0 = pe + 16 * tj;
                 Z16 acc;
                 z16_load(acc, i0, j0, [&](int i, int j) { return (i < n && j < n) ? M0[i + (size_t)j * ld] : zero; });
-                z16_mma(acc, i0, j0, p, pe,
-                        [&](int i, int k) { return i < n ? cneg(M0[i + (size_t)k * ld]) : zero; },
-                        [&](int k, int j) { return j < n ? cconj(M0[j + (size_t)k * ld]) : zero; });
+                z16_gemm<false, true, true>(acc, i0, j0, p, pe, M0, 1, ld, n, M0, ld, 1, n);
                 z16_store(acc, i0, j0, [&](int i, int j, double2 x) {
                     if (i < n && j < n && i >= j) M0[i + (size_t)j * ld] = x;
                 });
@@ -322,16 +503,17 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
     phase_mark(17);
 
     if (!code && a.stage >= 2) {
-        // ---- a3: X = L^-1 -> M1, block row r0..re at a time
+        // ---- a3: X = L^-1 -> M1, block row r0..re at a time; zeros above its
+        // diagonal, so that the products need no masks
+        for (int j = warp; j < n; j += kNW)
+            for (int i = lane; i < j; i += 32) M1[i + (size_t)j * ld] = zero;
         for (int r0 = 0; r0 < n; r0 += 16) {
             const int re = min(r0 + 16, n);
             for (int t = warp; t < (r0 >> 4); t += kNW) {
                 const int j0 = 16 * t;
                 Z16 acc;
                 z16_zero(acc);
-                z16_mma(acc, r0, j0, j0, r0,
-                        [&](int i, int k) { return i < n ? M0[i + (size_t)k * ld] : zero; },
-                        [&](int k, int j) { return k >= j ? M1[k + (size_t)j * ld] : zero; });
+                z16_gemm<false, false, false>(acc, r0, j0, j0, r0, M0, 1, ld, n, M1, 1, ld, n);
                 z16_store(acc, r0, j0, [&](int i, int j, double2 x) { if (i < n) M1[i + (size_t)j * ld] = x; });
             }
             __syncthreads();
@@ -381,13 +563,13 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
                 M2[i + (size_t)j * ld] = (i < m) ? x : cneg(x);
             }
         } else {
-            for (int t = warp; t < tn * tn; t += kNW) {
-                const int ti = t / tn, tj = t - ti * tn, i0 = 16 * ti, j0 = 16 * tj;
+            for (int t = warp; t < tile_blocks(tn, tn); t += kNW) {
+                int ti, tj;
+                if (!tile_at(t, tn, tn, ti, tj)) continue;
+                const int i0 = 16 * ti, j0 = 16 * tj;
                 Z16 acc;
                 z16_zero(acc);
-                z16_mma(acc, i0, j0, 0, min(n, j0 + 16),
-                        [&](int i, int k) { return i < n ? __ldg(Hb + i + (size_t)k * n) : zero; },
-                        [&](int k, int j) { return (j < n && k <= j) ? cconj(M1[j + (size_t)k * ld]) : zero; });
+                z16_gemm<false, false, true>(acc, i0, j0, 0, min(n, j0 + 16), Hb, 1, n, n, M1, ld, 1, n);
                 z16_store(acc, i0, j0, [&](int i, int j, double2 x) {
                     if (i < n && j < n) M2[i + (size_t)j * ld] = x;
                 });
@@ -396,15 +578,13 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
         __syncthreads();
         // C = X T, lower tiles; each lower element is written with its
         // mirror so that C is exactly Hermitian. L in M0 is dead by now.
-        for (int t = warp; t < tn * (tn + 1) / 2; t += kNW) {
+        for (int t = warp; t < tile_blocks(tn, tn); t += kNW) {
             int ti, tj;
-            tri_tile(t, ti, tj);
+            if (!tile_at(t, tn, tn, ti, tj) || ti < tj) continue;
             const int i0 = 16 * ti, j0 = 16 * tj;
             Z16 acc;
             z16_zero(acc);
-            z16_mma(acc, i0, j0, 0, min(n, i0 + 16),
-                    [&](int i, int k) { return (i < n && k <= i) ? M1[i + (size_t)k * ld] : zero; },
-                    [&](int k, int j) { return j < n ? M2[k + (size_t)j * ld] : zero; });
+            z16_gemm<false, false, false>(acc, i0, j0, 0, min(n, i0 + 16), M1, 1, ld, n, M2, 1, ld, n);
             z16_store(acc, i0, j0, [&](int i, int j, double2 x) {
                 if (i < n && j < n && i >= j) {
                     if (i == j) x.y = 0.0;
@@ -432,14 +612,13 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
     for (;;) {
         if (!code) {
             // ---- a5a: Householder tridiagonalisation of C (lower). Reflector
-            // k: I - tau_k v v^H on rows k+1.., v[k+1] = 1, v[k+2..] stored in
-            // column k of M0 below the subdiagonal. Small n: one rank-2
-            // update of the trailing matrix per column. Larger n: blocked as
-            // LAPACK's zhetrd/zlatrd, panels of up to 16 columns reduced
-            // against the panel-start trailing matrix A with the corrections
-            // of the panel's earlier columns (V = reflectors, W = their
-            // update vectors, W kept in M2 whose product T is dead by now),
-            // then A -= V W^H + W V^H on tensor-core tiles.
+            // k: I - tau_k v v^H on rows k+1.., v[k+1] = 1, stored in column k
+            // of M0 from row k+1 on. Blocked as LAPACK's zhetrd/zlatrd: panels
+            // of up to 16 columns reduced against the panel-start trailing
+            // matrix A with the corrections of the panel's earlier columns
+            // (V = reflectors, W = their update vectors, W kept in M2 whose
+            // product T is dead by now), then A -= V W^H + W V^H on
+            // tensor-core tiles. Only the lower triangle is read and written.
             if (use32) {
                 // Mixed form: the unblocked reduction in FP32 on a
                 // single-precision copy of C (reflectors kept in its columns;
@@ -524,266 +703,106 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
                     if (n == 1) v.tau[0] = zero;
                 }
                 __syncthreads();
-            } else if (n < kBlockedHetrdMinN) {
-                for (int k = 0; k < n - 1; ++k) {
-                    double2* ck = M0 + (size_t)k * ld;
-                    if (warp == 0) {
-                        double ss = 0.0;
-                        for (int i = k + 2 + lane; i < n; i += 32) { const double2 x = ck[i]; ss = fma(x.x, x.x, fma(x.y, x.y, ss)); }
-                        ss = warp_sum(ss);
-                        const double2 alpha = ck[k + 1];
-                        double2 taui, scal = zero;
-                        double beta;
-                        if (ss == 0.0 && alpha.y == 0.0) {
-                            taui = zero;
-                            beta = alpha.x;
-                        } else {
-                            beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + ss), alpha.x);
-                            const double rb = fast_rcp(beta);
-                            taui = c2((beta - alpha.x) * rb, -alpha.y * rb);
-                            const double2 z = c2(alpha.x - beta, alpha.y);
-                            const double inv = fast_rcp(z.x * z.x + z.y * z.y);
-                            scal = c2(z.x * inv, -z.y * inv);
-                        }
-                        for (int i = k + 2 + lane; i < n; i += 32) {
-                            const double2 vi = cmul(ck[i], scal);
-                            v.vb[i] = vi;
-                            ck[i] = vi;
-                        }
-                        if (lane == 0) {
-                            v.vb[k + 1] = c2(1.0, 0.0);
-                            v.tau[k] = taui;
-                            v.d[k] = ck[k].x;
-                            v.e[k] = beta;
-                        }
-                    }
-                    __syncthreads();
-                    const double2 taui = v.tau[k];
-                    if (taui.x == 0.0 && taui.y == 0.0) continue;
-                    // p = tau A22 v = tau sum_j v_j A(:, j) (A22 is kept as a full
-                    // Hermitian matrix): warp w takes the contiguous columns
-                    // j = k+1+w, +8, ..., lane l the rows k+1+l, +32, +64 (n < 96),
-                    // so each lane has a load per column in flight and no
-                    // shuffles; the 8 per-warp partials meet in shared memory (tb
-                    // and gb, contiguous, hold 768 >= 8 n entries) and warp 0 adds
-                    // them in a fixed order, then forms p^H v.
-                    double2* part = v.tb;
-                    {
-                        double2 acc[3] = {zero, zero, zero};
-    #pragma unroll 2
-                        for (int j = k + 1 + warp; j < n; j += kNW) {
-                            const double2* cj = M0 + (size_t)j * ld;
-                            const double2 vj = v.vb[j];
-    #pragma unroll
-                            for (int r = 0; r < 3; ++r) {
-                                const int i = k + 1 + lane + 32 * r;
-                                if (i < n) acc[r] = cfma(acc[r], cj[i], vj);
-                            }
-                        }
-    #pragma unroll
-                        for (int r = 0; r < 3; ++r) {
-                            const int i = k + 1 + lane + 32 * r;
-                            if (i < n) part[warp * n + i] = acc[r];
-                        }
-                    }
-                    __syncthreads();
-                    if (warp == 0) {
-                        double2 dot = zero;
-                        for (int i = k + 1 + lane; i < n; i += 32) {
-                            double2 sp = zero;
-    #pragma unroll
-                            for (int w = 0; w < kNW; ++w) sp = cadd(sp, part[w * n + i]);
-                            const double2 pi = cmul(taui, sp);
-                            v.pb[i] = pi;
-                            dot = cfmac(dot, pi, v.vb[i]);
-                        }
-                        dot = warp_sum2(dot);
-                        if (lane == 0) v.red[0] = cscale(cmul(taui, dot), -0.5);
-                    }
-                    __syncthreads();
-                    const double2 alpha2 = v.red[0];
-                    // A22 -= v w^H + w v^H, w = p + alpha2 v; a warp per column,
-                    // four columns per pass so that their loads are in flight together
-                    for (int j0 = k + 1 + warp; j0 < n; j0 += 4 * kNW) {
-                        double2 vj[4], wj[4];
-    #pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const int j = j0 + u * kNW;
-                            vj[u] = j < n ? v.vb[j] : zero;
-                            wj[u] = j < n ? cfma(v.pb[j], alpha2, vj[u]) : zero;
-                        }
-                        for (int i = k + 1 + lane; i < n; i += 32) {
-                            const double2 vi = v.vb[i], wi = cfma(v.pb[i], alpha2, vi);
-                            double2 x[4];
-    #pragma unroll
-                            for (int u = 0; u < 4; ++u) {
-                                const int j = j0 + u * kNW;
-                                x[u] = j < n ? M0[i + (size_t)j * ld] : zero;
-                            }
-    #pragma unroll
-                            for (int u = 0; u < 4; ++u) {
-                                const int j = j0 + u * kNW;
-                                if (j < n) M0[i + (size_t)j * ld] = cfms_bc(cfms_bc(x[u], vi, wj[u]), wi, vj[u]);
-                            }
-                        }
-                    }
-                    __syncthreads();
-                }
             } else {
+                // thread i owns row i of the vectors and of the panel (kNT >= n)
+                // V and W of the panel: columns Vp + c ld, Wp + c ld
                 double2* Wp = M2;
+                const int i = tid;
+                const bool row = i < n;
+                double* red = reinterpret_cast<double*>(v.red);   // 32 doubles for each of two sums
+                double2* t12 = v.tb;                               // W^H v at [0, c), V^H v at [16, 16 + c)
+                // (the divide and conquer's scratch is free until then: 2 n complex of its 7 n + 1 doubles)
+                double2* yx = reinterpret_cast<double2*>(v.dcd + (n & 1));
+                double2* const ydot[4] = {v.pb, v.gb, yx, yx + n};
                 for (int p = 0; p < n - 1; p += 16) {
                     const int w = min(16, n - 1 - p);
-                    // V(i, c) = v_{p+c}(i) for rows i > p + c
-                    auto Vp = [&](int i, int c) -> double2 {
-                        const int k = p + c;
-                        return (i <= k) ? zero : (i == k + 1) ? c2(1.0, 0.0) : M0[i + (size_t)k * ld];
-                    };
+                    double2* Vp = M0 + (size_t)p * ld;
                     for (int c = 0; c < w; ++c) {
                         const int k = p + c;
-                        double2* ck = M0 + (size_t)k * ld;
-                        // (1) a_k(k:n) -= V(k:n, 0:c) W(k, 0:c)^H + W(k:n, 0:c) V(k, 0:c)^H
-                        if (c > 0) {
-                            for (int i = k + tid; i < n; i += kNT) {
-                                double2 x = ck[i];
-                                for (int cc = 0; cc < c; ++cc) {
-                                    x = cfms_bc(x, Vp(i, cc), Wp[k + (size_t)cc * ld]);
-                                    x = cfms_bc(x, Wp[i + (size_t)cc * ld], Vp(k, cc));
-                                }
-                                ck[i] = x;
-                            }
-                            __syncthreads();
-                        }
-                        // (2) reflector from a_k(k+1:n), warp 0
-                        if (warp == 0) {
-                            double ss = 0.0;
-                            for (int i = k + 2 + lane; i < n; i += 32) { const double2 x = ck[i]; ss = fma(x.x, x.x, fma(x.y, x.y, ss)); }
-                            ss = warp_sum(ss);
-                            const double2 alpha = ck[k + 1];
-                            double2 taui, scal = zero;
-                            double beta;
-                            if (ss == 0.0 && alpha.y == 0.0) {
-                                taui = zero;
-                                beta = alpha.x;
-                            } else {
-                                beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + ss), alpha.x);
-                                const double rb = fast_rcp(beta);
-                                taui = c2((beta - alpha.x) * rb, -alpha.y * rb);
-                                const double2 z = c2(alpha.x - beta, alpha.y);
-                                const double inv = fast_rcp(z.x * z.x + z.y * z.y);
-                                scal = c2(z.x * inv, -z.y * inv);
-                            }
-                            for (int i = k + 2 + lane; i < n; i += 32) {
-                                const double2 vi = cmul(ck[i], scal);
-                                v.vb[i] = vi;
-                                ck[i] = vi;
-                            }
-                            if (lane == 0) {
-                                v.vb[k + 1] = c2(1.0, 0.0);
-                                v.tau[k] = taui;
-                                v.d[k] = ck[k].x;
-                                v.e[k] = beta;
-                            }
-                        }
-                        __syncthreads();
-                        const double2 taui = v.tau[k];
-                        // (3) y = A v (A: panel-start trailing matrix), t1 = W^H v and
-                        // t2 = V^H v over rows k+1..n. Up to kColMatvecMaxN, y is
-                        // formed column by column: warp w takes the contiguous
-                        // columns j = k+1+w, +8, ..., its lanes 4 rows each per
-                        // pass, so every lane keeps a load per row in flight and no
-                        // shuffles are needed; the 8 partials per row are added in
-                        // (4) in a fixed order. Above it, and for t1 / t2, one warp
-                        // per item reads down a column (y_i = sum_j conj(A(j, i)) v_j).
-                        const int m = n - k - 1;
-                        const bool colmv = n <= kColMatvecMaxN;
-                        if (colmv) {
-                            double2* part = v.part;
-                            for (int r0 = k + 1; r0 < n; r0 += 128) {
-                                double2 acc[4] = {zero, zero, zero, zero};
-    #pragma unroll 2
-                                for (int j = k + 1 + warp; j < n; j += kNW) {
-                                    const double2* cj = M0 + (size_t)j * ld;
-                                    const double2 vj = v.vb[j];
-    #pragma unroll
-                                    for (int u = 0; u < 4; ++u) {
-                                        const int i = r0 + lane + 32 * u;
-                                        if (i < n) acc[u] = cfma(acc[u], cj[i], vj);
-                                    }
-                                }
-    #pragma unroll
-                                for (int u = 0; u < 4; ++u) {
-                                    const int i = r0 + lane + 32 * u;
-                                    if (i < n) part[warp * n + i] = acc[u];
-                                }
-                            }
-                        }
-                        for (int it = (colmv ? m : 0) + warp; it < m + 2 * c; it += kNW) {
-                            double2 acc = zero;
-                            if (it < m) {
-                                const int i = k + 1 + it;
-                                const double2* ci = M0 + (size_t)i * ld;
-    #pragma unroll 4
-                                for (int j = k + 1 + lane; j < n; j += 32) acc = cfmac(acc, ci[j], v.vb[j]);
-                            } else if (it < m + c) {
-                                const double2* wc = Wp + (size_t)(it - m) * ld;
-                                for (int j = k + 1 + lane; j < n; j += 32) acc = cfmac(acc, wc[j], v.vb[j]);
-                            } else {
-                                const int cc = it - m - c;
-                                for (int j = k + 1 + lane; j < n; j += 32) acc = cfmac(acc, Vp(j, cc), v.vb[j]);
-                            }
-                            acc = warp_sum2(acc);
-                            if (lane == 0) {
-                                if (it < m) v.pb[k + 1 + it] = acc;
-                                else v.red[it - m] = acc;      // t1 at red[0..c), t2 at red[c..2c)
-                            }
-                        }
-                        __syncthreads();
-                        // (4) w = tau (y - V t1 - W t2) on rows k+1..n: the
-                        // current trailing matrix is A - V W^H - W V^H
-                        for (int i = k + 1 + tid; i < n; i += kNT) {
-                            double2 x = v.pb[i];
-                            if (colmv) {
-                                x = zero;
-    #pragma unroll
-                                for (int w = 0; w < kNW; ++w) x = cadd(x, v.part[w * n + i]);
-                            }
+                        // (1) column k of the current matrix:
+                        // a_k -= V(:, 0:c) W(k, 0:c)^H + W(:, 0:c) V(k, 0:c)^H
+                        // (rows k .. n-1 of V are stored whole)
+                        double2 x = zero;
+                        if (row && i >= k) {
+                            x = M0[i + (size_t)k * ld];
+#pragma unroll 4
                             for (int cc = 0; cc < c; ++cc) {
-                                x = cfms(x, Vp(i, cc), v.red[cc]);
-                                x = cfms(x, Wp[i + (size_t)cc * ld], v.red[c + cc]);
+                                x = cfms_bc(x, Vp[i + cc * ld], Wp[k + cc * ld]);
+                                x = cfms_bc(x, Wp[i + cc * ld], Vp[k + cc * ld]);
                             }
-                            v.pb[i] = cmul(taui, x);
+                        }
+                        if (i == k) { v.d[k] = x.x; M0[k + (size_t)k * ld] = x; }
+                        if (i == k + 1) v.gb[0] = x;
+                        // (2) reflector from a_k(k+1:n)
+                        const double ss = cta_sum<kNT>((row && i > k + 1) ? fma(x.x, x.x, x.y * x.y) : 0.0, red);
+                        const double2 alpha = v.gb[0];
+                        double2 taui = zero, scal = zero;
+                        double beta = alpha.x;
+                        if (!(ss == 0.0 && alpha.y == 0.0)) {
+                            const double nn = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, ss));
+                            const double rn = rsqrt(nn);
+                            beta = -copysign(nn * rn, alpha.x);
+                            const double rb = -copysign(rn, alpha.x);
+                            taui = c2((beta - alpha.x) * rb, -alpha.y * rb);
+                            const double2 z = c2(alpha.x - beta, alpha.y);
+                            const double inv = fast_rcp(fma(z.x, z.x, z.y * z.y));
+                            scal = c2(z.x * inv, -z.y * inv);
+                        }
+                        double2 vi = zero;
+                        if (row && i > k) {
+                            vi = i == k + 1 ? c2(1.0, 0.0) : cmul(x, scal);
+                            v.vb[i] = vi;
+                            M0[i + (size_t)k * ld] = vi;
+                        }
+                        if (tid == 0) { v.tau[k] = taui; v.e[k] = beta; }
+                        __syncthreads();
+                        // (3) y = A v (A: panel-start trailing matrix, lower
+                        // triangle), t1 = W^H v, t2 = V^H v
+                        sym_matvec<kNT>(M0, ld, n, k + 1, v.vb, v.part, ydot, v.ring);
+                        for (int it = warp; it < 2 * c; it += kNW) {
+                            const int cc = it >> 1;
+                            double2 acc = zero;
+                            const double2* col = (it & 1 ? Vp : Wp) + cc * ld;
+#pragma unroll 4
+                            for (int j = k + 1 + lane; j < n; j += 32) acc = cfmac(acc, col[j], v.vb[j]);
+                            acc = warp_sum2(acc);
+                            if (lane == 0) t12[16 * (it & 1) + cc] = acc;
                         }
                         __syncthreads();
-                        // (5) alpha2 = -tau/2 (w^H v)
-                        if (warp == 0) {
-                            double2 dot = zero;
-                            for (int i = k + 1 + lane; i < n; i += 32) dot = cfmac(dot, v.pb[i], v.vb[i]);
-                            dot = warp_sum2(dot);
-                            if (lane == 0) v.gb[0] = cscale(cmul(taui, dot), -0.5);
+                        // (4) w = tau (y - V t1 - W t2) + alpha2 v on rows k+1..n (the
+                        // current matrix is A - V W^H - W V^H), alpha2 =
+                        // -tau/2 (w^H v) = -|tau|^2/2 v^H A v; zero above
+                        double2 y = zero;
+                        if (row && i > k) {
+                            y = sym_matvec_row<kNT>(n, k + 1, i, v.part, ydot);
+#pragma unroll 4
+                            for (int cc = 0; cc < c; ++cc) {
+                                y = cfms(y, Vp[i + cc * ld], t12[cc]);
+                                y = cfms(y, Wp[i + cc * ld], t12[16 + cc]);
+                            }
                         }
-                        __syncthreads();
-                        // (6) W(:, c) = w + alpha2 v on rows k+1..n, zero above
-                        const double2 alpha2 = v.gb[0];
-                        for (int i = tid; i < n; i += kNT)
-                            Wp[i + (size_t)c * ld] = (i > k) ? cfma(v.pb[i], alpha2, v.vb[i]) : zero;
+                        const double h = -0.5 * fma(taui.x, taui.x, taui.y * taui.y) *
+                                         cta_sum<kNT>(fma(y.x, vi.x, y.y * vi.y), red + 32);
+                        if (row) {
+                            const double2 wt = cmul(taui, y);
+                            Wp[i + c * ld] = c2(fma(h, vi.x, wt.x), fma(h, vi.y, wt.y));
+                        }
                         __syncthreads();
                     }
-                    // trailing update A(q:n, q:n) -= V W^H + W V^H, q = p + w (all tiles)
+                    // trailing update, lower tiles: A(q:n, q:n) -= V W^H + W V^H, q = p + w
                     const int q = p + w, mq = n - q;
                     if (mq > 0) {
                         const int tq = (mq + 15) >> 4;
-                        for (int t = warp; t < tq * tq; t += kNW) {
-                            const int ti = t / tq, tj = t - ti * tq, i0 = q + 16 * ti, j0 = q + 16 * tj;
+                        for (int t = warp; t < tile_blocks(tq, tq); t += kNW) {
+                            int ti, tj;
+                            if (!tile_at(t, tq, tq, ti, tj) || ti < tj) continue;
+                            const int i0 = q + 16 * ti, j0 = q + 16 * tj;
                             Z16 acc;
-                            z16_load(acc, i0, j0, [&](int i, int j) { return (i < n && j < n) ? M0[i + (size_t)j * ld] : zero; });
-                            z16_mma(acc, i0, j0, 0, w,
-                                    [&](int i, int cc) { return i < n ? cneg(Vp(i, cc)) : zero; },
-                                    [&](int cc, int j) { return j < n ? cconj(Wp[j + (size_t)cc * ld]) : zero; });
-                            z16_mma(acc, i0, j0, 0, w,
-                                    [&](int i, int cc) { return i < n ? cneg(Wp[i + (size_t)cc * ld]) : zero; },
-                                    [&](int cc, int j) { return j < n ? cconj(Vp(j, cc)) : zero; });
-                            z16_store(acc, i0, j0, [&](int i, int j, double2 x) {
-                                if (i < n && j < n) M0[i + (size_t)j * ld] = x;
+                            z16_load(acc, i0, j0, [&](int r, int j) { return (r < n && j < n) ? M0[r + (size_t)j * ld] : zero; });
+                            z16_gemm<false, true, true>(acc, i0, j0, 0, w, Vp, 1, ld, n, Wp, ld, 1, n);
+                            z16_gemm<false, true, true>(acc, i0, j0, 0, w, Wp, 1, ld, n, Vp, ld, 1, n);
+                            z16_store(acc, i0, j0, [&](int r, int j, double2 x) {
+                                if (r < n && j < n && r >= j) M0[r + (size_t)j * ld] = x;
                             });
                         }
                     }
@@ -803,12 +822,12 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
             dc.Z = reinterpret_cast<double*>(M2); dc.ldz = ld;
             dc.U = dc.Z + mat;                    dc.ldu = ld;
             dc.Zo = Zo;
-            // tb, gb and the partial vectors are free here
-            dc.leaf = reinterpret_cast<double*>(v.tb);
-            dc.leaf_lanes = (int)((768 + tiled_part_elems(n)) * 2 / (kLeafStride * kLeaf)) * kLeaf;
+            // the work area is free here, else tb and gb are
+            dc.leaf = reinterpret_cast<double*>(a.work ? v.part : v.tb);
+            dc.leaf_lanes = (int)((a.work ? tiled_work_elems(n) : 768) * 2 / (kLeafStride * kLeaf)) * kLeaf;
             dc.d = v.d; dc.ds = 1; dc.e = v.e; dc.es = 1;
             dc_carve(dc, v.dcd, v.dci, n);
-            tiled_dc(n, dc);
+            tiled_dc<kNT>(n, dc);
             // a failed eigensolve shows as a non-finite value (every warp looks
             // at all of them: the verdict is uniform without a barrier)
             bool bad = false;
@@ -841,7 +860,7 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
                 return (i <= k) ? zero : (i == k + 1) ? c2(1.0, 0.0)
                      : use32 ? f2d(C32[i + (size_t)k * ld]) : M0[i + (size_t)k * ld];
             };
-            v.tb[tid] = zero;   // kNT == 256 == 16 x 16
+            if (tid < 256) v.tb[tid] = zero;
             // G = Y^H Y: warps 0 and 1 each sum half of the rows, and the two
             // halves are added in a fixed order (results are bitwise
             // reproducible from launch to launch)
@@ -856,7 +875,7 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
                 z16_store(acc, 0, 0, [&](int i, int j, double2 x) { v.gb[256 * warp + i + 16 * j] = x; });
             }
             __syncthreads();
-            v.gb[tid] = cadd(v.gb[tid], v.gb[256 + tid]);
+            if (tid < 256) v.gb[tid] = cadd(v.gb[tid], v.gb[256 + tid]);
             __syncthreads();
             // T_b (upper triangular, forward column-wise): T(j, j) = tau_j,
             // T(0:j, j) = T(0:j, 0:j) (-tau_j G(0:j, j))
@@ -880,8 +899,17 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
                 const int j0 = 16 * t;
                 Z16 acc;
                 z16_zero(acc);
-                z16_mma(acc, 0, j0, kb + 1, n, [&](int c, int i) { return cconj(Y(i, c)); },
-                        [&](int i, int j) { return j < n ? Ub[i + (size_t)j * n] : zero; });
+                if (use32) {
+                    z16_mma(acc, 0, j0, kb + 1, n, [&](int c, int i) { return cconj(Y(i, c)); },
+                            [&](int i, int j) { return j < n ? Ub[i + (size_t)j * n] : zero; });
+                } else {
+                    // the triangle of Y's first rows, then its full columns
+                    const int kt = min(n, kb + 17);
+                    z16_mma(acc, 0, j0, kb + 1, kt, [&](int c, int i) { return cconj(Y(i, c)); },
+                            [&](int i, int j) { return j < n ? Ub[i + (size_t)j * n] : zero; });
+                    if (kt < n)
+                        z16_gemm<true, false, false>(acc, 0, j0, kt, n, M0 + (size_t)kb * ld, ld, 1, w, Ub, 1, n, n);
+                }
                 z16_store(acc, 0, j0, [&](int c, int j, double2 x) { if (j < n) Wsc[c + 16 * j] = x; });
                 __syncwarp();
                 Z16 acc2;
@@ -898,8 +926,11 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
                 const int ti = rt0 + t / tn, tj = t % tn, i0 = 16 * ti, j0 = 16 * tj;
                 Z16 acc;
                 z16_load(acc, i0, j0, [&](int i, int j) { return (i < n && j < n) ? Ub[i + (size_t)j * n] : zero; });
-                z16_mma(acc, i0, j0, 0, 16, [&](int i, int c) { return cneg(Y(i, c)); },
-                        [&](int c, int j) { return j < n ? Wsc[c + 16 * j] : zero; });
+                if (use32 || i0 <= kb + 16)
+                    z16_mma(acc, i0, j0, 0, 16, [&](int i, int c) { return cneg(Y(i, c)); },
+                            [&](int c, int j) { return j < n ? Wsc[c + 16 * j] : zero; });
+                else
+                    z16_gemm<false, true, false>(acc, i0, j0, 0, w, M0 + (size_t)kb * ld, 1, ld, n, Wsc, 1, 16, n);
                 z16_store(acc, i0, j0, [&](int i, int j, double2 x) {
                     if (i < n && j < n) Ub[i + (size_t)j * n] = x;
                 });
@@ -930,8 +961,7 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
                         int ti, tj;
                         tri_tile(t, ti, tj);
                         const int i0 = 16 * ti, j0 = 16 * tj;
-                        z16_mma(acc, i0, j0, 0, n, [&](int i, int k) { return i < n ? cconj(Vh[k + (size_t)i * ldh]) : zero; },
-                                [&](int k, int j) { return j < n ? Vh[k + (size_t)j * ldh] : zero; });
+                        z16_gemm<true, false, false>(acc, i0, j0, 0, n, Vh, ldh, 1, n, Vh, 1, ldh, n);
                         z16_store(acc, i0, j0, [&](int i, int j, double2 x) {
                             if (i < n && j < n && i >= j) {
                                 x = c2((i == j ? 1.0 : 0.0) - x.x, i == j ? 0.0 : -x.y);
@@ -941,8 +971,7 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
                         });
                     } else {
                         const int t2 = t - tl, ti = t2 / tn, tj = t2 - ti * tn, i0 = 16 * ti, j0 = 16 * tj;
-                        z16_mma(acc, i0, j0, 0, n, [&](int i, int k) { return i < n ? M0[i + (size_t)k * ld] : zero; },
-                                [&](int k, int j) { return j < n ? Vh[k + (size_t)j * ldh] : zero; });
+                        z16_gemm<false, false, false>(acc, i0, j0, 0, n, M0, 1, ld, n, Vh, 1, ldh, n);
                         z16_store(acc, i0, j0, [&](int i, int j, double2 x) { if (i < n && j < n) Vn[i + (size_t)j * ldn] = x; });
                     }
                 }
@@ -953,8 +982,7 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
                     const int i0 = 16 * ti, j0 = 16 * tj;
                     Z16 acc;
                     z16_zero(acc);
-                    z16_mma(acc, i0, j0, 0, n, [&](int i, int k) { return i < n ? cconj(Vh[k + (size_t)i * ldh]) : zero; },
-                            [&](int k, int j) { return j < n ? Vn[k + (size_t)j * ldn] : zero; });
+                    z16_gemm<true, false, false>(acc, i0, j0, 0, n, Vh, ldh, 1, n, Vn, 1, ldn, n);
                     z16_store(acc, i0, j0, [&](int i, int j, double2 x) {
                         if (i < n && j < n && i >= j) {
                             if (i == j) x.y = 0.0;
@@ -1011,8 +1039,7 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
                     const int ti = t / tn, tj = t - ti * tn, i0 = 16 * ti, j0 = 16 * tj;
                     Z16 acc;
                     z16_load(acc, i0, j0, [&](int i, int j) { return (i < n && j < n) ? Vh[i + (size_t)j * ldh] : zero; });
-                    z16_mma(acc, i0, j0, 0, n, [&](int i, int k) { return i < n ? Vh[i + (size_t)k * ldh] : zero; },
-                            [&](int k, int j) { return j < n ? M2[k + (size_t)j * ld] : zero; });
+                    z16_gemm<false, false, false>(acc, i0, j0, 0, n, Vh, 1, ldh, n, M2, 1, ld, n);
                     z16_store(acc, i0, j0, [&](int i, int j, double2 x) { if (i < n && j < n) Vn[i + (size_t)j * ldn] = x; });
                 }
                 __syncthreads();
@@ -1077,13 +1104,13 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
     if (a.stage == 3) return;
 
     // ---- a6: U = X^H V -> M2, U(i, j) = sum_{k >= i} conj(X(k, i)) V(k, j); then to the output
-    for (int t = warp; t < tn * tn; t += kNW) {
-        const int ti = t / tn, tj = t - ti * tn, i0 = 16 * ti, j0 = 16 * tj;
+    for (int t = warp; t < tile_blocks(tn, tn); t += kNW) {
+        int ti, tj;
+        if (!tile_at(t, tn, tn, ti, tj)) continue;
+        const int i0 = 16 * ti, j0 = 16 * tj;
         Z16 acc;
         z16_zero(acc);
-        z16_mma(acc, i0, j0, i0, n,
-                [&](int i, int k) { return (i < n && k >= i) ? cconj(M1[k + (size_t)i * ld]) : zero; },
-                [&](int k, int j) { return j < n ? Ub[k + (size_t)j * n] : zero; });
+        z16_gemm<true, false, false>(acc, i0, j0, i0, n, M1, ld, 1, n, Ub, 1, n, n);
         z16_store(acc, i0, j0, [&](int i, int j, double2 x) { if (i < n && j < n) M2[i + (size_t)j * ld] = x; });
     }
     __syncthreads();

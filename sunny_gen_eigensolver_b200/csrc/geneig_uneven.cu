@@ -1,5 +1,6 @@
-// Persistent kernel for batches of pencils of uneven sizes (one launch for
-// the whole mix, but for the sizes whose pencils take a whole SM). The host groups the problems by size N (up to kMaxGroups
+// Batches of pencils of uneven sizes: a persistent kernel for the sizes several
+// of whose pencils fit an SM (one launch for all of them), beside the own
+// kernels of the larger sizes. The host groups the problems by size N (up to kMaxGroups
 // sizes, each group batch-contiguous in its own buffers, the layouts of
 // sunny_geneig_launch) and orders the groups by descending N. The groups are
 // cut into work items: one pencil for sizes in the l2-slot regime, `per_item`
@@ -83,8 +84,8 @@ __global__ void __launch_bounds__(kNT, 2) geneig_uneven_kernel(UnevenArgs a) {
             tiled::TiledArgs t;
             t.H = G.H; t.S = G.S; t.W = G.W; t.U = G.U; t.info = G.info;
             t.scratch = a.scratch; t.batch = G.count;
-            t.n = G.n; t.ld = G.n | 1; t.stage = 4; t.sigma = 0; t.mixed = 0; t.refine_max = 0;
-            for (long long b = b0; b < b1; ++b) tiled::tiled_solve(t, b, slot, smem_raw);
+            t.n = G.n; t.ld = G.n | 1; t.stage = 4; t.sigma = 0; t.mixed = 0; t.refine_max = 0; t.defer = 0; t.work = 1;
+            for (long long b = b0; b < b1; ++b) tiled::tiled_solve<kNT>(t, b, slot, smem_raw);
         } else {
             cta::CtaArgs c;
             c.H = G.H; c.S = G.S; c.W = G.W; c.U = G.U; c.info = G.info;
@@ -113,12 +114,12 @@ cudaError_t uneven_set_attributes(size_t smem) {
 }
 
 int uneven_kind(int n, bool l2slot) {
-    if (l2slot) return n > kCtaPreferredMaxN && n <= kResidentMaxN ? kUnevenResident : 5;
+    if (l2slot) return n <= kCtaPreferredMaxN ? 5 : n <= kResidentMaxN ? kUnevenResident : kUnevenBig;
     return n <= 16 ? 0 : n <= 32 ? 1 : n <= 48 ? 2 : n <= 56 ? 3 : 4;
 }
 
 size_t uneven_smem_bytes(int n, int kind) {
-    return kind == kUnevenResident ? 0
+    return kind >= kUnevenResident ? 0
          : kind == 5 ? tiled_vec_bytes(n)
                      : kind_teams(kind) * cta_smem_bytes(n);
 }
@@ -128,10 +129,10 @@ cudaError_t uneven_launch(const UnevenLaunch& L, unsigned long long* head, void*
     UnevenArgs a{};
     long long first = 0;
     int ng = 0;
-    bool resident = false;
+    int nside = 0;
     for (int i = 0; i < L.ngroups; ++i) {
         if (L.count[i] <= 0) continue;
-        if (L.kind[i] == kUnevenResident) { resident = true; continue; }
+        if (L.kind[i] >= kUnevenResident) { ++nside; continue; }
         UnevenGroup& G = a.g[ng++];
         G.H = static_cast<const double2*>(L.H[i]);
         G.S = static_cast<const double2*>(L.S[i]);
@@ -146,16 +147,25 @@ cudaError_t uneven_launch(const UnevenLaunch& L, unsigned long long* head, void*
         G.first_item = first;
         first += (G.count + G.per_item - 1) / G.per_item;
     }
-    // the persistent kernel first: its long items start at once, and the
-    // resident sizes fill the SMs that its CTAs leave
-    const bool both = resident && ng > 0;
-    cudaError_t e = cudaSuccess;
-    if (both) {
-        e = cudaEventRecord(side.fork, stream);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(side.stream, side.fork, 0);
+    // The side sizes first, largest first (the groups' order): their pencils
+    // take longest, and the persistent kernel's small ones fill the SMs that
+    // they leave.
+    const bool fork = nside + (ng > 0 ? 1 : 0) > 1;
+    cudaError_t e = fork ? cudaEventRecord(side.fork, stream) : cudaSuccess;
+    for (int i = 0, s = 0; i < L.ngroups; ++i) {
+        if (L.count[i] <= 0 || L.kind[i] < kUnevenResident) continue;
+        const cudaStream_t st = fork ? side.stream[s] : stream;
+        if (e == cudaSuccess && fork) e = cudaStreamWaitEvent(st, side.fork, 0);
         if (e != cudaSuccess) return e;
+        if (L.kind[i] == kUnevenResident)
+            e = cta_launch(L.n[i], cta_nmax_for(L.n[i]), 4, L.H[i], L.S[i], L.W[i], L.U[i], L.info[i], L.count[i], st);
+        else
+            e = tiled_launch(L.n[i], L.slots[i], 4, L.H[i], L.S[i], L.W[i], L.U[i], L.info[i],
+                             L.count[i], L.scratch[i], st, false);
+        if (e == cudaSuccess && fork) e = cudaEventRecord(side.join[s], st);
+        ++s;
     }
-    if (ng > 0) {
+    if (e == cudaSuccess && ng > 0) {
         a.ngroups = ng;
         a.nitems = first;
         a.head = head;
@@ -166,18 +176,8 @@ cudaError_t uneven_launch(const UnevenLaunch& L, unsigned long long* head, void*
         const long long g = first < grid ? first : grid;
         geneig_uneven_kernel<<<(unsigned)g, kNT, smem, stream>>>(a);
         e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
     }
-    const cudaStream_t st = both ? side.stream : stream;
-    for (int i = 0; i < L.ngroups && resident; ++i) {
-        if (L.count[i] <= 0 || L.kind[i] != kUnevenResident) continue;
-        e = cta_launch(L.n[i], cta_nmax_for(L.n[i]), 4, L.H[i], L.S[i], L.W[i], L.U[i], L.info[i], L.count[i], st);
-        if (e != cudaSuccess) return e;
-    }
-    if (both) {
-        e = cudaEventRecord(side.join, side.stream);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, side.join, 0);
-    }
+    for (int s = 0; fork && s < nside && e == cudaSuccess; ++s) e = cudaStreamWaitEvent(stream, side.join[s], 0);
     return e;
 }
 
