@@ -804,6 +804,7 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
                     Ub[i + (size_t)k * n] = i == k + 1 ? c2(1.0, 0.0) : M[i + k * ld];
         }
         team_sync<NT, BLOCK>();
+        phase_mark(9);
         // ---- a5b: divide and conquer; Z (real) and its workspace in M
         tridiag_dc<NT, NMAX, BLOCK, SPEC>(n, dc);
         // a failed eigensolve shows as a non-finite value (every warp looks at

@@ -112,36 +112,42 @@ __host__ __device__ __forceinline__ double lanes_prod(double v, unsigned mask) {
 }
 
 // Root i (0-based) of 1 + rho sum_j zz_j^2 / (dl_j - x) = 0 with dl ascending,
-// rho > 0, computed by P lanes together (lane qq sums the terms j = qq mod P).
-// Returns the offset tau of the root from pole `org`; the return value is the
-// number of iterations taken.
+// rho > 0, sum zz_j^2 <= 1 to rounding, computed by P lanes together (lane qq
+// sums the terms j = qq mod P). Returns the offset tau of the root from pole
+// `org`; the return value is the number of iterations taken.
+// The last root (no pole to its right, bracket rho long) takes the same path
+// with that pole's weight zero. Every sum runs over all poles with the left
+// ones' share picked by a select, so the lanes of a warp, which hold different
+// roots, do not diverge (N=54, one pencil on an SM, the three levels: 47.9 K
+// cycles, 64.0 K with two loops that meet at pole i).
 template <int P>
 __host__ __device__ inline int secular_root_p(int i, int K, const double* dl, const double* zz, double rho,
                                               int qq, unsigned mask, double& tau_out, int& org_out) {
     if (K == 1) { org_out = 0; tau_out = rho * zz[0] * zz[0]; return 0; }
-    int o;
-    double lo, hi, tau;
-    if (i < K - 1) {
-        const double gap = dl[i + 1] - dl[i];
-        const double mid = 0.5 * gap;
-        double gs = 0.0;
+    const bool right = i < K - 1;
+    const int ir = right ? i + 1 : i;
+    const double di = dl[i], gap = dl[ir] - di;
+    const double mid = 0.5 * (right ? gap : rho * (1.0 + 1e-10));
+    double gs = 0.0;
 #pragma unroll 2
-        for (int j = qq; j < K; j += P) {
-            const double del = (dl[j] - dl[i]) - mid;
-            gs = fma(rho * zz[j], zz[j] * fast_rcp(del), gs);
-        }
-        const double g = 1.0 + lanes_sum<P>(gs, mask);
-        if (g >= 0.0) { o = i;     lo = 0.0;  hi = mid; tau = mid; }
-        else          { o = i + 1; lo = -mid; hi = 0.0; tau = -mid; }
+    for (int j = qq; j < K; j += P) {
+        const double zj = zz[j];
+        gs = fma(zj, zj * fast_rcp((dl[j] - di) - mid), gs);
+    }
+    const double gm = fma(rho, lanes_sum<P>(gs, mask), 1.0);
+    const bool low = !right || gm >= 0.0;
+    const int o = low ? i : ir;
+    double lo = low ? 0.0 : -mid, hi = low ? (right ? mid : 2.0 * mid) : 0.0, tau = low ? hi : lo;
+    const double dlo = dl[o];
+    const double p = di - dlo, q = dl[ir] - dlo;       // one of them is 0
+    {
         // Starting point: the two nearest poles' terms exactly, the others
         // frozen at their midpoint value c (the fixed-weight start), i.e. the
         // root of c + a/(p - x) + b/(q - x) in origin coordinates, taken when
-        // it lies inside the bracket (otherwise the midpoint stays).
-        const double a = rho * zz[i] * zz[i], b = rho * zz[i + 1] * zz[i + 1];
-        const double rm = fast_rcp(mid);
-        const double c = g + (a - b) * rm;
-        const double p0 = dl[i] - dl[o], q0 = dl[i + 1] - dl[o];
-        const double B = -(c * (p0 + q0) + a + b), C = a * q0 + b * p0;
+        // it lies inside the bracket (otherwise the bracket's end stays).
+        const double a = rho * zz[i] * zz[i], b = right ? rho * zz[ir] * zz[ir] : 0.0;
+        const double c = fma(a - b, fast_rcp(mid), gm);
+        const double B = -(c * (p + q) + a + b), C = a * q + b * p;
         if (c != 0.0) {
             double disc = B * B - 4.0 * c * C;
             if (disc < 0.0) disc = 0.0;
@@ -150,88 +156,50 @@ __host__ __device__ inline int secular_root_p(int i, int K, const double* dl, co
             if (x1 > lo && x1 < hi) tau = x1;
             else if (x2 > lo && x2 < hi) tau = x2;
         }
-    } else {
-        double ss = 0.0;
-        for (int j = qq; j < K; j += P) ss += zz[j] * zz[j];
-        o = K - 1; lo = 0.0; hi = rho * lanes_sum<P>(ss, mask); tau = hi;
-        // Starting point: the last pole's term exactly, the others frozen at
-        // the bracket's midpoint m (c = f(m) - b / (-m)): the root of
-        // c + b / (-x) = 0, x = b / c, when it lies inside the bracket.
-        const double m = 0.5 * hi;
-        if (m > 0.0) {
-            double gs = 0.0;
-#pragma unroll 2
-            for (int j = qq; j < K; j += P) {
-                const double del = (dl[j] - dl[K - 1]) - m;
-                gs = fma(rho * zz[j], zz[j] * fast_rcp(del), gs);
-            }
-            const double b = rho * zz[K - 1] * zz[K - 1];
-            const double c = 1.0 + lanes_sum<P>(gs, mask) + b * fast_rcp(m);
-            if (c > 0.0) {
-                const double x = b * fast_rcp(c);
-                if (x > lo && x < hi) tau = x;
-            }
-        }
     }
-    const double dlo = dl[o];
-    const double p = dl[i] - dlo;
-    const double q = (i < K - 1) ? dl[i + 1] - dlo : 0.0;
     int it = 0;
     for (; it < 80; ++it) {
-        // poles up to i (left of the root) give psi <= 0, the others phi >= 0
-        double psi = 0.0, dpsi = 0.0, phi = 0.0, dphi = 0.0;
-        int j = qq;
+        // sums over all poles, and over those up to i (left of the root)
+        double tot = 0.0, dtot = 0.0, psi = 0.0, dpsi = 0.0;
 #pragma unroll 2
-        for (; j <= i; j += P) {
+        for (int j = qq; j < K; j += P) {
             const double zj = zz[j];
             const double t = zj * fast_rcp((dl[j] - dlo) - tau);
-            psi = fma(zj, t, psi);
-            dpsi = fma(t, t, dpsi);
+            const double tl = j <= i ? t : 0.0;
+            tot = fma(zj, t, tot);
+            dtot = fma(t, t, dtot);
+            psi = fma(zj, tl, psi);
+            dpsi = fma(tl, tl, dpsi);
         }
-#pragma unroll 2
-        for (; j < K; j += P) {
-            const double zj = zz[j];
-            const double t = zj * fast_rcp((dl[j] - dlo) - tau);
-            phi = fma(zj, t, phi);
-            dphi = fma(t, t, dphi);
-        }
+        tot = rho * lanes_sum<P>(tot, mask);
+        dtot = rho * lanes_sum<P>(dtot, mask);
         psi = rho * lanes_sum<P>(psi, mask);
         dpsi = rho * lanes_sum<P>(dpsi, mask);
-        phi = rho * lanes_sum<P>(phi, mask);
-        dphi = rho * lanes_sum<P>(dphi, mask);
-        const double erra = fabs(psi) + fabs(phi);
-        const double g = 1.0 + psi + phi;
-        const double err = kEps * (2.0 + 8.0 * erra + 3.0 * fabs(tau) * (dpsi + dphi));
+        const double phi = tot - psi, dphi = dtot - dpsi;      // psi <= 0 <= phi
+        const double g = 1.0 + tot;
+        const double err = kEps * (2.0 + 8.0 * (phi - psi) + 3.0 * fabs(tau) * dtot);
         if (fabs(g) <= err) break;
         if (g < 0.0) lo = tau; else hi = tau;
         if (hi - lo <= 2.0 * kEps * fmax(fabs(lo), fabs(hi))) break;
+        const double bpsi = dpsi * (p - tau) * (p - tau);
+        const double apsi = psi - dpsi * (p - tau);
+        const double bphi = right ? dphi * (q - tau) * (q - tau) : 0.0;
+        const double aphi = right ? phi - dphi * (q - tau) : 0.0;
+        const double c = 1.0 + apsi + aphi;
+        // c + bpsi/(p - x) + bphi/(q - x) = 0 in origin coordinates
+        // (one of p, q is 0, so p q = 0):
+        //   c x^2 - (c (p + q) + bpsi + bphi) x + (bpsi q + bphi p) = 0
+        const double B = -(c * (p + q) + bpsi + bphi);
+        const double C = bpsi * q + bphi * p;
         double tn;
-        if (i < K - 1) {
-            const double bpsi = dpsi * (p - tau) * (p - tau);
-            const double apsi = psi - dpsi * (p - tau);
-            const double bphi = dphi * (q - tau) * (q - tau);
-            const double aphi = phi - dphi * (q - tau);
-            const double c = 1.0 + apsi + aphi;
-            // c + bpsi/(p - x) + bphi/(q - x) = 0 in origin coordinates
-            // (one of p, q is 0, so p q = 0):
-            //   c x^2 - (c (p + q) + bpsi + bphi) x + (bpsi q + bphi p) = 0
-            const double B = -(c * (p + q) + bpsi + bphi);
-            const double C = bpsi * q + bphi * p;
-            tn = lo - 1.0;
-            if (c == 0.0) {
-                tn = -C * fast_rcp(B);
-            } else {
-                double disc = B * B - 4.0 * c * C;
-                if (disc < 0.0) disc = 0.0;
-                const double qq2 = -0.5 * (B + copysign(sqrt(disc), B));
-                const double x1 = qq2 * fast_rcp(c), x2 = (qq2 != 0.0) ? C * fast_rcp(qq2) : x1;
-                tn = (x1 > lo && x1 < hi) ? x1 : x2;
-            }
+        if (c == 0.0) {
+            tn = -C * fast_rcp(B);
         } else {
-            const double bpsi = dpsi * (p - tau) * (p - tau);
-            const double apsi = psi - dpsi * (p - tau);
-            const double den = 1.0 + apsi;
-            tn = (den > 0.0) ? p + bpsi * fast_rcp(den) : lo - 1.0;
+            double disc = B * B - 4.0 * c * C;
+            if (disc < 0.0) disc = 0.0;
+            const double qq2 = -0.5 * (B + copysign(sqrt(disc), B));
+            const double x1 = qq2 * fast_rcp(c), x2 = (qq2 != 0.0) ? C * fast_rcp(qq2) : x1;
+            tn = (x1 > lo && x1 < hi) ? x1 : x2;
         }
         // converged when the model step is within a few ulps of the iterate
         // (it may then round just outside the bracket)
@@ -410,45 +378,57 @@ __device__ __forceinline__ void dc_merge_tiled(int n, int half, int span, const 
 // lane of the leaf's group runs the same recurrence on the same data. Returns
 // false when it did not converge (non-finite input).
 __device__ __forceinline__ bool leaf_ql(int m, double* d, double* e, double* z) {
+    unsigned small = ~0u << (m - 1);                           // bit i: e[i] is negligible
+#pragma unroll 1
+    for (int i = 0; i < m - 1; ++i)
+        if (fabs(e[i]) <= kEps * (fabs(d[i]) + fabs(d[i + 1]))) small |= 1u << i;
 #pragma unroll 1
     for (int it = 0; it < 30 * kLeaf; ++it) {
-        unsigned small = ~0u << (m - 1);
-#pragma unroll 1
-        for (int i = 0; i < m - 1; ++i)
-            if (fabs(e[i]) <= kEps * (fabs(d[i]) + fabs(d[i + 1]))) small |= 1u << i;
         if (small == ~0u) return true;
         const int l = __ffs(~small) - 1;                       // first off-diagonal left
         const int top = l + __ffs(small >> l) - 1;             // its block is [l, top]
         const double dl = d[l], el = e[l];
         const double hd = 0.5 * (d[l + 1] - dl);
-        const double qs = hd + copysign(sqrt(fma(hd, hd, el * el)), hd);
-        double dnext = d[top];
+        double dnext = d[top], znext = z[top];
+        const double h2 = fma(hd, hd, el * el);
+        const double qs = hd + copysign(h2 > 0.0 ? h2 * rsqrt(h2) : 0.0, hd);
         double g = dnext - dl + (qs != 0.0 ? el * el * fast_rcp(qs) : 0.0);
-        double s = 1.0, c = 1.0, p = 0.0;
+        double s = 1.0, c = 1.0, p = 0.0, dabove = 0.0;        // |d| above the last rotation
         int i = top - 1;
-        double znext = z[top];
 #pragma unroll 1
         for (; i >= l; --i) {
             const double ei = e[i], di = d[i], zi = z[i];
             const double f = s * ei, b = c * ei;
             const double q = fma(f, f, g * g);
             if (q == 0.0) break;                               // the chase ended early: the block splits here
-            const double inv = rsqrt(q);
-            e[i + 1] = q * inv;
+            const double inv = rsqrt(q), en = q * inv;
+            e[i + 1] = en;
             s = f * inv;
             c = g * inv;
             g = dnext - p;
             const double r = fma(di - g, s, 2.0 * c * b);
             p = s * r;
-            d[i + 1] = g + p;
+            const double dn = g + p;
+            d[i + 1] = dn;
             g = fma(c, r, -b);
             z[i + 1] = fma(s, zi, c * znext);
             znext = fma(c, zi, -s * znext);
             dnext = di;
+            // e[i + 1] against its new neighbours (not for the first
+            // rotation: e[top] is outside the block)
+            if (i + 1 < top && en <= kEps * (fabs(dn) + dabove)) small |= 2u << i;
+            dabove = fabs(dn);
         }
+        const double dn = dnext - p;
         z[i + 1] = znext;
-        d[i + 1] = dnext - p;
-        if (i < l) e[l] = g; else e[i + 1] = 0.0;
+        d[i + 1] = dn;
+        if (i < l) {
+            e[l] = g;
+            if (fabs(g) <= kEps * (fabs(dn) + dabove)) small |= 1u << l;
+        } else {
+            e[i + 1] = 0.0;
+            small |= 2u << i;
+        }
         e[top] = 0.0;
     }
     return false;

@@ -23,9 +23,9 @@ from . import build as _build
 
 #: phase slot -> name (slots of geneig_cta.cu and geneig_dc.cuh)
 PHASES = {
-    0: "a1 load H, S", 1: "a2 Cholesky + L^-1", 2: "a3 T = H X^H", 3: "a4 C = X T",
+    0: "a1 load S", 1: "a2 Cholesky + L^-1", 2: "a3+a4 C = X H X^H", 3: "X^H to U, C mirrored",
     4: "a5a Householder tridiagonalisation", 5: "a5b D&C tail (finite check)",
-    6: "a5c rank + back-transform V = Q Z", 7: "a6 U = X^H V", 8: "a7 store U (+ loop barrier)",
+    6: "a5c rank + back-transform V = Q Z", 7: "a6 U = X^H V", 8: "a7 store U (+ loop barrier)", 9: "WY factors, reflectors to U",
     10: "D&C scale + leaves", 11: "D&C deflation (phase A)", 12: "D&C secular roots (phase B)",
     13: "D&C Loewner z (phase C)", 14: "D&C rank-one vectors (phase D)", 15: "D&C merge GEMMs (phase E)",
     # l2-slot (tiled) kernel
