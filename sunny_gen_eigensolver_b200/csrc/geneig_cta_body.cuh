@@ -78,9 +78,13 @@ __host__ __device__ inline size_t cta_dc_bytes(int n, bool spec) {   // (d, e) f
                      (size_t)dc_vec_ints(n) * 4;
     return (b + 15) & ~(size_t)15;
 }
+// The reduction's panel is two blocks wide where one pencil has the SM (its
+// shared memory) to itself anyway. N=108: 235 K cycles for one, 141 K for two.
+__host__ __device__ constexpr bool cta_two_panels(int nw) { return nw >= 16; }
 constexpr int kDElems = 72;       // an 8 x 8 tile with leading dimension 9
 __host__ __device__ inline size_t cta_work_bytes(int n, int nw, bool spec) {
-    const size_t panel = ((size_t)8 * (n | 1) + 2 * kDElems) * 16;
+    const size_t one = (size_t)8 * (n | 1);
+    const size_t panel = (cta_two_panels(nw) ? 2 * one : one + 2 * kDElems) * 16;
     const size_t hh = ((size_t)32 * nw + 3 * cta_rows(n, spec)) * 16;
     const size_t dc = cta_dc_bytes(n, spec) + (spec ? 0 : (size_t)((n + 7) / 8) * 36 * 16);
     const size_t m = panel > hh ? panel : hh;
@@ -434,78 +438,161 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
             }
             phase_mark(2);
         } else {
-            // ---- a3 + a4, one 8-column block of C at a time:
+            // ---- a3 + a4, one or two 8-column blocks of C at a time:
             // T(:, tj) = H X(tj, :)^H into `work` (H read in full, from global
             // memory, L2 after the first blocks), then C(ti, tj) = X(ti, :) T,
-            // ti >= tj. Two row tiles per warp share each fragment of X.
+            // ti >= tj.
             double2* Tp = work;
+            if constexpr (cta_two_panels(NW)) {
+                // Two blocks of C at a time, a row tile per warp: each element
+                // of H and of X serves both, and the sixteen warps meet half
+                // as often.
 #pragma unroll 1
-            for (int tj = 0; tj < nb; ++tj) {
+                for (int tj = 0; tj < nb; tj += 2) {
+                    const bool two = tj + 1 < nb;
+                    const int kend = two ? tj + 1 : tj;
 #pragma unroll 1
-                for (int t0 = warp; t0 < nb; t0 += 2 * NW) {
-                    const int i0 = 8 * t0 + fr, i1 = i0 + 8 * NW;
-                    double re0[2] = {0.0, 0.0}, im0[2] = {0.0, 0.0}, re1[2] = {0.0, 0.0}, im1[2] = {0.0, 0.0};
-                    const double2* xj = M + 8 * tj + fr;
-                    const double2* h0 = Hb + min(i0, n - 1);
-                    const double2* h1 = Hb + min(i1, n - 1);
-                    const bool two = t0 + NW < nb;
-                    double2 y0[2][2], y1[2][2];  // H of the next two k blocks, loaded ahead
+                    for (int t0 = warp; t0 < nb; t0 += NW) {
+                        const int i0 = 8 * t0 + fr;
+                        double re0[2] = {0.0, 0.0}, im0[2] = {0.0, 0.0}, re1[2] = {0.0, 0.0}, im1[2] = {0.0, 0.0};
+                        const double2* x0 = M + 8 * tj + fr;
+                        const double2* h0 = Hb + min(i0, n - 1);
+                        double2 y[4][2];         // H of the next four k blocks, loaded ahead
 #pragma unroll
-                    for (int p = 0; p < 2; ++p)
+                        for (int p = 0; p < 4; ++p)
 #pragma unroll
-                        for (int s = 0; s < 2; ++s) {
-                            const int k = min(8 * p + 2 * fq + s, n - 1);
-                            y0[p][s] = __ldg(h0 + k * n);
-                            y1[p][s] = __ldg(h1 + k * n);
+                            for (int s = 0; s < 2; ++s) y[p][s] = __ldg(h0 + min(8 * p + 2 * fq + s, n - 1) * n);
+#pragma unroll 1
+                        for (int kb = 0; kb <= kend; ++kb) {
+                            const double2 av[2] = {y[0][0], y[0][1]};
+#pragma unroll
+                            for (int p = 0; p < 3; ++p) {
+                                y[p][0] = y[p + 1][0];
+                                y[p][1] = y[p + 1][1];
+                            }
+                            if (kb + 4 <= kend) {
+#pragma unroll
+                                for (int s = 0; s < 2; ++s) y[3][s] = __ldg(h0 + min(8 * kb + 32 + 2 * fq + s, n - 1) * n);
+                            }
+#pragma unroll
+                            for (int s = 0; s < 2; ++s) {
+                                const int kr = 2 * fq + s;
+                                const double2* xk = x0 + (8 * kb + kr) * ld;
+                                if (kb <= tj) {
+                                    double2 bv = cconj(xk[0]);
+                                    if (kb == tj && kr > fr) bv = zero;
+                                    zmma(re0, im0, av[s], bv);
+                                }
+                                if (two) {
+                                    double2 bv = cconj(xk[8]);
+                                    if (kb == tj + 1 && kr > fr) bv = zero;
+                                    zmma(re1, im1, av[s], bv);
+                                }
+                            }
                         }
-#pragma unroll 1
-                    for (int kb = 0; kb <= tj; ++kb) {
-                        const double2 a0[2] = {y0[0][0], y0[0][1]}, a1[2] = {y1[0][0], y1[0][1]};
+                        if (i0 < n) {
 #pragma unroll
-                        for (int s = 0; s < 2; ++s) {
-                            const int k = min(8 * kb + 16 + 2 * fq + s, n - 1);
-                            y0[0][s] = y0[1][s];
-                            y1[0][s] = y1[1][s];
-                            if (kb + 2 <= tj) {
-                                y0[1][s] = __ldg(h0 + k * n);
-                                y1[1][s] = __ldg(h1 + k * n);
+                            for (int e = 0; e < 2; ++e) {
+                                double2* tc = Tp + (2 * fq + e) * ldp + i0;
+                                tc[0] = c2(re0[e], im0[e]);
+                                if (two) tc[8 * ldp] = c2(re1[e], im1[e]);
+                            }
+                        }
+                    }
+                    team_sync<NT, BLOCK>();
+#pragma unroll 1
+                    for (int ti = tj + warp; ti < nb; ti += NW) {
+                        double re0[2] = {0.0, 0.0}, im0[2] = {0.0, 0.0}, re1[2] = {0.0, 0.0}, im1[2] = {0.0, 0.0};
+                        const double2* xi = M + 8 * ti + fr;
+                        const double2* tc = Tp + fr * ldp;
+                        const bool both = two && ti > tj;
+#pragma unroll 1
+                        for (int kb = 0; kb <= ti; ++kb) {
+#pragma unroll
+                            for (int s = 0; s < 2; ++s) {
+                                const int kr = 2 * fq + s, k = 8 * kb + kr, kc = min(k, n - 1);
+                                double2 av = xi[k * ld];
+                                if (kb == ti && kr > fr) av = zero;
+                                zmma(re0, im0, av, tc[kc]);
+                                if (both) zmma(re1, im1, av, tc[8 * ldp + kc]);
+                            }
+                        }
+                        put_c(ti, tj, re0, im0);
+                        if (both) put_c(ti, tj + 1, re1, im1);
+                    }
+                    team_sync<NT, BLOCK>();
+                }
+            } else {
+                // One block at a time; two row tiles per warp share each
+                // fragment of X.
+#pragma unroll 1
+                for (int tj = 0; tj < nb; ++tj) {
+#pragma unroll 1
+                    for (int t0 = warp; t0 < nb; t0 += 2 * NW) {
+                        const int i0 = 8 * t0 + fr, i1 = i0 + 8 * NW;
+                        double re0[2] = {0.0, 0.0}, im0[2] = {0.0, 0.0}, re1[2] = {0.0, 0.0}, im1[2] = {0.0, 0.0};
+                        const double2* xj = M + 8 * tj + fr;
+                        const double2* h0 = Hb + min(i0, n - 1);
+                        const double2* h1 = Hb + min(i1, n - 1);
+                        const bool two = t0 + NW < nb;
+                        double2 y0[2][2], y1[2][2];  // H of the next two k blocks, loaded ahead
+#pragma unroll
+                        for (int p = 0; p < 2; ++p)
+#pragma unroll
+                            for (int s = 0; s < 2; ++s) {
+                                const int k = min(8 * p + 2 * fq + s, n - 1);
+                                y0[p][s] = __ldg(h0 + k * n);
+                                y1[p][s] = __ldg(h1 + k * n);
+                            }
+#pragma unroll 1
+                        for (int kb = 0; kb <= tj; ++kb) {
+                            const double2 a0[2] = {y0[0][0], y0[0][1]}, a1[2] = {y1[0][0], y1[0][1]};
+#pragma unroll
+                            for (int s = 0; s < 2; ++s) {
+                                const int k = min(8 * kb + 16 + 2 * fq + s, n - 1);
+                                y0[0][s] = y0[1][s];
+                                y1[0][s] = y1[1][s];
+                                if (kb + 2 <= tj) {
+                                    y0[1][s] = __ldg(h0 + k * n);
+                                    y1[1][s] = __ldg(h1 + k * n);
+                                }
+                            }
+#pragma unroll
+                            for (int s = 0; s < 2; ++s) {
+                                const int kr = 2 * fq + s;
+                                double2 bv = cconj(xj[(8 * kb + kr) * ld]);
+                                if (kb == tj && kr > fr) bv = zero;
+                                zmma(re0, im0, a0[s], bv);
+                                if (two) zmma(re1, im1, a1[s], bv);
                             }
                         }
 #pragma unroll
-                        for (int s = 0; s < 2; ++s) {
-                            const int kr = 2 * fq + s;
-                            double2 bv = cconj(xj[(8 * kb + kr) * ld]);
-                            if (kb == tj && kr > fr) bv = zero;
-                            zmma(re0, im0, a0[s], bv);
-                            if (two) zmma(re1, im1, a1[s], bv);
+                        for (int e = 0; e < 2; ++e) {
+                            double2* tc = Tp + (2 * fq + e) * ldp;
+                            if (i0 < n) tc[i0] = c2(re0[e], im0[e]);
+                            if (i1 < n) tc[i1] = c2(re1[e], im1[e]);
                         }
                     }
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        double2* tc = Tp + (2 * fq + e) * ldp;
-                        if (i0 < n) tc[i0] = c2(re0[e], im0[e]);
-                        if (i1 < n) tc[i1] = c2(re1[e], im1[e]);
-                    }
-                }
-                team_sync<NT, BLOCK>();
+                    team_sync<NT, BLOCK>();
 #pragma unroll 1
-                for (int ti = tj + warp; ti < nb; ti += NW) {
-                    double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
-                    const double2* xi = M + 8 * ti + fr;
-                    const double2* tc = Tp + fr * ldp;
+                    for (int ti = tj + warp; ti < nb; ti += NW) {
+                        double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
+                        const double2* xi = M + 8 * ti + fr;
+                        const double2* tc = Tp + fr * ldp;
 #pragma unroll 1
-                    for (int kb = 0; kb <= ti; ++kb) {
+                        for (int kb = 0; kb <= ti; ++kb) {
 #pragma unroll
-                        for (int s = 0; s < 2; ++s) {
-                            const int kr = 2 * fq + s, k = 8 * kb + kr;
-                            double2 av = xi[k * ld];
-                            if (kb == ti && kr > fr) av = zero;
-                            zmma(re, im, av, tc[min(k, n - 1)]);
+                            for (int s = 0; s < 2; ++s) {
+                                const int kr = 2 * fq + s, k = 8 * kb + kr;
+                                double2 av = xi[k * ld];
+                                if (kb == ti && kr > fr) av = zero;
+                                zmma(re, im, av, tc[min(k, n - 1)]);
+                            }
                         }
+                        put_c(ti, tj, re, im);
                     }
-                    put_c(ti, tj, re, im);
+                    team_sync<NT, BLOCK>();
                 }
-                team_sync<NT, BLOCK>();
             }
             phase_mark(2);
         }
@@ -623,13 +710,17 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
                     for (int t = 0; t < R; ++t) {
                         v[t] = vk[off[t]];
                         w[t] = zero;
-                        if (t < rb) {
-                            w[t] = pt[32 * t];
-#pragma unroll 1
-                            for (int g = 1; g < G; ++g) w[t] = cadd(w[t], pt[32 * (t + g * rb)]);
-                        }
-                        s = fma(w[t].x, v[t].x, fma(w[t].y, v[t].y, s));
                     }
+                    // (the loads of several classes in flight at sixteen warps,
+                    // n = 108: 5.3 K -> 4.8 K cycles a step)
+#pragma unroll (NW >= 16 ? 4 : NW >= 8 ? 2 : 1)
+                    for (int g = 0; g < G; ++g, pt += 32 * rb)
+#pragma unroll
+                        for (int t = 0; t < R; ++t)
+                            if (t < rb) w[t] = cadd(w[t], pt[32 * t]);
+#pragma unroll
+                    for (int t = 0; t < R; ++t)
+                        s = fma(w[t].x, v[t].x, fma(w[t].y, v[t].y, s));
                     const double h = -0.5 * fma(tau.x, tau.x, tau.y * tau.y) * warp_sum(s);
 #pragma unroll
                     for (int t = 0; t < R; ++t) {
