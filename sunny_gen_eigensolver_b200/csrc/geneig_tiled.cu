@@ -19,8 +19,8 @@
 //       the subdiagonal; for n >= 96 in 16-column panels whose trailing
 //       update A -= V W^H + W V^H is a GEMM), T = Z diag(w) Z^T by divide and conquer (Z and its
 //       merge workspace in M2, merge products through Zo), V = Q Z with
-//       compact-WY blocks of 16 reflectors, Q_b = I - Y T_b Y^H:
-//       W1 = Y^H V, W2 = T_b W1, V -= Y W2 (all GEMMs), V in the output U   (:250)
+//       compact-WY blocks of 16 reflectors, Q_b = I - Y T_b Y^H, two blocks
+//       at a time on strips of 8 columns of V, a warp each, V in the output U   (:250)
 //   a6  U = X^H V into M2, copied to the output                   (:252)
 //   a7  W ascending, U columns in the same order                  (:268-276)
 //

@@ -207,31 +207,8 @@ __device__ __forceinline__ void z16_step(Z16& c, const double2 (&a)[2], const do
         }
 }
 
-// c += A(i0:i0+16, k0:k1) B(k0:k1, j0:j0+16); a_at(i, k) and b_at(k, j)
-// return the operand elements (they must return 0 outside the operands;
-// k < k1 is checked here).
-template <class FA, class FB>
-__device__ __forceinline__ void z16_mma(Z16& c, int i0, int j0, int k0, int k1, FA a_at, FB b_at) {
-    const int lane = threadIdx.x & 31;
-    const int ar = i0 + (lane >> 2), bc = j0 + (lane >> 2), kq = lane & 3;
-#pragma unroll 4
-    for (int k = k0; k < k1; k += 4) {
-        const int kk = k + kq;
-        double2 a[2], b[2];
-        if (kk < k1) {
-            a[0] = a_at(ar, kk);
-            a[1] = a_at(ar + 8, kk);
-            b[0] = b_at(kk, bc);
-            b[1] = b_at(kk, bc + 8);
-        } else {
-            a[0] = a[1] = b[0] = b[1] = c2(0.0, 0.0);
-        }
-        z16_step(c, a, b);
-    }
-}
-
-// The same for operands in memory, A(i, k) at pa[i si + k sk] and B(k, j) at
-// pb[k tk + j tj], conjugated where CA / CB say so, A negated for NA. Rows and
+// c += A(i0:i0+16, k0:k1) B(k0:k1, j0:j0+16), A(i, k) at pa[i si + k sk], B(k, j)
+// at pb[k tk + j tj], conjugated where CA / CB say so, A negated for NA. Rows and
 // columns past ni, nj repeat the last one (they reach discarded results only);
 // k blocks are unmasked but for the last, whose A is zeroed past k1.
 template <bool CA, bool NA, bool CB>
@@ -280,6 +257,169 @@ __device__ __forceinline__ void tri_tile(int t, int& ti, int& tj) {
     while (r * (r + 1) / 2 > t) --r;
     ti = r;
     tj = t - r * (r + 1) / 2;
+}
+
+// ---------------------------------------------------------------- back-transform
+// Complex 8 x 8 x 4 step with four real ones.
+__device__ __forceinline__ void z8_step(double (&re)[2], double (&im)[2], double2 a, double2 b) {
+    dmma(re, a.x, b.x);
+    dmma(re, -a.y, b.y);
+    dmma(im, a.x, b.y);
+    dmma(im, a.y, b.x);
+}
+
+// T factor of the compact WY form I - Y T Y^H of w reflectors (Y: rows k0 .. n,
+// ones and zeros in place), forward column-wise: T(j, j) = tau_j, T(0:j, j) =
+// -tau_j T(0:j, 0:j) (Y^H Y)(0:j, j). 16 x 16, zero past w, by one warp.
+__device__ __forceinline__ void wy_factor(double2* tf, const double2* Y, int ld, int k0, int n, int w, const double2* tau) {
+    const int lane = threadIdx.x & 31;
+    Z16 acc;
+    z16_zero(acc);
+    z16_gemm<true, false, false>(acc, 0, 0, k0, n, Y, ld, 1, w, Y, 1, ld, w);
+    z16_store(acc, 0, 0, [&](int i, int j, double2 x) { tf[i + 16 * j] = i < j && j < w ? x : c2(0.0, 0.0); });
+    __syncwarp();
+#pragma unroll 1
+    for (int j = 0; j < w; ++j) {
+        const double2 tj = tau[j];
+        const double2 y = lane < j ? cneg(cmul(tj, tf[lane + 16 * j])) : c2(0.0, 0.0);
+        double2 s = c2(0.0, 0.0);
+#pragma unroll 2
+        for (int l = 0; l < j; ++l) {
+            const double2 yl = c2(__shfl_sync(0xffffffffu, y.x, l), __shfl_sync(0xffffffffu, y.y, l));
+            if (lane <= l) s = cfma(s, tf[lane + 16 * l], yl);
+        }
+        if (lane < j) tf[lane + 16 * j] = s;
+        if (lane == j) tf[j + 16 * j] = tj;
+        __syncwarp();
+    }
+}
+
+// V <- (I - Y1 T1 Y1^H) (I - Y2 T2 Y2^H) V on columns j0 .. j0 + 7 of V, by one
+// warp; Y1: reflectors k0 .. k0 + 15, Y2: the next 16 (two: they exist).
+// Worked on transposed, W^H = V^H Y, so that every accumulator is the next
+// product's A fragment (in each k block of 8 the MMA's slot q of step s is
+// index 2 q + s) and W stays in registers: nothing is shared, and the warps run
+// through all blocks without a barrier. Two blocks at a time, because a strip
+// of V is read twice and written once for each visit:
+//   W2 = T2 Y2^H V, W1 = T1 (Y1^H V - (Y1^H Y2) W2), V -= Y1 W1 + Y2 W2.
+// t1, t2: T factors, g12 = Y1^H Y2. Columns of Y past nref repeat the last one
+// (finite, and T is zero there); rows above a reflector are zero in Y.
+// Bound by the loads of V and Y from L2. N=216, the whole back-transform:
+// 2.06 M cycles block by block over all of V with five barriers each, 1.65 M
+// here; strips of 16 columns spill and are slower (N=384: 5 % of the solve).
+__device__ __forceinline__ void wy_strip(double2* V, int n, int j0, const double2* Y, int ld, int k0, int nref, bool two,
+                                         const double2* t1, const double2* t2, const double2* g12) {
+    const int lane = threadIdx.x & 31, fr = lane >> 2, fq = lane & 3;
+    double wr[2][2][2], wi[2][2][2];               // W^H of both blocks: column tiles of 8
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) wr[b][h][0] = wr[b][h][1] = wi[b][h][0] = wi[b][h][1] = 0.0;
+    const bool col = j0 + fr < n;
+    double2* vj = V + (size_t)min(j0 + fr, n - 1) * n;
+    const double2* yc[4];                          // columns of Y as right-hand operands
+#pragma unroll
+    for (int h = 0; h < 4; ++h) yc[h] = Y + (size_t)min(k0 + 8 * h + fr, nref - 1) * ld;
+#pragma unroll 1
+    for (int i0 = k0; i0 < n; i0 += 8) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const int i = i0 + 2 * fq + s, ic = min(i, n - 1);
+            double2 a = cconj(vj[ic]), y[4];
+            if (i >= n) a = c2(0.0, 0.0);
+#pragma unroll
+            for (int h = 0; h < 4; ++h) if (h < 2 || two) y[h] = yc[h][ic];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) if (h < 2 || two) z8_step(wr[h >> 1][h & 1], wi[h >> 1][h & 1], a, y[h]);
+        }
+    }
+    // out += sgn w m^H, m a 16 x 16 matrix (upper triangular if tri)
+    auto times = [&](double (&outr)[2][2], double (&outi)[2][2], const double (&r)[2][2], const double (&im)[2][2],
+                     const double2* m, double sgn, bool tri) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)                // k block (column of m)
+#pragma unroll
+            for (int s = 0; s < 2; ++s)
+#pragma unroll
+                for (int g = 0; g < 2; ++g) {      // column tile (row of m)
+                    if (tri && g > h) continue;
+                    const double2 bv = cconj(m[8 * g + fr + 16 * (8 * h + 2 * fq + s)]);
+                    z8_step(outr[g], outi[g], c2(sgn * r[h][s], sgn * im[h][s]), bv);
+                }
+    };
+    auto apply_t = [&](double (&r)[2][2], double (&im)[2][2], const double2* m) {
+        double nr[2][2] = {}, ni[2][2] = {};
+        times(nr, ni, r, im, m, 1.0, true);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                r[h][e] = nr[h][e];
+                im[h][e] = ni[h][e];
+            }
+    };
+    if (two) {
+        apply_t(wr[1], wi[1], t2);
+        times(wr[0], wi[0], wr[1], wi[1], g12, -1.0, false);
+    }
+    apply_t(wr[0], wi[0], t1);
+    const int ce = nref - 1 - k0;                  // last column of Y, from k0
+#pragma unroll 1
+    for (int i0 = k0; i0 < n; i0 += 8) {
+        double vr[2], vi[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const double2 x = vj[min(i0 + 2 * fq + e, n - 1)];
+            vr[e] = x.x;
+            vi[e] = x.y;
+        }
+        const double2* yi = Y + (size_t)k0 * ld + min(i0 + fr, n - 1);
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+            if (h < 2 || two)
+#pragma unroll
+                for (int s = 0; s < 2; ++s)
+                    z8_step(vr, vi, c2(-wr[h >> 1][h & 1][s], wi[h >> 1][h & 1][s]),
+                            yi[(size_t)min(8 * h + 2 * fq + s, ce) * ld]);
+        __syncwarp();
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+            if (col && i0 + 2 * fq + e < n) vj[i0 + 2 * fq + e] = c2(vr[e], vi[e]);
+    }
+    __syncwarp();
+}
+
+// V <- Q V, Q the product of the nref reflectors in Y. tf: room for the T
+// factors and, of each pair of blocks, Y1^H Y2, 256 elements each.
+template <int kNT>
+__device__ __forceinline__ void wy_apply(double2* V, int n, const double2* Y, int ld, int nref, const double2* tau,
+                                             double2* tf) {
+    constexpr int kNW = kNT / 32;
+    const int warp = threadIdx.x >> 5;
+    const int nblk = (nref + 15) >> 4, npair = (nblk + 1) >> 1;
+    double2* g12 = tf + 256 * nblk;
+#pragma unroll 1
+    for (int t = warp; t < nblk + (nblk >> 1); t += kNW) {
+        if (t < nblk) {
+            wy_factor(tf + 256 * t, Y + (size_t)16 * t * ld, ld, 16 * t + 1, n, min(16, nref - 16 * t), tau + 16 * t);
+        } else {
+            const int p = t - nblk, kb = 32 * p + 16, w = min(16, nref - kb);
+            Z16 acc;
+            z16_zero(acc);
+            z16_gemm<true, false, false>(acc, 0, 0, kb + 1, n, Y + (size_t)(kb - 16) * ld, ld, 1, 16,
+                                         Y + (size_t)kb * ld, 1, ld, w);
+            z16_store(acc, 0, 0, [&](int i, int j, double2 x) { g12[256 * p + i + 16 * j] = x; });
+        }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int j0 = 8 * warp; j0 < n; j0 += 8 * kNW)
+#pragma unroll 1
+        for (int p = npair - 1; p >= 0; --p) {
+            const double2 *t1 = tf + 512 * p, *t2 = t1 + 256, *g = g12 + 256 * p;
+            const bool two = 2 * p + 1 < nblk;
+            wy_strip(V, n, j0, Y, ld, 32 * p, nref, two, t1, t2, g);
+        }
 }
 
 // The divide and conquer with a register allocation of its own: inlined, it
@@ -413,6 +553,220 @@ __device__ __forceinline__ double cta_sum(double x, double* red) {
     return warp_sum(lane < kNT / 32 ? red[lane] : 0.0);
 }
 
+// X = L^-1 -> M1, block row r0..re at a time; zeros above its diagonal, so that
+// the products need no masks.
+template <int kNT>
+__device__ __forceinline__ void tiled_inverse(int n, int ld, const double2* M0, double2* M1, const double* rdg) {
+    constexpr int kNW = kNT / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const double2 zero = c2(0.0, 0.0);
+    for (int j = warp; j < n; j += kNW)
+        for (int i = lane; i < j; i += 32) M1[i + (size_t)j * ld] = zero;
+    for (int r0 = 0; r0 < n; r0 += 16) {
+        const int re = min(r0 + 16, n);
+        for (int t = warp; t < (r0 >> 4); t += kNW) {
+            const int j0 = 16 * t;
+            Z16 acc;
+            z16_zero(acc);
+            z16_gemm<false, false, false>(acc, r0, j0, j0, r0, M0, 1, ld, n, M1, 1, ld, n);
+            z16_store(acc, r0, j0, [&](int i, int j, double2 x) { if (i < n) M1[i + (size_t)j * ld] = x; });
+        }
+        __syncthreads();
+        for (int c = tid; c < re; c += kNT) {
+            double2 x[16];
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+                const int i = r0 + r;
+                x[r] = (i < re) ? ((c < r0) ? cneg(M1[i + (size_t)c * ld]) : c2(i == c ? 1.0 : 0.0, 0.0))
+                                : zero;
+            }
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+                const int i = r0 + r;
+                if (i < re) {
+                    double2 s = x[r];
+#pragma unroll
+                    for (int q = 0; q < r; ++q) s = cfms(s, M0[i + (size_t)(r0 + q) * ld], x[q]);
+                    x[r] = cscale(s, rdg[i]);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 16; ++r)
+                if (r0 + r < re) M1[r0 + r + (size_t)c * ld] = x[r];
+        }
+        __syncthreads();
+    }
+}
+
+// T = H X^H -> M2, T(i, j) = sum_{k <= j} H(i, k) conj(X(j, k)), then C = X T -> M0.
+template <int kNT>
+__device__ __forceinline__ void tiled_form_c(int n, int ld, int sigma, const double2* Hb, double2* M0, const double2* M1,
+                                                 double2* M2) {
+    constexpr int kNW = kNT / 32;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tn = (n + 15) >> 4;
+    const size_t nn = (size_t)n * n;
+    const double2 zero = c2(0.0, 0.0);
+    if (sigma) {
+        const int m = n >> 1;
+        for (int idx = tid; idx < (int)nn; idx += kNT) {
+            const int j = idx / n, i = idx - j * n;
+            const double2 x = (i <= j) ? cconj(M1[j + (size_t)i * ld]) : zero;
+            M2[i + (size_t)j * ld] = (i < m) ? x : cneg(x);
+        }
+    } else {
+        for (int t = warp; t < tile_blocks(tn, tn); t += kNW) {
+            int ti, tj;
+            if (!tile_at(t, tn, tn, ti, tj)) continue;
+            const int i0 = 16 * ti, j0 = 16 * tj;
+            Z16 acc;
+            z16_zero(acc);
+            z16_gemm<false, false, true>(acc, i0, j0, 0, min(n, j0 + 16), Hb, 1, n, n, M1, ld, 1, n);
+            z16_store(acc, i0, j0, [&](int i, int j, double2 x) {
+                if (i < n && j < n) M2[i + (size_t)j * ld] = x;
+            });
+        }
+    }
+    __syncthreads();
+    // C = X T, lower tiles; each lower element is written with its
+    // mirror so that C is exactly Hermitian. L in M0 is dead by now.
+    for (int t = warp; t < tile_blocks(tn, tn); t += kNW) {
+        int ti, tj;
+        if (!tile_at(t, tn, tn, ti, tj) || ti < tj) continue;
+        const int i0 = 16 * ti, j0 = 16 * tj;
+        Z16 acc;
+        z16_zero(acc);
+        z16_gemm<false, false, false>(acc, i0, j0, 0, min(n, i0 + 16), M1, 1, ld, n, M2, 1, ld, n);
+        z16_store(acc, i0, j0, [&](int i, int j, double2 x) {
+            if (i < n && j < n && i >= j) {
+                if (i == j) x.y = 0.0;
+                M0[i + (size_t)j * ld] = x;
+                M0[j + (size_t)i * ld] = cconj(x);
+            }
+        });
+    }
+    __syncthreads();
+}
+
+// The FP64 reduction of C (lower, M0) to tridiagonal form, reflectors in its
+// columns, (d, e, tau) to shared memory.
+template <int kNT>
+__device__ __forceinline__ void tiled_house(int n, int ld, double2* M0, double2* M2, unsigned char* smem_raw) {
+    constexpr int kNW = kNT / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const double2 zero = c2(0.0, 0.0);
+    const TVec v = tcarve(smem_raw, n);
+    // thread i owns row i of the vectors and of the panel (kNT >= n)
+    // V and W of the panel: columns Vp + c ld, Wp + c ld
+    double2* Wp = M2;
+    const int i = tid;
+    const bool row = i < n;
+    double* red = reinterpret_cast<double*>(v.red);   // 32 doubles for each of two sums
+    double2* t12 = v.tb;                               // W^H v at [0, c), V^H v at [16, 16 + c)
+    // (the divide and conquer's scratch is free until then: 2 n complex of its 7 n + 1 doubles)
+    double2* yx = reinterpret_cast<double2*>(v.dcd + (n & 1));
+    double2* const ydot[4] = {v.pb, v.gb, yx, yx + n};
+    for (int p = 0; p < n - 1; p += 16) {
+        const int w = min(16, n - 1 - p);
+        double2* Vp = M0 + (size_t)p * ld;
+        for (int c = 0; c < w; ++c) {
+            const int k = p + c;
+            // (1) column k of the current matrix:
+            // a_k -= V(:, 0:c) W(k, 0:c)^H + W(:, 0:c) V(k, 0:c)^H
+            // (rows k .. n-1 of V are stored whole)
+            double2 x = zero;
+            if (row && i >= k) {
+                x = M0[i + (size_t)k * ld];
+#pragma unroll 4
+                for (int cc = 0; cc < c; ++cc) {
+                    x = cfms_bc(x, Vp[i + cc * ld], Wp[k + cc * ld]);
+                    x = cfms_bc(x, Wp[i + cc * ld], Vp[k + cc * ld]);
+                }
+            }
+            if (i == k) { v.d[k] = x.x; M0[k + (size_t)k * ld] = x; }
+            if (i == k + 1) v.gb[0] = x;
+            // (2) reflector from a_k(k+1:n)
+            const double ss = cta_sum<kNT>((row && i > k + 1) ? fma(x.x, x.x, x.y * x.y) : 0.0, red);
+            const double2 alpha = v.gb[0];
+            double2 taui = zero, scal = zero;
+            double beta = alpha.x;
+            if (!(ss == 0.0 && alpha.y == 0.0)) {
+                const double nn = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, ss));
+                const double rn = rsqrt(nn);
+                beta = -copysign(nn * rn, alpha.x);
+                const double rb = -copysign(rn, alpha.x);
+                taui = c2((beta - alpha.x) * rb, -alpha.y * rb);
+                const double2 z = c2(alpha.x - beta, alpha.y);
+                const double inv = fast_rcp(fma(z.x, z.x, z.y * z.y));
+                scal = c2(z.x * inv, -z.y * inv);
+            }
+            double2 vi = zero;
+            if (row && i > k) {
+                vi = i == k + 1 ? c2(1.0, 0.0) : cmul(x, scal);
+                v.vb[i] = vi;
+                M0[i + (size_t)k * ld] = vi;
+            }
+            if (tid == 0) { v.tau[k] = taui; v.e[k] = beta; }
+            __syncthreads();
+            // (3) y = A v (A: panel-start trailing matrix, lower
+            // triangle), t1 = W^H v, t2 = V^H v
+            sym_matvec<kNT>(M0, ld, n, k + 1, v.vb, v.part, ydot, v.ring);
+            for (int it = warp; it < 2 * c; it += kNW) {
+                const int cc = it >> 1;
+                double2 acc = zero;
+                const double2* col = (it & 1 ? Vp : Wp) + cc * ld;
+#pragma unroll 4
+                for (int j = k + 1 + lane; j < n; j += 32) acc = cfmac(acc, col[j], v.vb[j]);
+                acc = warp_sum2(acc);
+                if (lane == 0) t12[16 * (it & 1) + cc] = acc;
+            }
+            __syncthreads();
+            // (4) w = tau (y - V t1 - W t2) + alpha2 v on rows k+1..n (the
+            // current matrix is A - V W^H - W V^H), alpha2 =
+            // -tau/2 (w^H v) = -|tau|^2/2 v^H A v; zero above
+            double2 y = zero;
+            if (row && i > k) {
+                y = sym_matvec_row<kNT>(n, k + 1, i, v.part, ydot);
+#pragma unroll 4
+                for (int cc = 0; cc < c; ++cc) {
+                    y = cfms(y, Vp[i + cc * ld], t12[cc]);
+                    y = cfms(y, Wp[i + cc * ld], t12[16 + cc]);
+                }
+            }
+            const double h = -0.5 * fma(taui.x, taui.x, taui.y * taui.y) *
+                             cta_sum<kNT>(fma(y.x, vi.x, y.y * vi.y), red + 32);
+            if (row) {
+                const double2 wt = cmul(taui, y);
+                Wp[i + c * ld] = c2(fma(h, vi.x, wt.x), fma(h, vi.y, wt.y));
+            }
+            __syncthreads();
+        }
+        // trailing update, lower tiles: A(q:n, q:n) -= V W^H + W V^H, q = p + w
+        const int q = p + w, mq = n - q;
+        if (mq > 0) {
+            const int tq = (mq + 15) >> 4;
+            for (int t = warp; t < tile_blocks(tq, tq); t += kNW) {
+                int ti, tj;
+                if (!tile_at(t, tq, tq, ti, tj) || ti < tj) continue;
+                const int i0 = q + 16 * ti, j0 = q + 16 * tj;
+                Z16 acc;
+                z16_load(acc, i0, j0, [&](int r, int j) { return (r < n && j < n) ? M0[r + (size_t)j * ld] : zero; });
+                z16_gemm<false, true, true>(acc, i0, j0, 0, w, Vp, 1, ld, n, Wp, ld, 1, n);
+                z16_gemm<false, true, true>(acc, i0, j0, 0, w, Wp, 1, ld, n, Vp, ld, 1, n);
+                z16_store(acc, i0, j0, [&](int r, int j, double2 x) {
+                    if (r < n && j < n && r >= j) M0[r + (size_t)j * ld] = x;
+                });
+            }
+        }
+        __syncthreads();
+    }
+    if (tid == 0) {
+        v.d[n - 1] = M0[(n - 1) + (size_t)(n - 1) * ld].x;
+        if (n == 1) v.tau[0] = zero;
+    }
+    __syncthreads();
+}
+
 // One pencil b, solved end to end by the whole CTA in its global-memory
 // slot `slot` (tiled_slot_elems(n, mixed) complex entries) with the
 // launch's dynamic shared memory as the vector area. kNT >= n.
@@ -429,7 +783,6 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
     double2* M3 = mixed ? M2 + mat : nullptr;       // mixed only
     double2* zob = mixed ? M3 + mat : M2 + mat;
     double*  Zo = reinterpret_cast<double*>(zob);
-    double2* Wsc = zob;                      // WY scratch (16 x n), shares Zo's storage
     // mixed only: FP32 copy of C after Zo; after the back-transform Zo and
     // it together hold one more n x ld complex matrix (M4)
     float2*  C32 = reinterpret_cast<float2*>(zob + tiled_zo_elems(n));
@@ -503,44 +856,8 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
     phase_mark(17);
 
     if (!code && a.stage >= 2) {
-        // ---- a3: X = L^-1 -> M1, block row r0..re at a time; zeros above its
-        // diagonal, so that the products need no masks
-        for (int j = warp; j < n; j += kNW)
-            for (int i = lane; i < j; i += 32) M1[i + (size_t)j * ld] = zero;
-        for (int r0 = 0; r0 < n; r0 += 16) {
-            const int re = min(r0 + 16, n);
-            for (int t = warp; t < (r0 >> 4); t += kNW) {
-                const int j0 = 16 * t;
-                Z16 acc;
-                z16_zero(acc);
-                z16_gemm<false, false, false>(acc, r0, j0, j0, r0, M0, 1, ld, n, M1, 1, ld, n);
-                z16_store(acc, r0, j0, [&](int i, int j, double2 x) { if (i < n) M1[i + (size_t)j * ld] = x; });
-            }
-            __syncthreads();
-            for (int c = tid; c < re; c += kNT) {
-                double2 x[16];
-#pragma unroll
-                for (int r = 0; r < 16; ++r) {
-                    const int i = r0 + r;
-                    x[r] = (i < re) ? ((c < r0) ? cneg(M1[i + (size_t)c * ld]) : c2(i == c ? 1.0 : 0.0, 0.0))
-                                    : zero;
-                }
-#pragma unroll
-                for (int r = 0; r < 16; ++r) {
-                    const int i = r0 + r;
-                    if (i < re) {
-                        double2 s = x[r];
-#pragma unroll
-                        for (int q = 0; q < r; ++q) s = cfms(s, M0[i + (size_t)(r0 + q) * ld], x[q]);
-                        x[r] = cscale(s, v.rdg[i]);
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < 16; ++r)
-                    if (r0 + r < re) M1[r0 + r + (size_t)c * ld] = x[r];
-            }
-            __syncthreads();
-        }
+        // ---- a3: X = L^-1 -> M1
+        tiled_inverse<kNT>(n, ld, M0, M1, v.rdg);
         phase_mark(18);
     }
 
@@ -554,46 +871,8 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
     }
 
     if (!code) {
-        // ---- a4: T = H X^H -> M2, T(i, j) = sum_{k <= j} H(i, k) conj(X(j, k))
-        if (a.sigma) {
-            const int m = n >> 1;
-            for (int idx = tid; idx < (int)nn; idx += kNT) {
-                const int j = idx / n, i = idx - j * n;
-                const double2 x = (i <= j) ? cconj(M1[j + (size_t)i * ld]) : zero;
-                M2[i + (size_t)j * ld] = (i < m) ? x : cneg(x);
-            }
-        } else {
-            for (int t = warp; t < tile_blocks(tn, tn); t += kNW) {
-                int ti, tj;
-                if (!tile_at(t, tn, tn, ti, tj)) continue;
-                const int i0 = 16 * ti, j0 = 16 * tj;
-                Z16 acc;
-                z16_zero(acc);
-                z16_gemm<false, false, true>(acc, i0, j0, 0, min(n, j0 + 16), Hb, 1, n, n, M1, ld, 1, n);
-                z16_store(acc, i0, j0, [&](int i, int j, double2 x) {
-                    if (i < n && j < n) M2[i + (size_t)j * ld] = x;
-                });
-            }
-        }
-        __syncthreads();
-        // C = X T, lower tiles; each lower element is written with its
-        // mirror so that C is exactly Hermitian. L in M0 is dead by now.
-        for (int t = warp; t < tile_blocks(tn, tn); t += kNW) {
-            int ti, tj;
-            if (!tile_at(t, tn, tn, ti, tj) || ti < tj) continue;
-            const int i0 = 16 * ti, j0 = 16 * tj;
-            Z16 acc;
-            z16_zero(acc);
-            z16_gemm<false, false, false>(acc, i0, j0, 0, min(n, i0 + 16), M1, 1, ld, n, M2, 1, ld, n);
-            z16_store(acc, i0, j0, [&](int i, int j, double2 x) {
-                if (i < n && j < n && i >= j) {
-                    if (i == j) x.y = 0.0;
-                    M0[i + (size_t)j * ld] = x;
-                    M0[j + (size_t)i * ld] = cconj(x);
-                }
-            });
-        }
-        __syncthreads();
+        // ---- a4: C = X H X^H -> M0
+        tiled_form_c<kNT>(n, ld, a.sigma, Hb, M0, M1, M2);
         phase_mark(19);
     }
 
@@ -704,116 +983,8 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
                 }
                 __syncthreads();
             } else {
-                // thread i owns row i of the vectors and of the panel (kNT >= n)
-                // V and W of the panel: columns Vp + c ld, Wp + c ld
-                double2* Wp = M2;
-                const int i = tid;
-                const bool row = i < n;
-                double* red = reinterpret_cast<double*>(v.red);   // 32 doubles for each of two sums
-                double2* t12 = v.tb;                               // W^H v at [0, c), V^H v at [16, 16 + c)
-                // (the divide and conquer's scratch is free until then: 2 n complex of its 7 n + 1 doubles)
-                double2* yx = reinterpret_cast<double2*>(v.dcd + (n & 1));
-                double2* const ydot[4] = {v.pb, v.gb, yx, yx + n};
-                for (int p = 0; p < n - 1; p += 16) {
-                    const int w = min(16, n - 1 - p);
-                    double2* Vp = M0 + (size_t)p * ld;
-                    for (int c = 0; c < w; ++c) {
-                        const int k = p + c;
-                        // (1) column k of the current matrix:
-                        // a_k -= V(:, 0:c) W(k, 0:c)^H + W(:, 0:c) V(k, 0:c)^H
-                        // (rows k .. n-1 of V are stored whole)
-                        double2 x = zero;
-                        if (row && i >= k) {
-                            x = M0[i + (size_t)k * ld];
-#pragma unroll 4
-                            for (int cc = 0; cc < c; ++cc) {
-                                x = cfms_bc(x, Vp[i + cc * ld], Wp[k + cc * ld]);
-                                x = cfms_bc(x, Wp[i + cc * ld], Vp[k + cc * ld]);
-                            }
-                        }
-                        if (i == k) { v.d[k] = x.x; M0[k + (size_t)k * ld] = x; }
-                        if (i == k + 1) v.gb[0] = x;
-                        // (2) reflector from a_k(k+1:n)
-                        const double ss = cta_sum<kNT>((row && i > k + 1) ? fma(x.x, x.x, x.y * x.y) : 0.0, red);
-                        const double2 alpha = v.gb[0];
-                        double2 taui = zero, scal = zero;
-                        double beta = alpha.x;
-                        if (!(ss == 0.0 && alpha.y == 0.0)) {
-                            const double nn = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, ss));
-                            const double rn = rsqrt(nn);
-                            beta = -copysign(nn * rn, alpha.x);
-                            const double rb = -copysign(rn, alpha.x);
-                            taui = c2((beta - alpha.x) * rb, -alpha.y * rb);
-                            const double2 z = c2(alpha.x - beta, alpha.y);
-                            const double inv = fast_rcp(fma(z.x, z.x, z.y * z.y));
-                            scal = c2(z.x * inv, -z.y * inv);
-                        }
-                        double2 vi = zero;
-                        if (row && i > k) {
-                            vi = i == k + 1 ? c2(1.0, 0.0) : cmul(x, scal);
-                            v.vb[i] = vi;
-                            M0[i + (size_t)k * ld] = vi;
-                        }
-                        if (tid == 0) { v.tau[k] = taui; v.e[k] = beta; }
-                        __syncthreads();
-                        // (3) y = A v (A: panel-start trailing matrix, lower
-                        // triangle), t1 = W^H v, t2 = V^H v
-                        sym_matvec<kNT>(M0, ld, n, k + 1, v.vb, v.part, ydot, v.ring);
-                        for (int it = warp; it < 2 * c; it += kNW) {
-                            const int cc = it >> 1;
-                            double2 acc = zero;
-                            const double2* col = (it & 1 ? Vp : Wp) + cc * ld;
-#pragma unroll 4
-                            for (int j = k + 1 + lane; j < n; j += 32) acc = cfmac(acc, col[j], v.vb[j]);
-                            acc = warp_sum2(acc);
-                            if (lane == 0) t12[16 * (it & 1) + cc] = acc;
-                        }
-                        __syncthreads();
-                        // (4) w = tau (y - V t1 - W t2) + alpha2 v on rows k+1..n (the
-                        // current matrix is A - V W^H - W V^H), alpha2 =
-                        // -tau/2 (w^H v) = -|tau|^2/2 v^H A v; zero above
-                        double2 y = zero;
-                        if (row && i > k) {
-                            y = sym_matvec_row<kNT>(n, k + 1, i, v.part, ydot);
-#pragma unroll 4
-                            for (int cc = 0; cc < c; ++cc) {
-                                y = cfms(y, Vp[i + cc * ld], t12[cc]);
-                                y = cfms(y, Wp[i + cc * ld], t12[16 + cc]);
-                            }
-                        }
-                        const double h = -0.5 * fma(taui.x, taui.x, taui.y * taui.y) *
-                                         cta_sum<kNT>(fma(y.x, vi.x, y.y * vi.y), red + 32);
-                        if (row) {
-                            const double2 wt = cmul(taui, y);
-                            Wp[i + c * ld] = c2(fma(h, vi.x, wt.x), fma(h, vi.y, wt.y));
-                        }
-                        __syncthreads();
-                    }
-                    // trailing update, lower tiles: A(q:n, q:n) -= V W^H + W V^H, q = p + w
-                    const int q = p + w, mq = n - q;
-                    if (mq > 0) {
-                        const int tq = (mq + 15) >> 4;
-                        for (int t = warp; t < tile_blocks(tq, tq); t += kNW) {
-                            int ti, tj;
-                            if (!tile_at(t, tq, tq, ti, tj) || ti < tj) continue;
-                            const int i0 = q + 16 * ti, j0 = q + 16 * tj;
-                            Z16 acc;
-                            z16_load(acc, i0, j0, [&](int r, int j) { return (r < n && j < n) ? M0[r + (size_t)j * ld] : zero; });
-                            z16_gemm<false, true, true>(acc, i0, j0, 0, w, Vp, 1, ld, n, Wp, ld, 1, n);
-                            z16_gemm<false, true, true>(acc, i0, j0, 0, w, Wp, 1, ld, n, Vp, ld, 1, n);
-                            z16_store(acc, i0, j0, [&](int r, int j, double2 x) {
-                                if (r < n && j < n && r >= j) M0[r + (size_t)j * ld] = x;
-                            });
-                        }
-                    }
-                    __syncthreads();
-                }
+                tiled_house<kNT>(n, ld, M0, M2, smem_raw);
             }
-            if (!use32 && tid == 0) {
-                v.d[n - 1] = M0[(n - 1) + (size_t)(n - 1) * ld].x;
-                if (n == 1) v.tau[0] = zero;
-            }
-            __syncthreads();
             phase_mark(20);
 
             // ---- a5b: divide and conquer on T: Z in M2 (real), its merge
@@ -851,92 +1022,22 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
         }
         __syncthreads();
         const int nref = n - 1;
-        for (int kb = nref > 0 ? ((nref - 1) / 16) * 16 : -1; kb >= 0; kb -= 16) {
-            const int w = min(16, nref - kb);
-            // Y(i, c) = v_{kb+c}(i): 0 above row kb+c+1, 1 there, stored below
-            auto Y = [&](int i, int c) -> double2 {
-                if (c >= w || i >= n) return zero;
-                const int k = kb + c;
-                return (i <= k) ? zero : (i == k + 1) ? c2(1.0, 0.0)
-                     : use32 ? f2d(C32[i + (size_t)k * ld]) : M0[i + (size_t)k * ld];
-            };
-            if (tid < 256) v.tb[tid] = zero;
-            // G = Y^H Y: warps 0 and 1 each sum half of the rows, and the two
-            // halves are added in a fixed order (results are bitwise
-            // reproducible from launch to launch)
-            if (warp < 2) {
-                const int r0 = kb + 1, rows = n - r0;
-                const int per = ((rows + 7) / 8) * 4;
-                const int k0 = r0 + warp * per, k1 = min(n, k0 + per);
-                Z16 acc;
-                z16_zero(acc);
-                z16_mma(acc, 0, 0, k0, k1, [&](int c, int i) { return cconj(Y(i, c)); },
-                        [&](int i, int c) { return Y(i, c); });
-                z16_store(acc, 0, 0, [&](int i, int j, double2 x) { v.gb[256 * warp + i + 16 * j] = x; });
-            }
+        {
+            // Y with its ones and zeros in place, so that the products need
+            // no masks: over the reduced C, or, for the mixed form, which
+            // still needs C, widened from the FP32 reduction into M3
+            double2* Y = use32 ? M3 : M0;
+            for (int k = warp; k < nref; k += kNW)
+                for (int i = lane; i < n; i += 32)
+                    if (use32 || i <= k + 1)
+                        Y[i + (size_t)k * ld] = i <= k ? zero : i == k + 1 ? c2(1.0, 0.0) : f2d(C32[i + (size_t)k * ld]);
             __syncthreads();
-            if (tid < 256) v.gb[tid] = cadd(v.gb[tid], v.gb[256 + tid]);
-            __syncthreads();
-            // T_b (upper triangular, forward column-wise): T(j, j) = tau_j,
-            // T(0:j, j) = T(0:j, 0:j) (-tau_j G(0:j, j))
-            if (warp == 0) {
-                for (int j = 0; j < w; ++j) {
-                    const double2 tj = v.tau[kb + j];
-                    const double2 y = (lane < j) ? cneg(cmul(tj, v.gb[lane + 16 * j])) : zero;
-                    double2 s = zero;
-                    for (int l = 0; l < j; ++l) {
-                        const double2 yl = c2(__shfl_sync(0xffffffffu, y.x, l), __shfl_sync(0xffffffffu, y.y, l));
-                        if (lane <= l) s = cfma(s, v.tb[lane + 16 * l], yl);
-                    }
-                    if (lane < j) v.tb[lane + 16 * j] = s;
-                    if (lane == j) v.tb[j + 16 * j] = tj;
-                    __syncwarp();
-                }
-            }
-            __syncthreads();
-            // W1 = Y^H V (16 x n) then W2 = T_b W1 in place, one column tile per warp
-            for (int t = warp; t < tn; t += kNW) {
-                const int j0 = 16 * t;
-                Z16 acc;
-                z16_zero(acc);
-                if (use32) {
-                    z16_mma(acc, 0, j0, kb + 1, n, [&](int c, int i) { return cconj(Y(i, c)); },
-                            [&](int i, int j) { return j < n ? Ub[i + (size_t)j * n] : zero; });
-                } else {
-                    // the triangle of Y's first rows, then its full columns
-                    const int kt = min(n, kb + 17);
-                    z16_mma(acc, 0, j0, kb + 1, kt, [&](int c, int i) { return cconj(Y(i, c)); },
-                            [&](int i, int j) { return j < n ? Ub[i + (size_t)j * n] : zero; });
-                    if (kt < n)
-                        z16_gemm<true, false, false>(acc, 0, j0, kt, n, M0 + (size_t)kb * ld, ld, 1, w, Ub, 1, n, n);
-                }
-                z16_store(acc, 0, j0, [&](int c, int j, double2 x) { if (j < n) Wsc[c + 16 * j] = x; });
-                __syncwarp();
-                Z16 acc2;
-                z16_zero(acc2);
-                z16_mma(acc2, 0, j0, 0, 16, [&](int c, int l) { return v.tb[c + 16 * l]; },
-                        [&](int l, int j) { return j < n ? Wsc[l + 16 * j] : zero; });
-                __syncwarp();
-                z16_store(acc2, 0, j0, [&](int c, int j, double2 x) { if (j < n) Wsc[c + 16 * j] = x; });
-            }
-            __syncthreads();
-            // V -= Y W2 on rows kb+1..n
-            const int rt0 = (kb + 1) >> 4, T = (tn - rt0) * tn;
-            for (int t = warp; t < T; t += kNW) {
-                const int ti = rt0 + t / tn, tj = t % tn, i0 = 16 * ti, j0 = 16 * tj;
-                Z16 acc;
-                z16_load(acc, i0, j0, [&](int i, int j) { return (i < n && j < n) ? Ub[i + (size_t)j * n] : zero; });
-                if (use32 || i0 <= kb + 16)
-                    z16_mma(acc, i0, j0, 0, 16, [&](int i, int c) { return cneg(Y(i, c)); },
-                            [&](int c, int j) { return j < n ? Wsc[c + 16 * j] : zero; });
-                else
-                    z16_gemm<false, true, false>(acc, i0, j0, 0, w, M0 + (size_t)kb * ld, 1, ld, n, Wsc, 1, 16, n);
-                z16_store(acc, i0, j0, [&](int i, int j, double2 x) {
-                    if (i < n && j < n) Ub[i + (size_t)j * n] = x;
-                });
-            }
+            // (M2 is free: Z is in the output; it holds the factors' 24 n from
+            // n = 34 on, tb and gb three of them)
+            wy_apply<kNT>(Ub, n, Y, ld, nref, v.tau, nref > 32 ? M2 : v.tb);
             __syncthreads();
         }
+        if (use32) phase_mark(22);
 
         if (use32) {
             // ---- a5d: Ogita-Aishima refinement in FP64 of the eigenpairs of
@@ -1091,7 +1192,7 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
 
         break;
     }
-    phase_mark(22);
+    phase_mark(use32 ? 25 : 22);
     if (code) {
         const double qnan = __longlong_as_double(0x7ff8000000000000LL);
         for (int idx = tid; idx < (int)nn; idx += kNT) Ub[idx] = c2(qnan, qnan);

@@ -31,8 +31,8 @@ PHASES = {
     # l2-slot (tiled) kernel
     16: "tiled a1 load S", 17: "tiled a2 blocked Cholesky", 18: "tiled a3 X = L^-1",
     19: "tiled a4 T = H X^H, C = X T", 20: "tiled a5a Householder", 21: "tiled a5b D&C tail + rank",
-    22: "tiled a5c WY back-transform (+ mixed refinement)", 23: "tiled a6 U = X^H V",
-    24: "tiled a7 store U (+ loop barrier)",
+    22: "tiled a5c WY back-transform", 23: "tiled a6 U = X^H V",
+    24: "tiled a7 store U (+ loop barrier)", 25: "tiled a5d mixed refinement",
 }
 #: event-counter slots (counts, not cycles)
 COUNTERS = {27: "D&C secular iterations", 28: "D&C secular iterations, slowest root per level",
