@@ -43,12 +43,18 @@ namespace sgeig {
 using namespace tiled;
 namespace {
 
-template <int NT>
+template <int NT, bool MIXED>
 __global__ void __launch_bounds__(NT, NT == kTiledWide ? 1 : 2) geneig_tiled_kernel(TiledArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double2* slot = a.scratch + (size_t)blockIdx.x * tiled_slot_elems(a.n, a.mixed != 0);
+    double2* slot = a.scratch + (size_t)blockIdx.x * tiled_slot_elems(a.n, MIXED);
     phase_start();
-    for (long long b = blockIdx.x; b < a.batch; b += gridDim.x) tiled_solve<NT>(a, b, slot, smem_raw);
+    for (long long b = blockIdx.x; b < a.batch; b += gridDim.x) tiled_solve<NT, MIXED>(a, b, slot, smem_raw);
+}
+
+using TiledKernelFn = void (*)(TiledArgs);
+TiledKernelFn tiled_kernel(int n, bool mixed) {
+    if (tiled_threads(n) == kTiledWide) return mixed ? geneig_tiled_kernel<kTiledWide, true> : geneig_tiled_kernel<kTiledWide, false>;
+    return mixed ? geneig_tiled_kernel<kTiledNarrow, true> : geneig_tiled_kernel<kTiledNarrow, false>;
 }
 
 }  // namespace
@@ -60,7 +66,8 @@ size_t tiled_vec_bytes(int n, bool work) { return tiled_base_bytes(n) + (work ? 
 // `smem` is the per-CTA shared-memory limit; the kernel's own static shared
 // memory (profiling builds have some) comes off the dynamic allowance.
 cudaError_t tiled_set_attributes(size_t smem) {
-    for (auto k : {geneig_tiled_kernel<kTiledNarrow>, geneig_tiled_kernel<kTiledWide>}) {
+    for (auto k : {tiled_kernel(1, false), tiled_kernel(1, true), tiled_kernel(kResidentMaxN + 1, false),
+                   tiled_kernel(kResidentMaxN + 1, true)}) {
         cudaFuncAttributes fa{};
         cudaError_t e = cudaFuncGetAttributes(&fa, k);
         if (e == cudaSuccess)
@@ -86,14 +93,13 @@ cudaError_t tiled_launch(int n, int slots, int stage, const void* H, const void*
     a.ld = n | 1;
     a.stage = stage;
     a.sigma = sigma ? 1 : 0;
-    a.mixed = mixed ? 1 : 0;
     a.refine_max = refine_max;
     a.defer = defer ? 1 : 0;
     a.work = defer ? 0 : 1;
-    const size_t smem = tiled_vec_bytes(n, !defer);
+    a.keep32 = defer && tiled_keep32(n) ? 1 : 0;
+    const size_t smem = tiled_vec_bytes(n, !defer) + (a.keep32 ? tiled_c32_bytes(n) : 0);
     const long long grid = batch < slots ? batch : slots;
-    if (tiled_threads(n) == kTiledWide) geneig_tiled_kernel<kTiledWide><<<(unsigned)grid, kTiledWide, smem, stream>>>(a);
-    else geneig_tiled_kernel<kTiledNarrow><<<(unsigned)grid, kTiledNarrow, smem, stream>>>(a);
+    tiled_kernel(n, mixed)<<<(unsigned)grid, tiled_threads(n), smem, stream>>>(a);
     return cudaGetLastError();
 }
 

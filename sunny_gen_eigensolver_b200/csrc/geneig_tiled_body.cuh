@@ -34,10 +34,10 @@ struct TiledArgs {
     long long batch;
     int n, ld, stage;
     int sigma;      // H = diag(I_{n/2}, -I_{n/2}), not read from memory
-    int mixed;      // FP32 Householder reduction + FP64 refinement
     int refine_max; // mixed: refinement steps before the FP64 fallback
     int defer;      // mixed: leave the fallback to the shared-memory kernel (info = kRetryInfo)
     int work;       // the launch's shared memory has the work area (tiled_work_elems)
+    int keep32;     // mixed: it has the FP32 copy of C instead (tiled_keep32)
 };
 
 // Ogita-Aishima refinement of the mixed form: it stops as soon as the current
@@ -121,6 +121,14 @@ __host__ __device__ inline size_t tiled_base_bytes(int n) {
     const size_t b = (size_t)n * 16 * 3 + 32 * 16 + 3 * 256 * 16 + (size_t)n * 8 * 3 + (size_t)dc_vec_doubles(n) * 8 +
                      (size_t)n * 4 + 8 * 4 + (size_t)dc_vec_ints(n) * 4;
     return (b + 15) & ~(size_t)15;
+}
+
+// The FP32 copy of C in the same place, for launches of the mixed form without
+// the work area and with two CTAs per SM (up to N = 101). N=54: the reduction
+// takes 333 K cycles on a copy in global memory, 191 K here.
+__host__ __device__ inline size_t tiled_c32_bytes(int n) { return ((size_t)n * (n | 1) * 8 + 15) & ~(size_t)15; }
+__host__ __device__ inline bool tiled_keep32(int n) {
+    return n <= kResidentMaxN && tiled_base_bytes(n) + tiled_c32_bytes(n) <= 112 * 1024;
 }
 
 __device__ inline TVec tcarve(unsigned char* p, int n) {
@@ -767,16 +775,145 @@ __device__ __forceinline__ void tiled_house(int n, int ld, double2* M0, double2*
     __syncthreads();
 }
 
+// Mixed form: the reduction of the FP32 copy of C (in shared memory, n <= 128),
+// by the smem-cta kernel's scheme: per step one warp forms w and the next
+// reflector from the partial products, then every warp, over its block of 32
+// rows and its class of columns, applies A -= v w^H + w v^H and multiplies the
+// updated elements by the new reflector in the same pass. Two barriers a step.
+// Reflectors stay in C32's columns; tau, d, e widened to FP64. part: 32 pairs
+// per warp, vb: 2 n, wb: n.
+template <int kNT>
+__device__ __forceinline__ void house32(int n, int ld, float2* C32, float2* part, float2* vb, float2* wb, double2* tauv,
+                                        double* dv, double* ev) {
+    constexpr int NW = kNT / 32, R = 4;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int last = n - 1 - lane;                 // row of block t: last - 32 t
+    const float2 zero = f2(0.0f, 0.0f);
+    for (int i = tid; i < n; i += kNT) vb[n + i] = wb[i] = zero;
+    __syncthreads();
+    int rb = 0, G = 0, myt = 0, myg = 0;
+    float2 tau = zero;                             // of reflector c - 1
+#pragma unroll 1
+    for (int c = 0; c < n; ++c) {
+        const float2* vk = vb + ((c + 1) & 1) * n;
+        float2* vc = vb + (c & 1) * n;
+        if (warp == 0) {
+            float2 x[R], w[R];
+            float2* mc = C32 + c * ld;
+            const int ic = n - 1 - c;              // slot of row c
+#pragma unroll
+            for (int t = 0; t < R; ++t) x[t] = mc[max(last - 32 * t, 0)];
+            if (c > 0) {
+                float2 v[R];
+                float s = 0.0f;
+#pragma unroll
+                for (int t = 0; t < R; ++t) {
+                    v[t] = vk[max(last - 32 * t, 0)];
+                    w[t] = zero;
+                }
+                const float2* pt = part + lane;
+#pragma unroll 2
+                for (int g = 0; g < G; ++g, pt += 32 * rb)
+#pragma unroll
+                    for (int t = 0; t < R; ++t)
+                        if (t < rb) w[t] = f2(w[t].x + pt[32 * t].x, w[t].y + pt[32 * t].y);
+#pragma unroll
+                for (int t = 0; t < R; ++t) s = fmaf(w[t].x, v[t].x, fmaf(w[t].y, v[t].y, s));
+                const float h = -0.5f * fmaf(tau.x, tau.x, tau.y * tau.y) * warp_sumf(s);
+                float2 wc = zero;
+#pragma unroll
+                for (int t = 0; t < R; ++t) {
+                    w[t] = fcmul(tau, w[t]);
+                    w[t] = f2(fmaf(h, v[t].x, w[t].x), fmaf(h, v[t].y, w[t].y));
+                    if (last - 32 * t >= 0) wb[last - 32 * t] = w[t];
+                    if ((ic >> 5) == t) wc = w[t];
+                }
+                wc = f2(__shfl_sync(0xffffffffu, wc.x, ic & 31), __shfl_sync(0xffffffffu, wc.y, ic & 31));
+#pragma unroll
+                for (int t = 0; t < R; ++t) {
+                    x[t] = fcfms_bc(x[t], v[t], wc);
+                    x[t] = f2(x[t].x - w[t].x, x[t].y - w[t].y);         // v(c) = 1
+                }
+            }
+            float2 xc = x[0], alpha = x[0];
+#pragma unroll
+            for (int t = 1; t < R; ++t) {
+                if ((ic >> 5) == t) xc = x[t];
+                if (((ic - 1) >> 5) == t) alpha = x[t];
+            }
+            float beta = 0.0f;
+            if (c < n - 1) {
+                alpha = f2(__shfl_sync(0xffffffffu, alpha.x, (ic - 1) & 31), __shfl_sync(0xffffffffu, alpha.y, (ic - 1) & 31));
+                float ss = 0.0f;
+#pragma unroll
+                for (int t = 0; t < R; ++t) {
+                    if (last - 32 * t <= c + 1) x[t] = zero;
+                    ss = fmaf(x[t].x, x[t].x, fmaf(x[t].y, x[t].y, ss));
+                }
+                ss = warp_sumf(ss);
+                float2 scal = zero;
+                tau = zero;
+                beta = alpha.x;
+                if (!(ss == 0.0f && alpha.y == 0.0f)) {
+                    beta = -copysignf(sqrtf(alpha.x * alpha.x + alpha.y * alpha.y + ss), alpha.x);
+                    tau = f2((beta - alpha.x) / beta, -alpha.y / beta);
+                    const float2 z = f2(alpha.x - beta, alpha.y);
+                    const float inv = 1.0f / (z.x * z.x + z.y * z.y);
+                    scal = f2(z.x * inv, -z.y * inv);
+                }
+#pragma unroll
+                for (int t = 0; t < R; ++t) {
+                    const int i = last - 32 * t;
+                    x[t] = fcmul(x[t], scal);
+                    if (i >= 0) vc[i] = i == c + 1 ? f2(1.0f, 0.0f) : x[t];
+                    if (i > c + 1) mc[i] = x[t];
+                }
+                if (lane == 0) tauv[c] = f2d(tau);
+            }
+            if (lane == (ic & 31)) {
+                dv[c] = (double)xc.x;
+                if (c < n - 1) ev[c] = (double)beta;
+            }
+        }
+        if (c >= n - 1) break;
+        __syncthreads();
+        if (const int r = (n - 1 - c + 31) >> 5; r != rb) {
+            rb = r;
+            G = NW / rb;
+            myg = warp / rb;
+            myt = warp - myg * rb;
+        }
+        if (myg < G) {
+            const int i = last - 32 * myt, o = max(i, 0);
+            const float2 vi = vk[o], wi = wb[o];
+            float2 y = zero;
+#pragma unroll 4
+            for (int j = c + 1 + myg; j < n; j += G) {
+                float2* q = C32 + o + j * ld;
+                const float2 z = fcfms_bc(fcfms_bc(*q, vi, wb[j]), wi, vk[j]);
+                if (i >= 0) *q = z;
+                y = fcfma(y, z, vc[j]);
+            }
+            part[32 * (myg * rb + myt) + lane] = y;
+        }
+        __syncthreads();
+    }
+    if (n == 1 && tid == 0) tauv[0] = c2(0.0, 0.0);
+    __syncthreads();
+}
+
 // One pencil b, solved end to end by the whole CTA in its global-memory
 // slot `slot` (tiled_slot_elems(n, mixed) complex entries) with the
 // launch's dynamic shared memory as the vector area. kNT >= n.
-template <int kNT>
+// MIXED: FP32 Householder reduction + FP64 refinement, an instance of its own
+// so that the FP64 form does not carry its pointers (n = 216: 1.6 %).
+template <int kNT, bool MIXED>
 __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long long b, double2* slot,
                                             unsigned char* smem_raw) {
     constexpr int kNW = kNT / 32;
     const int n = a.n, ld = a.ld;
     const size_t mat = (size_t)n * ld;
-    const bool mixed = a.mixed != 0;
+    constexpr bool mixed = MIXED;
     double2* M0 = slot;
     double2* M1 = M0 + mat;
     double2* M2 = M1 + mat;
@@ -785,9 +922,10 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
     double*  Zo = reinterpret_cast<double*>(zob);
     // mixed only: FP32 copy of C after Zo; after the back-transform Zo and
     // it together hold one more n x ld complex matrix (M4)
-    float2*  C32 = reinterpret_cast<float2*>(zob + tiled_zo_elems(n));
     double2* M4 = zob;
     TVec v = tcarve(smem_raw, n);
+    float2*  C32s = reinterpret_cast<float2*>(v.part);             // a.keep32
+    float2*  C32 = reinterpret_cast<float2*>(zob + tiled_zo_elems(n));
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tn = (n + 15) >> 4;
@@ -903,11 +1041,18 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
                 // single-precision copy of C (reflectors kept in its columns;
                 // tau, d, e widened to FP64). C itself stays in M0 for the
                 // refinement. The vectors live in pb's storage as float2.
-                for (int idx = tid; idx < (int)nn; idx += kNT) {
-                    const int j = idx / n, i = idx - j * n;
-                    const double2 x = M0[i + (size_t)j * ld];
-                    C32[i + (size_t)j * ld] = f2((float)x.x, (float)x.y);
-                }
+                for (int j = warp; j < n; j += kNW)
+                    for (int i = lane; i < n; i += 32) {
+                        const double2 x = M0[i + (size_t)j * ld];
+                        const float2 f = f2((float)x.x, (float)x.y);
+                        if (a.keep32) C32s[i + j * ld] = f;
+                        else C32[i + (size_t)j * ld] = f;
+                    }
+                if (a.keep32) {
+                    __syncthreads();
+                    house32<kNT>(n, ld, C32s, reinterpret_cast<float2*>(v.gb), reinterpret_cast<float2*>(v.vb),
+                                 reinterpret_cast<float2*>(v.pb), v.tau, v.d, v.e);
+                } else {
                 float2* vbf = reinterpret_cast<float2*>(v.pb);
                 float2* pbf = vbf + n;
                 const float2 fz = f2(0.0f, 0.0f);
@@ -982,6 +1127,7 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
                     if (n == 1) v.tau[0] = zero;
                 }
                 __syncthreads();
+                }
             } else {
                 tiled_house<kNT>(n, ld, M0, M2, smem_raw);
             }
@@ -1030,7 +1176,8 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
             for (int k = warp; k < nref; k += kNW)
                 for (int i = lane; i < n; i += 32)
                     if (use32 || i <= k + 1)
-                        Y[i + (size_t)k * ld] = i <= k ? zero : i == k + 1 ? c2(1.0, 0.0) : f2d(C32[i + (size_t)k * ld]);
+                        Y[i + (size_t)k * ld] = i <= k ? zero : i == k + 1 ? c2(1.0, 0.0)
+                                              : f2d(a.keep32 ? C32s[i + k * ld] : C32[i + (size_t)k * ld]);
             __syncthreads();
             // (M2 is free: Z is in the output; it holds the factors' 24 n from
             // n = 34 on, tb and gb three of them)
