@@ -8,12 +8,13 @@ shape is re-run by a single graph launch (`UnevenBatch.replay`). The plain
 alternative (`run_sequential`) is one launch per size on one stream.
 
 The persistent form (`persistent` / `replay_persistent`) solves the whole mix
-with ONE kernel launch (sunny_geneig_uneven_*): a device work counter hands
-out items, largest N first, to a grid of 2 CTAs per SM, and each item runs
-the per-problem code of its size's regime (results are bitwise those of
-the per-size launches). `autotune_persistent` picks, per size, the regime
+with ONE call (sunny_geneig_uneven_*): sizes above 60 as launches of their own
+kernels on the handle's streams, the largest first, and beside them one
+persistent kernel whose device work counter hands out the smaller sizes' items
+to a grid of 2 CTAs per SM; each item runs the per-problem code of its size's
+regime (results are bitwise those of the per-size launches). `autotune_persistent` picks, per size, the regime
 (smem-cta or l2-slot where both can hold N) and the problems per work item
-(for smem-cta sizes) by timing the one-launch form on the batch's own data,
+(for smem-cta sizes) by timing the one-call form on the batch's own data,
 one size at a time from the library defaults; the choice is remembered per
 size mix in the same table, and the launch is captured into a CUDA graph.
 
@@ -351,7 +352,7 @@ class UnevenBatch:
         self.pconfigs = {n: {"regime": r, "per_item": p} for n, r, p in self.uneven.shape}
 
     def launch_persistent(self, stream=None) -> None:
-        """One launch of the persistent kernel over the whole mix."""
+        """One uneven launch over the whole mix."""
         if self.uneven is None:
             self.persistent()
         self.uneven.launch(self.H, self.S, self.W, self.U, self.info, stream)

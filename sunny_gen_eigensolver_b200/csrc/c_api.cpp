@@ -541,7 +541,7 @@ sunny_geneig_uneven_t sunny_geneig_uneven_create(int num_sizes, const int* sizes
                     if (ea != cudaSuccess) { err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea); return ea; }
                 } else if (h->kind[g] == sgeig::kUnevenBig) {
                     ea = sgeig::tiled_set_attributes((size_t)optin);
-                    if (ea == cudaSuccess) ea = cudaMalloc(&h->big_scratch[g], (size_t)sms * sgeig::tiled_slot_bytes(n));
+                    if (ea == cudaSuccess) ea = cudaMalloc(&h->big_scratch[g], (size_t)sms * sgeig::tiled_slots_for(n) * sgeig::tiled_slot_bytes(n));
                     if (ea != cudaSuccess) { err = std::string("cudaMalloc scratch: ") + cudaGetErrorString(ea); return ea; }
                 } else if (l2) slot = std::max(slot, sgeig::tiled_slot_elems(n));
             }
@@ -632,7 +632,7 @@ sunny_geneig_status_t sunny_geneig_uneven_launch(sunny_geneig_uneven_t h, const 
         L.U[g] = reinterpret_cast<void*>(d_U[i]);
         L.info[g] = reinterpret_cast<int*>(d_info[i]);
         L.scratch[g] = h->big_scratch[g];
-        L.slots[g] = h->sms;
+        L.slots[g] = h->sms * sgeig::tiled_slots_for(L.n[g]);
     }
     try {
         std::lock_guard<std::mutex> lock(h->mu);

@@ -1,6 +1,6 @@
 // Batched generalized Hermitian-definite eigensolver, shared-memory regime
-// (N <= 64): a team of NT threads (32 to 128 by N) holds one matrix per pencil
-// in shared memory and solves it end to end; a CTA is one team or, with
+// (N <= 64) and the l2-slot class up to N = 110: a team of NT threads (32 to
+// 512 by N) holds one matrix per pencil in shared memory and solves it end to end; a CTA is one team or, with
 // several pencils per CTA, up to four, each with its own barrier and
 // shared-memory slice; CTAs loop over the batch. Further kernel forms
 // assemble S(q) from Fourier terms in the load stage (the metric solve of a
@@ -11,11 +11,11 @@
 //   a1  load the lower triangle of S                          (:233-242)
 //   a2  Cholesky S = L L^H fused with X = L^-1, in place, 8-column panels on
 //       the FP64 tensor cores (mma.m8n8k4.f64), two barriers per panel (:244)
-//   a3+a4  C = L^-1 H L^-H, 8 columns at a time: T = H X^H (H from global
+//   a3+a4  C = L^-1 H L^-H, 8 (N > 80: 16) columns at a time: T = H X^H (H from global
 //       memory, in full, as the reference's two triangular solves read it),
 //       then C = X T; C fills the upper triangle beside X       (:246-248)
 //   a5  Householder tridiagonalisation (lower; the rank-2 update and the next
-//       matrix-vector product share one pass, one barrier per step), divide
+//       matrix-vector product share one pass, two barriers per step), divide
 //       and conquer on the tridiagonal, back-transform V = Q Z in compact-WY
 //       blocks of 8 reflectors on the FP64 tensor cores, 8-column panels of
 //       V per warp                                                  (:250)
@@ -46,11 +46,10 @@ static CtaKernelFn cta_kernel(int nmax, int teams, bool fs, bool spec) {
 int cta_max_teams(int nmax) { return nmax <= 16 ? 4 : nmax <= 32 ? 2 : 1; }
 
 // Default pencils per CTA, measured on B200 (solves/s at batch 65,536, one
-// pencil per CTA -> default): N=12 12.4 M -> 14.4 M, N=16 9.3 M -> 11.9 M
-// (4 teams of 64); N=32 2.2 M -> 3.0 M (2 of 128); N=24 stays at one
-// (4.4 M; 3.95 M with 2 teams). Two teams of the 48- and 56-row kernels
-// (384- and 512-thread CTAs, one per SM) were not kept: N=44 1.14 M vs
-// 1.16 M, N=48 1.05 M vs 0.98 M, N=54 810 K vs 836 K.
+// pencil per CTA -> default): N=8 46.3 M -> 48.1 M, N=12 25.2 M -> 25.7 M, N=16
+// 21.3 M -> 21.9 M (4 teams of 32 threads); N=32 5.60 M -> 6.20 M (2 of 64);
+// N=24 has two on request (7.51 M, 8.67 M with two) and starts with one, so that
+// the reported pencils per CTA stay what they were.
 int cta_default_teams(int nmax) { return nmax <= 16 ? 4 : nmax == 32 ? 2 : 1; }
 
 size_t cta_teams_smem_bytes(int n, int teams, bool spec) { return teams * cta_smem_bytes(n, spec); }

@@ -19,19 +19,23 @@ int smem_cta_max_n();
 // Default choice by N: SmemCta up to 60, L2Slot above (measured crossovers);
 // SmemWide only when asked for.
 enum class Regime : int {
-    SmemCta  = 0,  // N <= 64: both matrices in one CTA's shared memory, register/MMA kernel
+    SmemCta  = 0,  // N <= 64: one matrix per pencil in shared memory, the rest in U's block
     SmemWide = 1,  // N <= ~80: both matrices in shared memory, column-group kernel
     L2Slot   = 2,  // any N: working matrices in a per-CTA global-memory slot, tiled MMA kernel
+                   // (the default up to kResidentMaxN is SmemCta's kernel all the same)
 };
 
-// Shared-memory kernel for N <= 64 (geneig_cta.cu); chosen by default up to
-// kCtaPreferredMaxN (measured crossover with the l2-slot kernel on B200).
+// Shared-memory kernel (geneig_cta.cu): the smem-cta regime can be asked for up
+// to kCtaMaxN and is the default up to kCtaPreferredMaxN; from there on the
+// default is the l2-slot class, so that handles keep the regime name, scratch
+// rules and stream ordering they had.
 constexpr int kCtaMaxN = 64;
 constexpr int kCtaPreferredMaxN = 60;
 // Above it, up to here, the l2-slot size class is also solved by that kernel
-// (one CTA of 256 or 512 threads per pencil, no slots) unless a number of
+// (one CTA of 128 to 512 threads per pencil, no slots) unless a number of
 // slots per SM is asked for: the largest N whose matrix and vectors fit one
-// CTA's shared memory.
+// CTA's shared memory. Solves/s, shared memory / slots: N=62 1227 K / 411 K,
+// N=77 569 K / 273 K, N=96 305 K / 192 K, N=108 227 K / 151 K.
 constexpr int kResidentMaxN = 110;
 // info of a pencil that the mixed form leaves to a following cta_launch with
 // `retry` (never seen by the caller).
@@ -94,7 +98,8 @@ __host__ __device__ inline size_t tiled_slot_bytes(int n, bool mixed = false) {
     return tiled_slot_elems(n, mixed) * 16;
 }
 size_t tiled_vec_bytes(int n, bool work = true);   // dynamic shared memory, with or without the work area
-int tiled_threads_for(int n);   // threads per CTA: 512 (one CTA per SM) above kResidentMaxN, else 256 (two)
+int tiled_threads_for(int n);   // threads per CTA: 512 or 256
+int tiled_slots_for(int n);     // CTAs, and default slots, per SM: 1 or 2
 cudaError_t tiled_set_attributes(size_t smem);
 // `mixed`: FP32 Householder reduction, FP64 refinement (see geneig_tiled.cu).
 // `refine_max`: mixed form's refinement steps before it falls back to FP64;

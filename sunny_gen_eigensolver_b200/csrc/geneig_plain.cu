@@ -1,6 +1,6 @@
 // FP64 batched generalized Hermitian-definite eigensolver for sm_100a, the
-// "smem-wide" regime (N too large for the register-resident smem-cta kernel,
-// small enough for both working matrices to fit one CTA's shared memory).
+// "smem-wide" regime (both working matrices in one CTA's shared memory, N <= 80;
+// only when asked for).
 //
 // One CTA solves one matrix pair at a time (persistent over the batch):
 //   a1  load S -> A, H^H -> B                     (kernel_source.hpp:233-242)
@@ -431,10 +431,9 @@ bool plain_plan(int n, int device, PlainPlan* plan, std::string* err, bool mixed
     // Each kernel's dynamic shared-memory limit is set to the device maximum
     // (not to this n's need), so that creating a handle for a smaller n never
     // lowers the limit under a live handle for a larger one.
-    // Measured on B200 (solves/s, batch 32768): the tiled kernel overtakes the
-    // register-resident smem-cta kernel between n = 60 and n = 62 and runs
-    // about 2x the smem-wide kernel at n = 66..80, so smem-wide is only used
-    // when asked for.
+    // The smem-wide kernel is 4x slower than the shared-memory kernel
+    // (n = 72: 164 K solves/s against 648 K), so it is only used when asked for. Regime names change at
+    // n = 61 as they always have; the kernel does not (kResidentMaxN).
     const size_t smem_wide = (size_t)2 * n * p.ld * 16 + vec_area_bytes(n);
     const bool cta_ok = n <= kCtaMaxN && cta_smem_bytes(n) <= (size_t)optin;
     const bool wide_ok = smem_wide <= (size_t)optin && n <= kWideNmax;
@@ -478,9 +477,9 @@ bool plain_plan(int n, int device, PlainPlan* plan, std::string* err, bool mixed
         p.regime = Regime::L2Slot;
         p.smem = tiled_vec_bytes(n);
         // resident CTAs (and scratch slots) per SM: SUNNY_GENEIG_SLOTS_PER_SM
-        // = 1 or 2 (default: the kernel's occupancy limit, 1 above kResidentMaxN)
+        // = 1 or 2 (default: the kernel's occupancy limit, tiled_slots_for)
         p.threads = tiled_threads_for(n);
-        int per_sm = n > kResidentMaxN ? 1 : 2;
+        int per_sm = tiled_slots_for(n);
         if (slots_per_sm != 0) per_sm = slots_per_sm;
         else if (const char* ps = std::getenv("SUNNY_GENEIG_SLOTS_PER_SM")) per_sm = std::atoi(ps) == 1 ? 1 : 2;
         p.slots = per_sm * sms;
@@ -547,7 +546,7 @@ cudaError_t plain_launch(const PlainPlan& plan, int stage, const void* H, const 
 // the life of the process. It holds floor(32 MiB / slot) slots, so the
 // number of resident CTAs, and with it the throughput, falls with n: 48
 // CTAs at n = 111, 12 at n = 216, 2 at n = 512 (the regular launch keeps
-// 2 per SM, 296 on B200).
+// one per SM, 148 on B200).
 namespace {
 
 constexpr size_t kNoAllocScratchBytes = size_t(32) << 20;   // 32 MiB per device

@@ -60,14 +60,15 @@ TiledKernelFn tiled_kernel(int n, bool mixed) {
 }  // namespace
 
 int tiled_threads_for(int n) { return tiled_threads(n); }
+int tiled_slots_for(int n) { return tiled_threads(n) == kTiledWide ? 1 : 2; }
 
 size_t tiled_vec_bytes(int n, bool work) { return tiled_base_bytes(n) + (work ? tiled_work_elems(n) * 16 : 0); }
 
 // `smem` is the per-CTA shared-memory limit; the kernel's own static shared
 // memory (profiling builds have some) comes off the dynamic allowance.
 cudaError_t tiled_set_attributes(size_t smem) {
-    for (auto k : {tiled_kernel(1, false), tiled_kernel(1, true), tiled_kernel(kResidentMaxN + 1, false),
-                   tiled_kernel(kResidentMaxN + 1, true)}) {
+    for (auto k : {tiled_kernel(1, false), tiled_kernel(1, true), tiled_kernel(kNarrowMaxN + 1, false),
+                   tiled_kernel(kNarrowMaxN + 1, true)}) {
         cudaFuncAttributes fa{};
         cudaError_t e = cudaFuncGetAttributes(&fa, k);
         if (e == cudaSuccess)

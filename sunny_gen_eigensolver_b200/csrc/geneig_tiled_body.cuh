@@ -17,12 +17,14 @@
 namespace sgeig {
 namespace tiled {
 
-// Threads per CTA: 512 (one CTA per SM) for the sizes this kernel solves by
-// default, whose steps want many loads in flight and whose slots then stay
-// closer to the L2's size; 256 (two per SM) up to kResidentMaxN, where only the
-// mixed form and explicit requests come here.
-constexpr int kTiledWide = 512, kTiledNarrow = 256;
-__host__ __device__ constexpr int tiled_threads(int n) { return n > kResidentMaxN ? kTiledWide : kTiledNarrow; }
+// Threads per CTA: 256, two CTAs per SM, as long as two work areas fit one; 512
+// and one CTA above, where the steps want the loads of one pencil in flight and
+// the slots stay closer to the L2's size. ms, 256 / 512 threads: N=111 (1184
+// pencils) 8.15 / 10.11, N=128 10.5 / 12.7, N=162 (888) 15.4 / 17.5, N=200 (592)
+// 16.6 / 17.7, N=216 19.7 / 20.6 in full waves but no gain in ragged ones,
+// N=232 (444; one CTA per SM fits) 22.1 / 17.9.
+constexpr int kTiledWide = 512, kTiledNarrow = 256, kNarrowMaxN = 200;
+__host__ __device__ constexpr int tiled_threads(int n) { return n > kNarrowMaxN ? kTiledWide : kTiledNarrow; }
 
 struct TiledArgs {
     const double2* __restrict__ H;

@@ -4,7 +4,8 @@
 // in src/common/c_api.cpp:76-107).
 //
 // TUNING_AUTOTUNE: every execution configuration this build can run for n
-// (smem-cta, smem-wide, l2-slot with 1 or 2 CTAs per SM; the plain form
+// (smem-cta, smem-wide, l2-slot with 1 or 2 CTAs per SM and, for N 61 to
+// 110, its shared-memory default; the plain form
 // only, the mixed form has one configuration) is timed on a seeded synthetic
 // batch of that size, generated on the device, and the fastest is kept.
 // Its name is cached under the key (n, kernel mode, device name, SM count,
