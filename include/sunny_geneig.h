@@ -60,7 +60,7 @@ typedef enum {
 /* replaces src/common/c_api.h:38-41. SUGGESTED: the execution
  * configuration is chosen by N from measured crossovers. AUTOTUNE: create
  * times every configuration that can hold N (smem-cta, smem-wide, l2-slot
- * with 1 or 2 CTAs per SM) on a seeded synthetic batch on the device and
+ * with 1 or 2 CTAs per SM and by default) on a seeded synthetic batch on the device and
  * keeps the fastest (cached per N, kernel mode, device and library build
  * as the cache mode says); the mixed form has a single configuration. */
 typedef enum {
@@ -271,16 +271,20 @@ sunny_geneig_status_t sunny_geneig_launch_fourier_sigma_intensity(
  * reference; its NVRTC autotuner picked launch shapes inside create).
  * `regime` is "smem-cta", "smem-wide" or "l2-slot" (NULL or "" = the default
  * choice by N); `slots_per_sm` is 1 or 2 resident CTAs per SM for the
- * l2-slot regime (0 = default). A configuration that cannot hold n returns
+ * l2-slot regime (0 = default: for N <= 110 the shared-memory kernel, which
+ * keeps no slots, 2 up to N = 200, then 1). A configuration that cannot hold n returns
  * NULL with the reason in sunny_geneig_last_error(). The uneven-batch
  * autotuner times the candidates per N through this call. */
 sunny_geneig_solver_t sunny_geneig_create_config(int n, int device_id, sunny_geneig_kernel_mode_t kernel_mode,
                                                  const char* regime, int slots_per_sm);
 
-/* Persistent solver for batches of uneven sizes (no counterpart in the
- * reference's C ABI). One launch solves problems of up to 8 different sizes,
+/* Solver for batches of uneven sizes (no counterpart in the
+ * reference's C ABI). One call solves problems of up to 8 different sizes,
  * each size's problems in their own buffers with the layouts, info codes and
- * NaN fill of sunny_geneig_launch: a device work counter hands out work
+ * NaN fill of sunny_geneig_launch. Sizes above 60 run as launches of their
+ * own kernels on streams of the handle, the larger the higher their priority,
+ * forked from and joined to `stream` by events; the smaller ones share a
+ * persistent kernel beside them: a device work counter hands out work
  * items, largest N first, to a grid of 2 CTAs per SM, each item solved by
  * the same per-problem code as that size's own kernel (results are bitwise
  * those of per-size launches in the same regime). A work item is one
@@ -289,8 +293,9 @@ sunny_geneig_solver_t sunny_geneig_create_config(int n, int device_id, sunny_gen
  *   create: sizes[i] distinct, 1 <= sizes[i] <= sunny_geneig_max_matrix_size();
  *     regimes[i] (NULL = all 0): 0 the default choice by N, 1 smem-cta
  *     (N <= 64), 2 l2-slot; per_item[i] (NULL or <= 0 = default: 4 in
- *     smem-cta, 1 in l2-slot). Reserves the l2-slot scratch for the largest
- *     such size and the work counter. NULL on failure (last_error).
+ *     smem-cta, 1 in l2-slot). Reserves the l2-slot scratch (one or two slots
+ *     per SM for each size above 110), the streams and the work counter. NULL on failure
+ *     (last_error).
  *   launch: arrays indexed like `sizes`; counts[i] >= 0 problems of size
  *     sizes[i] (0 skips the size, its buffers may then be NULL). The launch
  *     resets the counter on `stream` first (a memset node when captured).
@@ -312,8 +317,9 @@ int  sunny_geneig_uneven_shape(sunny_geneig_uneven_t solver, int* sizes, int* re
 int sunny_geneig_max_matrix_size(void);
 
 /* Name of the execution regime chosen at create time, e.g. "smem-cta"
- * (both matrices resident in one CTA's shared memory) or "l2-slot"
- * (matrices in a per-CTA global-memory slot). "" for NULL. */
+ * (the pencil's matrix in shared memory) or "l2-slot" (matrices in a per-CTA
+ * global-memory slot; up to N = 110 the default solves this class in shared
+ * memory too). "" for NULL. */
 const char* sunny_geneig_regime_name(sunny_geneig_solver_t solver);
 
 /* Self-test of the device reciprocal the eigensolver uses in place of FP64
