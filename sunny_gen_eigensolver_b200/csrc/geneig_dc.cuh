@@ -78,7 +78,7 @@ struct DCShared {
 __host__ __device__ inline int dc_vec_doubles(int n) { return 7 * n + 1; }
 __host__ __device__ inline int dc_vec_ints(int n) { return 6 * n; }
 
-__host__ __device__ inline int dc_leaf_doubles(int n) { return kLeafStride * kLeaf * ((n + kLeaf - 1) / kLeaf); }
+__host__ __device__ constexpr int dc_leaf_doubles(int n) { return kLeafStride * kLeaf * ((n + kLeaf - 1) / kLeaf); }
 
 // Points the scratch members at `dbl` (dc_vec_doubles(n), eigenvalues first)
 // and `ints` (dc_vec_ints(n)).

@@ -62,6 +62,13 @@ struct VecArea {
     int*     dci;   // divide-and-conquer ints (dc_vec_ints(n))
 };
 
+// Complex entries of B's storage: the matrix, or the rows of the divide and
+// conquer's leaves, which lie there before Z does and take more for n <= 13
+// and n = 17.
+__host__ __device__ constexpr size_t wide_b_elems(int n) {
+    const size_t mat = (size_t)n * (n | 1), leaf = ((size_t)dc_leaf_doubles(n) + 1) / 2;
+    return mat > leaf ? mat : leaf;
+}
 __host__ __device__ inline size_t vec_area_bytes(int n) {
     return (size_t)n * 16 * 3 + 32 * 16 + (size_t)n * 8 * 3 + (size_t)n * 4 + 8 * 4 +
            (size_t)dc_vec_doubles(n) * 8 + (size_t)dc_vec_ints(n) * 4;
@@ -108,7 +115,7 @@ __global__ void __launch_bounds__(kNT, 1) geneig_plain_kernel(PlainArgs a) {
 
     double2* A = reinterpret_cast<double2*>(smem_raw);
     double2* B = A + mat;
-    VecArea v = carve(reinterpret_cast<unsigned char*>(B + mat), n);
+    VecArea v = carve(reinterpret_cast<unsigned char*>(B + wide_b_elems(n)), n);
 
     const int tid  = threadIdx.x;
     const int g    = tid / kG;
@@ -385,14 +392,23 @@ int g_smem_optin = -1;
 
 constexpr int kWideNmax = 96;
 
+// A, B and the vectors.
+size_t wide_smem_bytes(int n) { return ((size_t)n * (n | 1) + wide_b_elems(n)) * 16 + vec_area_bytes(n); }
+
+constexpr bool leaves_fit_b() {
+    for (int n = 1; n <= kWideNmax; ++n)
+        if (2 * wide_b_elems(n) < (size_t)dc_leaf_doubles(n) || wide_b_elems(n) < (size_t)n * (n | 1)) return false;
+    return true;
+}
+static_assert(leaves_fit_b(), "B holds the matrix and the rows of the leaves");
+
 }  // namespace
 
 int smem_cta_max_n() {
     // largest n with 2*n*ld*16 + vectors <= 227 KB (ld = n | 1)
     int best = 0;
     for (int n = 1; n <= kMaxN; ++n) {
-        const int ld = n | 1;
-        const size_t bytes = (size_t)2 * n * ld * 16 + vec_area_bytes(n);
+        const size_t bytes = wide_smem_bytes(n);
         if (bytes <= 232448) best = n;
     }
     return best;
@@ -434,7 +450,7 @@ bool plain_plan(int n, int device, PlainPlan* plan, std::string* err, bool mixed
     // The smem-wide kernel is 4x slower than the shared-memory kernel
     // (n = 72: 164 K solves/s against 648 K), so it is only used when asked for. Regime names change at
     // n = 61 as they always have; the kernel does not (kResidentMaxN).
-    const size_t smem_wide = (size_t)2 * n * p.ld * 16 + vec_area_bytes(n);
+    const size_t smem_wide = wide_smem_bytes(n);
     const bool cta_ok = n <= kCtaMaxN && cta_smem_bytes(n) <= (size_t)optin;
     const bool wide_ok = smem_wide <= (size_t)optin && n <= kWideNmax;
     p.mixed = mixed;
