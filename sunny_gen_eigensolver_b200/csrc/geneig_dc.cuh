@@ -48,6 +48,11 @@ namespace sgeig {
 
 constexpr int kLeaf = 8;          // rows of a leaf
 constexpr int kLeafStride = 25;   // d, e and a row of z of a lane's leaf (odd: no bank conflicts)
+// Off-diagonals of the scaled T (max |T_ij| in [0.5, 1)) up to this are zero to
+// a leaf whatever its diagonal is, and so is a rotation's pair whose squares sum
+// to no more than its third power: squares that underflow lose the rotation's
+// bits, and beside a zero diagonal nothing is negligible by comparison.
+constexpr double kLeafTiny = 1e-100;
 constexpr int kRowsTracked = 8;   // ROWS: first row, last row, 6 caller rows per column slot
 
 struct DCShared {
@@ -389,7 +394,7 @@ __device__ __forceinline__ bool leaf_ql(int m, double* d, double* e, double* z) 
     unsigned small = ~0u << (m - 1);                           // bit i: e[i] is negligible
 #pragma unroll 1
     for (int i = 0; i < m - 1; ++i)
-        if (fabs(e[i]) <= kEps * (fabs(d[i]) + fabs(d[i + 1]))) small |= 1u << i;
+        if (fabs(e[i]) <= fma(kEps, fabs(d[i]) + fabs(d[i + 1]), kLeafTiny)) small |= 1u << i;
 #pragma unroll 1
     for (int it = 0; it < 30 * kLeaf; ++it) {
         if (small == ~0u) return true;
@@ -408,7 +413,9 @@ __device__ __forceinline__ bool leaf_ql(int m, double* d, double* e, double* z) 
             const double ei = e[i], di = d[i], zi = z[i];
             const double f = s * ei, b = c * ei;
             const double q = fma(f, f, g * g);
-            if (q == 0.0) break;                               // the chase ended early: the block splits here
+            // the chase ended early: the block splits here (never at the first
+            // rotation, whose f is above kLeafTiny)
+            if (q <= kLeafTiny * kLeafTiny * kLeafTiny) break;
             const double inv = rsqrt(q), en = q * inv;
             e[i + 1] = en;
             s = f * inv;
@@ -424,7 +431,7 @@ __device__ __forceinline__ bool leaf_ql(int m, double* d, double* e, double* z) 
             dnext = di;
             // e[i + 1] against its new neighbours (not for the first
             // rotation: e[top] is outside the block)
-            if (i + 1 < top && en <= kEps * (fabs(dn) + dabove)) small |= 2u << i;
+            if (i + 1 < top && en <= fma(kEps, fabs(dn) + dabove, kLeafTiny)) small |= 2u << i;
             dabove = fabs(dn);
         }
         const double dn = dnext - p;
@@ -432,8 +439,9 @@ __device__ __forceinline__ bool leaf_ql(int m, double* d, double* e, double* z) 
         d[i + 1] = dn;
         if (i < l) {
             e[l] = g;
-            if (fabs(g) <= kEps * (fabs(dn) + dabove)) small |= 1u << l;
+            if (fabs(g) <= fma(kEps, fabs(dn) + dabove, kLeafTiny)) small |= 1u << l;
         } else {
+            e[i] *= c;                                         // the last rotation's share
             e[i + 1] = 0.0;
             small |= 2u << i;
         }
