@@ -50,9 +50,9 @@ constexpr int kLeaf = 8;          // rows of a leaf
 constexpr int kLeafStride = 25;   // d, e and a row of z of a lane's leaf (odd: no bank conflicts)
 // Off-diagonals of the scaled T (max |T_ij| in [0.5, 1)) up to this are zero to
 // a leaf whatever its diagonal is, and so is a rotation's pair whose squares sum
-// to no more than its third power: squares that underflow lose the rotation's
-// bits, and beside a zero diagonal nothing is negligible by comparison.
-constexpr double kLeafTiny = 1e-100;
+// to less than 2^-996 (1e-300): squares that underflow lose the rotation's bits,
+// and beside a zero diagonal nothing is negligible by comparison.
+constexpr double kLeafTiny = 0x1p-332;
 constexpr int kRowsTracked = 8;   // ROWS: first row, last row, 6 caller rows per column slot
 
 struct DCShared {
@@ -394,7 +394,7 @@ __device__ __forceinline__ bool leaf_ql(int m, double* d, double* e, double* z) 
     unsigned small = ~0u << (m - 1);                           // bit i: e[i] is negligible
 #pragma unroll 1
     for (int i = 0; i < m - 1; ++i)
-        if (fabs(e[i]) <= fma(kEps, fabs(d[i]) + fabs(d[i + 1]), kLeafTiny)) small |= 1u << i;
+        if (fabs(e[i]) <= kEps * (fabs(d[i]) + fabs(d[i + 1])) + kLeafTiny) small |= 1u << i;
 #pragma unroll 1
     for (int it = 0; it < 30 * kLeaf; ++it) {
         if (small == ~0u) return true;
@@ -406,7 +406,7 @@ __device__ __forceinline__ bool leaf_ql(int m, double* d, double* e, double* z) 
         const double h2 = fma(hd, hd, el * el);
         const double qs = hd + copysign(h2 > 0.0 ? h2 * rsqrt(h2) : 0.0, hd);
         double g = dnext - dl + (qs != 0.0 ? el * el * fast_rcp(qs) : 0.0);
-        double s = 1.0, c = 1.0, p = 0.0, dabove = 0.0;        // |d| above the last rotation
+        double s = 1.0, c = 1.0, p = 0.0, dabove = 0.0;        // |d| above the last rotation, with the floor
         int i = top - 1;
 #pragma unroll 1
         for (; i >= l; --i) {
@@ -415,7 +415,7 @@ __device__ __forceinline__ bool leaf_ql(int m, double* d, double* e, double* z) 
             const double q = fma(f, f, g * g);
             // the chase ended early: the block splits here (never at the first
             // rotation, whose f is above kLeafTiny)
-            if (q <= kLeafTiny * kLeafTiny * kLeafTiny) break;
+            if (__double2hiint(q) < 0x01b00000) break;
             const double inv = rsqrt(q), en = q * inv;
             e[i + 1] = en;
             s = f * inv;
@@ -431,15 +431,15 @@ __device__ __forceinline__ bool leaf_ql(int m, double* d, double* e, double* z) 
             dnext = di;
             // e[i + 1] against its new neighbours (not for the first
             // rotation: e[top] is outside the block)
-            if (i + 1 < top && en <= fma(kEps, fabs(dn) + dabove, kLeafTiny)) small |= 2u << i;
-            dabove = fabs(dn);
+            if (i + 1 < top && en <= kEps * (fabs(dn) + dabove)) small |= 2u << i;
+            dabove = fabs(dn) + kLeafTiny / kEps;
         }
         const double dn = dnext - p;
         z[i + 1] = znext;
         d[i + 1] = dn;
         if (i < l) {
             e[l] = g;
-            if (fabs(g) <= fma(kEps, fabs(dn) + dabove, kLeafTiny)) small |= 1u << l;
+            if (fabs(g) <= kEps * (fabs(dn) + dabove)) small |= 1u << l;
         } else {
             e[i] *= c;                                         // the last rotation's share
             e[i + 1] = 0.0;
