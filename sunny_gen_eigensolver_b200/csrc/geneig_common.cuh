@@ -142,6 +142,52 @@ __device__ __forceinline__ void team_sync() {
 // spilled) across the phases of a long kernel.
 __device__ __forceinline__ void forget(int& x) { asm volatile("" : "+r"(x)); }
 
+// ---------------------------------------------------------------- reflectors
+// Householder's elementary reflector I - tau v v^H, v = (1, scal x), that takes
+// (alpha, x) to (beta, 0) with beta real (zlarfg), from rest = ||x||^2 +
+// Im(alpha)^2 and nn = rest + Re(alpha)^2.
+struct Reflector {
+    double2 tau, scal;
+    double beta;
+};
+// True where the squares neither underflow nor overflow and rest is not zero
+// (rest at least 2^-927, nn below 2^929, about 1e-279 and 1e+279; compares on the
+// exponents, false for NaN): reflector() holds, else
+// reflector_scaled().
+__device__ __forceinline__ bool squares_safe(double rest, double nn) {
+    return __double2hiint(rest) >= 0x06000000 && __double2hiint(nn) < 0x7a000000;
+}
+__device__ __forceinline__ Reflector reflector(double2 alpha, double nn) {
+    Reflector h;
+    const double rn = rsqrt(nn);                         // 1 / beta comes with the root
+    h.beta = -copysign(nn * rn, alpha.x);
+    const double rbeta = -copysign(rn, alpha.x);
+    h.tau = c2((h.beta - alpha.x) * rbeta, -alpha.y * rbeta);
+    const double2 z = c2(alpha.x - h.beta, alpha.y);
+    const double inv = fast_rcp(fma(z.x, z.x, z.y * z.y));
+    h.scal = c2(z.x * inv, -z.y * inv);
+    return h;
+}
+// The same from ss = ||f x||^2, f = column_scale(nn): for columns of zeros, those
+// that the rounding residues of a low-rank matrix leave (1e-16, 1e-32, 1e-48, ...
+// of its norm), and matrices of extreme scale. A column below 2^-1000 is zero.
+__device__ __forceinline__ double column_scale(double nn) {
+    return nn >= 0x1p-900 && nn <= 0x1p900 ? 1.0 : nn < 1.0 ? 0x1p700 : 0x1p-700;
+}
+__device__ __forceinline__ Reflector reflector_scaled(double2 alpha, double ss, double f) {
+    const double2 a = cscale(alpha, f);
+    const double rest = fma(a.y, a.y, ss), nn = fma(a.x, a.x, rest);
+    Reflector h;
+    h.tau = h.scal = c2(0.0, 0.0);
+    h.beta = alpha.x;
+    if (!(rest == 0.0 || (f > 1.0 && nn < 0x1p-600))) {
+        h = reflector(a, nn);
+        h.beta *= f > 1.0 ? 0x1p-700 : f < 1.0 ? 0x1p700 : 1.0;
+        h.scal = cscale(h.scal, f);
+    }
+    return h;
+}
+
 // ---------------------------------------------------------------- constants
 // LAPACK dlamch convention: eps = 2^-53 (relative machine precision).
 constexpr double kEps    = 1.1102230246251565e-16;

@@ -738,7 +738,7 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
                         if (SPEC && last - 32 * t >= n) mc[off[t]] = x[t];   // the final P of column c
                     }
                 }
-                // reflector c from column c (1 / beta comes with the root)
+                // reflector c from column c
                 double2 xc = x[0], alpha = x[0];
 #pragma unroll
                 for (int t = 1; t < R; ++t) {
@@ -757,24 +757,27 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
                         ss = fma(x[t].x, x[t].x, fma(x[t].y, x[t].y, ss));
                     }
                     ss = warp_sum(ss);
-                    double2 scal = zero, tau = zero;
-                    beta = alpha.x;
-                    if (!(ss == 0.0 && alpha.y == 0.0)) {
-                        const double nn = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, ss));
-                        const double rn = rsqrt(nn);
-                        beta = -copysign(nn * rn, alpha.x);
-                        const double rbeta = -copysign(rn, alpha.x);
-                        tau = c2((beta - alpha.x) * rbeta, -alpha.y * rbeta);
-                        const double2 z = c2(alpha.x - beta, alpha.y);
-                        const double inv = fast_rcp(fma(z.x, z.x, z.y * z.y));
-                        scal = c2(z.x * inv, -z.y * inv);
+                    const double rest = fma(alpha.y, alpha.y, ss), nn = fma(alpha.x, alpha.x, rest);
+                    Reflector h;
+                    if (squares_safe(rest, nn)) {
+                        h = reflector(alpha, nn);
+                    } else {
+                        const double f = column_scale(nn);
+                        ss = 0.0;
+#pragma unroll
+                        for (int t = 0; t < R; ++t) {
+                            const double2 y = cscale(x[t], f);
+                            ss = fma(y.x, y.x, fma(y.y, y.y, ss));
+                        }
+                        h = reflector_scaled(alpha, warp_sum(ss), f);
                     }
+                    beta = h.beta;
 #pragma unroll
                     for (int t = 0; t < R; ++t) {
                         const int i = last - 32 * t;
-                        x[t] = cmul(x[t], scal);
+                        x[t] = cmul(x[t], h.scal);
                         if (i >= 0) vc[i] = i == c + 1 ? c2(1.0, 0.0) : x[t];
-                        if (i > c && (!SPEC || i < n)) mc[i] = i == c + 1 ? tau : x[t];
+                        if (i > c && (!SPEC || i < n)) mc[i] = i == c + 1 ? h.tau : x[t];
                     }
                 }
                 if (lane == (ic & 31)) de[c * des] = c2(xc.x, beta);

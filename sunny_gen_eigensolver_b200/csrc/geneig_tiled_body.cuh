@@ -658,6 +658,19 @@ __device__ __forceinline__ void tiled_form_c(int n, int ld, int sigma, const dou
     __syncthreads();
 }
 
+// A reflector whose squares leave the range, from the column's elements x[lo .. n)
+// in shared memory, by every warp for itself; out of line to keep the caller's
+// registers (n = 216: 1 % of the solve).
+static __device__ __noinline__ Reflector column_out_of_range(const double2* x, int lo, int n, double2 alpha, double nn) {
+    const double f = column_scale(nn);
+    double ss = 0.0;
+    for (int i = lo + (int)(threadIdx.x & 31); i < n; i += 32) {
+        const double2 y = cscale(x[i], f);
+        ss = fma(y.x, y.x, fma(y.y, y.y, ss));
+    }
+    return reflector_scaled(alpha, warp_sum(ss), f);
+}
+
 // The FP64 reduction of C (lower, M0) to tridiagonal form, reflectors in its
 // columns, (d, e, tau) to shared memory.
 template <int kNT>
@@ -698,25 +711,24 @@ __device__ __forceinline__ void tiled_house(int n, int ld, double2* M0, double2*
             // (2) reflector from a_k(k+1:n)
             const double ss = cta_sum<kNT>((row && i > k + 1) ? fma(x.x, x.x, x.y * x.y) : 0.0, red);
             const double2 alpha = v.gb[0];
-            double2 taui = zero, scal = zero;
-            double beta = alpha.x;
-            if (!(ss == 0.0 && alpha.y == 0.0)) {
-                const double nn = fma(alpha.x, alpha.x, fma(alpha.y, alpha.y, ss));
-                const double rn = rsqrt(nn);
-                beta = -copysign(nn * rn, alpha.x);
-                const double rb = -copysign(rn, alpha.x);
-                taui = c2((beta - alpha.x) * rb, -alpha.y * rb);
-                const double2 z = c2(alpha.x - beta, alpha.y);
-                const double inv = fast_rcp(fma(z.x, z.x, z.y * z.y));
-                scal = c2(z.x * inv, -z.y * inv);
+            const double rest = fma(alpha.y, alpha.y, ss), nn = fma(alpha.x, alpha.x, rest);
+            Reflector refl;                                // the same in every thread
+            if (squares_safe(rest, nn)) {
+                refl = reflector(alpha, nn);
+            } else {
+                if (row) v.vb[i] = x;
+                __syncthreads();
+                refl = column_out_of_range(v.vb, k + 2, n, alpha, nn);
+                __syncthreads();
             }
+            const double2 taui = refl.tau;
             double2 vi = zero;
             if (row && i > k) {
-                vi = i == k + 1 ? c2(1.0, 0.0) : cmul(x, scal);
+                vi = i == k + 1 ? c2(1.0, 0.0) : cmul(x, refl.scal);
                 v.vb[i] = vi;
                 M0[i + (size_t)k * ld] = vi;
             }
-            if (tid == 0) { v.tau[k] = taui; v.e[k] = beta; }
+            if (tid == 0) { v.tau[k] = taui; v.e[k] = refl.beta; }
             __syncthreads();
             // (3) y = A v (A: panel-start trailing matrix, lower
             // triangle), t1 = W^H v, t2 = V^H v
