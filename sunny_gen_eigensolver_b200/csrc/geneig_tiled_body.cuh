@@ -1169,6 +1169,16 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
             phase_mark(21);
         }
 
+        if (use32 && code) {
+            // FP32 overflowed or underflowed (or the input is not finite): FP64 decides
+            code = 0;
+            if (a.defer) {
+                if (tid == 0) a.info[b] = kRetryInfo;
+                return;
+            }
+            use32 = false;
+            continue;
+        }
         if (code) break;
 
         // ---- a5c: V = Q Z in the output, columns in ascending eigenvalue order
