@@ -81,6 +81,7 @@ __host__ __device__ inline size_t cta_dc_bytes(int n, bool spec) {   // (d, e) f
 // The reduction's panel is two blocks wide where one pencil has the SM (its
 // shared memory) to itself anyway. N=108: 235 K cycles for one, 141 K for two.
 __host__ __device__ constexpr bool cta_two_panels(int nw) { return nw >= 16; }
+constexpr int kRefinePanel = 1 << 16;   // beside the failed minor's order in rank[0]
 constexpr int kDElems = 72;       // an 8 x 8 tile with leading dimension 9
 __host__ __device__ inline size_t cta_work_bytes(int n, int nw, bool spec) {
     const size_t one = (size_t)8 * (n | 1);
@@ -239,6 +240,7 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
     // panel p hold the Cholesky working matrix, columns up to p the inverse
     // accumulators Acc. With D = L_pp^-1 (from warp 0, in shared memory):
     //   L(i, p) = A(i, p) D^H  (i > p, into `work`),   X(p, c) = D Acc(p, c)  (c < p, in place)
+    //   where L_pp is ill-conditioned: L(i, p) += (A(i, p) - L(i, p) L_pp^H) D^H
     // barrier
     //   Acc(i, c) -= L(i, p) X(p, c)  (c < p),  Acc(i, p) = -L(i, p) D,  A(i, j) -= L(i, p) L(j, p)^H
     // barrier; warp 0 updates the next diagonal tile first and factors it
@@ -247,9 +249,40 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
     // four-lane group's registers took 90 K CTA cycles at n = 54 and needed
     // 256 threads. Fragment rows past n read whatever lies there: they reach
     // discarded rows or columns of the result only.
-    double2* Pn = work;                // n x 8 panel of L
+    // Rounding is amplified in column c of A(i, p) D^H by at most kappa_c,
+    // kappa_c^2 = sum_j A_jj |D(c, j)|^2 (|A(i, j)| <= ||L(i, :)|| sqrt(A_jj)). Where a
+    // lane's share of it passes 8 the panel takes one step of refinement. N = 16,
+    // cond(S) = 1e10, mean ||U^H S U - I||: 12.3e-8 without the step, 5.4e-8 with it,
+    // 7.5e-8 LAPACK's. At cond(S) = 100 (kappa^2 up to 9) it is not needed; taken in
+    // every panel it would cost N = 54 2.5 % of the solve, the test costs 0.6 %.
+    double2* Pn = work;                // n x 8 panel of L; rows 0 .. 7 (above every panel): L_pp
     const int ldp = n | 1;
     double2* Ds = work + 8 * ldp;      // D of even and odd panels: element (i, j) at i + 9 j
+    // warp 0: L of the diagonal tile at o into rows 0 .. 7 of Pn (an infinite
+    // pivot's column is zero)
+    auto tile_l = [&](int o) {
+        double2 x[2];
+#pragma unroll
+        for (int s = 0; s < 2; ++s) x[s] = 2 * fq + s <= fr ? M[o + fr + (o + 2 * fq + s) * ld] : zero;
+#pragma unroll 1
+        for (int h = 0; h < 4; ++h) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int c = 2 * h + u;
+                const double akk = __shfl_sync(0xffffffffu, x[u].x, 4 * c + h);
+                const double r = rsqrt(akk), l = akk * r;
+                const double2 aic = shfl2(x[u], (lane & 28) + h), aik = cscale(aic, r * r);
+                if (fq == h)
+                    Pn[fr + c * ldp] = fr > c ? cscale(aic, r)
+                                     : c2(fr == c && r > 0.0 ? fma(l, fma(-l, r, 1.0), l) : 0.0, 0.0);
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    const double2 ajc = shfl2(x[u], 4 * (2 * fq + s) + h);
+                    if (2 * fq + s > c && 2 * fq + s <= fr) x[s] = cfms_bc(x[s], aik, ajc);
+                }
+            }
+        }
+    };
     auto factor = [&](int p) {         // warp 0; lane: row fr, columns 2 fq + s of the tile
         const int o = 8 * p;
         double2* Dp = Ds + (p & 1) * kDElems;
@@ -259,6 +292,9 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
             const int j = 2 * fq + s;
             x[s] = (o + fr < n && j <= fr) ? M[o + fr + (o + j) * ld] : c2(fr == j ? 1.0 : 0.0, 0.0);
         }
+        double kap = 0.0, ajj[2];      // A's diagonal in this lane's columns
+#pragma unroll
+        for (int s = 0; s < 2; ++s) ajj[s] = __shfl_sync(0xffffffffu, x[s].x, 4 * (2 * fq + s) + fq);
         int bad = 0;
         double rr = 0.0;               // 1 / L of this lane's row
 #pragma unroll 1
@@ -291,12 +327,16 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
                 }
             }
         }
-        if (lane == 0) rank[0] = bad;
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
             const int j = 2 * fq + s;
-            Dp[fr + 9 * j] = j < fr ? cscale(x[s], rr) : c2(j == fr ? rr : 0.0, 0.0);
+            const double2 d = j < fr ? cscale(x[s], rr) : c2(j == fr ? rr : 0.0, 0.0);
+            Dp[fr + 9 * j] = d;
+            kap = fma(ajj[s], fma(d.x, d.x, d.y * d.y), kap);
         }
+        const bool refine = __any_sync(0xffffffffu, kap > 8.0) && o + 8 < n;
+        if (lane == 0) rank[0] = bad | (refine ? kRefinePanel : 0);
+        if (refine) tile_l(o);
     };
     int fail = 0;
 #pragma unroll 1
@@ -304,8 +344,10 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
         const int o = 8 * p;
         const double2* Dp = Ds + (p & 1) * kDElems;
         if (p >= 0) {
-            fail = rank[0];
+            const int st = rank[0];
+            fail = st & (kRefinePanel - 1);
             if (fail) break;
+            const bool refine = st >= kRefinePanel;
 #pragma unroll 1
             for (int t = warp; t < nb - 1; t += NW) {
                 double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
@@ -317,6 +359,20 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
                     const double2 dd = Dp[fr + 9 * k];
                     const double2 m = xt ? M[min(o + k, n - 1) + (8 * t + fr) * ld] : M[i + (o + k) * ld];
                     zmma(re, im, xt ? dd : m, xt ? m : cconj(dd));
+                }
+                if (refine && !xt) {
+                    double dr[2], di[2];   // A - L L_pp^H (an accumulator is laid out as the next A fragment)
+#pragma unroll
+                    for (int s = 0; s < 2; ++s) {
+                        const double2 m = M[i + (o + 2 * fq + s) * ld];
+                        dr[s] = m.x;
+                        di[s] = m.y;
+                    }
+#pragma unroll
+                    for (int s = 0; s < 2; ++s)
+                        zmma(dr, di, c2(-re[s], -im[s]), cconj(Pn[fr + (2 * fq + s) * ldp]));
+#pragma unroll
+                    for (int s = 0; s < 2; ++s) zmma(re, im, c2(dr[s], di[s]), cconj(Dp[fr + 9 * (2 * fq + s)]));
                 }
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
