@@ -108,8 +108,9 @@ void sunny_geneig_destroy(sunny_geneig_solver_t solver);
  * INVALID_ARG for a NULL solver, batch_size < 0, a NULL or misaligned
  * buffer with batch_size > 0; batch_size == 0 is a no-op returning OK;
  * LAUNCH_ERROR when the CUDA launch itself fails. One handle may be used
- * from several streams: for sizes whose solver keeps scratch slots (the
- * "l2-slot" regime) a launch on a different stream than the previous one
+ * from several streams: for handles of the "l2-slot" regime, which keep
+ * scratch slots (default handles up to N = 110 do not, and are ordered all
+ * the same), a launch on a different stream than the previous one
  * waits for it on the device, so launches of one such handle never overlap.
  * That ordering covers normal launches only: a launch captured into a CUDA
  * graph uses the same scratch slots when the graph is replayed, so the

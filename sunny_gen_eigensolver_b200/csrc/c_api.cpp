@@ -32,13 +32,14 @@ struct sunny_geneig_solver {
     bool tuned = false;          // configuration chosen by the autotuner
     sgeig::PlainPlan plan;
     void* scratch = nullptr;
-    // Scratch ordering across streams: a launch that uses the handle's
-    // scratch slots waits for the previous such launch when that one went to
-    // another stream (launches on one stream are ordered by the stream).
-    cudaEvent_t scratch_done = nullptr;
+    // Launch ordering across streams, for every handle of the l2-slot regime
+    // (the sizes that keep no slots included): a launch waits for the previous
+    // one when that went to another stream (launches on one stream are ordered
+    // by the stream).
+    cudaEvent_t done = nullptr;
     uintptr_t last_stream = 0;
-    bool scratch_used = false;
-    std::mutex scratch_mu;
+    bool used = false;
+    std::mutex mu;
 };
 
 // Handle of the persistent uneven-size solver (sunny_geneig_uneven_*).
@@ -181,7 +182,9 @@ sunny_geneig_solver_t create_impl(int n, int device_id, int bpb_request,
         if (s->plan.scratch_bytes) {
             cudaError_t ea = cudaMalloc(&s->scratch, s->plan.scratch_bytes);
             if (ea != cudaSuccess) { err = std::string("cudaMalloc scratch: ") + cudaGetErrorString(ea); return ea; }
-            ea = cudaEventCreateWithFlags(&s->scratch_done, cudaEventDisableTiming);
+        }
+        if (s->plan.regime == sgeig::Regime::L2Slot) {
+            const cudaError_t ea = cudaEventCreateWithFlags(&s->done, cudaEventDisableTiming);
             if (ea != cudaSuccess) { err = std::string("cudaEventCreate: ") + cudaGetErrorString(ea); return ea; }
         }
         return cudaSuccess;
@@ -189,7 +192,7 @@ sunny_geneig_solver_t create_impl(int n, int device_id, int bpb_request,
     if (e != cudaSuccess) {
         set_error(std::string(fn) + ": " + (err.empty() ? cudaGetErrorString(e) : err));
         if (s->scratch) with_device(device_id, [&]() { return cudaFree(s->scratch); });
-        if (s->scratch_done) with_device(device_id, [&]() { return cudaEventDestroy(s->scratch_done); });
+        if (s->done) with_device(device_id, [&]() { return cudaEventDestroy(s->done); });
         delete s;
         return nullptr;
     }
@@ -226,21 +229,21 @@ sunny_geneig_status_t launch_impl(sunny_geneig_solver_t s, int stage, uintptr_t 
                                        s->scratch, reinterpret_cast<cudaStream_t>(stream), sigma);
         };
         cudaError_t e;
-        if (s->scratch) {
-            std::lock_guard<std::mutex> lock(s->scratch_mu);
+        if (s->done) {
+            std::lock_guard<std::mutex> lock(s->mu);
             e = with_device(s->device, [&]() {
                 const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
                 cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
                 if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusActive)
                     return run();   // graph replays are ordered by the caller (see sunny_geneig_launch)
-                if (s->scratch_used && s->last_stream != stream) {
-                    cudaError_t w = cudaStreamWaitEvent(st, s->scratch_done, 0);
+                if (s->used && s->last_stream != stream) {
+                    cudaError_t w = cudaStreamWaitEvent(st, s->done, 0);
                     if (w != cudaSuccess) return w;
                 }
                 cudaError_t l = run();
                 if (l != cudaSuccess) return l;
-                l = cudaEventRecord(s->scratch_done, st);
-                if (l == cudaSuccess) { s->scratch_used = true; s->last_stream = stream; }
+                l = cudaEventRecord(s->done, st);
+                if (l == cudaSuccess) { s->used = true; s->last_stream = stream; }
                 return l;
             });
         } else {
@@ -362,14 +365,11 @@ sunny_geneig_solver_t sunny_geneig_create_ex(int n, int device_id, int batches_p
 void sunny_geneig_destroy(sunny_geneig_solver_t solver) {
     if (!solver) return;
     try {
-        if (solver->scratch) {
-            const int dev = solver->device;
-            void* p = solver->scratch;
-            cudaEvent_t ev = solver->scratch_done;
-            with_device(dev, [&]() {
-                if (ev) cudaEventSynchronize(ev);   // no launch may still use the slots
-                if (ev) cudaEventDestroy(ev);
-                return cudaFree(p);
+        if (solver->done) {
+            with_device(solver->device, [&]() {
+                cudaEventSynchronize(solver->done);   // no launch may still use the slots
+                cudaEventDestroy(solver->done);
+                return cudaFree(solver->scratch);
             });
         }
         delete solver;

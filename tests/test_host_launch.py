@@ -1,0 +1,73 @@
+"""Host side of the launches without a GPU: the C ABI (csrc/c_api.cpp) over a
+fake CUDA runtime and fake launchers (tests/host/fake_cuda.cpp), which log every
+record, wait and launch and can fail any of them."""
+import ctypes
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+REPO = Path(__file__).resolve().parents[1]
+CSRC = REPO / "sunny_gen_eigensolver_b200" / "csrc"
+CUDA = Path("/usr/local/cuda/include")
+U = ctypes.c_size_t
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    if shutil.which("g++") is None or not (CUDA / "cuda_runtime.h").exists():
+        pytest.skip("needs g++ and the CUDA headers")
+    out = tmp_path_factory.mktemp("host") / "libhost.so"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-Wl,-Bsymbolic", f"-I{REPO / 'include'}", f"-I{CSRC}",
+                    f"-I{CUDA}", str(CSRC / "c_api.cpp"), str(REPO / "tests" / "host" / "fake_cuda.cpp"), "-ldl", "-o", str(out)],
+                   check=True)
+    L = ctypes.CDLL(str(out))
+    for name in ("sunny_geneig_create_config", "sunny_geneig_uneven_create"):
+        getattr(L, name).restype = ctypes.c_void_p
+    L.sunny_geneig_create_config.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_char_p, ctypes.c_int]
+    L.sunny_geneig_launch.argtypes = [ctypes.c_void_p, U, U, U, U, U, ctypes.c_int, U]
+    L.sunny_geneig_destroy.argtypes = [ctypes.c_void_p]
+    L.fake_reset.argtypes = [ctypes.c_char_p, U]
+    L.fake_capture.argtypes = [U, ctypes.c_int]
+    L.fake_log.restype = ctypes.c_char_p
+    return L
+
+
+def reset(L, fail="", memory=1 << 40):
+    L.fake_reset(fail.encode(), memory)
+
+
+def log(L):
+    return L.fake_log().decode().splitlines()
+
+
+def launch(L, s, stream):
+    return L.sunny_geneig_launch(s, 4096, 8192, 12288, 16384, 20480, 3, stream)
+
+
+@pytest.mark.parametrize("n,mode,ordered", [(54, 0, False), (61, 0, True), (72, 0, True), (110, 0, True), (216, 0, True),
+                                            (54, 2, True)])
+def test_launches_of_an_l2_slot_handle_are_ordered_across_streams(lib, n, mode, ordered):
+    s = lib.sunny_geneig_create_config(n, 0, mode, b"", 0)
+    reset(lib)
+    for stream in (11, 11, 12, 11):
+        assert launch(lib, s, stream) == 0
+    lines = log(lib)
+    if not ordered:
+        assert lines == [f"launch {n} on {x}" for x in (11, 11, 12, 11)]
+    else:
+        ev = lines[1].split()[1]
+        assert lines == [f"launch {n} on 11", f"record {ev} on 11", f"launch {n} on 11", f"record {ev} on 11",
+                         f"wait {ev} on 12", f"launch {n} on 12", f"record {ev} on 12",
+                         f"wait {ev} on 11", f"launch {n} on 11", f"record {ev} on 11"]
+        reset(lib)
+        lib.fake_capture(12, 1)                      # replays are the caller's to order
+        assert launch(lib, s, 12) == 0
+        lib.fake_capture(12, 0)
+        assert log(lib) == [f"launch {n} on 12"]
+        reset(lib)
+        lib.sunny_geneig_destroy(s)
+        assert log(lib) == [f"sync_event {ev}"]
+        return
+    lib.sunny_geneig_destroy(s)
