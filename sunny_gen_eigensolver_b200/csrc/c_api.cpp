@@ -240,11 +240,11 @@ sunny_geneig_status_t launch_impl(sunny_geneig_solver_t s, int stage, uintptr_t 
                     cudaError_t w = cudaStreamWaitEvent(st, s->done, 0);
                     if (w != cudaSuccess) return w;
                 }
-                cudaError_t l = run();
-                if (l != cudaSuccess) return l;
-                l = cudaEventRecord(s->done, st);
-                if (l == cudaSuccess) { s->used = true; s->last_stream = stream; }
-                return l;
+                // (the mixed form is two kernels: the first may run although the
+                // second failed, so an error is recorded like a success)
+                const cudaError_t l = run(), r = cudaEventRecord(s->done, st);
+                if (r == cudaSuccess) { s->used = true; s->last_stream = stream; }
+                return l != cudaSuccess ? l : r;
             });
         } else {
             e = with_device(s->device, run);

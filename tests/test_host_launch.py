@@ -71,3 +71,16 @@ def test_launches_of_an_l2_slot_handle_are_ordered_across_streams(lib, n, mode, 
         assert log(lib) == [f"sync_event {ev}"]
         return
     lib.sunny_geneig_destroy(s)
+
+
+def test_launch_that_failed_is_still_waited_for(lib):
+    """The mixed form's launch is two kernels: when the second fails the first is
+    already using the handle's slots."""
+    s = lib.sunny_geneig_create_config(54, 0, 2, b"", 0)
+    reset(lib, fail="launch:0")
+    assert launch(lib, s, 11) != 0
+    assert launch(lib, s, 12) == 0
+    lines = log(lib)
+    ev = lines[1].split()[1]
+    assert lines == ["launch 54 on 11 FAILS", f"record {ev} on 11", f"wait {ev} on 12", "launch 54 on 12", f"record {ev} on 12"]
+    lib.sunny_geneig_destroy(s)
