@@ -22,8 +22,8 @@ TIMERS_LIB_PATH = LIB_DIR / "libsunny_geneig_timers.so"
 INCLUDE = REPO_DIR / "include"
 
 SOURCES = ["geneig_cta.cu", "geneig_cta_small.cu", "geneig_cta_mid.cu", "geneig_cta_wide.cu", "geneig_cta_spec.cu",
-           "geneig_plain.cu", "geneig_tiled.cu", "geneig_uneven.cu", "selftest.cu", "tune.cu",
-           "c_api.cpp"]
+           "geneig_plain.cu", "geneig_tiled.cu", "geneig_uneven.cu", "geneig_uneven_launch.cpp",
+           "selftest.cu", "tune.cu", "c_api.cpp"]
 HEADERS = ["geneig_common.cuh", "geneig_dc.cuh", "geneig_kernels.h", "geneig_cta_body.cuh",
            "geneig_cta_kernel.cuh", "geneig_tiled_body.cuh"]
 

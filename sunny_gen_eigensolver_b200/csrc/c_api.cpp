@@ -645,11 +645,11 @@ sunny_geneig_status_t sunny_geneig_uneven_launch(sunny_geneig_uneven_t h, const 
                 cudaError_t w = cudaStreamWaitEvent(st, h->done, 0);
                 if (w != cudaSuccess) return w;
             }
-            cudaError_t l = sgeig::uneven_launch(L, h->head, h->scratch, h->slot_elems, h->grid, h->smem, st, h->side);
-            if (l != cudaSuccess || capturing) return l;
-            l = cudaEventRecord(h->done, st);
-            if (l == cudaSuccess) { h->used = true; h->last_stream = stream; }
-            return l;
+            const cudaError_t l = sgeig::uneven_launch(L, h->head, h->scratch, h->slot_elems, h->grid, h->smem, st, h->side);
+            if (capturing) return l;
+            const cudaError_t r = cudaEventRecord(h->done, st);   // on an error too: some sizes may run
+            if (r == cudaSuccess) { h->used = true; h->last_stream = stream; }
+            return l != cudaSuccess ? l : r;
         });
         if (e != cudaSuccess) {
             set_error(std::string(fn) + ": launch failed: " + cudaGetErrorString(e));

@@ -207,6 +207,10 @@ struct UnevenSide {
     cudaEvent_t join[kUnevenMaxGroups] = {};
     cudaEvent_t fork = nullptr;
 };
+cudaError_t uneven_persistent_launch(const UnevenLaunch& L, unsigned long long* head, void* scratch, size_t slot_elems,
+                                     int grid, size_t smem, cudaStream_t stream);   // the sizes of kinds 0 .. 5
+// All sizes (geneig_uneven_launch.cpp). On an error, too, `stream` waits for
+// everything that was launched.
 cudaError_t uneven_launch(const UnevenLaunch& L, unsigned long long* head, void* scratch, size_t slot_elems,
                           int grid, size_t smem, cudaStream_t stream, const UnevenSide& side);
 

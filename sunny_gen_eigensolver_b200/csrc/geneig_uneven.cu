@@ -124,16 +124,12 @@ size_t uneven_smem_bytes(int n, int kind) {
                      : kind_teams(kind) * cta_smem_bytes(n);
 }
 
-cudaError_t uneven_launch(const UnevenLaunch& L, unsigned long long* head, void* scratch, size_t slot_elems,
-                          int grid, size_t smem, cudaStream_t stream, const UnevenSide& side) {
+cudaError_t uneven_persistent_launch(const UnevenLaunch& L, unsigned long long* head, void* scratch, size_t slot_elems,
+                                     int grid, size_t smem, cudaStream_t stream) {
     UnevenArgs a{};
-    long long first = 0;
-    int ng = 0;
-    int nside = 0;
     for (int i = 0; i < L.ngroups; ++i) {
-        if (L.count[i] <= 0) continue;
-        if (L.kind[i] >= kUnevenResident) { ++nside; continue; }
-        UnevenGroup& G = a.g[ng++];
+        if (L.count[i] <= 0 || L.kind[i] >= kUnevenResident) continue;
+        UnevenGroup& G = a.g[a.ngroups++];
         G.H = static_cast<const double2*>(L.H[i]);
         G.S = static_cast<const double2*>(L.S[i]);
         G.W = L.W[i];
@@ -144,41 +140,17 @@ cudaError_t uneven_launch(const UnevenLaunch& L, unsigned long long* head, void*
         G.kind = L.kind[i];
         G.per_item = L.per_item[i] > 0 ? L.per_item[i] : 1;
         G.slice = G.kind == 5 ? 0 : cta_smem_bytes(G.n);
-        G.first_item = first;
-        first += (G.count + G.per_item - 1) / G.per_item;
+        G.first_item = a.nitems;
+        a.nitems += (G.count + G.per_item - 1) / G.per_item;
     }
-    // The side sizes first, largest first (the groups' order): their pencils
-    // take longest, and the persistent kernel's small ones fill the SMs that
-    // they leave.
-    const bool fork = nside + (ng > 0 ? 1 : 0) > 1;
-    cudaError_t e = fork ? cudaEventRecord(side.fork, stream) : cudaSuccess;
-    for (int i = 0, s = 0; i < L.ngroups; ++i) {
-        if (L.count[i] <= 0 || L.kind[i] < kUnevenResident) continue;
-        const cudaStream_t st = fork ? side.stream[s] : stream;
-        if (e == cudaSuccess && fork) e = cudaStreamWaitEvent(st, side.fork, 0);
-        if (e != cudaSuccess) return e;
-        if (L.kind[i] == kUnevenResident)
-            e = cta_launch(L.n[i], cta_nmax_for(L.n[i]), 4, L.H[i], L.S[i], L.W[i], L.U[i], L.info[i], L.count[i], st);
-        else
-            e = tiled_launch(L.n[i], L.slots[i], 4, L.H[i], L.S[i], L.W[i], L.U[i], L.info[i],
-                             L.count[i], L.scratch[i], st, false);
-        if (e == cudaSuccess && fork) e = cudaEventRecord(side.join[s], st);
-        ++s;
-    }
-    if (e == cudaSuccess && ng > 0) {
-        a.ngroups = ng;
-        a.nitems = first;
-        a.head = head;
-        a.scratch = static_cast<double2*>(scratch);
-        a.slot_elems = slot_elems;
-        e = cudaMemsetAsync(head, 0, sizeof(unsigned long long), stream);
-        if (e != cudaSuccess) return e;
-        const long long g = first < grid ? first : grid;
-        geneig_uneven_kernel<<<(unsigned)g, kNT, smem, stream>>>(a);
-        e = cudaGetLastError();
-    }
-    for (int s = 0; fork && s < nside && e == cudaSuccess; ++s) e = cudaStreamWaitEvent(stream, side.join[s], 0);
-    return e;
+    a.head = head;
+    a.scratch = static_cast<double2*>(scratch);
+    a.slot_elems = slot_elems;
+    const cudaError_t e = cudaMemsetAsync(head, 0, sizeof(unsigned long long), stream);
+    if (e != cudaSuccess) return e;
+    const long long g = a.nitems < grid ? a.nitems : grid;
+    geneig_uneven_kernel<<<(unsigned)g, kNT, smem, stream>>>(a);
+    return cudaGetLastError();
 }
 
 }  // namespace sgeig

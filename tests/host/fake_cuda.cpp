@@ -108,9 +108,14 @@ cudaError_t uneven_set_attributes(size_t) { return cudaSuccess; }
 int tiled_slots_for(int n) { return n > 200 ? 1 : 2; }
 int uneven_kind(int n, bool l2) { return !l2 ? 0 : n <= kCtaPreferredMaxN ? 5 : n <= kResidentMaxN ? kUnevenResident : kUnevenBig; }
 size_t uneven_smem_bytes(int, int) { return 1024; }
-#ifndef UNEVEN_LAUNCH
-cudaError_t uneven_launch(const UnevenLaunch&, unsigned long long*, void*, size_t, int, size_t, cudaStream_t s,
-                          const UnevenSide&) { return result(say("uneven", "on " + num(s))); }
-#endif
+cudaError_t cta_launch(int n, int, int, const void*, const void*, double*, void*, int*, long long, cudaStream_t s, bool,
+                       int, bool) { return result(say("cta", std::to_string(n) + " on " + num(s))); }
+cudaError_t tiled_launch(int n, int, int, const void*, const void*, double*, void*, int*, long long, void* scratch,
+                         cudaStream_t s, bool, bool, int, bool) {
+    return result(say("tiled", std::to_string(n) + " on " + num(s) + " slots " + num(scratch)));
+}
+cudaError_t uneven_persistent_launch(const UnevenLaunch&, unsigned long long*, void*, size_t, int, size_t, cudaStream_t s) {
+    return result(say("persistent", "on " + num(s)));
+}
 
 }  // namespace sgeig

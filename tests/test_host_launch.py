@@ -1,5 +1,5 @@
-"""Host side of the launches without a GPU: the C ABI (csrc/c_api.cpp) over a
-fake CUDA runtime and fake launchers (tests/host/fake_cuda.cpp), which log every
+"""Host side of the launches without a GPU: the C ABI (csrc/c_api.cpp) and the
+uneven-size launch (csrc/geneig_uneven_launch.cpp) over a fake CUDA runtime and fake launchers (tests/host/fake_cuda.cpp), which log every
 record, wait and launch and can fail any of them."""
 import ctypes
 import shutil
@@ -20,7 +20,8 @@ def lib(tmp_path_factory):
         pytest.skip("needs g++ and the CUDA headers")
     out = tmp_path_factory.mktemp("host") / "libhost.so"
     subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-Wl,-Bsymbolic", f"-I{REPO / 'include'}", f"-I{CSRC}",
-                    f"-I{CUDA}", str(CSRC / "c_api.cpp"), str(REPO / "tests" / "host" / "fake_cuda.cpp"), "-ldl", "-o", str(out)],
+                    f"-I{CUDA}", str(CSRC / "c_api.cpp"),
+                    str(CSRC / "geneig_uneven_launch.cpp"), str(REPO / "tests" / "host" / "fake_cuda.cpp"), "-ldl", "-o", str(out)],
                    check=True)
     L = ctypes.CDLL(str(out))
     for name in ("sunny_geneig_create_config", "sunny_geneig_uneven_create"):
@@ -28,6 +29,10 @@ def lib(tmp_path_factory):
     L.sunny_geneig_create_config.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_char_p, ctypes.c_int]
     L.sunny_geneig_launch.argtypes = [ctypes.c_void_p, U, U, U, U, U, ctypes.c_int, U]
     L.sunny_geneig_destroy.argtypes = [ctypes.c_void_p]
+    A = ctypes.POINTER(U)
+    L.sunny_geneig_uneven_create.argtypes = [ctypes.c_int] + [ctypes.POINTER(ctypes.c_int)] * 3 + [ctypes.c_int]
+    L.sunny_geneig_uneven_launch.argtypes = [ctypes.c_void_p, A, A, A, A, A, ctypes.POINTER(ctypes.c_int), U]
+    L.sunny_geneig_uneven_destroy.argtypes = [ctypes.c_void_p]
     L.fake_reset.argtypes = [ctypes.c_char_p, U]
     L.fake_capture.argtypes = [U, ctypes.c_int]
     L.fake_log.restype = ctypes.c_char_p
@@ -84,3 +89,53 @@ def test_launch_that_failed_is_still_waited_for(lib):
     ev = lines[1].split()[1]
     assert lines == ["launch 54 on 11 FAILS", f"record {ev} on 11", f"wait {ev} on 12", "launch 54 on 12", f"record {ev} on 12"]
     lib.sunny_geneig_destroy(s)
+
+
+SIZES = [12, 54, 72, 108, 162, 216]
+
+
+def uneven_create(L, sizes=SIZES):
+    return L.sunny_geneig_uneven_create(len(sizes), (ctypes.c_int * len(sizes))(*sizes), None, None, 0)
+
+
+def uneven_launch(L, h, stream, sizes=SIZES, counts=None):
+    k = len(sizes)
+    p = (U * k)(*[4096] * k)
+    return L.sunny_geneig_uneven_launch(h, p, p, p, p, p, (ctypes.c_int * k)(*(counts or [5] * k)), stream)
+
+
+def unjoined(lines, stream):
+    """Work that `stream` does not wait for at the end of the log: kernels on other streams after the last
+    record of an event that `stream` waits for later."""
+    kernels = [(i, x.split(" on ")[1].split()[0]) for i, x in enumerate(lines)
+               if x.split()[0] in ("cta", "tiled", "persistent") and not x.endswith("FAILS")]
+    bad = []
+    for i, st in kernels:
+        if st == str(stream):
+            continue
+        joins = [j for j, x in enumerate(lines) if j > i and x.startswith("record") and x.endswith(f" on {st}")]
+        waited = any(x == f"wait {lines[j].split()[1]} on {stream}" for j in joins for x in lines[j:])
+        if not waited and not any(x == f"sync_stream {st}" for x in lines[i:]):
+            bad.append(lines[i])
+    return bad
+
+
+FAILURES = [f"{c}:{k}" for c, n in (("cta", 2), ("tiled", 2), ("persistent", 1), ("wait", 9), ("record", 6)) for k in range(n)]
+
+
+@pytest.mark.parametrize("fail", [""] + FAILURES)
+def test_uneven_launch_joins_its_streams_whatever_fails(lib, fail):
+    h = uneven_create(lib)
+    reset(lib, fail=fail)
+    st = uneven_launch(lib, h, 11)
+    lines = log(lib)
+    assert (st == 0) == (not any(x.endswith("FAILS") for x in lines))
+    assert unjoined(lines, 11) == []
+    if not fail:
+        assert sum(x.startswith(("cta", "tiled", "persistent")) for x in lines) == 5
+    if not fail.startswith("record") and any(x.split()[0] in ("cta", "tiled", "persistent") for x in lines):
+        # the next call on another stream waits for this one
+        reset(lib)
+        assert uneven_launch(lib, h, 12) == 0
+        assert log(lib)[0].startswith("wait") and log(lib)[0].endswith("on 12")
+    lib.sunny_geneig_uneven_destroy(h)
