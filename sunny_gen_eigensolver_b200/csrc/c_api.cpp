@@ -645,7 +645,8 @@ sunny_geneig_status_t sunny_geneig_uneven_launch(sunny_geneig_uneven_t h, const 
                 cudaError_t w = cudaStreamWaitEvent(st, h->done, 0);
                 if (w != cudaSuccess) return w;
             }
-            const cudaError_t l = sgeig::uneven_launch(L, h->head, h->scratch, h->slot_elems, h->grid, h->smem, st, h->side);
+            const cudaError_t l = sgeig::uneven_launch(L, h->head, h->scratch, h->slot_elems, h->grid, h->smem, st,
+                                                       h->side, capturing);
             if (capturing) return l;
             const cudaError_t r = cudaEventRecord(h->done, st);   // on an error too: some sizes may run
             if (r == cudaSuccess) { h->used = true; h->last_stream = stream; }

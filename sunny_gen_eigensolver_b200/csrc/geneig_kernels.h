@@ -210,8 +210,9 @@ struct UnevenSide {
 cudaError_t uneven_persistent_launch(const UnevenLaunch& L, unsigned long long* head, void* scratch, size_t slot_elems,
                                      int grid, size_t smem, cudaStream_t stream);   // the sizes of kinds 0 .. 5
 // All sizes (geneig_uneven_launch.cpp). On an error, too, `stream` waits for
-// everything that was launched.
+// everything that was launched. `capturing`: `stream` is being captured; `side`
+// stays untouched then.
 cudaError_t uneven_launch(const UnevenLaunch& L, unsigned long long* head, void* scratch, size_t slot_elems,
-                          int grid, size_t smem, cudaStream_t stream, const UnevenSide& side);
+                          int grid, size_t smem, cudaStream_t stream, const UnevenSide& side, bool capturing);
 
 }  // namespace sgeig

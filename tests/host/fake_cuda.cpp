@@ -15,7 +15,10 @@ using namespace sgeig;
 
 static std::string g_log, g_fail;      // "name:k": the k-th call (from 0) of `name` fails
 static std::map<std::string, int> g_calls;
-static std::set<size_t> g_capturing;
+// Captures: the origin of each capturing stream; the origin of each event recorded in one; and each
+// capturing stream's current dependencies (nodes are numbers).
+static std::map<size_t, size_t> g_capturing, g_event;
+static std::map<size_t, std::vector<cudaGraphNode_t>> g_deps;
 static size_t g_next = 100, g_memory = (size_t)1 << 40, g_used = 0;
 static std::map<size_t, size_t> g_blocks;
 
@@ -27,6 +30,18 @@ static bool say(const std::string& name, const std::string& rest = "") {
 }
 static std::string num(const void* p) { return std::to_string((size_t)p); }
 template <class T> static T fresh() { return reinterpret_cast<T>(++g_next); }
+// A kernel on stream s: in a capture a node after the stream's dependencies.
+static cudaError_t kernel(const std::string& name, const std::string& what, cudaStream_t s, const std::string& rest = "") {
+    std::string line = what + "on " + std::to_string((size_t)s) + rest;
+    if (g_capturing.count((size_t)s)) {
+        auto& d = g_deps[(size_t)s];
+        const auto node = fresh<cudaGraphNode_t>();
+        line += " node " + num(node) + " after";
+        for (auto n : d) line += " " + num(n);
+        d = {node};
+    }
+    return say(name, line) ? cudaErrorLaunchFailure : cudaSuccess;
+}
 static cudaError_t result(bool fails) { return fails ? cudaErrorLaunchFailure : cudaSuccess; }
 
 extern "C" {
@@ -36,7 +51,18 @@ void fake_reset(const char* fail, size_t memory) {
     g_fail = fail;
     g_memory = memory;
 }
-void fake_capture(size_t stream, int on) { if (on) g_capturing.insert(stream); else g_capturing.erase(stream); }
+void fake_capture(size_t stream, int on) {
+    if (on) { g_capturing[stream] = stream; g_deps[stream] = {fresh<cudaGraphNode_t>()}; return; }
+    std::map<size_t, size_t> left;
+    for (auto& c : g_capturing) if (c.second != stream) left.insert(c);
+    g_capturing = left;
+}
+const char* fake_dependencies(size_t stream) {
+    static std::string out;
+    out.clear();
+    for (auto n : g_deps[stream]) out += num(n) + " ";
+    return out.c_str();
+}
 const char* fake_log() { return g_log.c_str(); }
 size_t fake_memory_used() { return g_used; }
 
@@ -64,8 +90,35 @@ cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { *e = fresh<cuda
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t e) { return result(say("sync_event", num(e))); }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { return result(say("sync_stream", num(s))); }
-cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { return result(say("record", num(e) + " on " + num(s))); }
-cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) { return result(say("wait", num(e) + " on " + num(s))); }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+    if (say("record", num(e) + " on " + num(s))) return cudaErrorLaunchFailure;
+    g_event.erase((size_t)e);
+    if (g_capturing.count((size_t)s)) g_event[(size_t)e] = g_capturing[(size_t)s];
+    return cudaSuccess;
+}
+cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
+    if (say("wait", num(e) + " on " + num(s))) return cudaErrorLaunchFailure;
+    const bool in = g_event.count((size_t)e);
+    if (!in && g_capturing.count((size_t)s)) return cudaErrorStreamCaptureIsolation;
+    if (in && g_capturing.count((size_t)s) && g_capturing[(size_t)s] != g_event[(size_t)e]) return cudaErrorStreamCaptureMerge;
+    if (in) g_capturing[(size_t)s] = g_event[(size_t)e];
+    return cudaSuccess;
+}
+cudaError_t cudaStreamGetCaptureInfo_v2(cudaStream_t s, cudaStreamCaptureStatus* cs, unsigned long long*, cudaGraph_t*,
+                                        const cudaGraphNode_t** nodes, size_t* count) {
+    const bool in = g_capturing.count((size_t)s);
+    *cs = in ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+    if (in) { *nodes = g_deps[(size_t)s].data(); *count = g_deps[(size_t)s].size(); }
+    return result(say("capture_info"));
+}
+cudaError_t cudaStreamUpdateCaptureDependencies(cudaStream_t s, cudaGraphNode_t* nodes, size_t count, unsigned flags) {
+    if (say("set_dependencies")) return cudaErrorLaunchFailure;
+    if (!g_capturing.count((size_t)s)) return cudaErrorIllegalState;
+    auto& d = g_deps[(size_t)s];
+    if (flags == cudaStreamSetCaptureDependencies) d.clear();
+    d.insert(d.end(), nodes, nodes + count);
+    return cudaSuccess;
+}
 cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus* cs) {
     *cs = g_capturing.count((size_t)s) ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
     return cudaSuccess;
@@ -109,13 +162,13 @@ int tiled_slots_for(int n) { return n > 200 ? 1 : 2; }
 int uneven_kind(int n, bool l2) { return !l2 ? 0 : n <= kCtaPreferredMaxN ? 5 : n <= kResidentMaxN ? kUnevenResident : kUnevenBig; }
 size_t uneven_smem_bytes(int, int) { return 1024; }
 cudaError_t cta_launch(int n, int, int, const void*, const void*, double*, void*, int*, long long, cudaStream_t s, bool,
-                       int, bool) { return result(say("cta", std::to_string(n) + " on " + num(s))); }
+                       int, bool) { return kernel("cta", std::to_string(n) + " ", s); }
 cudaError_t tiled_launch(int n, int, int, const void*, const void*, double*, void*, int*, long long, void* scratch,
                          cudaStream_t s, bool, bool, int, bool) {
-    return result(say("tiled", std::to_string(n) + " on " + num(s) + " slots " + num(scratch)));
+    return kernel("tiled", std::to_string(n) + " ", s, " slots " + num(scratch));
 }
 cudaError_t uneven_persistent_launch(const UnevenLaunch&, unsigned long long*, void*, size_t, int, size_t, cudaStream_t s) {
-    return result(say("persistent", "on " + num(s)));
+    return kernel("persistent", "", s);
 }
 
 }  // namespace sgeig

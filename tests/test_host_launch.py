@@ -35,7 +35,8 @@ def lib(tmp_path_factory):
     L.sunny_geneig_uneven_destroy.argtypes = [ctypes.c_void_p]
     L.fake_reset.argtypes = [ctypes.c_char_p, U]
     L.fake_capture.argtypes = [U, ctypes.c_int]
-    L.fake_log.restype = ctypes.c_char_p
+    L.fake_log.restype = L.fake_dependencies.restype = ctypes.c_char_p
+    L.fake_dependencies.argtypes = [U]
     return L
 
 
@@ -138,4 +139,42 @@ def test_uneven_launch_joins_its_streams_whatever_fails(lib, fail):
         reset(lib)
         assert uneven_launch(lib, h, 12) == 0
         assert log(lib)[0].startswith("wait") and log(lib)[0].endswith("on 12")
+    lib.sunny_geneig_uneven_destroy(h)
+
+
+def test_captured_uneven_launch_keeps_to_the_callers_stream(lib):
+    """Each size is a branch of the graph from the point of the call, and what follows comes after all of them; the
+    handle's streams and events stay out of the capture, so that its launches go on elsewhere while it lasts."""
+    h = uneven_create(lib)
+    reset(lib)
+    lib.fake_capture(11, 1)
+    root = lib.fake_dependencies(11).decode().split()
+    assert uneven_launch(lib, h, 11) == 0
+    kernels = [x.split() for x in log(lib) if x.split()[0] in ("cta", "tiled", "persistent")]
+    assert len(kernels) == 5 and not any(x.startswith(("record", "wait")) for x in log(lib))
+    assert all(k[k.index("on") + 1] == "11" and k[k.index("after") + 1:] == root for k in kernels)
+    nodes = sorted(k[k.index("node") + 1] for k in kernels)
+    assert sorted(lib.fake_dependencies(11).decode().split()) == nodes
+    assert uneven_launch(lib, h, 12) == 0                 # not captured
+    lib.fake_capture(13, 1)                                # a second capture
+    assert uneven_launch(lib, h, 13) == 0 and uneven_launch(lib, h, 12) == 0
+    assert uneven_launch(lib, h, 11) == 0                 # the first one goes on
+    again = [x.split() for x in log(lib) if " on 11 " in x and "node" in x][5:]
+    assert all(sorted(k[k.index("after") + 1:]) == nodes for k in again) and len(again) == 5
+    lib.fake_capture(11, 0)
+    lib.fake_capture(13, 0)
+    lib.sunny_geneig_uneven_destroy(h)
+
+
+@pytest.mark.parametrize("fail", [f"{c}:{k}" for c, n in (("cta", 2), ("tiled", 2), ("persistent", 1), ("capture_info", 5),
+                                                        ("set_dependencies", 4)) for k in range(n)])
+def test_captured_uneven_launch_joins_its_branches_whatever_fails(lib, fail):
+    h = uneven_create(lib)
+    reset(lib, fail=fail)
+    lib.fake_capture(11, 1)
+    assert uneven_launch(lib, h, 11) != 0
+    nodes = [x.split() for x in log(lib) if "node" in x and not x.endswith("FAILS")]
+    left = lib.fake_dependencies(11).decode().split()
+    assert all(k[k.index("node") + 1] in left for k in nodes)
+    lib.fake_capture(11, 0)
     lib.sunny_geneig_uneven_destroy(h)
