@@ -283,7 +283,7 @@ sunny_geneig_solver_t sunny_geneig_create_config(int n, int device_id, sunny_gen
  * reference's C ABI). One call solves problems of up to 8 different sizes,
  * each size's problems in their own buffers with the layouts, info codes and
  * NaN fill of sunny_geneig_launch. Sizes above 60 run as launches of their
- * own kernels on streams of the handle, the larger the higher their priority,
+ * own kernels on streams of the handle, of default priority, the largest first,
  * forked from and joined to `stream` by events; the smaller ones share a
  * persistent kernel beside them: a device work counter hands out work
  * items, largest N first, to a grid of 2 CTAs per SM, each item solved by

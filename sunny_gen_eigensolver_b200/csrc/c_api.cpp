@@ -560,14 +560,8 @@ sunny_geneig_uneven_t sunny_geneig_uneven_create(int num_sizes, const int* sizes
             int nside = 0;
             for (int g = 0; g < num_sizes; ++g) nside += h->kind[g] >= sgeig::kUnevenResident;
             if (num_sizes < 2) nside = 0;      // a lone size runs on the caller's stream
-            // The larger a size, the higher its stream's priority: in back-to-back
-            // calls all launches are pending when the fork event fires, and the
-            // one that takes longest has to get its SMs first (12 to 216 rows, 4000
-            // pencils: 10.9 -> 9.95 ms a call, as fast as a call on its own).
-            int least = 0, greatest = 0;
-            if (nside) ea = cudaDeviceGetStreamPriorityRange(&least, &greatest);
             for (int i = 0; i < nside && ea == cudaSuccess; ++i) {
-                ea = cudaStreamCreateWithPriority(&h->side.stream[i], cudaStreamNonBlocking, std::min(greatest + i, least));
+                ea = cudaStreamCreateWithFlags(&h->side.stream[i], cudaStreamNonBlocking);
                 if (ea == cudaSuccess) ea = cudaEventCreateWithFlags(&h->side.join[i], cudaEventDisableTiming);
             }
             if (ea == cudaSuccess && nside) ea = cudaEventCreateWithFlags(&h->side.fork, cudaEventDisableTiming);

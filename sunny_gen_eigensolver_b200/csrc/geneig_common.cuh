@@ -8,6 +8,24 @@
 
 namespace sgeig {
 
+// A kernel launch; `started` (may be NULL) is recorded when the last of its CTAs
+// has begun.
+template <class... Args>
+inline cudaError_t launch_with_event(void (*kernel)(Args...), unsigned grid, int threads, size_t smem,
+                                     cudaStream_t stream, cudaEvent_t started, const Args&... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeLaunchCompletionEvent;
+    at.val.launchCompletionEvent.event = started;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3((unsigned)threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    c.attrs = &at;
+    c.numAttrs = started ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, args...);
+}
+
 // ---------------------------------------------------------------- complex FP64
 __device__ __forceinline__ double2 c2(double re, double im) { return make_double2(re, im); }
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return c2(a.x + b.x, a.y + b.y); }

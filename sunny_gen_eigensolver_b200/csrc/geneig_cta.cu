@@ -73,16 +73,16 @@ cudaError_t cta_set_attributes(int nmax, size_t smem) {
 }
 
 static cudaError_t cta_start(const CtaArgs& a, const CtaFourier& f, int nmax, int teams, bool fs, bool spec,
-                             cudaStream_t stream) {
+                             cudaStream_t stream, cudaEvent_t started = nullptr) {
     const long long ctas = (a.batch + teams - 1) / teams;
     const long long grid = ctas < 0x7fffffffLL ? ctas : 0x7fffffffLL;
-    cta_kernel(nmax, teams, fs, spec)<<<(unsigned)grid, teams * cta_threads_for(nmax),
-                                        cta_teams_smem_bytes(a.n, teams, spec), stream>>>(a, f);
-    return cudaGetLastError();
+    return launch_with_event(cta_kernel(nmax, teams, fs, spec), (unsigned)grid, teams * cta_threads_for(nmax),
+                             cta_teams_smem_bytes(a.n, teams, spec), stream, started, a, f);
 }
 
 cudaError_t cta_launch(int n, int nmax, int stage, const void* H, const void* S, double* W, void* U,
-                       int* info, long long batch, cudaStream_t stream, bool sigma, int teams, bool retry) {
+                       int* info, long long batch, cudaStream_t stream, bool sigma, int teams, bool retry,
+                       cudaEvent_t started) {
     CtaArgs a{};
     a.H = static_cast<const double2*>(H);
     a.S = static_cast<const double2*>(S);
@@ -95,7 +95,7 @@ cudaError_t cta_launch(int n, int nmax, int stage, const void* H, const void* S,
     a.stage = stage;
     a.sigma = sigma ? 1 : 0;
     a.retry = retry ? 1 : 0;
-    return cta_start(a, CtaFourier{}, nmax, teams, false, false, stream);
+    return cta_start(a, CtaFourier{}, nmax, teams, false, false, stream, started);
 }
 
 // Arguments of the intensity form (no U).

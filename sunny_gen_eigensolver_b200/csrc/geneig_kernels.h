@@ -53,9 +53,10 @@ cudaError_t cta_set_attributes(int nmax, size_t smem);   // every teams form of 
 // `sigma`: H is the metric diag(I_{n/2}, -I_{n/2}) and is not read (H may be NULL).
 // `teams`: pencils per CTA (1, or up to cta_max_teams(nmax)). `retry`: only
 // pencils whose info is kRetryInfo.
+// `started`: recorded when the last CTA has begun.
 cudaError_t cta_launch(int n, int nmax, int stage, const void* H, const void* S, double* W, void* U,
                        int* info, long long batch, cudaStream_t stream, bool sigma = false, int teams = 1,
-                       bool retry = false);
+                       bool retry = false, cudaEvent_t started = nullptr);
 
 // Spin-wave metric solve that reduces the eigenvectors to the spectrum
 // S(q, E) on the device (no U output): O is 3 x n complex per problem,
@@ -103,11 +104,13 @@ int tiled_slots_for(int n);     // CTAs, and default slots, per SM: 1 or 2
 cudaError_t tiled_set_attributes(size_t smem);
 // `mixed`: FP32 Householder reduction, FP64 refinement (see geneig_tiled.cu).
 // `refine_max`: mixed form's refinement steps before it falls back to FP64;
-// `defer`: a pencil that needs it gets info = kRetryInfo instead.
+// `defer`: a pencil that needs it gets info = kRetryInfo instead. `started`: as in
+// cta_launch.
 constexpr int kRefineMaxIters = 8;
 cudaError_t tiled_launch(int n, int slots, int stage, const void* H, const void* S, double* W, void* U,
                          int* info, long long batch, void* scratch, cudaStream_t stream, bool sigma,
-                         bool mixed = false, int refine_max = kRefineMaxIters, bool defer = false);
+                         bool mixed = false, int refine_max = kRefineMaxIters, bool defer = false,
+                         cudaEvent_t started = nullptr);
 
 struct PlainPlan {
     int    n        = 0;

@@ -80,7 +80,7 @@ cudaError_t tiled_set_attributes(size_t smem) {
 
 cudaError_t tiled_launch(int n, int slots, int stage, const void* H, const void* S, double* W, void* U,
                          int* info, long long batch, void* scratch, cudaStream_t stream, bool sigma, bool mixed,
-                         int refine_max, bool defer) {
+                         int refine_max, bool defer, cudaEvent_t started) {
     if (batch <= 0) return cudaSuccess;
     TiledArgs a;
     a.H = static_cast<const double2*>(H);
@@ -100,8 +100,7 @@ cudaError_t tiled_launch(int n, int slots, int stage, const void* H, const void*
     a.keep32 = defer && tiled_keep32(n) ? 1 : 0;
     const size_t smem = tiled_vec_bytes(n, !defer) + (a.keep32 ? tiled_c32_bytes(n) : 0);
     const long long grid = batch < slots ? batch : slots;
-    tiled_kernel(n, mixed)<<<(unsigned)grid, tiled_threads(n), smem, stream>>>(a);
-    return cudaGetLastError();
+    return launch_with_event(tiled_kernel(n, mixed), (unsigned)grid, tiled_threads(n), smem, stream, started, a);
 }
 
 }  // namespace sgeig

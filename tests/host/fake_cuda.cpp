@@ -19,6 +19,7 @@ static std::map<std::string, int> g_calls;
 // capturing stream's current dependencies (nodes are numbers).
 static std::map<size_t, size_t> g_capturing, g_event;
 static std::map<size_t, std::vector<cudaGraphNode_t>> g_deps;
+static std::map<size_t, std::vector<cudaGraphEdgeData>> g_edges;
 static size_t g_next = 100, g_memory = (size_t)1 << 40, g_used = 0;
 static std::map<size_t, size_t> g_blocks;
 
@@ -37,8 +38,10 @@ static cudaError_t kernel(const std::string& name, const std::string& what, cuda
         auto& d = g_deps[(size_t)s];
         const auto node = fresh<cudaGraphNode_t>();
         line += " node " + num(node) + " after";
-        for (auto n : d) line += " " + num(n);
+        for (size_t i = 0; i < d.size(); ++i)
+            line += " " + num(d[i]) + (g_edges[(size_t)s][i].from_port ? "-begun" : "");
         d = {node};
+        g_edges[(size_t)s] = {cudaGraphEdgeData{}};
     }
     return say(name, line) ? cudaErrorLaunchFailure : cudaSuccess;
 }
@@ -52,7 +55,7 @@ void fake_reset(const char* fail, size_t memory) {
     g_memory = memory;
 }
 void fake_capture(size_t stream, int on) {
-    if (on) { g_capturing[stream] = stream; g_deps[stream] = {fresh<cudaGraphNode_t>()}; return; }
+    if (on) { g_capturing[stream] = stream; g_deps[stream] = {fresh<cudaGraphNode_t>()}; g_edges[stream] = {cudaGraphEdgeData{}}; return; }
     std::map<size_t, size_t> left;
     for (auto& c : g_capturing) if (c.second != stream) left.insert(c);
     g_capturing = left;
@@ -104,19 +107,22 @@ cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
     if (in) g_capturing[(size_t)s] = g_event[(size_t)e];
     return cudaSuccess;
 }
-cudaError_t cudaStreamGetCaptureInfo_v2(cudaStream_t s, cudaStreamCaptureStatus* cs, unsigned long long*, cudaGraph_t*,
-                                        const cudaGraphNode_t** nodes, size_t* count) {
+cudaError_t cudaStreamGetCaptureInfo_v3(cudaStream_t s, cudaStreamCaptureStatus* cs, unsigned long long*, cudaGraph_t*,
+                                        const cudaGraphNode_t** nodes, const cudaGraphEdgeData** edges, size_t* count) {
     const bool in = g_capturing.count((size_t)s);
     *cs = in ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
-    if (in) { *nodes = g_deps[(size_t)s].data(); *count = g_deps[(size_t)s].size(); }
+    if (in) { *nodes = g_deps[(size_t)s].data(); *edges = g_edges[(size_t)s].data(); *count = g_deps[(size_t)s].size(); }
     return result(say("capture_info"));
 }
-cudaError_t cudaStreamUpdateCaptureDependencies(cudaStream_t s, cudaGraphNode_t* nodes, size_t count, unsigned flags) {
+cudaError_t cudaStreamUpdateCaptureDependencies_v2(cudaStream_t s, cudaGraphNode_t* nodes, const cudaGraphEdgeData* edges,
+                                                   size_t count, unsigned flags) {
     if (say("set_dependencies")) return cudaErrorLaunchFailure;
     if (!g_capturing.count((size_t)s)) return cudaErrorIllegalState;
     auto& d = g_deps[(size_t)s];
-    if (flags == cudaStreamSetCaptureDependencies) d.clear();
+    auto& x = g_edges[(size_t)s];
+    if (flags == cudaStreamSetCaptureDependencies) { d.clear(); x.clear(); }
     d.insert(d.end(), nodes, nodes + count);
+    x.insert(x.end(), edges, edges + count);
     return cudaSuccess;
 }
 cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus* cs) {
@@ -133,6 +139,7 @@ cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 
 namespace sgeig {
 
+static void started(cudaEvent_t e, cudaStream_t s) { if (e) g_log += "starts " + num(e) + " with " + num(s) + "\n"; }
 bool plain_plan(int n, int, PlainPlan* p, std::string*, bool mixed, const char* regime, int slots, int) {
     p->n = n;
     p->mixed = mixed;
@@ -162,9 +169,10 @@ int tiled_slots_for(int n) { return n > 200 ? 1 : 2; }
 int uneven_kind(int n, bool l2) { return !l2 ? 0 : n <= kCtaPreferredMaxN ? 5 : n <= kResidentMaxN ? kUnevenResident : kUnevenBig; }
 size_t uneven_smem_bytes(int, int) { return 1024; }
 cudaError_t cta_launch(int n, int, int, const void*, const void*, double*, void*, int*, long long, cudaStream_t s, bool,
-                       int, bool) { return kernel("cta", std::to_string(n) + " ", s); }
+                       int, bool, cudaEvent_t e) { started(e, s); return kernel("cta", std::to_string(n) + " ", s); }
 cudaError_t tiled_launch(int n, int, int, const void*, const void*, double*, void*, int*, long long, void* scratch,
-                         cudaStream_t s, bool, bool, int, bool) {
+                         cudaStream_t s, bool, bool, int, bool, cudaEvent_t e) {
+    started(e, s);
     return kernel("tiled", std::to_string(n) + " ", s, " slots " + num(scratch));
 }
 cudaError_t uneven_persistent_launch(const UnevenLaunch&, unsigned long long*, void*, size_t, int, size_t, cudaStream_t s) {

@@ -152,15 +152,21 @@ def test_captured_uneven_launch_keeps_to_the_callers_stream(lib):
     assert uneven_launch(lib, h, 11) == 0
     kernels = [x.split() for x in log(lib) if x.split()[0] in ("cta", "tiled", "persistent")]
     assert len(kernels) == 5 and not any(x.startswith(("record", "wait")) for x in log(lib))
-    assert all(k[k.index("on") + 1] == "11" and k[k.index("after") + 1:] == root for k in kernels)
-    nodes = sorted(k[k.index("node") + 1] for k in kernels)
+    # largest first, each from the point of the call and when the one before it has begun
+    assert [k[1] for k in kernels] == ["216", "162", "108", "72", "on"]
+    nodes = [k[k.index("node") + 1] for k in kernels]
+    for i, k in enumerate(kernels):
+        assert k[k.index("on") + 1] == "11" and k[k.index("after") + 1:] == root + [f"{x}-begun" for x in nodes[max(i - 1, 0):i]]
+    nodes.sort()
     assert sorted(lib.fake_dependencies(11).decode().split()) == nodes
     assert uneven_launch(lib, h, 12) == 0                 # not captured
     lib.fake_capture(13, 1)                                # a second capture
     assert uneven_launch(lib, h, 13) == 0 and uneven_launch(lib, h, 12) == 0
     assert uneven_launch(lib, h, 11) == 0                 # the first one goes on
     again = [x.split() for x in log(lib) if " on 11 " in x and "node" in x][5:]
-    assert all(sorted(k[k.index("after") + 1:]) == nodes for k in again) and len(again) == 5
+    assert len(again) == 5
+    for k in again:
+        assert sorted(x for x in k[k.index("after") + 1:] if not x.endswith("begun")) == nodes
     lib.fake_capture(11, 0)
     lib.fake_capture(13, 0)
     lib.sunny_geneig_uneven_destroy(h)
@@ -177,4 +183,27 @@ def test_captured_uneven_launch_joins_its_branches_whatever_fails(lib, fail):
     left = lib.fake_dependencies(11).decode().split()
     assert all(k[k.index("node") + 1] in left for k in nodes)
     lib.fake_capture(11, 0)
+    lib.sunny_geneig_uneven_destroy(h)
+
+
+def test_branches_start_largest_first_without_priorities(lib):
+    """Each side stream waits for the launch completion of the size before it, and no stream is put above the
+    caller's (priority 0 is the lowest)."""
+    reset(lib)
+    h = uneven_create(lib)
+    assert [x for x in log(lib) if x.startswith("stream")] and all(x.endswith("priority 0") for x in log(lib))
+    reset(lib)
+    assert uneven_launch(lib, h, 11) == 0
+    lines = log(lib)
+    fork = lines[0].split()[1]
+    assert lines[0] == f"record {fork} on 11"
+    before, i = fork, 1
+    for n in (216, 162, 108, 72):
+        st = lines[i].split()[3]
+        assert lines[i] == f"wait {before} on {st}" and st != "11"
+        before = lines[i + 1].split()[1]
+        assert lines[i + 1] == f"starts {before} with {st}" and lines[i + 2].split()[:4] == [
+            "cta" if n <= 110 else "tiled", str(n), "on", st]
+        i += 3
+    assert lines[i] == f"wait {before} on 11" and lines[i + 1] == "persistent on 11"
     lib.sunny_geneig_uneven_destroy(h)
