@@ -295,8 +295,10 @@ sunny_geneig_solver_t sunny_geneig_create_config(int n, int device_id, sunny_gen
  *     regimes[i] (NULL = all 0): 0 the default choice by N, 1 smem-cta
  *     (N <= 64), 2 l2-slot; per_item[i] (NULL or <= 0 = default: 4 in
  *     smem-cta, 1 in l2-slot). Reserves the l2-slot scratch (one or two slots
- *     per SM for each size above 110), the streams and the work counter. NULL on failure
- *     (last_error).
+ *     per SM for each size above 110: 0.4 GB for N = 216, 15 GB for eight sizes
+ *     from 442 to 512), the streams and the work counter. Where the device has no
+ *     room for all of that, it reserves the largest size's alone and the handle
+ *     runs its sizes one after another. NULL on failure (last_error).
  *   launch: arrays indexed like `sizes`; counts[i] >= 0 problems of size
  *     sizes[i] (0 skips the size, its buffers may then be NULL). The launch
  *     resets the counter on `stream` first (a memset node when captured).

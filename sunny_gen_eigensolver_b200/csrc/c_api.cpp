@@ -50,7 +50,10 @@ struct sunny_geneig_uneven {
     int n[sgeig::kUnevenMaxGroups] = {};
     int kind[sgeig::kUnevenMaxGroups] = {};
     int per_item[sgeig::kUnevenMaxGroups] = {};
-    void* big_scratch[sgeig::kUnevenMaxGroups] = {};   // kUnevenBig sizes: one slot per SM
+    // l2-slot scratch: an array for each kUnevenBig size and one for the
+    // persistent kernel's, or, where those do not fit the device, one array
+    // (`scratch`) for all, which then run one after another (no `side`).
+    void* big_scratch[sgeig::kUnevenMaxGroups] = {};
     int sms = 0;
     size_t smem = 0;
     int grid = 0;
@@ -93,6 +96,15 @@ void release_side(sgeig::UnevenSide& s) {
     for (cudaStream_t st : s.stream) if (st) cudaStreamDestroy(st);
     for (cudaEvent_t ev : s.join) if (ev) cudaEventDestroy(ev);
     if (s.fork) cudaEventDestroy(s.fork);
+}
+
+void release_scratch(sunny_geneig_uneven* h) {
+    for (void*& p : h->big_scratch) {
+        if (p != h->scratch) cudaFree(p);
+        p = nullptr;
+    }
+    cudaFree(h->scratch);
+    h->scratch = nullptr;
 }
 
 // NVTX range around each entry point (header-only NVTX v3: a no-op unless a
@@ -527,7 +539,7 @@ sunny_geneig_uneven_t sunny_geneig_uneven_create(int num_sizes, const int* sizes
             cudaError_t ea = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_id);
             if (ea == cudaSuccess) ea = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_id);
             if (ea != cudaSuccess) return ea;
-            size_t slot = 0;
+            size_t slot = 0, big[sgeig::kUnevenMaxGroups] = {};
             for (int g = 0; g < num_sizes; ++g) {
                 const int i = h->order[g], n = sizes[i];
                 const int r = regimes ? regimes[i] : 0;
@@ -541,8 +553,8 @@ sunny_geneig_uneven_t sunny_geneig_uneven_create(int num_sizes, const int* sizes
                     if (ea != cudaSuccess) { err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea); return ea; }
                 } else if (h->kind[g] == sgeig::kUnevenBig) {
                     ea = sgeig::tiled_set_attributes((size_t)optin);
-                    if (ea == cudaSuccess) ea = cudaMalloc(&h->big_scratch[g], (size_t)sms * sgeig::tiled_slots_for(n) * sgeig::tiled_slot_bytes(n));
-                    if (ea != cudaSuccess) { err = std::string("cudaMalloc scratch: ") + cudaGetErrorString(ea); return ea; }
+                    if (ea != cudaSuccess) { err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea); return ea; }
+                    big[g] = (size_t)sms * sgeig::tiled_slots_for(n) * sgeig::tiled_slot_bytes(n);
                 } else if (l2) slot = std::max(slot, sgeig::tiled_slot_elems(n));
             }
             if (h->smem > (size_t)optin) { err = "the mix needs more shared memory than a CTA has"; return cudaErrorInvalidValue; }
@@ -551,15 +563,28 @@ sunny_geneig_uneven_t sunny_geneig_uneven_create(int num_sizes, const int* sizes
             h->grid = 2 * sms;
             h->sms = sms;
             h->slot_elems = slot;
-            if (slot) {
-                ea = cudaMalloc(&h->scratch, (size_t)h->grid * slot * 16);
-                if (ea != cudaSuccess) { err = std::string("cudaMalloc scratch: ") + cudaGetErrorString(ea); return ea; }
+            const size_t small = (size_t)h->grid * slot * 16;
+            size_t largest = small;
+            ea = small ? cudaMalloc(&h->scratch, small) : cudaSuccess;
+            for (int g = 0; g < num_sizes; ++g) {
+                largest = std::max(largest, big[g]);
+                if (big[g] && ea == cudaSuccess) ea = cudaMalloc(&h->big_scratch[g], big[g]);
             }
+            bool together = true;              // the sizes may run at the same time
+            if (ea == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                release_scratch(h);
+                together = false;
+                ea = cudaMalloc(&h->scratch, largest);
+                for (int g = 0; g < num_sizes && ea == cudaSuccess; ++g)
+                    if (big[g]) h->big_scratch[g] = h->scratch;
+            }
+            if (ea != cudaSuccess) { err = std::string("cudaMalloc scratch: ") + cudaGetErrorString(ea); return ea; }
             ea = cudaMalloc(reinterpret_cast<void**>(&h->head), sizeof(unsigned long long));
             if (ea != cudaSuccess) { err = std::string("cudaMalloc counter: ") + cudaGetErrorString(ea); return ea; }
             int nside = 0;
             for (int g = 0; g < num_sizes; ++g) nside += h->kind[g] >= sgeig::kUnevenResident;
-            if (num_sizes < 2) nside = 0;      // a lone size runs on the caller's stream
+            if (num_sizes < 2 || !together) nside = 0;   // all on the caller's stream
             for (int i = 0; i < nside && ea == cudaSuccess; ++i) {
                 ea = cudaStreamCreateWithFlags(&h->side.stream[i], cudaStreamNonBlocking);
                 if (ea == cudaSuccess) ea = cudaEventCreateWithFlags(&h->side.join[i], cudaEventDisableTiming);
@@ -571,9 +596,8 @@ sunny_geneig_uneven_t sunny_geneig_uneven_create(int num_sizes, const int* sizes
         if (e != cudaSuccess) {
             set_error(std::string(fn) + ": " + (err.empty() ? cudaGetErrorString(e) : err));
             with_device(device_id, [&]() {
-                cudaFree(h->scratch);
+                release_scratch(h);
                 cudaFree(h->head);
-                for (void* p : h->big_scratch) cudaFree(p);
                 release_side(h->side);
                 if (h->done) cudaEventDestroy(h->done);
                 return cudaSuccess;
@@ -663,9 +687,8 @@ void sunny_geneig_uneven_destroy(sunny_geneig_uneven_t h) {
         with_device(h->device, [&]() {
             if (h->done) { cudaEventSynchronize(h->done); cudaEventDestroy(h->done); }
             release_side(h->side);
-            cudaFree(h->scratch);
+            release_scratch(h);
             cudaFree(h->head);
-            for (void* p : h->big_scratch) cudaFree(p);
             return cudaSuccess;
         });
         delete h;

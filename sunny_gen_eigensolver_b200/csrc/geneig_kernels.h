@@ -205,6 +205,7 @@ cudaError_t uneven_set_attributes(size_t smem);
 // kResidentMaxN, the shared-memory kernel; kind 7, above, the tiled kernel with
 // L.slots[i] slots at L.scratch[i].
 constexpr int kUnevenResident = 6, kUnevenBig = 7;
+// Without a fork event all sizes follow one another on the caller's stream.
 struct UnevenSide {
     cudaStream_t stream[kUnevenMaxGroups] = {};
     cudaEvent_t join[kUnevenMaxGroups] = {};

@@ -121,7 +121,8 @@ cudaError_t uneven_launch(const UnevenLaunch& L, unsigned long long* head, void*
     Fork fork(stream, side, capturing);
     cudaStream_t st = stream;
     cudaEvent_t started = nullptr;
-    cudaError_t e = nside + (nsmall > 0 ? 1 : 0) > 1 ? fork.begin() : cudaSuccess;
+    const bool several = nside + (nsmall > 0 ? 1 : 0) > 1;
+    cudaError_t e = several && side.fork ? fork.begin() : cudaSuccess;
     for (int i = 0; i < L.ngroups && e == cudaSuccess; ++i) {
         if (L.count[i] <= 0 || L.kind[i] < kUnevenResident) continue;
         e = fork.next(&st, &started);

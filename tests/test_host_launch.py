@@ -207,3 +207,41 @@ def test_branches_start_largest_first_without_priorities(lib):
         i += 3
     assert lines[i] == f"wait {before} on 11" and lines[i + 1] == "persistent on 11"
     lib.sunny_geneig_uneven_destroy(h)
+
+
+def _slots(n):
+    mat = n * (n | 1)
+    return 148 * (1 if n > 200 else 2) * 16 * (3 * mat + max((mat + 1) // 2, 16 * n))
+
+
+def test_uneven_handle_falls_back_to_one_slot_array(lib):
+    """Each size above 110 has slots of its own where they fit; where they do not, the largest size's are enough and
+    everything runs on the caller's stream."""
+    lib.fake_memory_used.restype = U
+    sizes = [442, 452, 462, 472, 482, 492, 502, 512]
+    all_, one = sum(map(_slots, sizes)), max(map(_slots, sizes))
+    reset(lib, memory=all_ + 4096)
+    h = uneven_create(lib, sizes)
+    assert h and lib.fake_memory_used() == all_ + 8
+    lib.sunny_geneig_uneven_destroy(h)
+    assert lib.fake_memory_used() == 0
+    reset(lib, memory=one + 4096)
+    h = uneven_create(lib, sizes)
+    assert h and lib.fake_memory_used() == one + 8
+    assert not any(x.startswith("stream") for x in log(lib))
+    reset(lib)
+    assert uneven_launch(lib, h, 11, sizes) == 0
+    lines = log(lib)
+    slots = lines[0].split()[-1]
+    assert lines[:-1] == [f"tiled {n} on 11 slots {slots}" for n in reversed(sizes)] and lines[-1].startswith("record")
+    reset(lib)
+    lib.fake_capture(11, 1)
+    assert uneven_launch(lib, h, 11, sizes) == 0
+    kernels = [x.split() for x in log(lib)]
+    for before, k in zip(kernels, kernels[1:]):          # a chain
+        assert k[k.index("after") + 1:] == [before[before.index("node") + 1]]
+    lib.fake_capture(11, 0)
+    lib.sunny_geneig_uneven_destroy(h)
+    assert lib.fake_memory_used() == 0
+    reset(lib, memory=one - 1)
+    assert not uneven_create(lib, sizes) and lib.fake_memory_used() == 0
