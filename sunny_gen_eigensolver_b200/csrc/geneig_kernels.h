@@ -98,7 +98,7 @@ __host__ __device__ inline size_t tiled_slot_elems(int n, bool mixed = false) {
 __host__ __device__ inline size_t tiled_slot_bytes(int n, bool mixed = false) {
     return tiled_slot_elems(n, mixed) * 16;
 }
-size_t tiled_vec_bytes(int n, bool work = true);   // dynamic shared memory, with or without the work area
+size_t tiled_vec_bytes(int n, bool mixed = false);   // dynamic shared memory
 int tiled_threads_for(int n);   // threads per CTA: 512 or 256
 int tiled_slots_for(int n);     // CTAs, and default slots, per SM: 1 or 2
 cudaError_t tiled_set_attributes(size_t smem);

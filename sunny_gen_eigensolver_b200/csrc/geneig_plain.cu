@@ -491,7 +491,7 @@ bool plain_plan(int n, int device, PlainPlan* plan, std::string* err, bool mixed
         e = cta_set_attributes(p.nmax, (size_t)optin);
     } else {
         p.regime = Regime::L2Slot;
-        p.smem = tiled_vec_bytes(n);
+        p.smem = tiled_vec_bytes(n, mixed);
         // resident CTAs (and scratch slots) per SM: SUNNY_GENEIG_SLOTS_PER_SM
         // = 1 or 2 (default: the kernel's occupancy limit, tiled_slots_for)
         p.threads = tiled_threads_for(n);

@@ -43,18 +43,20 @@ namespace sgeig {
 using namespace tiled;
 namespace {
 
-template <int NT, bool MIXED>
+template <int NT, bool MIXED, bool ROWS>
 __global__ void __launch_bounds__(NT, NT == kTiledWide ? 1 : 2) geneig_tiled_kernel(TiledArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* slot = a.scratch + (size_t)blockIdx.x * tiled_slot_elems(a.n, MIXED);
     phase_start();
-    for (long long b = blockIdx.x; b < a.batch; b += gridDim.x) tiled_solve<NT, MIXED>(a, b, slot, smem_raw);
+    for (long long b = blockIdx.x; b < a.batch; b += gridDim.x) tiled_solve<NT, MIXED, ROWS>(a, b, slot, smem_raw);
 }
 
 using TiledKernelFn = void (*)(TiledArgs);
 TiledKernelFn tiled_kernel(int n, bool mixed) {
-    if (tiled_threads(n) == kTiledWide) return mixed ? geneig_tiled_kernel<kTiledWide, true> : geneig_tiled_kernel<kTiledWide, false>;
-    return mixed ? geneig_tiled_kernel<kTiledNarrow, true> : geneig_tiled_kernel<kTiledNarrow, false>;
+    constexpr int W = kTiledWide, N = kTiledNarrow;
+    if (tiled_threads(n) == W) return mixed ? geneig_tiled_kernel<W, true, false> : geneig_tiled_kernel<W, false, false>;
+    if (tiled_rows(n, mixed)) return mixed ? geneig_tiled_kernel<N, true, true> : geneig_tiled_kernel<N, false, true>;
+    return mixed ? geneig_tiled_kernel<N, true, false> : geneig_tiled_kernel<N, false, false>;
 }
 
 }  // namespace
@@ -62,13 +64,16 @@ TiledKernelFn tiled_kernel(int n, bool mixed) {
 int tiled_threads_for(int n) { return tiled_threads(n); }
 int tiled_slots_for(int n) { return tiled_threads(n) == kTiledWide ? 1 : 2; }
 
-size_t tiled_vec_bytes(int n, bool work) { return tiled_base_bytes(n) + (work ? tiled_work_elems(n) * 16 : 0); }
+size_t tiled_vec_bytes(int n, bool mixed) {
+    return tiled_base_bytes(n) + (!tiled_rows(n, mixed) ? tiled_work_elems(n) * 16
+                                : mixed && tiled_keep32(n) ? tiled_c32_bytes(n) : 0);
+}
 
 // `smem` is the per-CTA shared-memory limit; the kernel's own static shared
 // memory (profiling builds have some) comes off the dynamic allowance.
 cudaError_t tiled_set_attributes(size_t smem) {
-    for (auto k : {tiled_kernel(1, false), tiled_kernel(1, true), tiled_kernel(kNarrowMaxN + 1, false),
-                   tiled_kernel(kNarrowMaxN + 1, true)}) {
+    for (int n : {1, kNarrowMaxN, kNarrowMaxN + 1})
+    for (auto k : {tiled_kernel(n, false), tiled_kernel(n, true)}) {
         cudaFuncAttributes fa{};
         cudaError_t e = cudaFuncGetAttributes(&fa, k);
         if (e == cudaSuccess)
@@ -96,9 +101,9 @@ cudaError_t tiled_launch(int n, int slots, int stage, const void* H, const void*
     a.sigma = sigma ? 1 : 0;
     a.refine_max = refine_max;
     a.defer = defer ? 1 : 0;
-    a.work = defer ? 0 : 1;
-    a.keep32 = defer && tiled_keep32(n) ? 1 : 0;
-    const size_t smem = tiled_vec_bytes(n, !defer) + (a.keep32 ? tiled_c32_bytes(n) : 0);
+    a.work = tiled_rows(n, mixed) ? 0 : 1;
+    a.keep32 = mixed && tiled_keep32(n) ? 1 : 0;
+    const size_t smem = tiled_vec_bytes(n, mixed);
     const long long grid = batch < slots ? batch : slots;
     return launch_with_event(tiled_kernel(n, mixed), (unsigned)grid, tiled_threads(n), smem, stream, started, a);
 }

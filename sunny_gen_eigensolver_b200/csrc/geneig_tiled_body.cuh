@@ -38,8 +38,9 @@ struct TiledArgs {
     int sigma;      // H = diag(I_{n/2}, -I_{n/2}), not read from memory
     int refine_max; // mixed: refinement steps before the FP64 fallback
     int defer;      // mixed: leave the fallback to the shared-memory kernel (info = kRetryInfo)
-    int work;       // the launch's shared memory has the work area (tiled_work_elems)
-    int keep32;     // mixed: it has the FP32 copy of C instead (tiled_keep32)
+    // (arguments rather than functions of n in the kernel: n = 216 2.5 % faster)
+    int work;       // the launch's shared memory has the work area (not tiled_rows)
+    int keep32;     // mixed: it has the FP32 copy of C (tiled_keep32)
 };
 
 // Ogita-Aishima refinement of the mixed form: it stops as soon as the current
@@ -114,9 +115,14 @@ struct TVec {
 constexpr int kMvRows = 128, kMvDepth = 3;
 __host__ __device__ inline size_t tiled_part_elems(int n) { return (size_t)(tiled_threads(n) / 32) * kMvRows; }
 __host__ __device__ inline size_t tiled_ring_elems(int n) { return (size_t)kMvDepth * (kMvRows / 32) * tiled_threads(n); }
-// The work area of the FP64 reduction, last in shared memory: launches of the
-// mixed form that leave their fallback to the shared-memory kernel go without
-// it, which leaves the SM's L1 to the refinement's products (N=54: 7 %).
+// The work area of the blocked FP64 reduction (tiled_house), last in shared
+// memory. Small sizes are reduced by house_rows and go without it, which leaves
+// the SM's L1 to the matrices. ms, two slots per SM, house_rows / tiled_house:
+// N=16 (4096 pencils) 1.36 / 1.82, N=54 (1024) 1.68 / 2.39, N=80 (592) 2.08 / 2.26,
+// N=90 2.75 / 2.87, N=96 3.16 / 3.09, N=108 4.15 / 3.90. The mixed form needs the
+// FP64 reduction for few pencils and keeps to house_rows up to kResidentMaxN
+// (U over H, 592 pencils of N=108: 6.48 / 7.20).
+__host__ __device__ constexpr bool tiled_rows(int n, bool mixed) { return n <= (mixed ? kResidentMaxN : 95); }
 __host__ __device__ inline size_t tiled_work_elems(int n) { return tiled_part_elems(n) + tiled_ring_elems(n); }
 
 __host__ __device__ inline size_t tiled_base_bytes(int n) {
@@ -125,9 +131,9 @@ __host__ __device__ inline size_t tiled_base_bytes(int n) {
     return (b + 15) & ~(size_t)15;
 }
 
-// The FP32 copy of C in the same place, for launches of the mixed form without
-// the work area and with two CTAs per SM (up to N = 101). N=54: the reduction
-// takes 333 K cycles on a copy in global memory, 191 K here.
+// The mixed form's FP32 copy of C in the same place, as long as two CTAs fit an
+// SM (up to N = 103). N=54: the reduction takes 333 K cycles on a copy in global
+// memory, 191 K here.
 __host__ __device__ inline size_t tiled_c32_bytes(int n) { return ((size_t)n * (n | 1) * 8 + 15) & ~(size_t)15; }
 __host__ __device__ inline bool tiled_keep32(int n) {
     return n <= kResidentMaxN && tiled_base_bytes(n) + tiled_c32_bytes(n) <= 112 * 1024;
@@ -789,100 +795,153 @@ __device__ __forceinline__ void tiled_house(int n, int ld, double2* M0, double2*
     __syncthreads();
 }
 
-// Mixed form: the reduction of the FP32 copy of C (in shared memory, n <= 128),
-// by the smem-cta kernel's scheme: per step one warp forms w and the next
-// reflector from the partial products, then every warp, over its block of 32
-// rows and its class of columns, applies A -= v w^H + w v^H and multiplies the
-// updated elements by the new reflector in the same pass. Two barriers a step.
-// Reflectors stay in C32's columns; tau, d, e widened to FP64. part: 32 pairs
+// The same names for both precisions.
+__device__ __forceinline__ float2 xmul(float2 a, float2 b) { return fcmul(a, b); }
+__device__ __forceinline__ double2 xmul(double2 a, double2 b) { return cmul(a, b); }
+__device__ __forceinline__ float2 xfma(float2 acc, float2 a, float2 b) { return fcfma(acc, a, b); }
+__device__ __forceinline__ double2 xfma(double2 acc, double2 a, double2 b) { return cfma(acc, a, b); }
+__device__ __forceinline__ float2 xfms_bc(float2 acc, float2 a, float2 b) { return fcfms_bc(acc, a, b); }
+__device__ __forceinline__ double2 xfms_bc(double2 acc, double2 a, double2 b) { return cfms_bc(acc, a, b); }
+__device__ __forceinline__ float xfma(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double xfma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float xsum(float v) { return warp_sumf(v); }
+__device__ __forceinline__ double xsum(double v) { return warp_sum(v); }
+__device__ __forceinline__ double2 widen(float2 a) { return f2d(a); }
+__device__ __forceinline__ double2 widen(double2 a) { return a; }
+template <class T2> __device__ __forceinline__ T2 xshfl(T2 v, int src) {
+    v.x = __shfl_sync(0xffffffffu, v.x, src);
+    v.y = __shfl_sync(0xffffffffu, v.y, src);
+    return v;
+}
+
+// Reflector from a column (alpha, x) whose elements, x from row lo on, the lanes
+// hold and `column` has room for; ss = ||x||^2.
+__device__ __forceinline__ void column_reflector(float2 alpha, float ss, float2& tau, float2& scal, float& beta) {
+    tau = scal = f2(0.0f, 0.0f);
+    beta = alpha.x;
+    if (!(ss == 0.0f && alpha.y == 0.0f)) {
+        beta = -copysignf(sqrtf(alpha.x * alpha.x + alpha.y * alpha.y + ss), alpha.x);
+        tau = f2((beta - alpha.x) / beta, -alpha.y / beta);
+        const float2 z = f2(alpha.x - beta, alpha.y);
+        const float inv = 1.0f / (z.x * z.x + z.y * z.y);
+        scal = f2(z.x * inv, -z.y * inv);
+    }
+}
+template <class Store>
+__device__ __forceinline__ void column_reflector(double2 alpha, double ss, double2& tau, double2& scal, double& beta,
+                                                 const double2* column, int lo, int n, Store store) {
+    const double rest = fma(alpha.y, alpha.y, ss), nn = fma(alpha.x, alpha.x, rest);
+    Reflector h;
+    if (squares_safe(rest, nn)) {
+        h = reflector(alpha, nn);
+    } else {
+        store();
+        __syncwarp();
+        h = column_out_of_range(column, lo, n, alpha, nn);
+        __syncwarp();
+    }
+    tau = h.tau;
+    scal = h.scal;
+    beta = h.beta;
+}
+
+// The reduction of a small C to tridiagonal form (n <= 128) by the smem-cta
+// kernel's scheme: per step one warp forms w and the next reflector from the
+// partial products, then every warp, over its block of 32 rows and its class of
+// columns, applies A -= v w^H + w v^H and multiplies the updated elements by the
+// new reflector in the same pass. Two barriers a step. The mixed form runs it on
+// the FP32 copy of C (in shared memory), the FP64 form on C in the slot
+// (tiled_rows). Reflectors stay in A's columns; tau, d, e in FP64. part: 32 values
 // per warp, vb: 2 n, wb: n.
-template <int kNT>
-__device__ __forceinline__ void house32(int n, int ld, float2* C32, float2* part, float2* vb, float2* wb, double2* tauv,
-                                        double* dv, double* ev) {
+template <int kNT, class T2>
+__device__ __forceinline__ void house_rows(int n, int ld, T2* A, T2* part, T2* vb, T2* wb, double2* tauv, double* dv,
+                                           double* ev) {
+    using T = decltype(T2::x);
     constexpr int NW = kNT / 32, R = 4;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int last = n - 1 - lane;                 // row of block t: last - 32 t
-    const float2 zero = f2(0.0f, 0.0f);
+    const T2 zero{0, 0}, one{1, 0};
     for (int i = tid; i < n; i += kNT) vb[n + i] = wb[i] = zero;
     __syncthreads();
     int rb = 0, G = 0, myt = 0, myg = 0;
-    float2 tau = zero;                             // of reflector c - 1
+    T2 tau = zero;                                 // of reflector c - 1
 #pragma unroll 1
     for (int c = 0; c < n; ++c) {
-        const float2* vk = vb + ((c + 1) & 1) * n;
-        float2* vc = vb + (c & 1) * n;
+        const T2* vk = vb + ((c + 1) & 1) * n;
+        T2* vc = vb + (c & 1) * n;
         if (warp == 0) {
-            float2 x[R], w[R];
-            float2* mc = C32 + c * ld;
+            T2 x[R], w[R];
+            T2* mc = A + c * ld;
             const int ic = n - 1 - c;              // slot of row c
 #pragma unroll
             for (int t = 0; t < R; ++t) x[t] = mc[max(last - 32 * t, 0)];
             if (c > 0) {
-                float2 v[R];
-                float s = 0.0f;
+                T2 v[R];
+                T s = 0;
 #pragma unroll
                 for (int t = 0; t < R; ++t) {
                     v[t] = vk[max(last - 32 * t, 0)];
                     w[t] = zero;
                 }
-                const float2* pt = part + lane;
+                const T2* pt = part + lane;
 #pragma unroll 2
                 for (int g = 0; g < G; ++g, pt += 32 * rb)
 #pragma unroll
                     for (int t = 0; t < R; ++t)
-                        if (t < rb) w[t] = f2(w[t].x + pt[32 * t].x, w[t].y + pt[32 * t].y);
+                        if (t < rb) { w[t].x += pt[32 * t].x; w[t].y += pt[32 * t].y; }
 #pragma unroll
-                for (int t = 0; t < R; ++t) s = fmaf(w[t].x, v[t].x, fmaf(w[t].y, v[t].y, s));
-                const float h = -0.5f * fmaf(tau.x, tau.x, tau.y * tau.y) * warp_sumf(s);
-                float2 wc = zero;
+                for (int t = 0; t < R; ++t) s = xfma(w[t].x, v[t].x, xfma(w[t].y, v[t].y, s));
+                const T h = T(-0.5) * xfma(tau.x, tau.x, tau.y * tau.y) * xsum(s);
+                T2 wc = zero;
 #pragma unroll
                 for (int t = 0; t < R; ++t) {
-                    w[t] = fcmul(tau, w[t]);
-                    w[t] = f2(fmaf(h, v[t].x, w[t].x), fmaf(h, v[t].y, w[t].y));
+                    w[t] = xmul(tau, w[t]);
+                    w[t].x = xfma(h, v[t].x, w[t].x);
+                    w[t].y = xfma(h, v[t].y, w[t].y);
                     if (last - 32 * t >= 0) wb[last - 32 * t] = w[t];
                     if ((ic >> 5) == t) wc = w[t];
                 }
-                wc = f2(__shfl_sync(0xffffffffu, wc.x, ic & 31), __shfl_sync(0xffffffffu, wc.y, ic & 31));
+                wc = xshfl(wc, ic & 31);
 #pragma unroll
                 for (int t = 0; t < R; ++t) {
-                    x[t] = fcfms_bc(x[t], v[t], wc);
-                    x[t] = f2(x[t].x - w[t].x, x[t].y - w[t].y);         // v(c) = 1
+                    x[t] = xfms_bc(x[t], v[t], wc);
+                    x[t].x -= w[t].x;                                    // v(c) = 1
+                    x[t].y -= w[t].y;
                 }
             }
-            float2 xc = x[0], alpha = x[0];
+            T2 xc = x[0], alpha = x[0];
 #pragma unroll
             for (int t = 1; t < R; ++t) {
                 if ((ic >> 5) == t) xc = x[t];
                 if (((ic - 1) >> 5) == t) alpha = x[t];
             }
-            float beta = 0.0f;
+            T beta = 0;
             if (c < n - 1) {
-                alpha = f2(__shfl_sync(0xffffffffu, alpha.x, (ic - 1) & 31), __shfl_sync(0xffffffffu, alpha.y, (ic - 1) & 31));
-                float ss = 0.0f;
+                alpha = xshfl(alpha, (ic - 1) & 31);
+                T ss = 0;
 #pragma unroll
                 for (int t = 0; t < R; ++t) {
                     if (last - 32 * t <= c + 1) x[t] = zero;
-                    ss = fmaf(x[t].x, x[t].x, fmaf(x[t].y, x[t].y, ss));
+                    ss = xfma(x[t].x, x[t].x, xfma(x[t].y, x[t].y, ss));
                 }
-                ss = warp_sumf(ss);
-                float2 scal = zero;
-                tau = zero;
-                beta = alpha.x;
-                if (!(ss == 0.0f && alpha.y == 0.0f)) {
-                    beta = -copysignf(sqrtf(alpha.x * alpha.x + alpha.y * alpha.y + ss), alpha.x);
-                    tau = f2((beta - alpha.x) / beta, -alpha.y / beta);
-                    const float2 z = f2(alpha.x - beta, alpha.y);
-                    const float inv = 1.0f / (z.x * z.x + z.y * z.y);
-                    scal = f2(z.x * inv, -z.y * inv);
+                ss = xsum(ss);
+                T2 scal;
+                if constexpr (sizeof(T) == 8) {
+                    column_reflector(alpha, ss, tau, scal, beta, vc, c + 2, n, [&]() {
+#pragma unroll
+                        for (int t = 0; t < R; ++t) if (last - 32 * t >= 0) vc[last - 32 * t] = x[t];
+                    });
+                } else {
+                    column_reflector(alpha, ss, tau, scal, beta);
                 }
 #pragma unroll
                 for (int t = 0; t < R; ++t) {
                     const int i = last - 32 * t;
-                    x[t] = fcmul(x[t], scal);
-                    if (i >= 0) vc[i] = i == c + 1 ? f2(1.0f, 0.0f) : x[t];
+                    x[t] = xmul(x[t], scal);
+                    if (i >= 0) vc[i] = i == c + 1 ? one : x[t];
                     if (i > c + 1) mc[i] = x[t];
                 }
-                if (lane == 0) tauv[c] = f2d(tau);
+                if (lane == 0) tauv[c] = widen(tau);
             }
             if (lane == (ic & 31)) {
                 dv[c] = (double)xc.x;
@@ -899,14 +958,14 @@ __device__ __forceinline__ void house32(int n, int ld, float2* C32, float2* part
         }
         if (myg < G) {
             const int i = last - 32 * myt, o = max(i, 0);
-            const float2 vi = vk[o], wi = wb[o];
-            float2 y = zero;
+            const T2 vi = vk[o], wi = wb[o];
+            T2 y = zero;
 #pragma unroll 4
             for (int j = c + 1 + myg; j < n; j += G) {
-                float2* q = C32 + o + j * ld;
-                const float2 z = fcfms_bc(fcfms_bc(*q, vi, wb[j]), wi, vk[j]);
+                T2* q = A + o + j * ld;
+                const T2 z = xfms_bc(xfms_bc(*q, vi, wb[j]), wi, vk[j]);
                 if (i >= 0) *q = z;
-                y = fcfma(y, z, vc[j]);
+                y = xfma(y, z, vc[j]);
             }
             part[32 * (myg * rb + myt) + lane] = y;
         }
@@ -921,7 +980,8 @@ __device__ __forceinline__ void house32(int n, int ld, float2* C32, float2* part
 // launch's dynamic shared memory as the vector area. kNT >= n.
 // MIXED: FP32 Householder reduction + FP64 refinement, an instance of its own
 // so that the FP64 form does not carry its pointers (n = 216: 1.6 %).
-template <int kNT, bool MIXED>
+// ROWS: tiled_rows(n, MIXED), the FP64 reduction is house_rows.
+template <int kNT, bool MIXED, bool ROWS>
 __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long long b, double2* slot,
                                             unsigned char* smem_raw) {
     constexpr int kNW = kNT / 32;
@@ -1064,7 +1124,7 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
                     }
                 if (a.keep32) {
                     __syncthreads();
-                    house32<kNT>(n, ld, C32s, reinterpret_cast<float2*>(v.gb), reinterpret_cast<float2*>(v.vb),
+                    house_rows<kNT>(n, ld, C32s, reinterpret_cast<float2*>(v.gb), reinterpret_cast<float2*>(v.vb),
                                  reinterpret_cast<float2*>(v.pb), v.tau, v.d, v.e);
                 } else {
                 float2* vbf = reinterpret_cast<float2*>(v.pb);
@@ -1142,6 +1202,8 @@ __device__ SGEIG_TILED_BODY_INLINE void tiled_solve(const TiledArgs& a, long lon
                 }
                 __syncthreads();
                 }
+            } else if constexpr (ROWS) {
+                house_rows<kNT>(n, ld, M0, v.gb, v.vb, reinterpret_cast<double2*>(v.dcd + (n & 1)), v.tau, v.d, v.e);
             } else {
                 tiled_house<kNT>(n, ld, M0, M2, smem_raw);
             }

@@ -84,8 +84,8 @@ __global__ void __launch_bounds__(kNT, 2) geneig_uneven_kernel(UnevenArgs a) {
             tiled::TiledArgs t;
             t.H = G.H; t.S = G.S; t.W = G.W; t.U = G.U; t.info = G.info;
             t.scratch = a.scratch; t.batch = G.count;
-            t.n = G.n; t.ld = G.n | 1; t.stage = 4; t.sigma = 0; t.refine_max = 0; t.defer = 0; t.work = 1; t.keep32 = 0;
-            for (long long b = b0; b < b1; ++b) tiled::tiled_solve<kNT, false>(t, b, slot, smem_raw);
+            t.n = G.n; t.ld = G.n | 1; t.stage = 4; t.sigma = 0; t.refine_max = 0; t.defer = 0; t.work = 0; t.keep32 = 0;
+            for (long long b = b0; b < b1; ++b) tiled::tiled_solve<kNT, false, true>(t, b, slot, smem_raw);   // (kind 5 is N <= 60)
         } else {
             cta::CtaArgs c;
             c.H = G.H; c.S = G.S; c.W = G.W; c.U = G.U; c.info = G.info;
