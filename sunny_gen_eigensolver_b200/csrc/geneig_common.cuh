@@ -5,6 +5,9 @@
 
 #include <cuda_runtime.h>
 #include <cstdint>
+#ifdef SGEIG_PHASE_TIMERS
+#include <vector>
+#endif
 
 namespace sgeig {
 
@@ -261,7 +264,8 @@ __device__ __forceinline__ void phase_level_flush(int slot) {
         phase_level() = 0;
     }
 }
-// Adds this translation unit's counters to `out` (and clears them).
+// Adds this translation unit's counters to `out` (and clears them). Each unit
+// that includes this header puts its own into phase_readers().
 static inline cudaError_t add_phase_cycles(unsigned long long* out, int count, bool reset) {
     unsigned long long mine[kPhaseSlots] = {};
     cudaError_t e = cudaMemcpyFromSymbol(mine, g_phase_cycles, sizeof(mine));
@@ -272,6 +276,12 @@ static inline cudaError_t add_phase_cycles(unsigned long long* out, int count, b
     }
     return e;
 }
+using PhaseReader = cudaError_t (*)(unsigned long long* out, int count, bool reset);
+inline std::vector<PhaseReader>& phase_readers() {
+    static std::vector<PhaseReader> r;
+    return r;
+}
+static const bool g_phase_registered = (phase_readers().push_back(add_phase_cycles), true);
 #else
 __device__ __forceinline__ void phase_start() {}
 __device__ __forceinline__ void phase_mark(int) {}

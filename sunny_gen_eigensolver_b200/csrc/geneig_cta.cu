@@ -161,7 +161,7 @@ extern "C" int sunny_geneig_phase_cycles(unsigned long long* out, int count, int
     if (count > kPhaseSlots) count = kPhaseSlots;
     cudaError_t e = cudaDeviceSynchronize();
     unsigned long long sum[kPhaseSlots] = {};
-    for (auto f : {cta_small_phase_cycles, cta_mid_phase_cycles, cta_wide_phase_cycles, tiled_phase_cycles})
+    for (PhaseReader f : phase_readers())
         if (e == cudaSuccess) e = f(sum, kPhaseSlots, reset != 0);
     for (int i = 0; out && i < count; ++i) out[i] = sum[i];
     return e == cudaSuccess ? 0 : -1;

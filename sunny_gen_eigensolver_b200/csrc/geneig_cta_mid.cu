@@ -12,8 +12,4 @@ CtaKernelFn cta_kernel_mid(int nmax) {
     }
 }
 
-#ifdef SGEIG_PHASE_TIMERS
-cudaError_t cta_mid_phase_cycles(unsigned long long* out, int count, bool reset) { return add_phase_cycles(out, count, reset); }
-#endif
-
 }  // namespace sgeig

@@ -109,9 +109,3 @@ cudaError_t tiled_launch(int n, int slots, int stage, const void* H, const void*
 }
 
 }  // namespace sgeig
-
-#ifdef SGEIG_PHASE_TIMERS
-namespace sgeig {
-cudaError_t tiled_phase_cycles(unsigned long long* out, int count, bool reset) { return add_phase_cycles(out, count, reset); }
-}  // namespace sgeig
-#endif
