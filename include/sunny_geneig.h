@@ -80,8 +80,7 @@ typedef enum {
 /* replaces src/common/c_api.h:50-55 (impl c_api.cpp:76-107).
  * Returns NULL on failure (message in sunny_geneig_last_error()).
  * batches_per_block_request: matrix pairs one CTA solves at a time. 0:
- * automatic (4 for N <= 16, 2 for N = 25..32, else 1: the fastest measured
- * on B200). 1: one per CTA. 2 or more: 2 for N <= 32, 4 for N <= 16 (the
+ * automatic (4 for N <= 16, 2 for N = 25..32, else 1). 1: one per CTA. 2 or more: 2 for N <= 32, 4 for N <= 16 (the
  * largest form at or below the request that the shared-memory kernel has;
  * 1 otherwise and in the global-memory regime).
  * sunny_geneig_batches_per_block reports the choice. */
@@ -337,17 +336,17 @@ sunny_geneig_status_t sunny_geneig_selftest_reciprocal(uintptr_t d_x, uintptr_t 
  * that forbid cudaMalloc from plugins, graph-replay setups that must not
  * touch the allocator. Same buffers, layouts, info codes and error
  * behaviour as sunny_geneig_launch, on the calling thread's current device,
- * with no handle. For n <= 60 it runs the shared-memory kernel, which needs
+ * with no handle. For n <= 110 it runs the shared-memory kernel, which needs
  * no scratch at all; above that, the L2-slot kernel with its per-CTA scratch
  * taken from a fixed 32 MiB device array built into the library (held by
  * every GPU that loads the library until the process exits), so it
  * allocates nothing. The array holds floor(32 MiB / slot) slots, so the
  * number of CTAs in flight, and with it the throughput, falls as n grows:
- * 161 at n = 61, 12 at n = 216, 2 at n = 512 (a regular handle keeps two
- * per SM). n outside [1, 512] is rejected with INVALID_ARG. The first call
+ * 48 at n = 111, 12 at n = 216, 2 at n = 512 (a regular handle keeps two
+ * per SM up to n = 200 and one above). n outside [1, 512] is rejected with INVALID_ARG. The first call
  * on a device resolves the array's address and sets the kernels'
  * shared-memory limits; make that first call before any stream capture.
- * All calls share the one array: calls whose kernels overlap on the GPU
+ * All calls with n > 110 share the one array: calls whose kernels overlap on the GPU
  * (other streams, other host threads) race on it and must be serialised by
  * the caller. */
 sunny_geneig_status_t sunny_geneig_launch_noalloc(

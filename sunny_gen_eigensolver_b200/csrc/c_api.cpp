@@ -552,7 +552,7 @@ sunny_geneig_uneven_t sunny_geneig_uneven_create(int num_sizes, const int* sizes
                     ea = sgeig::cta_set_attributes(sgeig::cta_nmax_for(n), (size_t)optin);
                     if (ea != cudaSuccess) { err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea); return ea; }
                 } else if (h->kind[g] == sgeig::kUnevenBig) {
-                    ea = sgeig::tiled_set_attributes((size_t)optin);
+                    ea = sgeig::tiled_set_attributes(n, false, (size_t)optin);
                     if (ea != cudaSuccess) { err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea); return ea; }
                     big[g] = (size_t)sms * sgeig::tiled_slots_for(n) * sgeig::tiled_slot_bytes(n);
                 } else if (l2) slot = std::max(slot, sgeig::tiled_slot_elems(n));

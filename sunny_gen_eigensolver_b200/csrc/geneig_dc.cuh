@@ -221,12 +221,6 @@ __host__ __device__ inline int secular_root_p(int i, int K, const double* dl, co
     return it;
 }
 
-// Single-lane form (host tests and callers without lane groups).
-__host__ __device__ inline int secular_root(int i, int K, const double* dl, const double* zz, double rho,
-                                            double& tau_out, int& org_out) {
-    return secular_root_p<1>(i, K, dl, zz, rho, 0, 0u, tau_out, org_out);
-}
-
 // Phase E of a level for NMAX > 0: the merges' products on the FP64 tensor
 // cores (mma.m8n8k4.f64), a warp per 8-row tile with all K columns of the
 // result in registers, so that the tile is read (and its old columns used up)

@@ -12,8 +12,6 @@ namespace sgeig {
 
 // Largest N accepted at create time.
 constexpr int kMaxN = 512;
-// Largest N whose two working matrices fit one CTA's shared memory.
-int smem_cta_max_n();
 
 // How one solve is laid out on the device.
 // Default choice by N: SmemCta up to 60, L2Slot above (measured crossovers);
@@ -22,7 +20,8 @@ enum class Regime : int {
     SmemCta  = 0,  // N <= 64: one matrix per pencil in shared memory, the rest in U's block
     SmemWide = 1,  // N <= ~80: both matrices in shared memory, column-group kernel
     L2Slot   = 2,  // any N: working matrices in a per-CTA global-memory slot, tiled MMA kernel
-                   // (the default up to kResidentMaxN is SmemCta's kernel all the same)
+                   // (the default up to kResidentMaxN is SmemCta's kernel all the same);
+                   // launches of one handle are ordered across streams
 };
 
 // Shared-memory kernel (geneig_cta.cu): the smem-cta regime can be asked for up
@@ -33,9 +32,10 @@ constexpr int kCtaMaxN = 64;
 constexpr int kCtaPreferredMaxN = 60;
 // Above it, up to here, the l2-slot size class is also solved by that kernel
 // (one CTA of 128 to 512 threads per pencil, no slots) unless a number of
-// slots per SM is asked for: the largest N whose matrix and vectors fit one
-// CTA's shared memory. Solves/s, shared memory / slots: N=62 1227 K / 411 K,
-// N=77 569 K / 273 K, N=96 305 K / 192 K, N=108 227 K / 151 K.
+// slots per SM is asked for. Its matrix and vectors fit one CTA's shared memory
+// (those of 111 and 112 would too; they run in slots). Solves/s, shared memory /
+// two slots per SM: N=62 1232 K / 565 K, N=77 566 K / 308 K, N=96 303 K / 193 K,
+// N=108 227 K / 152 K.
 constexpr int kResidentMaxN = 110;
 // info of a pencil that the mixed form leaves to a following cta_launch with
 // `retry` (never seen by the caller).
@@ -101,7 +101,7 @@ __host__ __device__ inline size_t tiled_slot_bytes(int n, bool mixed = false) {
 size_t tiled_vec_bytes(int n, bool mixed = false);   // dynamic shared memory
 int tiled_threads_for(int n);   // threads per CTA: 512 or 256
 int tiled_slots_for(int n);     // CTAs, and default slots, per SM: 1 or 2
-cudaError_t tiled_set_attributes(size_t smem);
+cudaError_t tiled_set_attributes(int n, bool mixed, size_t smem);   // of the size's kernel
 // `mixed`: FP32 Householder reduction, FP64 refinement (see geneig_tiled.cu).
 // `refine_max`: mixed form's refinement steps before it falls back to FP64;
 // `defer`: a pencil that needs it gets info = kRetryInfo instead. `started`: as in

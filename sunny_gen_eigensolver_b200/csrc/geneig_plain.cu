@@ -388,8 +388,6 @@ __global__ void __launch_bounds__(kNT, 1) geneig_plain_kernel(PlainArgs a) {
     }
 }
 
-int g_smem_optin = -1;
-
 constexpr int kWideNmax = 96;
 
 // A, B and the vectors.
@@ -404,16 +402,6 @@ static_assert(leaves_fit_b(), "B holds the matrix and the rows of the leaves");
 
 }  // namespace
 
-int smem_cta_max_n() {
-    // largest n with 2*n*ld*16 + vectors <= 227 KB (ld = n | 1)
-    int best = 0;
-    for (int n = 1; n <= kMaxN; ++n) {
-        const size_t bytes = wide_smem_bytes(n);
-        if (bytes <= 232448) best = n;
-    }
-    return best;
-}
-
 bool plain_plan(int n, int device, PlainPlan* plan, std::string* err, bool mixed, const char* regime,
                 int slots_per_sm, int pencils_per_cta) {
     if (n < 1 || n > kMaxN) {
@@ -425,7 +413,6 @@ bool plain_plan(int n, int device, PlainPlan* plan, std::string* err, bool mixed
     if (e != cudaSuccess) { *err = std::string("cudaDeviceGetAttribute: ") + cudaGetErrorString(e); return false; }
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) { *err = std::string("cudaDeviceGetAttribute: ") + cudaGetErrorString(e); return false; }
-    g_smem_optin = optin;
 
     // Optional override for measurements: SUNNY_GENEIG_REGIME = smem-cta |
     // smem-wide | l2-slot picks that regime wherever it can hold n.
@@ -500,7 +487,7 @@ bool plain_plan(int n, int device, PlainPlan* plan, std::string* err, bool mixed
         else if (const char* ps = std::getenv("SUNNY_GENEIG_SLOTS_PER_SM")) per_sm = std::atoi(ps) == 1 ? 1 : 2;
         p.slots = per_sm * sms;
         p.scratch_bytes = (size_t)p.slots * tiled_slot_bytes(n, mixed);
-        e = tiled_set_attributes((size_t)optin);
+        e = tiled_set_attributes(n, mixed, (size_t)optin);
         if (mixed && n <= kResidentMaxN && cta_smem_bytes(n) <= (size_t)optin) {
             p.nmax = cta_nmax_for(n);
             if (e == cudaSuccess) e = cta_set_attributes(p.nmax, (size_t)optin);
@@ -562,7 +549,7 @@ cudaError_t plain_launch(const PlainPlan& plan, int stage, const void* H, const 
 // the life of the process. It holds floor(32 MiB / slot) slots, so the
 // number of resident CTAs, and with it the throughput, falls with n: 48
 // CTAs at n = 111, 12 at n = 216, 2 at n = 512 (the regular launch keeps
-// one per SM, 148 on B200).
+// two per SM up to n = 200 and one above, 296 or 148 on B200).
 namespace {
 
 constexpr size_t kNoAllocScratchBytes = size_t(32) << 20;   // 32 MiB per device
@@ -593,7 +580,8 @@ cudaError_t noalloc_setup(int dev, NoAllocDevice** out, std::string* err) {
         int optin = 0;
         e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         if (e != cudaSuccess) { *err = std::string("cudaDeviceGetAttribute: ") + cudaGetErrorString(e); return e; }
-        e = tiled_set_attributes((size_t)optin);
+        for (int n : {kResidentMaxN + 1, kMaxN})            // both of its kernels
+            if (e == cudaSuccess) e = tiled_set_attributes(n, false, (size_t)optin);
         for (int nmax : {16, 24, 32, 40, 48, 56, 64, 72, 80, 96, 112})
             if (e == cudaSuccess) e = cta_set_attributes(nmax, (size_t)optin);
         if (e != cudaSuccess) { *err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e); return e; }

@@ -16,11 +16,12 @@
 //       C = L^-1 H L^-H; for the spin-wave metric H = diag(I, -I) the first
 //       product is a sign flip of X^H                              (:248)
 //   a5  C = Q T Q^H (Householder, lower; v_k kept in column k of M0 below
-//       the subdiagonal; for n >= 96 in 16-column panels whose trailing
-//       update A -= V W^H + W V^H is a GEMM), T = Z diag(w) Z^T by divide and conquer (Z and its
-//       merge workspace in M2, merge products through Zo), V = Q Z with
-//       compact-WY blocks of 16 reflectors, Q_b = I - Y T_b Y^H, two blocks
-//       at a time on strips of 8 columns of V, a warp each, V in the output U   (:250)
+//       the subdiagonal; in 16-column panels whose trailing update A -= V W^H +
+//       W V^H is a GEMM, small n (tiled_rows) in one pass per column),
+//       T = Z diag(w) Z^T by divide and conquer (Z and its merge workspace in
+//       M2, merge products through Zo), V = Q Z with compact-WY
+//       blocks of 16 reflectors, Q_b = I - Y T_b Y^H, two blocks at a time on
+//       strips of 8 columns of V, a warp each, V in the output U   (:250)
 //   a6  U = X^H V into M2, copied to the output                   (:252)
 //   a7  W ascending, U columns in the same order                  (:268-276)
 //
@@ -32,8 +33,8 @@
 // and conquer, the back-transform and everything else stay FP64; then
 // Ogita-Aishima refinement steps (FP64 tensor-core GEMMs against the FP64 C,
 // repeated until the correction is negligible) recover FP64 eigenpairs of C
-// before U = X^H V. A pencil whose refinement does not converge is solved in
-// FP64: from C in this kernel, or (`defer`) by the shared-memory kernel, which
+// before U = X^H V. A pencil whose refinement does not converge, or that FP32
+// cannot hold, is solved in FP64: from C in this kernel, or (`defer`) by the shared-memory kernel, which
 // is the plain form of the sizes it holds.
 
 #include "geneig_tiled_body.cuh"
@@ -71,16 +72,12 @@ size_t tiled_vec_bytes(int n, bool mixed) {
 
 // `smem` is the per-CTA shared-memory limit; the kernel's own static shared
 // memory (profiling builds have some) comes off the dynamic allowance.
-cudaError_t tiled_set_attributes(size_t smem) {
-    for (int n : {1, kNarrowMaxN, kNarrowMaxN + 1})
-    for (auto k : {tiled_kernel(n, false), tiled_kernel(n, true)}) {
-        cudaFuncAttributes fa{};
-        cudaError_t e = cudaFuncGetAttributes(&fa, k);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem - fa.sharedSizeBytes));
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+cudaError_t tiled_set_attributes(int n, bool mixed, size_t smem) {
+    const TiledKernelFn k = tiled_kernel(n, mixed);
+    cudaFuncAttributes fa{};
+    const cudaError_t e = cudaFuncGetAttributes(&fa, k);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem - fa.sharedSizeBytes));
 }
 
 cudaError_t tiled_launch(int n, int slots, int stage, const void* H, const void* S, double* W, void* U,
