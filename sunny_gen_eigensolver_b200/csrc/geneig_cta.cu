@@ -58,8 +58,8 @@ int cta_threads_for(int nmax) { return cta_team_threads(nmax); }
 
 // `smem` is the per-CTA shared-memory limit; the kernel's own static shared
 // memory (profiling builds have some) comes off the dynamic allowance.
-cudaError_t cta_set_attributes(int nmax, size_t smem) {
-    for (int form = 0; form < (nmax > kCtaMaxN ? 1 : 4); ++form)
+cudaError_t cta_set_attributes(int nmax, size_t smem, bool extra) {
+    for (int form = 0; form < (extra ? 4 : 1); ++form)
         for (int teams = 1; teams <= cta_max_teams(nmax); teams *= 2) {
             const CtaKernelFn k = cta_kernel(nmax, teams, (form & 1) != 0, (form & 2) != 0);
             cudaFuncAttributes fa{};

@@ -49,7 +49,10 @@ int cta_threads_for(int nmax);   // threads per pencil (per team) of that row bo
 int cta_max_teams(int nmax);
 int cta_default_teams(int nmax);   // pencils per CTA when none is requested
 size_t cta_teams_smem_bytes(int n, int teams, bool spec = false);
-cudaError_t cta_set_attributes(int nmax, size_t smem);   // every teams form of the row bound
+// Every teams form of the row bound; `extra`: with the Fourier and intensity
+// forms, for handles that launch them (each kernel is loaded at this point, which
+// takes milliseconds once per process).
+cudaError_t cta_set_attributes(int nmax, size_t smem, bool extra = false);
 // `sigma`: H is the metric diag(I_{n/2}, -I_{n/2}) and is not read (H may be NULL).
 // `teams`: pencils per CTA (1, or up to cta_max_teams(nmax)). `retry`: only
 // pencils whose info is kRetryInfo.

@@ -462,7 +462,7 @@ bool plain_plan(int n, int device, PlainPlan* plan, std::string* err, bool mixed
         p.teams = teams;
         p.smem = cta_teams_smem_bytes(n, teams);
         p.threads = teams * cta_threads_for(p.nmax);
-        e = cta_set_attributes(p.nmax, (size_t)optin);
+        e = cta_set_attributes(p.nmax, (size_t)optin, true);
     } else if (!mixed && wide_ok && want == "smem-wide") {
         p.regime = Regime::SmemWide;
         p.smem = smem_wide;

@@ -162,7 +162,7 @@ bool tune_lookup(const std::string&, int, std::string*) { return false; }
 void tune_store(const std::string&, int, const std::string&) {}
 int tune_pick(int, int, const std::vector<std::pair<std::string, int>>&, std::string*) { return 0; }
 int cta_nmax_for(int) { return 0; }
-cudaError_t cta_set_attributes(int, size_t) { return cudaSuccess; }
+cudaError_t cta_set_attributes(int, size_t, bool) { return cudaSuccess; }
 cudaError_t tiled_set_attributes(int, bool, size_t) { return cudaSuccess; }
 cudaError_t uneven_set_attributes(size_t) { return cudaSuccess; }
 int tiled_slots_for(int n) { return n > 200 ? 1 : 2; }
