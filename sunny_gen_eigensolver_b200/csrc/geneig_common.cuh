@@ -173,8 +173,7 @@ struct Reflector {
 };
 // True where the squares neither underflow nor overflow and rest is not zero
 // (rest at least 2^-927, nn below 2^929, about 1e-279 and 1e+279; compares on the
-// exponents, false for NaN): reflector() holds, else
-// reflector_scaled().
+// exponents, false for NaN): reflector() holds.
 __device__ __forceinline__ bool squares_safe(double rest, double nn) {
     return __double2hiint(rest) >= 0x06000000 && __double2hiint(nn) < 0x7a000000;
 }
@@ -189,22 +188,21 @@ __device__ __forceinline__ Reflector reflector(double2 alpha, double nn) {
     h.scal = c2(z.x * inv, -z.y * inv);
     return h;
 }
-// The same from ss = ||f x||^2, f = column_scale(nn): for columns of zeros, those
-// that the rounding residues of a low-rank matrix leave (1e-16, 1e-32, 1e-48, ...
-// of its norm), and matrices of extreme scale. A column below 2^-1000 is zero.
-__device__ __forceinline__ double column_scale(double nn) {
-    return nn >= 0x1p-900 && nn <= 0x1p900 ? 1.0 : nn < 1.0 ? 0x1p700 : 0x1p-700;
-}
-__device__ __forceinline__ Reflector reflector_scaled(double2 alpha, double ss, double f) {
-    const double2 a = cscale(alpha, f);
-    const double rest = fma(a.y, a.y, ss), nn = fma(a.x, a.x, rest);
+// Otherwise the same from the column times f = column_scale(nn) (as = f alpha,
+// rest its sum): columns of zeros, those that the rounding residues of a low-rank
+// matrix leave (1e-16, 1e-32, 1e-48, ... of its norm), and matrices of extreme
+// scale. A column below 2^-1000 is zero, and so is one whose x underflows beside an
+// alpha above 2^-200.
+__device__ __forceinline__ double column_scale(double nn) { return nn < 0x1p-400 ? 0x1p700 : 0x1p-700; }
+__device__ __forceinline__ Reflector reflector_scaled(double2 alpha, double2 as, double rest, double f) {
+    const double nn = fma(as.x, as.x, rest);
     Reflector h;
     h.tau = h.scal = c2(0.0, 0.0);
     h.beta = alpha.x;
     if (!(rest == 0.0 || (f > 1.0 && nn < 0x1p-600))) {
-        h = reflector(a, nn);
-        h.beta *= f > 1.0 ? 0x1p-700 : f < 1.0 ? 0x1p700 : 1.0;
-        h.scal = cscale(h.scal, f);
+        h = reflector(as, nn);
+        h.beta *= f > 1.0 ? 0x1p-700 : 0x1p700;
+        h.scal = cscale(h.scal, f);                      // scal is applied to x itself
     }
     return h;
 }

@@ -81,7 +81,6 @@ __host__ __device__ inline size_t cta_dc_bytes(int n, bool spec) {   // (d, e) f
 // The reduction's panel is two blocks wide where one pencil has the SM (its
 // shared memory) to itself anyway. N=108: 235 K cycles for one, 141 K for two.
 __host__ __device__ constexpr bool cta_two_panels(int nw) { return nw >= 16; }
-constexpr int kRefinePanel = 1 << 16;   // beside the failed minor's order in rank[0]
 constexpr int kDElems = 72;       // an 8 x 8 tile with leading dimension 9
 __host__ __device__ inline size_t cta_work_bytes(int n, int nw, bool spec) {
     const size_t one = (size_t)8 * (n | 1);
@@ -254,34 +253,32 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
     // lane's share of it passes 8 the panel takes one step of refinement. N = 16,
     // cond(S) = 1e10, mean ||U^H S U - I||: 12.3e-8 without the step, 5.4e-8 with it,
     // 7.5e-8 LAPACK's. At cond(S) = 100 (kappa^2 up to 9) it is not needed; taken in
-    // every panel it would cost N = 54 2.5 % of the solve, the test costs 0.6 %.
+    // every panel it would cost N = 54 2.5 % of the solve.
     double2* Pn = work;                // n x 8 panel of L; rows 0 .. 7 (above every panel): L_pp
     const int ldp = n | 1;
     double2* Ds = work + 8 * ldp;      // D of even and odd panels: element (i, j) at i + 9 j
-    // warp 0: L of the diagonal tile at o into rows 0 .. 7 of Pn (an infinite
-    // pivot's column is zero)
-    auto tile_l = [&](int o) {
-        double2 x[2];
-#pragma unroll
-        for (int s = 0; s < 2; ++s) x[s] = 2 * fq + s <= fr ? M[o + fr + (o + 2 * fq + s) * ld] : zero;
+    // warp 0: L of the diagonal tile at o, row by lane, into rows 0 .. 7 of Pn, in
+    // the same operations as factor() (D has to be this L's inverse; the scales are
+    // D's diagonal; an infinite pivot's column is zero)
+    auto tile_l = [&](int o, const double2* Dp) {
+        double2* row = Pn + (lane & 7);
 #pragma unroll 1
-        for (int h = 0; h < 4; ++h) {
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const int c = 2 * h + u;
-                const double akk = __shfl_sync(0xffffffffu, x[u].x, 4 * c + h);
-                const double r = rsqrt(akk), l = akk * r;
-                const double2 aic = shfl2(x[u], (lane & 28) + h), aik = cscale(aic, r * r);
-                if (fq == h)
-                    Pn[fr + c * ldp] = fr > c ? cscale(aic, r)
-                                     : c2(fr == c && r > 0.0 ? fma(l, fma(-l, r, 1.0), l) : 0.0, 0.0);
-#pragma unroll
-                for (int s = 0; s < 2; ++s) {
-                    const double2 ajc = shfl2(x[u], 4 * (2 * fq + s) + h);
-                    if (2 * fq + s > c && 2 * fq + s <= fr) x[s] = cfms_bc(x[s], aik, ajc);
-                }
+        for (int c = -1; c < 8; ++c) {
+#pragma unroll 1
+            for (int j = c + 1; j < 8 && lane < 8; ++j) {
+                const double r = c < 0 ? 0.0 : Dp[10 * c].x;
+                if (c < 0) row[j * ldp] = j <= lane ? M[o + lane + (o + j) * ld] : zero;
+                else if (lane >= j) row[j * ldp] = cfms_bc(row[j * ldp], cscale(row[c * ldp], r * r), Pn[j + c * ldp]);
             }
+            __syncwarp();
         }
+#pragma unroll 1
+        for (int j = 0; j <= lane && lane < 8; ++j) {
+            const double2 v = row[j * ldp];
+            const double r = Dp[10 * j].x, l = v.x * r;
+            row[j * ldp] = j < lane ? cscale(v, r) : c2(r > 0.0 ? fma(l, fma(-l, r, 1.0), l) : 0.0, 0.0);
+        }
+        __syncwarp();
     };
     auto factor = [&](int p) {         // warp 0; lane: row fr, columns 2 fq + s of the tile
         const int o = 8 * p;
@@ -292,9 +289,6 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
             const int j = 2 * fq + s;
             x[s] = (o + fr < n && j <= fr) ? M[o + fr + (o + j) * ld] : c2(fr == j ? 1.0 : 0.0, 0.0);
         }
-        double kap = 0.0, ajj[2];      // A's diagonal in this lane's columns
-#pragma unroll
-        for (int s = 0; s < 2; ++s) ajj[s] = __shfl_sync(0xffffffffu, x[s].x, 4 * (2 * fq + s) + fq);
         int bad = 0;
         double rr = 0.0;               // 1 / L of this lane's row
 #pragma unroll 1
@@ -327,16 +321,12 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
                 }
             }
         }
+        if (lane == 0) rank[0] = bad;
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
             const int j = 2 * fq + s;
-            const double2 d = j < fr ? cscale(x[s], rr) : c2(j == fr ? rr : 0.0, 0.0);
-            Dp[fr + 9 * j] = d;
-            kap = fma(ajj[s], fma(d.x, d.x, d.y * d.y), kap);
+            Dp[fr + 9 * j] = j < fr ? cscale(x[s], rr) : c2(j == fr ? rr : 0.0, 0.0);
         }
-        const bool refine = __any_sync(0xffffffffu, kap > 8.0) && o + 8 < n;
-        if (lane == 0) rank[0] = bad | (refine ? kRefinePanel : 0);
-        if (refine) tile_l(o);
     };
     int fail = 0;
 #pragma unroll 1
@@ -344,10 +334,17 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
         const int o = 8 * p;
         const double2* Dp = Ds + (p & 1) * kDElems;
         if (p >= 0) {
-            const int st = rank[0];
-            fail = st & (kRefinePanel - 1);
+            fail = rank[0];
             if (fail) break;
-            const bool refine = st >= kRefinePanel;
+            // (A's diagonal is in M until warp 0 puts D there below)
+            double kap = 0.0;
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                const int k = 2 * fq + s;
+                const double2 d = Dp[fr + 9 * k];
+                kap = fma(M[min(o + k, n - 1) * (ld + 1)].x, fma(d.x, d.x, d.y * d.y), kap);
+            }
+            const bool refine = __any_sync(0xffffffffu, kap > 8.0) && o + 8 < n;
 #pragma unroll 1
             for (int t = warp; t < nb - 1; t += NW) {
                 double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
@@ -360,26 +357,46 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
                     const double2 m = xt ? M[min(o + k, n - 1) + (8 * t + fr) * ld] : M[i + (o + k) * ld];
                     zmma(re, im, xt ? dd : m, xt ? m : cconj(dd));
                 }
-                if (refine && !xt) {
-                    double dr[2], di[2];   // A - L L_pp^H (an accumulator is laid out as the next A fragment)
-#pragma unroll
-                    for (int s = 0; s < 2; ++s) {
-                        const double2 m = M[i + (o + 2 * fq + s) * ld];
-                        dr[s] = m.x;
-                        di[s] = m.y;
-                    }
-#pragma unroll
-                    for (int s = 0; s < 2; ++s)
-                        zmma(dr, di, c2(-re[s], -im[s]), cconj(Pn[fr + (2 * fq + s) * ldp]));
-#pragma unroll
-                    for (int s = 0; s < 2; ++s) zmma(re, im, c2(dr[s], di[s]), cconj(Dp[fr + 9 * (2 * fq + s)]));
-                }
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const int j = 2 * fq + e;
                     if (xt) {
                         if (o + fr < n) M[o + fr + (8 * t + j) * ld] = c2(re[e], im[e]);
                     } else if (i < n) {
+                        Pn[i + j * ldp] = c2(re[e], im[e]);
+                        if (a.stage == 1) Ub[i + (size_t)(o + j) * n] = c2(re[e], im[e]);
+                    }
+                }
+            }
+            if (refine) {                  // the same verdict in every warp
+                if (warp == 0) tile_l(o, Dp);
+                team_sync<NT, BLOCK>();
+                // every lane on the elements of L that it has just written (an
+                // accumulator is laid out as the next A fragment)
+#pragma unroll 1
+                for (int t = warp; t < nb - 1; t += NW) {
+                    if (t < p) continue;
+                    const int i = 8 * (t + 1) + fr;
+                    double re[2], im[2], dr[2], di[2];
+                    double2 l[2];
+#pragma unroll
+                    for (int s = 0; s < 2; ++s) {
+                        l[s] = Pn[i + (2 * fq + s) * ldp];
+                        re[s] = l[s].x;
+                        im[s] = l[s].y;
+                        const double2 m = M[i + (o + 2 * fq + s) * ld];
+                        dr[s] = m.x;
+                        di[s] = m.y;
+                    }
+#pragma unroll
+                    for (int s = 0; s < 2; ++s)          // A - L L_pp^H
+                        zmma(dr, di, c2(-l[s].x, -l[s].y), cconj(Pn[fr + (2 * fq + s) * ldp]));
+#pragma unroll
+                    for (int s = 0; s < 2; ++s) zmma(re, im, c2(dr[s], di[s]), cconj(Dp[fr + 9 * (2 * fq + s)]));
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int j = 2 * fq + e;
+                        if (i >= n) continue;
                         Pn[i + j * ldp] = c2(re[e], im[e]);
                         if (a.stage == 1) Ub[i + (size_t)(o + j) * n] = c2(re[e], im[e]);
                     }
@@ -814,18 +831,19 @@ __device__ SGEIG_CTA_BODY_INLINE void cta_solve(const CtaArgs& a, long long b, u
                     }
                     ss = warp_sum(ss);
                     const double rest = fma(alpha.y, alpha.y, ss), nn = fma(alpha.x, alpha.x, rest);
-                    Reflector h;
-                    if (squares_safe(rest, nn)) {
-                        h = reflector(alpha, nn);
-                    } else {
+                    // (the test comes after the reflector, out of its chain: N=54, batch 100, 1 %)
+                    Reflector h = reflector(alpha, nn);
+                    if (!squares_safe(rest, nn)) {
                         const double f = column_scale(nn);
+                        const double2 as = cscale(alpha, f);
                         ss = 0.0;
 #pragma unroll
                         for (int t = 0; t < R; ++t) {
                             const double2 y = cscale(x[t], f);
                             ss = fma(y.x, y.x, fma(y.y, y.y, ss));
                         }
-                        h = reflector_scaled(alpha, warp_sum(ss), f);
+                        const double rs = fma(as.y, as.y, warp_sum(ss));
+                        h = reflector_scaled(alpha, as, rs, f);
                     }
                     beta = h.beta;
 #pragma unroll

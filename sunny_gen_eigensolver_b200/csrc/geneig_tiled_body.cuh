@@ -674,7 +674,8 @@ static __device__ __noinline__ Reflector column_out_of_range(const double2* x, i
         const double2 y = cscale(x[i], f);
         ss = fma(y.x, y.x, fma(y.y, y.y, ss));
     }
-    return reflector_scaled(alpha, warp_sum(ss), f);
+    const double2 as = cscale(alpha, f);
+    return reflector_scaled(alpha, as, fma(as.y, as.y, warp_sum(ss)), f);
 }
 
 // The FP64 reduction of C (lower, M0) to tridiagonal form, reflectors in its
