@@ -46,9 +46,9 @@ static CtaKernelFn cta_kernel(int nmax, int teams, bool fs, bool spec) {
 int cta_max_teams(int nmax) { return nmax <= 16 ? 4 : nmax <= 32 ? 2 : 1; }
 
 // Default pencils per CTA, measured on B200 (solves/s at batch 65,536, one
-// pencil per CTA -> default): N=8 46.3 M -> 48.1 M, N=12 25.2 M -> 25.7 M, N=16
-// 21.3 M -> 21.9 M (4 teams of 32 threads); N=32 5.60 M -> 6.20 M (2 of 64);
-// N=24 has two on request (7.51 M, 8.67 M with two) and starts with one, so that
+// pencil per CTA -> default): N=8 45.6 M -> 47.2 M, N=12 24.7 M -> 25.4 M, N=16
+// 20.9 M -> 21.7 M (4 teams of 32 threads); N=32 5.30 M -> 6.09 M (2 of 64);
+// N=24 has two on request (7.17 M, 8.51 M with two) and starts with one, so that
 // the reported pencils per CTA stay what they were.
 int cta_default_teams(int nmax) { return nmax <= 16 ? 4 : nmax == 32 ? 2 : 1; }
 
